@@ -138,6 +138,29 @@ exl3_had_rows_kernel(const TI* __restrict__ x, int ldx, const __half* __restrict
   st4(y + static_cast<size_t>(r) * ldy + c0, v);
 }
 
+// Rows of a prompt batch in expert order: y[i] = had128(x[perm[i] / top_k] * suh[expert of pair perm[i]]), fp16.  The gather, the
+// row-to-expert lookup and the transform are one pass (before: a bf16 gather, four index kernels and exl3_had_rows).
+__global__ void __launch_bounds__(256)
+exl3_had_gather_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __restrict__ perm, const int* __restrict__ ids, int top_k,
+                       const __half* __restrict__ suh, long long suh_stride, __half* __restrict__ y, int ldy, int nblk, long long total) {
+  const int lane = threadIdx.x & 31;
+  const long long w = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // (row, 128-block) of this warp
+  if (w >= total) return;
+  const int r = static_cast<int>(w / nblk), blk = static_cast<int>(w - static_cast<long long>(r) * nblk);
+  const int pair = perm[r], e = max(ids[pair], 0);           // filler rows past this rank's pairs may name an expert elsewhere
+  const int c0 = blk * 128 + lane * 4;
+  float v[4];
+  ld4(x + static_cast<size_t>(pair / top_k) * ldx + c0, v);
+  const uint2 sraw = *reinterpret_cast<const uint2*>(suh + e * suh_stride + c0);
+  const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.x));
+  const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.y));
+  v[0] *= s01.x; v[1] *= s01.y; v[2] *= s23.x; v[3] *= s23.y;
+  fwht128_warp(v, lane);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] *= INV_SQRT_128;
+  st4(y + static_cast<size_t>(r) * ldy + c0, v);
+}
+
 }  // namespace spark
 
 using namespace spark;
@@ -174,5 +197,17 @@ extern "C" int spark_exl3_had_rows(const void* x, int ldx, const void* scale, vo
   const unsigned grid = static_cast<unsigned>((total + 7) / 8);
   if (!post) exl3_had_rows_kernel<__nv_bfloat16, __half><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (const __half*)scale, (__half*)y, ldy, 0, row_expert, expert_stride, nblk, total);
   else exl3_had_rows_kernel<float, __nv_bfloat16><<<grid, 256, 0, s>>>((const float*)x, ldx, (const __half*)scale, (__nv_bfloat16*)y, ldy, 1, row_expert, expert_stride, nblk, total);
+  return spark_launch_rc(__func__);
+}
+
+// x bf16 [rows, C] -> y fp16 [P, C]: row i is pair perm[i] of the routing table `ids` [rows, top_k], scaled by its expert's vector.
+extern "C" int spark_exl3_had_gather(const void* x, int ldx, const int* perm, const int* ids, int top_k, const void* suh,
+                                     long long suh_stride, void* y, int ldy, int P, int C, cudaStream_t s) {
+  if (P <= 0) return 0;
+  if ((C & 127) || (ldx & 3) || (ldy & 3) || top_k < 1) return -5;
+  const int nblk = C / 128;
+  const long long total = static_cast<long long>(P) * nblk;
+  exl3_had_gather_kernel<<<static_cast<unsigned>((total + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)x, ldx, perm, ids, top_k, (const __half*)suh,
+                                                                               suh_stride, (__half*)y, ldy, nblk, total);
   return spark_launch_rc(__func__);
 }

@@ -62,7 +62,8 @@ _SIGS = {
     "spark_attn_prefill": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp],
     "spark_attn_prefill_masked": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp, vp, i32, i32, vp,
                                   i32, vp],
-    "spark_exl3_mgemm": [vp, i32, vp, vp, i64, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, i32, vp],
+    "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp],
+    "spark_exl3_had_gather": [vp, i32, vp, vp, i32, vp, i64, vp, i32, i32, i32, vp],
     "spark_gdn_chunk_prefill": [vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32,
                                 i32, f32, vp],
     "spark_attn_prep": [vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp, vp, vp, vp,
@@ -465,29 +466,27 @@ def exl3_fold(w: Exl3Weight) -> torch.Tensor:
     return b.t().contiguous()
 
 
-def _pick_mg_slices(K: int, target: int) -> int:
-    """K-slices (cluster size) of the grouped EXL3 GEMM: the smallest of 1/2/4/8 that brings the slice to <= target."""
-    blocks = K // 128
-    best = 1
-    for s in (1, 2, 4, 8):
-        if blocks % s == 0:
-            best = s
-            if K // s <= target:
-                break
-    return best
+def exl3_had_gather(x, scale, perm, ids, expert_stride):
+    """fp16 rows in expert order: row i is row perm[i] // top_k of `x` through the input transform of expert ids[perm[i]]."""
+    Pn, Cn = perm.shape[0], x.shape[1]
+    if dbg.CHECK:
+        dbg.check_index("exl3_had_gather pairs", perm, 0, ids.numel())
+    y = torch.empty(Pn, Cn, dtype=torch.float16, device=x.device)
+    rc = lib().spark_exl3_had_gather(P(x), x.stride(0), P(perm), P(ids), ids.shape[-1], P(scale), expert_stride, P(y), Cn, Pn, Cn, stream())
+    check(rc, "spark_exl3_had_gather")
+    return y
 
 
-def exl3_mgemm(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, rows_per_item=64):
-    """Rows in expert order (fp16, input Hadamard applied) x expert trellises -> [P, N]; output Hadamard fused."""
+def exl3_tc(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, glu: Optional[Exl3Weight] = None, limit=0.0):
+    """Rows in expert order (fp16, input transform applied) x expert trellises on tcgen05 -> [P, N], output transform applied.
+    `glu`: w is [gate | up]; the result is the fp16 input [P, F] of the product with `glu` (gated, its input transform applied)."""
     Pn, K = xh.shape
-    y = torch.empty(Pn, w.n, dtype=torch.float32 if out_f32 else torch.bfloat16, device=xh.device)
-    t = w.trellis
-    # slice depth: two (64-row items) or three (32-row items) CTAs per SM must fit their rows + reduction buffers
-    target = int(os.environ.get("SPARK_MG_KS", "512" if rows_per_item == 32 else "256"))
-    rc = lib().spark_exl3_mgemm(P(xh), xh.stride(0), P(t), P(w.svh), (K // 16) * (w.n // 16) * 32, w.n, P(tiles),
-                                P(ntile), max_tiles, P(y), w.n, int(out_f32), K, w.n, _pick_mg_slices(K, target),
-                                0 if w.kind == "mul1" else 1, rows_per_item, stream())
-    check(rc, "spark_exl3_mgemm")
+    n = w.n // 2 if glu is not None else w.n
+    y = torch.empty(Pn, n, dtype=torch.float16 if glu is not None else torch.float32 if out_f32 else torch.bfloat16, device=xh.device)
+    rc = lib().spark_exl3_tc(P(xh), xh.stride(0), Pn, P(w.trellis), P(w.svh), (K // 16) * (w.n // 16) * 32, w.n,
+                             P(glu.suh) if glu is not None else None, n, P(tiles), P(ntile), max_tiles, P(y), n, int(out_f32), K, w.n,
+                             int(glu is not None), float(limit), 0 if w.kind == "mul1" else 1, P(status_word(xh.device)), stream())
+    check(rc, "spark_exl3_tc")
     return y
 
 
@@ -936,15 +935,15 @@ def moe(h, w, c, defer: bool = False):
         inv = None
     else:
         perm, inv, offs, tiles, ntile, max_tiles = moe_sort(ids.view(-1), (ep[1] - ep[0]) if ep else c.n_experts)
-        src = torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32)
-        a = gather_rows(h, src)
+        gathered = lambda: gather_rows(h, torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32))
         if isinstance(wgu, Exl3Weight):
             from .exl3_moe import exl3_grouped_experts
-            y = exl3_grouped_experts(a, wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
+            y = exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
         elif isinstance(wgu, QuantWeight):
             from . import mx
-            y = mx.grouped_experts(a, wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
+            y = mx.grouped_experts(gathered(), wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
         else:
+            a = gathered()
             E, F2, K = wgu.shape
             act = grouped_gemm(a, wgu.view(E * F2, K), tiles, ntile, max_tiles, E, F2, F2 // 2, 1, c.swiglu_limit)
             y = grouped_gemm(act, wd.view(E * H, F2 // 2), tiles, ntile, max_tiles, E, H, H, 0)
