@@ -393,46 +393,96 @@ __global__ void mx_dequant_kernel(const uint8_t* __restrict__ W, const void* __r
 }
 
 // ------------------------------------------------------------------------------------------ activation quant
-// One warp per (row, block).  BLOCK 128 -> e4m3 + fp32 scale (amax/448, clamp 1e-4; optionally rounded up to a
-// power of two); BLOCK 32 -> e4m3 + E8M0 scale byte (MXFP8: 2^ceil(log2(amax/448))).  act 1: x = [gate | up].
-template <int BLOCK, typename TI>
-__global__ void act_quant_kernel(const TI* __restrict__ x, int ldx, uint8_t* __restrict__ q, void* __restrict__ scales, int R,
-                                 int K, int pow2, int act, float limit) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int nb = K / BLOCK;
-  if (warp >= R * nb) return;
-  const int r = warp / nb, b = warp - r * nb;
-  constexpr int PER = BLOCK / 32;
-  float v[PER];
-  float amax = 0.f;
-  const TI* xr = x + static_cast<size_t>(r) * ldx;
+// BLOCK 128 -> e4m3 + fp32 scale (amax/448, clamp 1e-4; optionally rounded up to a power of two); BLOCK 32 -> e4m3 + E8M0 scale
+// byte (MXFP8: 2^ceil(log2(amax/448))).  act 1: x = [gate | up].
+// A lane owns PER consecutive elements of a block.  PER = 8 (16- or 32-byte loads, one 8-byte store; the scale's division, logarithm
+// and exponential are paid once per 8 elements): prompts, bound by memory; the four calls of an MXFP4 layer on 2048 rows (2048 and
+// 16384 rows, 4096 and 2048 wide) took 494 us with one element per lane and take 123.  PER = 2: what does not fill the GPU with
+// eight, where the chain of one lane is the time (the two calls of four streams, 4 and 24 rows: 4.0 us each with eight, 3.5 with two).  A power-of-two scale is
+// divided by through its reciprocal, which is exact.
+// `vec` 0: rows or outputs that do not start on a vector take the same elements one at a time.
+template <int PER, typename TI>
+__device__ __forceinline__ void aq_load(const TI* p, int vec, float (&v)[PER]) {
+  if (!vec) {
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int k = b * BLOCK + lane * PER + j;
-    float a = static_cast<float>(xr[k]);
-    if (act) {
-      float u = static_cast<float>(xr[K + k]);
-      if (limit > 0.f) { a = fminf(a, limit); u = fminf(fmaxf(u, -limit), limit); }
-      a = a / (1.f + __expf(-a)) * u;
-    }
-    v[j] = a;
-    amax = fmaxf(amax, fabsf(a));
+    for (int j = 0; j < PER; ++j) v[j] = static_cast<float>(p[j]);
+  } else if (sizeof(TI) == 4) {
+#pragma unroll
+    for (int j = 0; j < PER; j += 2) { const float2 f = reinterpret_cast<const float2*>(p)[j / 2]; v[j] = f.x; v[j + 1] = f.y; }
+  } else {
+    __nv_bfloat162 h[PER / 2];
+    if (PER == 8) *reinterpret_cast<uint4*>(h) = *reinterpret_cast<const uint4*>(p);
+    else *reinterpret_cast<uint32_t*>(h) = *reinterpret_cast<const uint32_t*>(p);
+#pragma unroll
+    for (int j = 0; j < PER / 2; ++j) { const float2 f = __bfloat1622float2(h[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
   }
-  amax = warp_max(amax);
+}
+
+template <int BLOCK, typename TI, int PER>
+__global__ void __launch_bounds__(256)
+act_quant_kernel(const TI* __restrict__ x, int ldx, uint8_t* __restrict__ q, void* __restrict__ scales, int R,
+                 int K, int pow2, int act, float limit, int vec) {
+  const int pr = K / PER;                                    // lanes of a row (a multiple of BLOCK / PER)
+  const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, total = static_cast<long long>(R) * pr;
+  if (id - (threadIdx.x & 31) >= total) return;              // whole warps leave: the others shuffle
+  const bool live = id < total;
+  const int r = live ? static_cast<int>(id / pr) : R - 1, k = live ? static_cast<int>(id - static_cast<long long>(r) * pr) * PER : 0;
+  const TI* xr = x + static_cast<size_t>(r) * ldx + k;
+  constexpr int LANES = BLOCK / PER;                          // lanes of a block
+  float v[PER];
+  aq_load<PER>(xr, vec, v);
+  if (act) {
+    float u[PER];
+    aq_load<PER>(xr + K, vec, u);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      float a = v[j], b = u[j];
+      if (limit > 0.f) { a = fminf(a, limit); b = fminf(fmaxf(b, -limit), limit); }
+      v[j] = a / (1.f + __expf(-a)) * b;
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) amax = fmaxf(amax, fabsf(v[j]));
+#pragma unroll
+  for (int m = 1; m < LANES; m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
   amax = fmaxf(amax, 1e-4f);
   float sc = amax / 448.f;
-  if (BLOCK == 32 || pow2) sc = exp2f(ceilf(log2f(sc)));
-  if (lane == 0) {
-    if (BLOCK == 32) reinterpret_cast<uint8_t*>(scales)[static_cast<size_t>(r) * nb + b] =
-        static_cast<uint8_t>(__float_as_uint(sc) >> 23);
-    else reinterpret_cast<float*>(scales)[static_cast<size_t>(r) * nb + b] = sc;
+  const bool p2 = BLOCK == 32 || pow2;
+  if (p2) sc = exp2f(ceilf(log2f(sc)));
+  if (!live) return;
+  const int nb = K / BLOCK;
+  if ((k & (BLOCK - 1)) == 0) {
+    const size_t o = static_cast<size_t>(r) * nb + k / BLOCK;
+    if (BLOCK == 32) reinterpret_cast<uint8_t*>(scales)[o] = static_cast<uint8_t>(__float_as_uint(sc) >> 23);
+    else reinterpret_cast<float*>(scales)[o] = sc;
   }
+  const float inv = 1.f / sc;
+  uint32_t w[(PER + 3) / 4] = {};
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
-    const float s = fminf(fmaxf(v[j] / sc, -448.f), 448.f);
-    q[static_cast<size_t>(r) * K + b * BLOCK + lane * PER + j] =
-        static_cast<uint8_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3));
+    const float s = fminf(fmaxf(p2 ? v[j] * inv : v[j] / sc, -448.f), 448.f);
+    w[j >> 2] |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3)) << (8 * (j & 3));
   }
+  uint8_t* dst = q + static_cast<size_t>(r) * K + k;
+  if (!vec) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) dst[j] = static_cast<uint8_t>(w[j >> 2] >> (8 * (j & 3)));
+  } else if (PER == 8) {
+    *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[PER == 8 ? 1 : 0]);
+  } else {
+    *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(w[0]);
+  }
+}
+
+template <int BLOCK, typename TI>
+static void launch_act_quant(const void* x, int ldx, uint8_t* q, void* scales, int R, int K, int pow2, int act, float limit, cudaStream_t s) {
+  // eight elements a lane once that still is a warp for every scheduler of the GPU
+  const int vec = ((reinterpret_cast<uintptr_t>(x) & 15) | (static_cast<size_t>(ldx) * sizeof(TI) & 15) | (reinterpret_cast<uintptr_t>(q) & 7)) == 0;
+  const bool many = static_cast<long long>(R) * K >= 148LL * 4 * 32 * 8;
+  const unsigned blocks = static_cast<unsigned>((static_cast<long long>(R) * (K / (many || BLOCK == 128 ? 8 : 2)) + 255) / 256);
+  if (many || BLOCK == 128) act_quant_kernel<BLOCK, TI, 8><<<blocks, 256, 0, s>>>((const TI*)x, ldx, q, scales, R, K, pow2, act, limit, vec);
+  else act_quant_kernel<BLOCK, TI, BLOCK == 128 ? 8 : 2><<<blocks, 256, 0, s>>>((const TI*)x, ldx, q, scales, R, K, pow2, act, limit, vec);
 }
 
 }  // namespace spark
@@ -470,9 +520,7 @@ extern "C" int spark_act_quant(const void* x, int ldx, int in_f32, void* q, void
                                int act, float limit, cudaStream_t s) {
   if (R <= 0) return 0;
   if ((block != 128 && block != 32) || K % block) return -5;
-  const long long warps = static_cast<long long>(R) * (K / block);
-  const unsigned blocks = static_cast<unsigned>((warps * 32 + 255) / 256);
-#define SPARK_AQ(B, T) act_quant_kernel<B, T><<<blocks, 256, 0, s>>>((const T*)x, ldx, (uint8_t*)q, scales, R, K, pow2, act, limit)
+#define SPARK_AQ(B, T) launch_act_quant<B, T>(x, ldx, (uint8_t*)q, scales, R, K, pow2, act, limit, s)
   if (block == 128) { if (in_f32) SPARK_AQ(128, float); else SPARK_AQ(128, __nv_bfloat16); }
   else { if (in_f32) SPARK_AQ(32, float); else SPARK_AQ(32, __nv_bfloat16); }
 #undef SPARK_AQ
