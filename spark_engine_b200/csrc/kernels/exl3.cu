@@ -71,94 +71,109 @@ __global__ void exl3_reconstruct_bits_kernel(const uint32_t* __restrict__ trelli
 }
 
 // y[r, :] = had128(x[r, :] * scale[:]) (pre) or had128(x[r, :]) * scale[:] (post); 128-blocks along the row.
-// One warp per 128-block: a lane keeps 4 consecutive elements (one 8- or 16-byte load), the strides 1 and 2 of the
-// butterfly run in registers and the strides 4..64 through five shuffles -- the same additions in the same order as a
-// shared-memory butterfly, without its 14 barriers per block (this pass was 0.76 TB/s as one block per CTA).
-template <typename T> __device__ __forceinline__ void ld4(const T* p, float (&v)[4]);
-template <> __device__ __forceinline__ void ld4<float>(const float* p, float (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+// Eight lanes per 128-block, four blocks per warp: a lane moves 16 consecutive elements as 16-byte vectors.  With one block per
+// warp (four elements a lane, five shuffle stages, an index division per 128 elements) the pass was bound by issue and shuffles:
+// 4096 rows of 12288
+// and of 2048 columns out (fp32 -> bf16) 99 -> 74 us, 4096 rows in (bf16 -> fp16) 21 -> 13 us.
+__device__ __forceinline__ void ld16(const float* p, float (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 t = reinterpret_cast<const float4*>(p)[i];
+    v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+  }
 }
-template <> __device__ __forceinline__ void ld4<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[4]) {
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
-  const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
-  v[0] = a.x; v[1] = a.y; v[2] = c.x; v[3] = c.y;
+template <typename T2, typename T> __device__ __forceinline__ float2 up2(uint32_t w);
+template <> __device__ __forceinline__ float2 up2<__nv_bfloat162, __nv_bfloat16>(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+template <> __device__ __forceinline__ float2 up2<__half2, __half>(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+// 16 elements of 16 bits; rows are aligned to 8 bytes (`wide`: to 16)
+template <typename T2, typename T>
+__device__ __forceinline__ void ld16h(const T* p, bool wide, float (&v)[16]) {
+  uint32_t w[8];
+  if (wide) {
+    const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const uint2 a = reinterpret_cast<const uint2*>(p)[i]; w[2 * i] = a.x; w[2 * i + 1] = a.y; }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { const float2 f = up2<T2, T>(w[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
 }
-__device__ __forceinline__ void st4(__half* p, const float (&v)[4]) {
-  const __half2 a = __floats2half2_rn(v[0], v[1]), c = __floats2half2_rn(v[2], v[3]);
-  uint2 o; o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&c);
-  *reinterpret_cast<uint2*>(p) = o;
+__device__ __forceinline__ void ld16(const __nv_bfloat16* p, bool wide, float (&v)[16]) { ld16h<__nv_bfloat162>(p, wide, v); }
+__device__ __forceinline__ void ld16(const __half* p, bool wide, float (&v)[16]) { ld16h<__half2>(p, wide, v); }
+__device__ __forceinline__ void ld16(const float* p, bool, float (&v)[16]) { ld16(p, v); }
+__device__ __forceinline__ uint32_t pk(const __half*, float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ uint32_t pk(const __nv_bfloat16*, float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
+template <typename T> __device__ __forceinline__ void st16(T* p, bool wide, const float (&v)[16]) {
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = pk(p, v[2 * i], v[2 * i + 1]);
+  if (wide) {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) reinterpret_cast<uint2*>(p)[i] = make_uint2(w[2 * i], w[2 * i + 1]);
+  }
 }
-__device__ __forceinline__ void st4(__nv_bfloat16* p, const float (&v)[4]) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), c = __floats2bfloat162_rn(v[2], v[3]);
-  uint2 o; o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&c);
-  *reinterpret_cast<uint2*>(p) = o;
+
+// thread id -> (row, 128-block); lanes past the end take part in the shuffles with the last block's values
+struct HadAt { int r, c0; bool live; };
+__device__ __forceinline__ HadAt had_at(int R, int nblk) {
+  const long long b = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) >> 3, total = static_cast<long long>(R) * nblk;
+  HadAt h;
+  h.live = b < total;
+  const long long bb = h.live ? b : total - 1;
+  // R * nblk < 2^31 in all that fits a device: 32-bit division
+  h.r = static_cast<int>(static_cast<uint32_t>(bb) / static_cast<uint32_t>(nblk));
+  h.c0 = static_cast<int>(bb - static_cast<long long>(h.r) * nblk) * 128 + (threadIdx.x & 7) * 16;
+  return h;
 }
 
 template <typename TI, typename TOUT>
 __global__ void __launch_bounds__(256)
 exl3_had_rows_kernel(const TI* __restrict__ x, int ldx, const __half* __restrict__ scale, TOUT* __restrict__ y, int ldy,
-                     int post, const int* __restrict__ row_expert, long long expert_stride, int nblk, long long total) {
-  const int lane = threadIdx.x & 31;
-  const long long w = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // (row, 128-block) of this warp
-  if (w >= total) return;
-  const int r = static_cast<int>(w / nblk), blk = static_cast<int>(w - static_cast<long long>(r) * nblk);
-  const int c0 = blk * 128 + lane * 4;
-  float v[4];
-  ld4(x + static_cast<size_t>(r) * ldx + c0, v);
-  const __half* srow = scale + (row_expert ? row_expert[r] * expert_stride : 0);
-  const uint2 sraw = *reinterpret_cast<const uint2*>(srow + c0);
-  const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.x));
-  const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.y));
-  const float sc[4] = {s01.x, s01.y, s23.x, s23.y};
+                     int post, const int* __restrict__ row_expert, long long expert_stride, int R, int nblk, int wide) {
+  const HadAt at = had_at(R, nblk);
+  float v[16], sc[16];
+  ld16(x + static_cast<size_t>(at.r) * ldx + at.c0, wide & 1, v);
+  ld16(scale + (row_expert ? row_expert[at.r] * expert_stride : 0) + at.c0, wide & 4, sc);
   if (!post) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] *= sc[i];
+    for (int i = 0; i < 16; ++i) v[i] *= sc[i];
   }
-  // strides 1, 2: inside the lane (element i pairs with i ^ stride; the upper one takes lower - upper)
-  {
-    const float a0 = v[0] + v[1], a1 = v[0] - v[1], a2 = v[2] + v[3], a3 = v[2] - v[3];
-    v[0] = a0 + a2; v[1] = a1 + a3; v[2] = a0 - a2; v[3] = a1 - a3;
-  }
-  // strides 4 .. 64: lane ^ 1 .. lane ^ 16
+  fwht128_oct(v, threadIdx.x & 31);
 #pragma unroll
-  for (int m = 1; m < 32; m <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, v[i], m);
-      v[i] = (lane & m) ? other - v[i] : v[i] + other;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[i] *= 0.08838834764831845f;
+  for (int i = 0; i < 16; ++i) {
+    v[i] *= INV_SQRT_128;
     if (post) v[i] *= sc[i];
   }
-  st4(y + static_cast<size_t>(r) * ldy + c0, v);
+  if (at.live) st16(y + static_cast<size_t>(at.r) * ldy + at.c0, wide & 2, v);
 }
 
 // Rows of a prompt batch in expert order: y[i] = had128(x[perm[i] / top_k] * suh[expert of pair perm[i]]), fp16.  The gather, the
 // row-to-expert lookup and the transform are one pass (before: a bf16 gather, four index kernels and exl3_had_rows).
+// Bound by writing y: 81920 rows of 2048 took 278 us with one block per warp and take 139 (2.4 TB/s written).
 __global__ void __launch_bounds__(256)
 exl3_had_gather_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __restrict__ perm, const int* __restrict__ ids, int top_k,
-                       const __half* __restrict__ suh, long long suh_stride, __half* __restrict__ y, int ldy, int nblk, long long total) {
-  const int lane = threadIdx.x & 31;
-  const long long w = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // (row, 128-block) of this warp
-  if (w >= total) return;
-  const int r = static_cast<int>(w / nblk), blk = static_cast<int>(w - static_cast<long long>(r) * nblk);
-  const int pair = perm[r], e = max(ids[pair], 0);           // filler rows past this rank's pairs may name an expert elsewhere
-  const int c0 = blk * 128 + lane * 4;
-  float v[4];
-  ld4(x + static_cast<size_t>(pair / top_k) * ldx + c0, v);
-  const uint2 sraw = *reinterpret_cast<const uint2*>(suh + e * suh_stride + c0);
-  const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.x));
-  const float2 s23 = __half22float2(*reinterpret_cast<const __half2*>(&sraw.y));
-  v[0] *= s01.x; v[1] *= s01.y; v[2] *= s23.x; v[3] *= s23.y;
-  fwht128_warp(v, lane);
+                       const __half* __restrict__ suh, long long suh_stride, __half* __restrict__ y, int ldy, int R, int nblk, int wide) {
+  const HadAt at = had_at(R, nblk);
+  const int pair = perm[at.r], e = max(ids[pair], 0);        // filler rows past this rank's pairs may name an expert elsewhere
+  float v[16], sc[16];
+  ld16(x + static_cast<size_t>(pair / top_k) * ldx + at.c0, wide & 1, v);
+  ld16(suh + e * suh_stride + at.c0, wide & 4, sc);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] *= INV_SQRT_128;
-  st4(y + static_cast<size_t>(r) * ldy + c0, v);
+  for (int i = 0; i < 16; ++i) v[i] *= sc[i];
+  fwht128_oct(v, threadIdx.x & 31);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] *= INV_SQRT_128;
+  if (at.live) st16(y + static_cast<size_t>(at.r) * ldy + at.c0, wide & 2, v);
+}
+
+// bit 0: rows of x start on 16 bytes, bit 1: rows of y, bit 2: scale vectors
+static int had_wide(const void* x, size_t x_row_bytes, const void* y, size_t y_row_bytes, const void* sc, long long sc_row_bytes) {
+  auto ok = [](const void* p, size_t row) { return ((reinterpret_cast<uintptr_t>(p) | row) & 15) == 0; };
+  return (ok(x, x_row_bytes) ? 1 : 0) | (ok(y, y_row_bytes) ? 2 : 0) | (ok(sc, static_cast<size_t>(sc_row_bytes)) ? 4 : 0);
 }
 
 }  // namespace spark
@@ -194,9 +209,11 @@ extern "C" int spark_exl3_had_rows(const void* x, int ldx, const void* scale, vo
   if ((ldx & 3) || (ldy & 3)) return -5;               // 8- / 16-byte vector accesses along the rows
   const int nblk = C / 128;
   const long long total = static_cast<long long>(R) * nblk;
-  const unsigned grid = static_cast<unsigned>((total + 7) / 8);
-  if (!post) exl3_had_rows_kernel<__nv_bfloat16, __half><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (const __half*)scale, (__half*)y, ldy, 0, row_expert, expert_stride, nblk, total);
-  else exl3_had_rows_kernel<float, __nv_bfloat16><<<grid, 256, 0, s>>>((const float*)x, ldx, (const __half*)scale, (__nv_bfloat16*)y, ldy, 1, row_expert, expert_stride, nblk, total);
+  if (total > 0x7fffffffLL) return -5;
+  const unsigned grid = static_cast<unsigned>((total * 8 + 255) / 256);
+  const int wide = had_wide(x, static_cast<size_t>(ldx) * (post ? 4 : 2), y, static_cast<size_t>(ldy) * 2, scale, row_expert ? expert_stride * 2 : 0);
+  if (!post) exl3_had_rows_kernel<__nv_bfloat16, __half><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (const __half*)scale, (__half*)y, ldy, 0, row_expert, expert_stride, R, nblk, wide);
+  else exl3_had_rows_kernel<float, __nv_bfloat16><<<grid, 256, 0, s>>>((const float*)x, ldx, (const __half*)scale, (__nv_bfloat16*)y, ldy, 1, row_expert, expert_stride, R, nblk, wide);
   return spark_launch_rc(__func__);
 }
 
@@ -207,7 +224,9 @@ extern "C" int spark_exl3_had_gather(const void* x, int ldx, const int* perm, co
   if ((C & 127) || (ldx & 3) || (ldy & 3) || top_k < 1) return -5;
   const int nblk = C / 128;
   const long long total = static_cast<long long>(P) * nblk;
-  exl3_had_gather_kernel<<<static_cast<unsigned>((total + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)x, ldx, perm, ids, top_k, (const __half*)suh,
-                                                                               suh_stride, (__half*)y, ldy, nblk, total);
+  if (total > 0x7fffffffLL) return -5;
+  exl3_had_gather_kernel<<<static_cast<unsigned>((total * 8 + 255) / 256), 256, 0, s>>>(
+      (const __nv_bfloat16*)x, ldx, perm, ids, top_k, (const __half*)suh, suh_stride, (__half*)y, ldy, P, nblk,
+      had_wide(x, static_cast<size_t>(ldx) * 2, y, static_cast<size_t>(ldy) * 2, suh, suh_stride * 2));
   return spark_launch_rc(__func__);
 }

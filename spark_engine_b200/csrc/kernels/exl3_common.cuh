@@ -77,4 +77,21 @@ __device__ __forceinline__ void fwht128_warp(float (&v)[4], int lane) {
   }
 }
 
+// The same transform of one 128-block by eight lanes: lane l & 7 owns elements 16 (l & 7) .. + 15.  Strides 1 .. 8 stay in the lane
+// and only three cross lanes, 0.38 shuffles per element instead of 0.63; a stage is one shuffle and one exact fused multiply-add
+// (by +-1).  Same pairs in the same order as fwht128_warp, so the same bits.
+__device__ __forceinline__ void fwht128_oct(float (&v)[16], int lane) {
+#pragma unroll
+  for (int st = 1; st < 16; st <<= 1)
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (!(i & st)) { const float a = v[i], b = v[i | st]; v[i] = a + b; v[i | st] = a - b; }
+#pragma unroll
+  for (int m = 1; m < 8; m <<= 1) {
+    const float sg = (lane & m) ? -1.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = fmaf(sg, v[i], __shfl_xor_sync(0xffffffffu, v[i], m));
+  }
+}
+
 }  // namespace spark
