@@ -12,69 +12,77 @@
 
 namespace spark {
 
-constexpr int ROUTE_THREADS = 256;
-constexpr int ROUTE_MAXE_PER_THREAD = 4;     // up to 1024 experts
+constexpr int ROUTE_MAXE = 1024;
+constexpr int ROUTE_ROWS = 8;                // rows (warps) per CTA
+
+// Best of a lane's EPL selection scores and the lowest position that holds it: a max tree and a bit mask, not a serial compare chain.
+// A score that is no number is never the best.
+template <int EPL>
+__device__ __forceinline__ void lane_best(const float (&s)[EPL], float& best, int& bj) {
+  float m[EPL];
+#pragma unroll
+  for (int j = 0; j < EPL; ++j) m[j] = s[j];
+#pragma unroll
+  for (int w = EPL / 2; w >= 1; w >>= 1)
+#pragma unroll
+    for (int j = 0; j < w; ++j) m[j] = fmaxf(m[j], m[j + w]);
+  best = m[0] == m[0] ? m[0] : -INFINITY;
+  unsigned mask = 0u;
+#pragma unroll
+  for (int j = 0; j < EPL; ++j) mask |= (s[j] == best ? 1u : 0u) << j;
+  bj = __ffs(mask) - 1;
+  if (bj < 0) bj = 0;
+}
 
 // kind: 0 softmax, 1 sigmoid+bias, 2 sqrt(softplus)+bias, 3 softmax+bias (the bias enters the choice only), 4 sigmoid, not
 // renormalised (ranked by the logits, which a saturated sigmoid would tie), 5 softmax over the chosen logits alone (bias, if any,
 // added to the logits; ranked by them, and only the chosen ones are exponentiated, against the largest).
 // The last n_self of the E router outputs are identity experts: they leave -1 in `ids` and their weight in self_w[row].
-__global__ void __launch_bounds__(ROUTE_THREADS)
-moe_route_kernel(const float* __restrict__ logits, int ld, int E, int top_k, int kind, const float* __restrict__ bias,
+// One warp per row, EPL experts per lane; a choice is two warp reductions (the largest score's order-preserving key, the lowest expert
+// among the lanes that hold it).  A CTA per row with three block barriers per choice took 107 us for 8192 rows of 512 experts, top
+// 10; this takes 31.
+template <int EPL>
+__global__ void __launch_bounds__(ROUTE_ROWS * 32)
+moe_route_kernel(const float* __restrict__ logits, int ld, int R, int E, int top_k, int kind, const float* __restrict__ bias,
                  float scale, int shared_gate, float* __restrict__ wts, int* __restrict__ ids,
                  int* __restrict__ pair_row, float* __restrict__ sg, int e_lo, int e_hi, int n_self, float* __restrict__ self_w) {
-  __shared__ float rv[ROUTE_THREADS / 32];
-  __shared__ int ri[ROUTE_THREADS / 32];
-  __shared__ float bv; __shared__ int bidx;
-  __shared__ float sel_p[32];
-  __shared__ int sel_self[32];
-  const int r = blockIdx.x, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int r = blockIdx.x * ROUTE_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= R) return;
   const float* x = logits + static_cast<size_t>(r) * ld;
-  float p[ROUTE_MAXE_PER_THREAD], s[ROUTE_MAXE_PER_THREAD];
+  float p[EPL], s[EPL];                                     // p: what the weights are made of; s: selection score
   float mx = -INFINITY;
 #pragma unroll
-  for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) {
-    const int e = t + j * ROUTE_THREADS;
+  for (int j = 0; j < EPL; ++j) {
+    const int e = lane + 32 * j;
     p[j] = e < E ? x[e] : -INFINITY;
     if (kind == 5 && bias && e < E) p[j] += bias[e];
     mx = fmaxf(mx, p[j]);
   }
   if (kind == 0 || kind == 3) {
     mx = warp_max(mx);
-    if (lane == 0) rv[warp] = mx;
-    __syncthreads();
-    mx = rv[0];
-    for (int w = 1; w < ROUTE_THREADS / 32; ++w) mx = fmaxf(mx, rv[w]);
-    __syncthreads();
     float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) {
-      const int e = t + j * ROUTE_THREADS;
-      p[j] = e < E ? expf(p[j] - mx) : 0.f;
+    for (int j = 0; j < EPL; ++j) {
+      p[j] = lane + 32 * j < E ? expf(p[j] - mx) : 0.f;
       sum += p[j];
     }
     sum = warp_sum(sum);
-    if (lane == 0) rv[warp] = sum;
-    __syncthreads();
-    sum = 0.f;
-    for (int w = 0; w < ROUTE_THREADS / 32; ++w) sum += rv[w];
-    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) {
+    for (int j = 0; j < EPL; ++j) {
       p[j] = p[j] / sum;
       s[j] = p[j];
-      if (kind == 3 && t + j * ROUTE_THREADS < E) s[j] += bias[t + j * ROUTE_THREADS];
+      if (kind == 3 && lane + 32 * j < E) s[j] += bias[lane + 32 * j];
     }
   } else if (kind == 4) {
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) { s[j] = p[j]; p[j] = 1.f / (1.f + expf(-p[j])); }
+    for (int j = 0; j < EPL; ++j) { s[j] = p[j]; p[j] = 1.f / (1.f + expf(-p[j])); }
   } else if (kind == 5) {
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) s[j] = p[j];
+    for (int j = 0; j < EPL; ++j) s[j] = p[j];
   } else {
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) {
-      const int e = t + j * ROUTE_THREADS;
+    for (int j = 0; j < EPL; ++j) {
+      const int e = lane + 32 * j;
       if (e < E) {
         const float v = p[j];
         if (kind == 1) p[j] = 1.f / (1.f + expf(-v));
@@ -84,57 +92,47 @@ moe_route_kernel(const float* __restrict__ logits, int ld, int E, int top_k, int
     }
   }
 #pragma unroll
-  for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) if (t + j * ROUTE_THREADS >= E) s[j] = -INFINITY;
+  for (int j = 0; j < EPL; ++j) if (lane + 32 * j >= E) s[j] = -INFINITY;
+  float selp = 0.f, best; int seli = 0x7fffffff, bj;          // lane k keeps slot k's weight numerator and expert
+  lane_best(s, best, bj);
   for (int k = 0; k < top_k; ++k) {
-    float best = -INFINITY; int bi = 0x7fffffff; float bp = 0.f;
+    const uint32_t bits = __float_as_uint(best + 0.f);        // -0 ranks as 0
+    const uint32_t key = best == -INFINITY ? 0u : (bits ^ ((bits >> 31) ? 0xffffffffu : 0x80000000u));
+    const uint32_t wmax = __reduce_max_sync(0xffffffffu, key);
+    const int cand = (key == wmax && key != 0u) ? lane + 32 * bj : 0x7fffffff;
+    const int wi = __reduce_min_sync(0xffffffffu, cand);
+    float bp = 0.f;
+    if (wi == cand && wi != 0x7fffffff) {                     // this lane owns the winner
 #pragma unroll
-    for (int j = 0; j < ROUTE_MAXE_PER_THREAD; ++j) {
-      const int e = t + j * ROUTE_THREADS;
-      if (s[j] > best || (s[j] == best && e < bi && s[j] != -INFINITY)) { best = s[j]; bi = e; }
+      for (int j = 0; j < EPL; ++j) if (j == bj) { bp = p[j]; s[j] = -INFINITY; }
+      lane_best(s, best, bj);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (lane == 0) { rv[warp] = best; ri[warp] = bi; }
-    __syncthreads();
-    if (t == 0) {
-      for (int w = 1; w < ROUTE_THREADS / 32; ++w)
-        if (rv[w] > best || (rv[w] == best && ri[w] < bi)) { best = rv[w]; bi = ri[w]; }
-      bv = best; bidx = bi;
-    }
-    __syncthreads();
-    const int win = bidx;
-    if ((win % ROUTE_THREADS) == t) {
-      const int j = win / ROUTE_THREADS;
-#pragma unroll
-      for (int jj = 0; jj < ROUTE_MAXE_PER_THREAD; ++jj) if (jj == j) { bp = p[jj]; s[jj] = -INFINITY; }
-      sel_p[k] = bp;
-      sel_self[k] = win >= E - n_self;
-      // expert-parallel ranks keep only their own experts [e_lo, e_hi): others become -1 (skipped downstream)
-      ids[static_cast<size_t>(r) * top_k + k] = (win >= e_lo && win < e_hi) ? win - e_lo : -1;
-      if (pair_row) pair_row[static_cast<size_t>(r) * top_k + k] = r;
-    }
-    __syncthreads();
+    const float wp = __shfl_sync(0xffffffffu, bp, wi & 31);
+    if (lane == k) { selp = wp; seli = wi; }
   }
-  if (t == 0) {
-    float sum = 0.f;
-    if (kind == 5) {                                         // the first one chosen is the largest
-      const float top = sel_p[0];
-      for (int k = 0; k < top_k; ++k) sel_p[k] = expf(sel_p[k] - top);
-    }
-    for (int k = 0; k < top_k; ++k) sum += sel_p[k];
-    sum = kind == 4 ? 1.f : fmaxf(sum, 1e-20f);
-    float own = 0.f;
+  if (kind == 5) {                                            // the first one chosen is the largest
+    const float top = __shfl_sync(0xffffffffu, selp, 0);
+    selp = lane < top_k ? expf(selp - top) : 0.f;
+  }
+  float sum = 0.f, own = 0.f;
+  for (int k = 0; k < top_k; ++k) sum += __shfl_sync(0xffffffffu, selp, k);      // slot order
+  sum = kind == 4 ? 1.f : fmaxf(sum, 1e-20f);
+  const float w = selp / sum * scale;
+  if (self_w) {
     for (int k = 0; k < top_k; ++k) {
-      const float w = sel_p[k] / sum * scale;
-      wts[static_cast<size_t>(r) * top_k + k] = w;
-      if (sel_self[k]) own += w;
+      const float wk = __shfl_sync(0xffffffffu, w, k);
+      if (__shfl_sync(0xffffffffu, seli, k) >= E - n_self) own += wk;
     }
-    if (self_w) self_w[r] = own;
-    if (shared_gate) sg[r] = 1.f / (1.f + expf(-x[E]));
+    if (lane == 0) self_w[r] = own;
   }
+  if (lane < top_k) {
+    const size_t o = static_cast<size_t>(r) * top_k + lane;
+    wts[o] = w;
+    // expert-parallel ranks keep only their own experts [e_lo, e_hi): others become -1 (skipped downstream)
+    ids[o] = (seli >= e_lo && seli < e_hi) ? seli - e_lo : -1;
+    if (pair_row) pair_row[o] = r;
+  }
+  if (lane == 0 && shared_gate) sg[r] = 1.f / (1.f + expf(-x[E]));
 }
 
 
@@ -247,25 +245,9 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
   __syncthreads();
   if (!last_s) return;
   // (the writers fenced before they arrived; the logits are read with L2 loads, so no reader-side fence)
-  // EPL experts per lane (E <= 32 * EPL).  The k selection rounds are a serial chain, so each round is kept short: the
-  // lane's best candidate comes from a max TREE over its EPL scores and a bit mask of the positions that hold it
-  // (lowest position = lowest expert id), not from a serial compare chain (timed inside the kernel: the serial form spent 5.8 us per group of rows).
+  // EPL experts per lane (E <= 32 * EPL).  The k selection rounds are a serial chain, so each round is kept short (lane_best: a
+  // serial compare chain in its place spent 5.8 us per group of rows).
   const int nj = (a.E + 31) >> 5;
-  auto lane_best = [&](const float (&s)[EPL], float& best, int& bj) {
-    float m[EPL];
-#pragma unroll
-    for (int j = 0; j < EPL; ++j) m[j] = s[j];
-#pragma unroll
-    for (int w = EPL / 2; w >= 1; w >>= 1)
-#pragma unroll
-      for (int j = 0; j < w; ++j) m[j] = fmaxf(m[j], m[j + w]);
-    best = m[0];
-    unsigned mask = 0u;
-#pragma unroll
-    for (int j = 0; j < EPL; ++j) mask |= (s[j] == best ? 1u : 0u) << j;
-    bj = __ffs(mask) - 1;
-    if (bj < 0) bj = 0;
-  };
   for (int r = warp; r < R; r += 8) {
     const float* lg = a.logits + static_cast<size_t>(r) * a.ld;
     float p[EPL], s[EPL];                                   // p: what the weights are made of; s: selection score
@@ -487,7 +469,17 @@ moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restric
   int mine = 0;
   if (e < E) {
     int acc = 0;
-    for (int b = 0; b < nblocks; ++b) { int c = block_hist[static_cast<size_t>(b) * E + e]; block_hist[static_cast<size_t>(b) * E + e] = acc; acc += c; }
+    // sixteen counts are asked for before the first is overwritten (one at a time: 40 us for the 320 blocks of 8192 rows, top 10)
+    for (int b0 = 0; b0 < nblocks; b0 += 16) {
+      int c[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) c[u] = b0 + u < nblocks ? block_hist[static_cast<size_t>(b0 + u) * E + e] : 0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        if (b0 + u < nblocks) block_hist[static_cast<size_t>(b0 + u) * E + e] = acc;
+        acc += c[u];
+      }
+    }
     tot[e] = acc;
     mine = acc;
   }
@@ -525,28 +517,87 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, int P, int E, cons
 
 // ---------------------------------------------------------------------------------- combine
 // res[R,H] += sum_slot w[r,slot] * y[pair_pos(r,slot), :] (+ sg[r] * shared[r,:]).  y fp32 or bf16.
-template <typename TY>
-__global__ void moe_combine_kernel(float* __restrict__ res, const TY* __restrict__ y, const int* __restrict__ inv_perm,
-                                   const float* __restrict__ wts, int top_k, const __nv_bfloat16* __restrict__ shared,
-                                   const float* __restrict__ sg, int H, __nv_bfloat16* __restrict__ out_bf16,
-                                   const int* __restrict__ pair_expert) {
-  const int r = blockIdx.x;
-  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < H; i += gridDim.y * blockDim.x) {
-    float acc = 0.f;
-#pragma unroll 4
-    for (int k = 0; k < top_k; ++k) {
-      const int pi = r * top_k + k;
-      if (pair_expert && pair_expert[pi] < 0) continue;          // expert lives on another rank
-      const int row = inv_perm ? inv_perm[pi] : pi;
-      acc = fmaf(wts[pi], static_cast<float>(y[static_cast<size_t>(row) * H + i]), acc);
+// A thread owns V consecutive columns (one 16-byte load of y per slot; V = 1 where H or an address does not allow it) and asks for
+// four slots before it adds them, in slot order.  Bound by reading y: 8192 rows of 2048, ten bf16 slots, took 224 us with one
+// column per thread and take 110 (3.4 TB/s); 2048 rows of 4096, eight fp32 slots, 91 -> 49.
+template <int V, typename T> __device__ __forceinline__ void ldv(const T* p, float (&v)[V]) {
+  if (V * sizeof(T) == 16) {
+    const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
+    if (sizeof(T) == 4) {
+      v[0] = __uint_as_float(r.x); v[1 % V] = __uint_as_float(r.y); v[2 % V] = __uint_as_float(r.z); v[3 % V] = __uint_as_float(r.w);
+    } else {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
     }
-    if (shared) {
-      const float s = __bfloat162float(shared[static_cast<size_t>(r) * H + i]);
-      acc += sg ? sg[r] * s : s;
-    }
-    if (res) res[static_cast<size_t>(r) * H + i] += acc;
-    if (out_bf16) out_bf16[static_cast<size_t>(r) * H + i] = __float2bfloat16(acc);
+  } else {
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = static_cast<float>(p[i]);
   }
+}
+
+template <typename TY, int V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(float* __restrict__ res, const TY* __restrict__ y, const int* __restrict__ inv_perm,
+                   const float* __restrict__ wts, int top_k, const __nv_bfloat16* __restrict__ shared,
+                   const float* __restrict__ sg, int H, __nv_bfloat16* __restrict__ out_bf16,
+                   const int* __restrict__ pair_expert) {
+  const int r = blockIdx.x;
+  const float gate = shared && sg ? sg[r] : 1.f;
+  for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * V; i < H; i += gridDim.y * blockDim.x * V) {
+    float acc[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] = 0.f;
+    for (int k0 = 0; k0 < top_k; k0 += 4) {
+      float v[4][V], w[4];
+      bool live[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int pi = r * top_k + min(k0 + u, top_k - 1);
+        live[u] = k0 + u < top_k && !(pair_expert && pair_expert[pi] < 0);       // else: no slot, or the expert lives on another rank
+        const int row = inv_perm ? inv_perm[pi] : pi;
+        w[u] = wts[pi];
+        if (live[u]) ldv<V>(y + static_cast<size_t>(row) * H + i, v[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (live[u]) {
+#pragma unroll
+          for (int j = 0; j < V; ++j) acc[j] = fmaf(w[u], v[u][j], acc[j]);
+        }
+    }
+    const size_t o = static_cast<size_t>(r) * H + i;
+    if (shared) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const float s = __bfloat162float(shared[o + j]);
+        acc[j] += sg ? gate * s : s;
+      }
+    }
+    if (res) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) res[o + j] += acc[j];
+    }
+    if (out_bf16) {
+      if (V == 1) {
+        out_bf16[o] = __float2bfloat16(acc[0]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; j += 4) {
+          const __nv_bfloat162 b0 = __floats2bfloat162_rn(acc[j % V], acc[(j + 1) % V]), b1 = __floats2bfloat162_rn(acc[(j + 2) % V], acc[(j + 3) % V]);
+          *reinterpret_cast<uint2*>(out_bf16 + o + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
+        }
+      }
+    }
+  }
+}
+
+template <typename TY, int V>
+static void launch_combine(float* res, const void* y, const int* inv_perm, const float* wts, int R, int top_k, const void* shared, const float* sg,
+                           int H, void* out, const int* pair_expert, cudaStream_t s) {
+  const int per = 256 * V;
+  moe_combine_kernel<TY, V><<<dim3(R, (H + per - 1) / per), 256, 0, s>>>(res, (const TY*)y, inv_perm, wts, top_k, (const __nv_bfloat16*)shared, sg,
+                                                                         H, (__nv_bfloat16*)out, pair_expert);
 }
 
 }  // namespace spark
@@ -557,8 +608,10 @@ extern "C" int spark_moe_route(const float* logits, int ld, int R, int E, int to
                                float scale, int shared_gate, float* wts, int* ids, int* pair_row, float* sg,
                                cudaStream_t s, int e_lo, int e_hi, int n_self, float* self_w) {
   if (R <= 0) return 0;
-  if (E > ROUTE_THREADS * ROUTE_MAXE_PER_THREAD || top_k > 32 || top_k > E || (kind == 3 && !bias)) return -5;
-  moe_route_kernel<<<R, ROUTE_THREADS, 0, s>>>(logits, ld, E, top_k, kind, bias, scale, shared_gate, wts, ids, pair_row, sg, e_lo, e_hi, n_self, self_w);
+  if (E > ROUTE_MAXE || top_k > 32 || top_k > E || (kind == 3 && !bias)) return -5;
+  auto kern = E <= 64 ? moe_route_kernel<2> : E <= 512 ? moe_route_kernel<16> : moe_route_kernel<32>;
+  kern<<<(R + ROUTE_ROWS - 1) / ROUTE_ROWS, ROUTE_ROWS * 32, 0, s>>>(logits, ld, R, E, top_k, kind, bias, scale, shared_gate, wts, ids, pair_row, sg,
+                                                                   e_lo, e_hi, n_self, self_w);
   return spark_launch_rc(__func__);
 }
 
@@ -582,12 +635,11 @@ extern "C" int spark_moe_combine(float* res, const void* y, int y_f32, const int
                                  int top_k, const void* shared, const float* sg, int H, void* out_bf16, cudaStream_t s,
                                  const int* pair_expert) {
   if (R <= 0) return 0;
-  if (y_f32)
-    moe_combine_kernel<float><<<dim3(R, (H + 255) / 256), 256, 0, s>>>(res, (const float*)y, inv_perm, wts, top_k, (const __nv_bfloat16*)shared, sg, H,
-                                                (__nv_bfloat16*)out_bf16, pair_expert);
-  else
-    moe_combine_kernel<__nv_bfloat16><<<dim3(R, (H + 255) / 256), 256, 0, s>>>(res, (const __nv_bfloat16*)y, inv_perm, wts, top_k,
-                                                        (const __nv_bfloat16*)shared, sg, H, (__nv_bfloat16*)out_bf16, pair_expert);
+  const bool wide = H % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out_bf16)) & 15) == 0;
+#define SPARK_CMB(T, V) launch_combine<T, V>(res, y, inv_perm, wts, R, top_k, shared, sg, H, out_bf16, pair_expert, s)
+  if (y_f32) { if (wide) SPARK_CMB(float, 4); else SPARK_CMB(float, 1); }
+  else { if (wide) SPARK_CMB(__nv_bfloat16, 8); else SPARK_CMB(__nv_bfloat16, 1); }
+#undef SPARK_CMB
   return spark_launch_rc(__func__);
 }
 
