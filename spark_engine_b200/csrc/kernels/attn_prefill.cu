@@ -1,215 +1,390 @@
-// Causal GQA attention for prefill segments (dense context, bf16 KV cache): flash-style streaming softmax on
-// tensor cores.  One CTA = 64 query rows of one q head; 4 warps x 16 rows; key/value tiles of 64 tokens are
-// double-buffered with cp.async; S = Q K^T and O += P V run on mma.sync m16n8k16 (bf16, fp32 accumulate) with
-// ldmatrix-fed fragments; P never leaves registers.  The rows of a segment see the committed prefix of their
-// sequence (already in the cache) plus the rows before them in the segment (stored by the prep kernel of the same
-// step).  Epilogue: 1/l, optional sigmoid output gate, bf16 store.  One CTA owns a (row tile, head) from first key
-// to last, so results are run-to-run identical.
-// Serves: GQA / QSA layers while the context is below the sparse-selection threshold (engine-rs/shim/qwen_qsa.cu
-// attn paths; the reference runs prefill rows through the same per-row kernel as decode).
+// Causal GQA attention for prefill segments (bf16 KV cache): streaming softmax on tcgen05.  One CTA = 128 query rows of one q head,
+// key/value tiles of 64 tokens.
+//   warp 0      TMA: the query tile, then key and value tiles into a ring of four slots in the order the products use them;
+//               values past the last key of a ragged tile are zeroed in shared memory (a masked probability of 0 times whatever
+//               the cache holds there would otherwise not be 0)
+//   warp 1      issues S = Q K^T one tile ahead of O += P V (P in tensor memory, V as an N-major operand straight from its rows)
+//   warps 2..5  softmax, one query row per thread: a row's 64 scores are one tensor-memory load, maximum and sum stay in the thread
+// The accumulator is rescaled only where a row's maximum has grown by more than 2^8 since its reference (the sums stay exact: every
+// term of a row uses the same reference), so most tiles never touch it.
+// The rows of a segment see the committed prefix of their sequence (already in the cache) plus the rows before them in the segment
+// (stored by the prep kernel of the same step).  One CTA owns a (row tile, head) from first key to last, so results are run-to-run
+// identical.  What bounds it: L2.  Every tile brings 64 KB of keys and values to 128 rows (D = 256), 2140 cycles at the 30 bytes per
+// cycle and SM that 148 of them get together; the softmax of a tile takes 900, its products 770.  4000 rows of 16 heads (2 for keys),
+// D = 256: 214 us, 612 TFLOP/s (64-row tiles on warp-level products: 828 us with block masks).
+// Serves: GQA / QSA layers (engine-rs/shim/qwen_qsa.cu attn paths; the reference runs prefill rows through the same per-row kernel
+// as decode).
 #include "../common/ptx.cuh"
 
 namespace spark {
 
-constexpr int PF_BM = 64, PF_BN = 64;
+int make_tmap_rows64(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
 
-__device__ __forceinline__ void pf_cp16(void* smem_dst, const void* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+constexpr int PF_BM = 128, PF_BN = 64, PF_THREADS = 192;
+constexpr float PF_GROW = 8.f;          // log2 of how far a maximum may outgrow its reference
+
+// D = 256: the queries are a tensor-memory operand (a product of 64 keys reads 2 KB of shared memory per step instead of 6: 74 -> 25
+// cycles of issue each) and the ring has the room; 64 / 128: 256 columns hold everything with the queries in shared memory, and two
+// CTAs share an SM
+template <int D> struct Pf {
+  static constexpr bool QT = D == 256;
+  static constexpr int SLOTS = QT ? 6 : 4, SLOT = PF_BN * D * 2, Q_BYTES = QT ? 0 : PF_BM * D * 2;
+  static constexpr int SMEM = Q_BYTES + SLOTS * SLOT + 256 + 1024;
+  static constexpr int COLS = QT ? 512 : 256, S_COL = 0, P_COL = 64, O_COL = 128, Q_COL = 384;
+};
+
+struct PrefillArgs {
+  const __nv_bfloat16* q;                             // [R, Hq, D]
+  const long long* row_kv; const int* seg;            // cache row of a sequence's first token per row; [nseg][4]
+  const __nv_bfloat16* qkv; int ld, gated;            // gate columns
+  __nv_bfloat16* out;
+  int Hq, Hkv; float scale_log2;
+  const uint32_t* bmask; int mw;                      // MASK: a bit per 4-token key block, mw words per row
+  int* status;
+};
+
+__device__ __forceinline__ void pf_mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void pf_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void pf_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+__device__ __forceinline__ void pf_tmem_st_x32(uint32_t addr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+        "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
+__device__ __forceinline__ void pf_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ uint32_t pf_pack(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
+// N-major operand, 128-byte swizzle: 64 n are a 128-byte row per k; chunks of 64 n `chunk` bytes apart, groups of 8 k 1024 bytes
+__device__ __forceinline__ uint64_t pf_desc_nmajor(uint32_t addr, uint32_t chunk) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((addr & 0x3FFFF) >> 4);
+  d |= static_cast<uint64_t>(chunk >> 4) << 16;
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
 }
 
-// grid (row tiles, Hq, segments); 128 threads.  MASK: rows also carry a bit per 4-token key block (bmask [R, mw] words,
-// bit b of a row = block b may be attended): block-sparse selections of a few thousand tokens run through the dense
-// tiles with the unselected blocks masked, which beats one gathering CTA per row while the context is short enough.
+// grid (Hq, row tiles, segments)
 template <int D, bool MASK>
-__global__ void __launch_bounds__(128)
-attn_prefill_kernel(const __nv_bfloat16* __restrict__ qbuf,        // [R, Hq, D]
-                    const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc,   // [tokens, Hkv, D]
-                    const long long* __restrict__ row_kv, const int* __restrict__ seg,
-                    const __nv_bfloat16* __restrict__ qkv, int ld, int gated,
-                    __nv_bfloat16* __restrict__ out, int Hq, int Hkv, float scale_log2,
-                    const uint32_t* __restrict__ bmask, int mw) {
-  constexpr int LDS = D + 8;                                // smem row stride (elements): 16 bytes past a 128-byte multiple
-  extern __shared__ __align__(16) uint8_t smem_pf[];
-  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_pf);        // [64][LDS]
-  __nv_bfloat16* Ks = Qs + PF_BM * LDS;                                  // [2][64][LDS]
-  __nv_bfloat16* Vs = Ks + 2 * PF_BN * LDS;                              // [2][64][LDS]
-  const int sg = blockIdx.z, h = blockIdx.y;
-  const int qt = gridDim.x - 1 - blockIdx.x;                 // longest row tiles (most key tiles) are scheduled first
-  const int r0 = seg[sg * 4 + 1], n = seg[sg * 4 + 2], pos0 = seg[sg * 4 + 3];
+__global__ void __launch_bounds__(PF_THREADS, D == 256 ? 1 : 2)
+attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ PrefillArgs a) {
+  using L = Pf<D>;
+  constexpr int CH = D / 64, SLOT = L::SLOT, SLOTS = L::SLOTS, KV_CHUNK = PF_BN * 128, Q_CHUNK = PF_BM * 128;
+  constexpr int COLS = L::COLS, O_COL = L::O_COL;
+  const int sg = blockIdx.z, h = blockIdx.x;
+  const int qt = gridDim.y - 1 - blockIdx.y;                 // longest row tiles (most key tiles) are scheduled first
+  const int r0 = a.seg[sg * 4 + 1], n = a.seg[sg * 4 + 2], pos0 = a.seg[sg * 4 + 3];
   if (qt * PF_BM >= n) return;
-  const int hk = h / (Hq / Hkv);
-  const long long base = row_kv[r0];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int rows_valid = min(PF_BM, n - qt * PF_BM);
   const int nkeys = pos0 + qt * PF_BM + rows_valid;           // keys visible to the last valid row of the tile
   const int ntiles = (nkeys + PF_BN - 1) / PF_BN;
-  constexpr int VPR = D / 8;                                  // 16-byte vectors per row
 
-  auto load_kv = [&](int j, int buf) {
-    __nv_bfloat16* kd = Ks + buf * PF_BN * LDS;
-    __nv_bfloat16* vd = Vs + buf * PF_BN * LDS;
-    for (int i = tid; i < PF_BN * VPR; i += 128) {
-      const int r = i / VPR, v = i - r * VPR;
-      const int key = j * PF_BN + r;
-      if (key < nkeys) {
-        const size_t off = (static_cast<size_t>(base + key) * Hkv + hk) * D + v * 8;
-        pf_cp16(kd + r * LDS + v * 8, kc + off);
-        pf_cp16(vd + r * LDS + v * 8, vc + off);
-      } else {
-        *reinterpret_cast<uint4*>(kd + r * LDS + v * 8) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(vd + r * LDS + v * 8) = make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-  };
-  for (int i = tid; i < PF_BM * VPR; i += 128) {
-    const int r = i / VPR, v = i - r * VPR;
-    const int rr = min(r, rows_valid - 1);                     // padded rows repeat the last valid row
-    pf_cp16(Qs + r * LDS + v * 8, qbuf + (static_cast<size_t>(r0 + qt * PF_BM + rr) * Hq + h) * D + v * 8);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = smem + L::Q_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + SLOTS * SLOT);
+  uint64_t* empty = full + SLOTS;
+  uint64_t* q_full = empty + SLOTS;
+  uint64_t* v_fixed = q_full + 1;
+  uint64_t* s_full = v_fixed + 1;
+  uint64_t* s_read = s_full + 1;
+  uint64_t* p_full = s_read + 1;
+  uint64_t* o_full = p_full + 2;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_full + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    if (!L::QT) tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+    for (int s = 0; s < SLOTS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(q_full, L::QT ? 4 : 1); mbar_init(v_fixed, 1); mbar_init(s_full, 1); mbar_init(s_read, 4);
+    for (int s = 0; s < 2; ++s) { mbar_init(&p_full[s], 4); mbar_init(&o_full[s], 1); }
+    fence_barrier_init();
   }
-  load_kv(0, 0);
-  pf_commit();
+  if (warp == 1) { tmem_alloc<COLS>(tmem_ptr); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
 
-  float o[D / 8][4];
-#pragma unroll
-  for (int i = 0; i < D / 8; ++i) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
-  float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
-  // query positions of this thread's two rows (padded rows: the last valid row's)
-  const int p_lo = pos0 + qt * PF_BM + min(warp * 16 + g, rows_valid - 1);
-  const int p_hi = pos0 + qt * PF_BM + min(warp * 16 + g + 8, rows_valid - 1);
-  const uint32_t* bm_lo = MASK ? bmask + static_cast<size_t>(r0 + p_lo - pos0) * mw : nullptr;
-  const uint32_t* bm_hi = MASK ? bmask + static_cast<size_t>(r0 + p_hi - pos0) * mw : nullptr;
-
-  for (int j = 0; j < ntiles; ++j) {
-    const int buf = j & 1;
-    pf_wait<0>();
-    __syncthreads();
-    if (j + 1 < ntiles) { load_kv(j + 1, buf ^ 1); pf_commit(); }
-    const __nv_bfloat16* kb = Ks + buf * PF_BN * LDS;
-    const __nv_bfloat16* vb = Vs + buf * PF_BN * LDS;
-    // ---- S = Q K^T : 16 rows x 64 keys per warp
-    float s[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { s[i][0] = 0.f; s[i][1] = 0.f; s[i][2] = 0.f; s[i][3] = 0.f; }
-#pragma unroll
-    for (int ks = 0; ks < D / 16; ++ks) {
-      uint32_t a[4];
-      ldsm4(a, Qs + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDS + ks * 16 + (lane >> 4) * 8);
-#pragma unroll
-      for (int np = 0; np < 4; ++np) {
-        uint32_t b[4];
-        ldsm4(b, kb + (np * 16 + (lane >> 4) * 8 + (lane & 7)) * LDS + ks * 16 + ((lane >> 3) & 1) * 8);
-        mma_bf16(s[2 * np], a, b[0], b[1]);
-        mma_bf16(s[2 * np + 1], a, b[2], b[3]);
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer
+    const int hk = h / (a.Hq / a.Hkv);
+    const int base = static_cast<int>(a.row_kv[r0]);
+    int slot = 0; uint32_t ph = 0; bool ok = true;
+    if (!L::QT && lane == 0) {
+      mbar_arrive_expect_tx(q_full, PF_BM * D * 2);
+      for (int c = 0; c < CH; ++c) tma_load_2d(smem + c * Q_CHUNK, &tmQ, q_full, h * D + c * 64, r0 + qt * PF_BM);
+    }
+    int last_slot = 0; uint32_t last_ph = 0;
+    for (int i = 0; i < 2 * ntiles; ++i) {                    // K0 K1 V0 K2 V1 .. K(n-1) V(n-2) V(n-1)
+      const bool is_v = i == 2 * ntiles - 1 || (i >= 2 && !(i & 1));
+      const int j = i == 0 ? 0 : i == 2 * ntiles - 1 ? ntiles - 1 : is_v ? i / 2 - 1 : (i + 1) / 2;
+      ok = __all_sync(0xffffffffu, mbar_wait(&empty[slot], ph ^ 1));
+      if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, blockIdx.y, i); break; }
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&full[slot], SLOT);
+        for (int c = 0; c < CH; ++c)
+          tma_load_2d(ring + slot * SLOT + c * KV_CHUNK, is_v ? &tmV : &tmK, &full[slot], hk * D + c * 64, base + j * PF_BN);
+      }
+      __syncwarp();
+      last_slot = slot; last_ph = ph;
+      if (++slot == SLOTS) { slot = 0; ph ^= 1; }
+    }
+    const int keep = nkeys - (ntiles - 1) * PF_BN;
+    if (ok && keep < PF_BN) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[last_slot], last_ph));
+      if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -1);
+      if (ok) {
+        const int per = (PF_BN - keep) * 8;                   // 16-byte units of a chunk's rows past the last key
+        for (int u = lane; u < CH * per; u += 32)
+          *reinterpret_cast<uint4*>(ring + last_slot * SLOT + (u / per) * KV_CHUNK + keep * 128 + (u % per) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(v_fixed);
       }
     }
-    // ---- scale, causal mask, streaming softmax
-    const int k0 = j * PF_BN;
-    const bool need_mask = k0 + PF_BN - 1 > pos0 + qt * PF_BM;
-    // 16 block bits of this 64-key tile for the thread's two rows (a word covers two tiles)
-    const uint32_t sel_lo = MASK ? (__ldg(bm_lo + (j >> 1)) >> ((j & 1) * 16)) : 0u;
-    const uint32_t sel_hi = MASK ? (__ldg(bm_hi + (j >> 1)) >> ((j & 1) * 16)) : 0u;
-    float mx_lo = m_lo, mx_hi = m_hi;
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      const uint32_t id_s = make_idesc(1, 1, PF_BM, PF_BN), id_o = make_idesc(1, 1, PF_BM, D) | (1u << 16);
+      int slot = 0; uint32_t ph = 0;
+      bool ok = mbar_wait(q_full, 0);
+      if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -2);
+      const uint32_t qs = smem_u32(smem), rs = smem_u32(ring);
+      for (int j = -1; j < ntiles && ok; ++j) {
+        if (j + 1 < ntiles) {
+          // the scores have one buffer, free as soon as every warp has loaded those of tile j
+          if (!mbar_wait(&full[slot], ph) || (j >= 0 && !mbar_wait(s_read, j & 1))) {
+            set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+          for (int c = 0; c < CH; ++c) {
+            const uint64_t kd = make_smem_desc_sw128(rs + slot * SLOT + c * KV_CHUNK);
+            if (L::QT) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float v = s[i][e] * scale_log2;
-        if (need_mask) {
-          const int key = k0 + i * 8 + 2 * t + (e & 1);
-          if (key > ((e >> 1) ? p_hi : p_lo)) v = -INFINITY;
+              for (int k = 0; k < 4; ++k) pf_mma_ts(tmem + L::S_COL, tmem + L::Q_COL + c * 32 + k * 8, kd + 2 * k, id_s, (c | k) != 0);
+            } else {
+              const uint64_t qd = make_smem_desc_sw128(qs + c * Q_CHUNK);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) umma_f16(tmem + L::S_COL, qd + 2 * k, kd + 2 * k, id_s, (c | k) != 0);
+            }
+          }
+          umma_commit(&empty[slot]);
+          umma_commit(s_full);
+          if (++slot == SLOTS) { slot = 0; ph ^= 1; }
         }
-        if (MASK && !((((e >> 1) ? sel_hi : sel_lo) >> (i * 2 + (t >> 1))) & 1u)) v = -INFINITY;
-        s[i][e] = v;
+        if (j < 0) continue;
+        if (!mbar_wait(&full[slot], ph) || !mbar_wait(&p_full[j & 1], (j >> 1) & 1) ||
+            (j == ntiles - 1 && nkeys < ntiles * PF_BN && !mbar_wait(v_fixed, 0))) {
+          set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t p = tmem + L::P_COL + (j & 1) * 32;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          pf_mma_ts(tmem + O_COL, p + k * 8, pf_desc_nmajor(rs + slot * SLOT + k * 2048, KV_CHUNK), id_o, (j | k) != 0);
+        umma_commit(&empty[slot]);
+        umma_commit(&o_full[j & 1]);
+        if (++slot == SLOTS) { slot = 0; ph ^= 1; }
       }
-      mx_lo = fmaxf(mx_lo, fmaxf(s[i][0], s[i][1]));
-      mx_hi = fmaxf(mx_hi, fmaxf(s[i][2], s[i][3]));
     }
-    mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1)); mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-    mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1)); mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    // dense: key 0 is visible to every row, so mx is finite.  Masked: a row may have seen no key yet (mx = -inf):
-    // exponentials are then taken against 0, every term is exp2(-inf) = 0 and the running sums stay 0.
-    const float f_lo = (MASK && mx_lo == -INFINITY) ? 0.f : mx_lo, f_hi = (MASK && mx_hi == -INFINITY) ? 0.f : mx_hi;
-    const float c_lo = exp2f(m_lo - f_lo), c_hi = exp2f(m_hi - f_hi);
-    m_lo = mx_lo; m_hi = mx_hi;
-    float sum_lo = 0.f, sum_hi = 0.f;
+  } else {
+    // ------------------------------------------------------------ softmax, one query row per thread
+    const int q = warp & 3, row = q * 32 + lane;
+    const uint32_t t_lane = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    const int pos = pos0 + qt * PF_BM + min(row, rows_valid - 1);          // padded rows: the last valid row's mask
+    const uint32_t* bm = MASK ? a.bmask + static_cast<size_t>(r0 + pos - pos0) * a.mw : nullptr;
+    if (L::QT) {                                               // this thread's query: column c holds dimensions 2 c and 2 c + 1
+      const uint4* qp = reinterpret_cast<const uint4*>(a.q + (static_cast<size_t>(r0 + qt * PF_BM + min(row, rows_valid - 1)) * a.Hq + h) * D);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      s[i][0] = exp2f(s[i][0] - f_lo); s[i][1] = exp2f(s[i][1] - f_lo);
-      s[i][2] = exp2f(s[i][2] - f_hi); s[i][3] = exp2f(s[i][3] - f_hi);
-      sum_lo += s[i][0] + s[i][1]; sum_hi += s[i][2] + s[i][3];
+      for (int c = 0; c < D / 2; c += 32) {
+        uint32_t w[32];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 v = __ldg(qp + c / 4 + i);
+          w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+        pf_tmem_st_x32(t_lane + L::Q_COL + c, w);
+      }
+      pf_tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
     }
-    l_lo = l_lo * c_lo + sum_lo; l_hi = l_hi * c_hi + sum_hi;
+    // the gates are wanted at the end: from DRAM they took longer than the rest of the epilogue, so they are asked into L2 now
+    if (a.gated && row < rows_valid) {
+      const __nv_bfloat16* gp = a.qkv + static_cast<size_t>(r0 + qt * PF_BM + row) * a.ld + h * 2 * D + D;
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) { o[i][0] *= c_lo; o[i][1] *= c_lo; o[i][2] *= c_hi; o[i][3] *= c_hi; }
-    // ---- O += P V : P from the score registers (bf16), V fragments via transposed ldmatrix
+      for (int c = 0; c < D; c += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + c));
+    }
+    float m = -INFINITY, l = 0.f;
+    uint32_t word = MASK ? __ldg(bm) : 0u;
+    bool ok = true;
+    for (int j = 0; j < ntiles; ++j) {
+      uint32_t next = 0u;
+      if (MASK && (j & 1) && j + 1 < ntiles) next = __ldg(bm + ((j + 1) >> 1));
+      ok = __all_sync(0xffffffffu, mbar_wait(s_full, j & 1));
+      if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
+      tc_fence_after();
+      uint32_t raw[2][32];
+      tmem_ld_32x32(t_lane + L::S_COL, raw[0]);
+      tmem_ld_32x32(t_lane + L::S_COL + 32, raw[1]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_read);
+      float s[64];
 #pragma unroll
-    for (int kk = 0; kk < PF_BN / 16; ++kk) {
-      uint32_t a[4];
-      a[0] = pack_bf16(s[2 * kk][0], s[2 * kk][1]); a[1] = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
-      a[2] = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]); a[3] = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+      for (int i = 0; i < 64; ++i) s[i] = __uint_as_float(raw[i >> 5][i & 31]);
+      const int k0 = j * PF_BN;
+      if (MASK) {
+        const uint32_t sel = word >> ((j & 1) * 16);           // 16 block bits of this tile (a word covers two tiles)
 #pragma unroll
-      for (int np = 0; np < D / 16; ++np) {
-        uint32_t b[4];
-        ldsm4t(b, vb + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * LDS + np * 16 + (lane >> 4) * 8);
-        mma_bf16(o[2 * np], a, b[0], b[1]);
-        mma_bf16(o[2 * np + 1], a, b[2], b[3]);
+        for (int b = 0; b < 16; ++b) {
+          const bool on = (sel >> b) & 1u;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[b * 4 + e] = on ? s[b * 4 + e] : -INFINITY;
+        }
+        if (j & 1) word = next;
+      }
+      if (k0 + PF_BN - 1 > pos0 + qt * PF_BM) {                // a tile on the diagonal, or past the last key
+        const int seen = pos - k0;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) s[i] = i <= seen ? s[i] : -INFINITY;
+      }
+      float mx[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mx[i] = s[i];
+#pragma unroll
+      for (int i = 8; i < 64; ++i) mx[i & 7] = fmaxf(mx[i & 7], s[i]);
+      const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7]))) * a.scale_log2;
+      // m stays the reference until a maximum outgrows it; m = -inf: this row has seen no key yet
+      const bool grow = top > m + PF_GROW;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float c = grow ? pf_exp2(m - top) : 1.f;
+        if (grow) { m = top; l *= c; }
+        if (j > 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1));
+          if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
+          tc_fence_after();
+#pragma unroll 1
+          for (int cc = 0; cc < D; cc += 32) {
+            uint32_t o[32];
+            tmem_ld_32x32(t_lane + O_COL + cc, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * c);
+            pf_tmem_st_x32(t_lane + O_COL + cc, o);
+          }
+        }
+      }
+      const float ref = m == -INFINITY ? 0.f : m;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t p[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float e0 = pf_exp2(fmaf(s[2 * i], a.scale_log2, -ref)), e1 = pf_exp2(fmaf(s[2 * i + 1], a.scale_log2, -ref));
+        sum[i & 1] += e0; sum[2 + (i & 1)] += e1;
+        p[i] = pf_pack(e0, e1);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      // P's buffer: the product of two tiles back has read it
+      if (j >= 2) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[j & 1], ((j - 2) >> 1) & 1));
+        if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
+      }
+      pf_tmem_st_x32(t_lane + L::P_COL + (j & 1) * 32, p);
+      pf_tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
+    }
+    // ---- epilogue: normalise, gate, store
+    if (ok) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1));
+      if (!ok) set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, ntiles);
+    }
+    if (ok) {
+      tc_fence_after();
+      // through shared memory (queries, keys and values are used up), so that a row's columns are read and written together
+      constexpr int LX = D + 1, CW = D / 64;                   // 64-column pieces of a row: a lane has columns 2 lane, 2 lane + 1 of each
+      float* x = reinterpret_cast<float*>(smem) + q * (32 * LX);
+      const float inv = 1.f / l;
+      const int live = min(32, rows_valid - q * 32);
+      const size_t rw = static_cast<size_t>(r0 + qt * PF_BM + q * 32);
+#pragma unroll 1
+      for (int cc = 0; cc < D; cc += 32) {
+        uint32_t o[32];
+        tmem_ld_32x32(t_lane + O_COL + cc, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[lane * LX + cc + i] = __uint_as_float(o[i]) * inv;
+      }
+      __syncwarp();
+      // eight rows' gates are asked for before the first is used
+#pragma unroll 1
+      for (int i0 = 0; i0 < live; i0 += 8) {
+        uint32_t gate[8][CW];
+        if (a.gated) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const __nv_bfloat16* gp = a.qkv + (rw + min(i0 + i, live - 1)) * a.ld + h * 2 * D + D + 2 * lane;
+#pragma unroll
+            for (int c = 0; c < CW; ++c) gate[i][c] = __ldg(reinterpret_cast<const uint32_t*>(gp + c * 64));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          __nv_bfloat16* dst = a.out + ((rw + i0 + i) * a.Hq + h) * D + 2 * lane;
+#pragma unroll
+          for (int c = 0; c < CW; ++c) {
+            float v0 = x[(i0 + i) * LX + c * 64 + 2 * lane], v1 = x[(i0 + i) * LX + c * 64 + 2 * lane + 1];
+            if (a.gated) {
+              const float2 gt = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gate[i][c]));
+              v0 = __fdividef(v0, 1.f + __expf(-gt.x)); v1 = __fdividef(v1, 1.f + __expf(-gt.y));
+            }
+            if (i0 + i < live) *reinterpret_cast<uint32_t*>(dst + c * 64) = pf_pack(v0, v1);
+          }
+        }
       }
     }
   }
-  // ---- epilogue: row sums over the quad, normalise, gate, store
-  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1); l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1); l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-  const float inv_lo = 1.f / l_lo, inv_hi = 1.f / l_hi;
-#pragma unroll
-  for (int hh = 0; hh < 2; ++hh) {
-    const int rl = warp * 16 + g + hh * 8;
-    if (rl >= rows_valid) continue;
-    const size_t r = static_cast<size_t>(r0 + qt * PF_BM + rl);
-    const float inv = hh ? inv_hi : inv_lo;
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      const int d = i * 8 + 2 * t;
-      float v0 = o[i][2 * hh] * inv, v1 = o[i][2 * hh + 1] * inv;
-      if (gated) {
-        const float2 gt = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(qkv + r * ld + h * 2 * D + D + d));
-        v0 = v0 / (1.f + __expf(-gt.x)); v1 = v1 / (1.f + __expf(-gt.y));
-      }
-      *reinterpret_cast<__nv_bfloat162*>(out + (r * Hq + h) * D + d) = __floats2bfloat162_rn(v0, v1);
-    }
-  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc<COLS>(tmem); }
 }
 
 template <int D, bool MASK>
-static int launch_prefill(const void* qbuf, const void* kc, const void* vc, const long long* row_kv, const int* seg, int nseg,
-                          int max_rows, const void* qkv, int ld, int gated, void* out, int Hq, int Hkv, float scale,
-                          cudaStream_t s, const uint32_t* bmask = nullptr, int mw = 0) {
+static int launch_prefill(const void* qbuf, int R, const void* kc, const void* vc, long long tokens, int nseg, int max_rows,
+                          const PrefillArgs& a, cudaStream_t s) {
+  CUtensorMap tq, tk, tv;
+  const uint64_t wq = static_cast<uint64_t>(a.Hq) * D, wk = static_cast<uint64_t>(a.Hkv) * D;
+  if (int r = make_tmap_rows64(&tq, qbuf, R, wq, wq, PF_BM, 1)) return r;
+  if (int r = make_tmap_rows64(&tk, kc, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_rows64(&tv, vc, tokens, wk, wk, PF_BN, 1)) return r;
   auto kern = attn_prefill_kernel<D, MASK>;
-  constexpr int smem = (PF_BM + 4 * PF_BN) * (D + 8) * 2;
   static bool done = false;
-  if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); done = true; }
-  dim3 grid((max_rows + PF_BM - 1) / PF_BM, Hq, nseg);
-  kern<<<grid, 128, smem, s>>>((const __nv_bfloat16*)qbuf, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, row_kv, seg,
-                               (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv,
-                               scale * 1.4426950408889634f, bmask, mw);
+  if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Pf<D>::SMEM); done = true; }
+  kern<<<dim3(a.Hq, (max_rows + PF_BM - 1) / PF_BM, nseg), PF_THREADS, Pf<D>::SMEM, s>>>(tq, tk, tv, a);
   return spark_launch_rc(__func__);
 }
 
@@ -236,17 +411,26 @@ sel_blockmask_kernel(const int* __restrict__ sel, const int* __restrict__ sel_n,
 
 using namespace spark;
 
-// Dense causal attention over bf16 caches for whole segments.  seg: int [nseg][4] = slot, first row, rows, first
-// position; max_rows = longest segment.  head_dim 64, 128 or 256.
+template <bool MASK>
+static int prefill(const void* qbuf, int R, const void* kc, const void* vc, long long tokens, int nseg, int max_rows, int D,
+                   const PrefillArgs& a, cudaStream_t s) {
+  if (tokens <= 0 || tokens > 0x7fffffffLL || a.Hkv <= 0 || a.Hq % a.Hkv || (a.gated && (a.ld & 1))) return -5;
+  if (D == 256) return launch_prefill<256, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
+  if (D == 128) return launch_prefill<128, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
+  if (D == 64) return launch_prefill<64, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
+  return -5;
+}
+
+// Dense causal attention over bf16 caches for whole segments.  seg: int [nseg][4] = slot, first row, rows, first position; R: rows of
+// qbuf; max_rows = longest segment; tokens: cache rows that may be touched (past the last key of every segment: what lies
+// between is read and masked, what lies beyond is not read).  head_dim 64, 128 or 256.
 extern "C" int spark_attn_prefill(const void* qbuf, const void* kc, const void* vc, const long long* row_kv, const int* seg,
                                   int nseg, int max_rows, const void* qkv, int ld, int gated, void* out, int Hq, int Hkv,
-                                  int D, float scale, cudaStream_t s) {
-  if (nseg <= 0 || max_rows <= 0) return 0;
-  if (Hq % Hkv) return -5;
-  if (D == 256) return launch_prefill<256, false>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s);
-  if (D == 128) return launch_prefill<128, false>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s);
-  if (D == 64) return launch_prefill<64, false>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s);
-  return -5;
+                                  int D, float scale, int R, long long tokens, int* status, cudaStream_t s) {
+  if (nseg <= 0 || max_rows <= 0 || R <= 0) return 0;
+  const PrefillArgs a{(const __nv_bfloat16*)qbuf, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
+                      nullptr, 0, status};
+  return prefill<false>(qbuf, R, kc, vc, tokens, nseg, max_rows, D, a, s);
 }
 
 // The same tiles for rows with a block-sparse selection (4-token blocks): sel / sel_n are the per-row token lists of the
@@ -254,12 +438,11 @@ extern "C" int spark_attn_prefill(const void* qbuf, const void* kc, const void* 
 extern "C" int spark_attn_prefill_masked(const void* qbuf, const void* kc, const void* vc, const long long* row_kv,
                                          const int* seg, int nseg, int max_rows, const void* qkv, int ld, int gated, void* out,
                                          int Hq, int Hkv, int D, float scale, const int* sel, const int* sel_n, int sel_ld,
-                                         int R, unsigned* bmask, int mw, cudaStream_t s) {
+                                         int R, unsigned* bmask, int mw, long long tokens, int* status, cudaStream_t s) {
   if (nseg <= 0 || max_rows <= 0 || R <= 0) return 0;
-  if (Hq % Hkv || mw <= 0 || mw > 8192 || !sel || !sel_n || !bmask) return -5;
+  if (mw <= 0 || mw > 8192 || !sel || !sel_n || !bmask) return -5;
   sel_blockmask_kernel<<<R, 256, mw * 4, s>>>(sel, sel_n, sel_ld, bmask, mw);
-  if (D == 256) return launch_prefill<256, true>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s, bmask, mw);
-  if (D == 128) return launch_prefill<128, true>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s, bmask, mw);
-  if (D == 64) return launch_prefill<64, true>(qbuf, kc, vc, row_kv, seg, nseg, max_rows, qkv, ld, gated, out, Hq, Hkv, scale, s, bmask, mw);
-  return -5;
+  const PrefillArgs a{(const __nv_bfloat16*)qbuf, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
+                      bmask, mw, status};
+  return prefill<true>(qbuf, R, kc, vc, tokens, nseg, max_rows, D, a, s);
 }

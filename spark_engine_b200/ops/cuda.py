@@ -59,9 +59,9 @@ _SIGS = {
     "spark_kda_chunk_prefill": [vp, i32, vp, vp, i32, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32,
                                 i32, i32, vp],
     "spark_kda_seq": [vp, i32, vp, vp, i32, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, vp, vp, i32, i32],
-    "spark_attn_prefill": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp],
+    "spark_attn_prefill": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, i32, i64, vp, vp],
     "spark_attn_prefill_masked": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp, vp, i32, i32, vp,
-                                  i32, vp],
+                                  i32, i64, vp, vp],
     "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp],
     "spark_exl3_had_gather": [vp, i32, vp, vp, i32, vp, i64, vp, i32, i32, i32, vp],
     "spark_gdn_chunk_prefill": [vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32,
@@ -1285,6 +1285,12 @@ def tree_ancestor_masks(plan, device) -> torch.Tensor:
     return torch.from_numpy(m.view(np.int32)).to(device)
 
 
+def _keys_end(plan, seqs):
+    """First cache row behind every key of the plan: whole tiles may be read up to here (a cache that grows on demand is backed up
+    to its highest lease)."""
+    return max(seqs[s.slot].kv_base + s.pos0 + s.n for s in plan.segs)
+
+
 def attn_mixer(mixer, qkv, plan, seqs):
     c = mixer.c
     dev = qkv.device
@@ -1329,18 +1335,19 @@ def attn_mixer(mixer, qkv, plan, seqs):
         max_ctx = sel_ld
     if (sel is None and not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.head_dim in (64, 128, 256)
             and min(s.n for s in plan.segs) >= ATTN_PREFILL_MIN_ROWS):
-        # whole segments, dense context: flash-style tensor-core kernel (one CTA per 64 rows of a head)
+        # whole segments, dense context: streaming softmax on tcgen05 (one CTA per 128 rows of a head)
         out = torch.empty(R, c.n_q_heads * c.head_dim, dtype=torch.bfloat16, device=dev)
         rc = lib().spark_attn_prefill(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
                                       max(s.n for s in plan.segs), P(qkv), qkv.stride(0), int(c.gated), P(out),
-                                      c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), stream())
+                                      c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), R,
+                                      _keys_end(plan, seqs), P(status_word(dev)), stream())
         check(rc, "spark_attn_prefill")
         return out
     if (sel is not None and not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.block == 4
             and c.head_dim in (64, 128, 256) and min(s.n for s in plan.segs) >= ATTN_PREFILL_MIN_ROWS
             and max(s.pos0 + s.n // 2 for s in plan.segs) <= ATTN_MASKED_MAX_KEYS):
         # block-sparse rows on a context of a few thousand tokens: the dense tiles with the unselected blocks masked
-        # (64 rows share every key tile) beat one gathering CTA per row, which is bound by L2 bandwidth
+        # (128 rows share every key tile) beat one gathering CTA per row, which is bound by L2 bandwidth
         mw = (d["max_ctx"] + 127) // 128
         bmask = scratch("attn_block_mask", R * mw, torch.int32, dev)
         out = torch.empty(R, c.n_q_heads * c.head_dim, dtype=torch.bfloat16, device=dev)
@@ -1348,7 +1355,8 @@ def attn_mixer(mixer, qkv, plan, seqs):
         rc = lib().spark_attn_prefill_masked(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
                                              max(s.n for s in plan.segs), P(qkv), qkv.stride(0), int(c.gated), P(out),
                                              c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), P(sel),
-                                             P(sel_n), sel_ld, R, P(bmask), mw, stream())
+                                             P(sel_n), sel_ld, R, P(bmask), mw, _keys_end(plan, seqs), P(status_word(dev)),
+                                             stream())
         check(rc, "spark_attn_prefill_masked")
         return out
     nsplit, chunks = (max_ctx + ATT_TS - 1) // ATT_TS, 1
