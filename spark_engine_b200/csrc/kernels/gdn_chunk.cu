@@ -9,7 +9,7 @@
 //     O = diag(D) Q S0^T + P U,                           P_tj = (D_t/D_j) (q_t.k_j)         (j <= t)
 //     S_C = D_C S0 + U^T diag(D_C / D) K
 // so with T = (I + A)^-1 everything that does not involve S0 is computed for all chunks in parallel:
-//   kernel 1 (chunk, head):  conv(k=4)+SiLU, L2 norms, gates;  K K^T, Q K^T -> A, P;  T by forward substitution;
+//   kernel 1 (chunk, head):  conv(k=4)+SiLU, L2 norms, gates;  K K^T, Q K^T -> A, P;  T by blocks;
 //                            W = T diag(beta D) K,  Ut = T diag(beta) V,  Qt = diag(D) Q,  Kt = diag(D_C/D) K
 //   kernel 2 (v-slice, head, segment), sequential over the chunks of one sequence, S kept in registers:
 //                            U = Ut - W S0^T;  O = Qt S0^T + P U;  S <- D_C S + U^T Kt
@@ -44,27 +44,65 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], float a0, float a1, floa
                : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)),
                  "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
-__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }      // rounded to TF32 next
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------- kernel 1
-// grid (chunks, Hv); 256 threads
-__global__ void __launch_bounds__(256)
+// grid (chunks, Hv); 256 threads.  Two CTAs share an SM (107 KB each): A and T take the place of Q once its products are through.
+// What bounds it: the chain of its phases, of which the convolution is the longest (a row of a warp is 95 instructions for four
+// channels), hidden only by the second CTA; 302 MB are written at 1.5 TB/s.  64 chunks of 32 heads: 544 -> 198 us (one CTA per SM,
+// one channel per lane with its rows loaded one after the other: 20 us for the convolution of a CTA).
+constexpr int SM_AT = GC * LD128, SM_AT_EXTRA = 2 * GC * LD64 - SM_AT;      // floats of A and T past the end of Q
+constexpr int PREP_SMEM = (3 * GC * LD128 + SM_AT_EXTRA + 3 * GC) * 4;
+
+// Rows 8 warp - 3 .. 8 warp + 7 of four consecutive channels as they are in memory (zero outside the segment)
+__device__ __forceinline__ void gdn_load_rows(const __nv_bfloat16* __restrict__ proj, int ldp, int r0, int first, int n, int ch, uint2 (&x)[11]) {
+#pragma unroll
+  for (int j = 0; j < 11; ++j) {
+    const int p = first + j;
+    x[j] = p >= 0 && p < n ? __ldg(reinterpret_cast<const uint2*>(proj + static_cast<size_t>(r0 + p) * ldp + ch)) : make_uint2(0u, 0u);
+  }
+}
+// The same in fp32, rows before the segment's start from the slot's history
+__device__ __forceinline__ void gdn_widen_rows(const uint2 (&u)[11], const float* __restrict__ hist, size_t hist_ld, int first, float4 (&x)[11]) {
+#pragma unroll
+  for (int j = 0; j < 11; ++j) {
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[j].x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[j].y));
+    x[j] = make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
+  if (first < 0) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (first + j < 0) x[j] = *reinterpret_cast<const float4*>(hist + static_cast<size_t>(first + j + 3) * hist_ld);
+  }
+}
+// conv(k = 4) + SiLU of row i (x[i .. i + 3]); w[c]: taps of channel c
+__device__ __forceinline__ float4 gdn_conv(const float4 (&x)[11], int i, const float4 (&w)[4]) {
+  return make_float4(silu(x[i].x * w[0].x + x[i + 1].x * w[0].y + x[i + 2].x * w[0].z + x[i + 3].x * w[0].w),
+                     silu(x[i].y * w[1].x + x[i + 1].y * w[1].y + x[i + 2].y * w[1].z + x[i + 3].y * w[1].w),
+                     silu(x[i].z * w[2].x + x[i + 1].z * w[2].y + x[i + 2].z * w[2].z + x[i + 3].z * w[2].w),
+                     silu(x[i].w * w[3].x + x[i + 1].w * w[3].y + x[i + 2].w * w[3].z + x[i + 3].w * w[3].w));
+}
+__device__ __forceinline__ float4 scale_tf32(float4 v, float f) { return make_float4(tf32r(v.x * f), tf32r(v.y * f), tf32r(v.z * f), tf32r(v.w * f)); }
+
+// w_wide: the convolution's taps start on 16 bytes
+__global__ void __launch_bounds__(256, 2)
 gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __nv_bfloat16* __restrict__ ab, int ldab,
                       const float* __restrict__ conv_w, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                       const float* __restrict__ tail, const int* __restrict__ seg, const int* __restrict__ chunks,
-                      float* __restrict__ ws, int Hk, int Hv, float eps) {
+                      float* __restrict__ ws, int Hk, int Hv, float eps, int w_wide) {
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;                          // [64][136]
-  float* Ks = Qs + GC * LD128;
+  float* As = sm;                          // [64][72]   A, over Q
+  float* Ts = As + GC * LD64;              // [64][72]   T
+  float* Ks = sm + SM_AT + SM_AT_EXTRA;
   float* Vs = Ks + GC * LD128;
-  float* As = Vs + GC * LD128;             // [64][72]   A, later T diag(beta D)
-  float* Ts = As + GC * LD64;              // [64][72]   T, later T diag(beta)
-  float* beta_s = Ts + GC * LD64;          // [64]
+  float* beta_s = Vs + GC * LD128;         // [64]
   float* G_s = beta_s + GC;                // [64] cumulative log decay
+  float* D_s = G_s + GC;                   // [64] exp of it
   const int ci = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sg = chunks[2 * ci], c = chunks[2 * ci + 1];
   const int slot = seg[sg * 4], r0 = seg[sg * 4 + 1], n = seg[sg * 4 + 2];
@@ -72,86 +110,75 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
   const int hk = h / (Hv / Hk);
   float* wsb = ws + (static_cast<size_t>(ci) * Hv + h) * WS_STRIDE;
 
-  // ---- conv + SiLU + L2 norms: warp w owns rows 8w..8w+7 (sliding window), lane owns channels lane+32cc
-  {
-    const float* tl = tail + (static_cast<size_t>(slot) * 3 * Hv + h) * 3 * GD;
-    const float qscale = rsqrtf(static_cast<float>(GD));
-    float hq[4][3], hk_[4][3], hv[4][3], wq[4][4], wk[4][4], wv[4][4];
-    int chq[4], chk[4], chv[4];
+  // ---- inputs of this warp's eight rows are asked for first: a lane owns four channels of q, of k and of v
+  const float* hist = tail + (static_cast<size_t>(slot) * 3 * Hv + h) * 3 * GD + lane * 4;
+  const size_t hist_ld = static_cast<size_t>(Hv) * 3 * GD;
+  const int first = t0 + warp * 8 - 3;
+  const int chq = hk * GD + lane * 4, chk = Hk * GD + chq, chv = 2 * Hk * GD + h * GD + lane * 4;
+  uint2 raw[3][11];
+  gdn_load_rows(proj, ldp, r0, first, n, chq, raw[0]);
+  gdn_load_rows(proj, ldp, r0, first, n, chk, raw[1]);
+  gdn_load_rows(proj, ldp, r0, first, n, chv, raw[2]);
+  // ---- gates and the prefix sum of the log decays: warp 0, two rows per lane
+  if (warp == 0) {
+    float beta[2], lg[2];
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      const int i = lane + 32 * cc;
-      chq[cc] = hk * GD + i; chk[cc] = Hk * GD + hk * GD + i; chv[cc] = 2 * Hk * GD + h * GD + i;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        wq[cc][j] = conv_w[chq[cc] * 4 + j]; wk[cc][j] = conv_w[chk[cc] * 4 + j]; wv[cc][j] = conv_w[chv[cc] * 4 + j];
-      }
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int p = t0 + warp * 8 - 3 + j;            // position in the segment of history entry j
-        if (p < 0) {
-          const float* t = tl + static_cast<size_t>(p + 3) * Hv * 3 * GD;
-          hq[cc][j] = t[i]; hk_[cc][j] = t[GD + i]; hv[cc][j] = t[2 * GD + i];
-        } else if (p < n) {
-          const __nv_bfloat16* pr = proj + static_cast<size_t>(r0 + p) * ldp;
-          hq[cc][j] = __bfloat162float(pr[chq[cc]]); hk_[cc][j] = __bfloat162float(pr[chk[cc]]);
-          hv[cc][j] = __bfloat162float(pr[chv[cc]]);
-        } else { hq[cc][j] = 0.f; hk_[cc][j] = 0.f; hv[cc][j] = 0.f; }
-      }
-    }
-    for (int rr = 0; rr < 8; ++rr) {
-      const int r = warp * 8 + rr;
-      float q[4], k[4], v[4], q2 = 0.f, k2 = 0.f;
+    for (int i = 0; i < 2; ++i) {
+      const int r = lane * 2 + i;
+      beta[i] = 0.f; lg[i] = 0.f;
       if (r < nv) {
-        const __nv_bfloat16* pr = proj + static_cast<size_t>(r0 + t0 + r) * ldp;
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const float xq = __bfloat162float(pr[chq[cc]]), xk = __bfloat162float(pr[chk[cc]]), xv = __bfloat162float(pr[chv[cc]]);
-          q[cc] = silu(hq[cc][0] * wq[cc][0] + hq[cc][1] * wq[cc][1] + hq[cc][2] * wq[cc][2] + xq * wq[cc][3]);
-          k[cc] = silu(hk_[cc][0] * wk[cc][0] + hk_[cc][1] * wk[cc][1] + hk_[cc][2] * wk[cc][2] + xk * wk[cc][3]);
-          v[cc] = silu(hv[cc][0] * wv[cc][0] + hv[cc][1] * wv[cc][1] + hv[cc][2] * wv[cc][2] + xv * wv[cc][3]);
-          hq[cc][0] = hq[cc][1]; hq[cc][1] = hq[cc][2]; hq[cc][2] = xq;
-          hk_[cc][0] = hk_[cc][1]; hk_[cc][1] = hk_[cc][2]; hk_[cc][2] = xk;
-          hv[cc][0] = hv[cc][1]; hv[cc][1] = hv[cc][2]; hv[cc][2] = xv;
-          q2 = fmaf(q[cc], q[cc], q2); k2 = fmaf(k[cc], k[cc], k2);
-        }
-        q2 = warp_sum(q2); k2 = warp_sum(k2);
-        const float qn = rsqrtf(q2 + eps) * qscale, kn = rsqrtf(k2 + eps);
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) { q[cc] *= qn; k[cc] *= kn; }
-      } else {
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) { q[cc] = 0.f; k[cc] = 0.f; v[cc] = 0.f; }
-      }
-#pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
-        const int i = lane + 32 * cc;
-        Qs[r * LD128 + i] = tf32r(q[cc]); Ks[r * LD128 + i] = tf32r(k[cc]); Vs[r * LD128 + i] = tf32r(v[cc]);
+        const float bl = __bfloat162float(ab[static_cast<size_t>(r0 + t0 + r) * ldab + h]);
+        const float al = __bfloat162float(ab[static_cast<size_t>(r0 + t0 + r) * ldab + Hv + h]);
+        beta[i] = 1.f / (1.f + __expf(-bl));
+        const float xa = al + dt_bias[h];
+        const float sp = xa > 20.f ? xa : log1pf(__expf(xa));
+        lg[i] = -__expf(A_log[h]) * sp;
       }
     }
-  }
-  if (tid < GC) {
-    float beta = 0.f, lg = 0.f;
-    if (tid < nv) {
-      const float bl = __bfloat162float(ab[static_cast<size_t>(r0 + t0 + tid) * ldab + h]);
-      const float al = __bfloat162float(ab[static_cast<size_t>(r0 + t0 + tid) * ldab + Hv + h]);
-      beta = 1.f / (1.f + __expf(-bl));
-      const float xa = al + dt_bias[h];
-      const float sp = xa > 20.f ? xa : log1pf(__expf(xa));
-      lg = -__expf(A_log[h]) * sp;
-    }
-    beta_s[tid] = beta;
-    G_s[tid] = lg;
+    float inc = lg[0] + lg[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += u; }
+    float before = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) before = 0.f;
+    const float G0 = before + lg[0], G1 = G0 + lg[1];
+    *reinterpret_cast<float2*>(beta_s + lane * 2) = make_float2(beta[0], beta[1]);
+    *reinterpret_cast<float2*>(G_s + lane * 2) = make_float2(G0, G1);
+    *reinterpret_cast<float2*>(D_s + lane * 2) = make_float2(__expf(G0), __expf(G1));
   }
   __syncthreads();
-  {                                                  // inclusive prefix sum of the log decays
-    float gsum = 0.f;
-    if (tid < GC)
-      for (int j = 0; j <= tid; ++j) gsum += G_s[j];
-    __syncthreads();
-    if (tid < GC) G_s[tid] = gsum;
-    __syncthreads();
+  // ---- conv + SiLU + L2 norms -> shared memory (TF32), Qt = diag(D) Q and Kt = diag(D_C / D) K -> workspace
+  {
+    const float Gl = G_s[GC - 1];
+    float4 w[4];
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {                  // q, k, v
+      const int ch = part == 0 ? chq : part == 1 ? chk : chv;
+      float4 x[11];
+      gdn_widen_rows(raw[part], hist + part * GD, hist_ld, first, x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float* p = conv_w + static_cast<size_t>(ch + i) * 4;
+        w[i] = w_wide ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(p[0], p[1], p[2], p[3]);
+      }
+      float* dst = (part == 0 ? Qs : part == 1 ? Ks : Vs) + warp * 8 * LD128 + lane * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = warp * 8 + i;
+        float4 y = r < nv ? gdn_conv(x, i, w) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float f = 1.f;
+        if (part < 2) {
+          const float ss = warp_sum(fmaf(y.w, y.w, fmaf(y.z, y.z, fmaf(y.y, y.y, y.x * y.x))));
+          f = rsqrtf(ss + eps) * (part == 0 ? rsqrtf(static_cast<float>(GD)) : 1.f);
+        }
+        y = scale_tf32(y, f);
+        *reinterpret_cast<float4*>(dst + i * LD128) = y;
+        if (part < 2)
+          *reinterpret_cast<float4*>(wsb + (part == 0 ? WS_QT : WS_KT) + r * GD + lane * 4) = scale_tf32(y, part == 0 ? D_s[r] : __expf(Gl - G_s[r]));
+      }
+    }
+    if (tid == 0) wsb[WS_DC] = __expf(Gl);
   }
+  __syncthreads();
 
   const int g = lane >> 2, t = lane & 3;
   // ---- K K^T and Q K^T (lower triangle only): warp -> m-tile (warp&3), n-tiles 4*(warp>>2) .. +4
@@ -162,77 +189,133 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
     for (int a = 0; a < 4; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) { ckk[a][b] = 0.f; cqk[a][b] = 0.f; }
-    const float* ka = Ks + (mt * 16 + g) * LD128 + t;
-    const float* qa = Qs + (mt * 16 + g) * LD128 + t;
-    for (int ks = 0; ks < GD / 8; ++ks) {
-      const float k0 = ka[ks * 8], k1 = ka[8 * LD128 + ks * 8], k2 = ka[ks * 8 + 4], k3 = ka[8 * LD128 + ks * 8 + 4];
-      const float q0 = qa[ks * 8], q1 = qa[8 * LD128 + ks * 8], q2 = qa[ks * 8 + 4], q3 = qa[8 * LD128 + ks * 8 + 4];
+    if (nt0 * 8 <= mt * 16 + 15) {
+      const float* ka = Ks + (mt * 16 + g) * LD128 + t;
+      const float* qa = Qs + (mt * 16 + g) * LD128 + t;
+#pragma unroll 4
+      for (int ks = 0; ks < GD / 8; ++ks) {
+        const float k0 = ka[ks * 8], k1 = ka[8 * LD128 + ks * 8], k2 = ka[ks * 8 + 4], k3 = ka[8 * LD128 + ks * 8 + 4];
+        const float q0 = qa[ks * 8], q1 = qa[8 * LD128 + ks * 8], q2 = qa[ks * 8 + 4], q3 = qa[8 * LD128 + ks * 8 + 4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int nt = nt0 + a;
-        if (nt * 8 > mt * 16 + 15) continue;                      // strictly above the diagonal
-        const float* kb = Ks + (nt * 8 + g) * LD128 + ks * 8 + t;
-        const float b0 = kb[0], b1 = kb[4];
-        mma_tf32(ckk[a], k0, k1, k2, k3, b0, b1);
-        mma_tf32(cqk[a], q0, q1, q2, q3, b0, b1);
+        for (int a = 0; a < 4; ++a) {
+          const int nt = nt0 + a;
+          if (nt * 8 > mt * 16 + 15) continue;                      // strictly above the diagonal
+          const float* kb = Ks + (nt * 8 + g) * LD128 + ks * 8 + t;
+          const float b0 = kb[0], b1 = kb[4];
+          mma_tf32(ckk[a], k0, k1, k2, k3, b0, b1);
+          mma_tf32(cqk[a], q0, q1, q2, q3, b0, b1);
+        }
       }
     }
+    __syncthreads();                                                // Q is read: A takes its place
     float* Pg = wsb + WS_P;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      const int nt = nt0 + a;
+      const int col = (nt0 + a) * 8 + 2 * t;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int row = mt * 16 + g + (e >> 1) * 8, col = nt * 8 + 2 * t + (e & 1);
-        float av = 0.f, pv = 0.f;
-        if (col <= row) {
-          const float dec = __expf(G_s[row] - G_s[col]);
-          pv = dec * cqk[a][e];
-          if (col < row) av = beta_s[row] * dec * ckk[a][e];
+      for (int e = 0; e < 2; ++e) {
+        const int row = mt * 16 + g + e * 8;
+        float av[2], pv[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          av[u] = 0.f; pv[u] = 0.f;
+          if (col + u <= row) {
+            const float dec = __expf(G_s[row] - G_s[col + u]);
+            pv[u] = tf32r(dec * cqk[a][e * 2 + u]);
+            if (col + u < row) av[u] = beta_s[row] * dec * ckk[a][e * 2 + u];
+          }
         }
-        As[row * LD64 + col] = av;
-        Pg[row * GC + col] = tf32r(pv);
+        *reinterpret_cast<float2*>(As + row * LD64 + col) = make_float2(av[0], av[1]);
+        *reinterpret_cast<float2*>(Pg + row * GC + col) = make_float2(pv[0], pv[1]);
       }
     }
   }
   __syncthreads();
-  // ---- T = (I + A)^-1: thread c owns column c (forward substitution, column in registers)
+  // ---- T = (I + A)^-1 by blocks, all in fp32: the four 16 x 16 blocks on the diagonal by forward substitution (a thread per
+  // column), then twice T21 = -T22 (A21 T11).  A's unused upper blocks hold A21 T11.  (One thread per column of the whole matrix
+  // was a chain of 2016 steps on two warps.)
   if (tid < GC) {
-    float tc[GC];
+    const int b0 = tid & ~15, cc = tid & 15;
+    float tc[16];
 #pragma unroll
-    for (int i = 0; i < GC; ++i) {
-      float s = (i == tid) ? 1.f : 0.f;
+    for (int i = 0; i < 16; ++i) {
+      const float4* row = reinterpret_cast<const float4*>(As + (b0 + i) * LD64 + b0);
+      float s0 = i == cc ? 1.f : 0.f, s1 = 0.f;
 #pragma unroll
-      for (int j = 0; j < i; ++j) s = fmaf(-As[i * LD64 + j], tc[j], s);
-      tc[i] = s;
+      for (int j = 0; j < i; j += 4) {
+        const float4 av = row[j >> 2];
+        s0 = fmaf(-av.x, tc[j], s0);
+        if (j + 1 < i) s1 = fmaf(-av.y, tc[j + 1 < 16 ? j + 1 : 15], s1);
+        if (j + 2 < i) s0 = fmaf(-av.z, tc[j + 2 < 16 ? j + 2 : 15], s0);
+        if (j + 3 < i) s1 = fmaf(-av.w, tc[j + 3 < 16 ? j + 3 : 15], s1);
+      }
+      tc[i] = s0 + s1;
     }
 #pragma unroll
-    for (int i = 0; i < GC; ++i) Ts[i * LD64 + tid] = tc[i];
+    for (int i = 0; i < 16; ++i) Ts[(b0 + i) * LD64 + tid] = tc[i];
   }
   __syncthreads();
-  // As <- T diag(beta D), Ts <- T diag(beta)
-  for (int idx = tid; idx < GC * GC; idx += 256) {
-    const int i = idx >> 6, j = idx & 63;
-    const float tv = Ts[i * LD64 + j];
-    As[i * LD64 + j] = tf32r(tv * beta_s[j] * __expf(G_s[j]));
-    Ts[i * LD64 + j] = tf32r(tv * beta_s[j]);
+  {
+    const int o = (tid >> 7) * 32, i = (tid >> 3) & 15, j = (tid & 7) * 2;      // 32-blocks at (o, o): rows 16 + i, columns j, j + 1
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const float av = As[(o + 16 + i) * LD64 + o + k];
+      const float2 tv = *reinterpret_cast<const float2*>(Ts + (o + k) * LD64 + o + j);
+      s0 = fmaf(av, tv.x, s0); s1 = fmaf(av, tv.y, s1);
+    }
+    *reinterpret_cast<float2*>(As + (o + i) * LD64 + o + 16 + j) = make_float2(s0, s1);
+    __syncthreads();
+    s0 = 0.f; s1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const float tv = Ts[(o + 16 + i) * LD64 + o + 16 + k];
+      const float2 xv = *reinterpret_cast<const float2*>(As + (o + k) * LD64 + o + 16 + j);
+      s0 = fmaf(-tv, xv.x, s0); s1 = fmaf(-tv, xv.y, s1);
+    }
+    *reinterpret_cast<float2*>(Ts + (o + 16 + i) * LD64 + o + j) = make_float2(s0, s1);
+    *reinterpret_cast<float2*>(Ts + (o + i) * LD64 + o + 16 + j) = make_float2(0.f, 0.f);
   }
   __syncthreads();
-  // ---- W = As K, Ut = Ts V: warp -> m-tile (warp&3), n-tiles 8*(warp>>2) .. +8; k-steps up to the diagonal
+  {
+    const int i = tid >> 3, j = (tid & 7) * 4;                                  // rows 32 + i, columns j .. j + 3
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+      const float av = As[(32 + i) * LD64 + k];
+      const float4 tv = *reinterpret_cast<const float4*>(Ts + k * LD64 + j);
+      s.x = fmaf(av, tv.x, s.x); s.y = fmaf(av, tv.y, s.y); s.z = fmaf(av, tv.z, s.z); s.w = fmaf(av, tv.w, s.w);
+    }
+    *reinterpret_cast<float4*>(As + i * LD64 + 32 + j) = s;
+    __syncthreads();
+    s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+      const float tv = Ts[(32 + i) * LD64 + 32 + k];
+      const float4 xv = *reinterpret_cast<const float4*>(As + k * LD64 + 32 + j);
+      s.x = fmaf(-tv, xv.x, s.x); s.y = fmaf(-tv, xv.y, s.y); s.z = fmaf(-tv, xv.z, s.z); s.w = fmaf(-tv, xv.w, s.w);
+    }
+    *reinterpret_cast<float4*>(Ts + (32 + i) * LD64 + j) = s;
+  }
+  __syncthreads();
+  // ---- W = T diag(beta D) K, Ut = T diag(beta) V: warp -> m-tile (warp&3), n-tiles 8*(warp>>2) .. +8; k-steps up to the diagonal
+  // (the diagonals are multiplied into the fragments of T)
   {
     const int mt = warp & 3, nt0 = (warp >> 2) * 8;
+    const float* aa = Ts + (mt * 16 + g) * LD64 + t;
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {
-      const float* Am = which == 0 ? As : Ts;
       const float* Bm = which == 0 ? Ks : Vs;
       float acc[8][4];
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-      const float* aa = Am + (mt * 16 + g) * LD64 + t;
       for (int ks = 0; ks < 2 * (mt + 1); ++ks) {
-        const float a0 = aa[ks * 8], a1 = aa[8 * LD64 + ks * 8], a2 = aa[ks * 8 + 4], a3 = aa[8 * LD64 + ks * 8 + 4];
+        const float e0 = which == 0 ? D_s[ks * 8 + t] : 1.f, e1 = which == 0 ? D_s[ks * 8 + t + 4] : 1.f;
+        const float f0 = beta_s[ks * 8 + t], f1 = beta_s[ks * 8 + t + 4];
+        const float a0 = tf32r(aa[ks * 8] * f0 * e0), a1 = tf32r(aa[8 * LD64 + ks * 8] * f0 * e0);
+        const float a2 = tf32r(aa[ks * 8 + 4] * f1 * e1), a3 = tf32r(aa[8 * LD64 + ks * 8 + 4] * f1 * e1);
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
           const float* bb = Bm + (ks * 8 + t) * LD128 + (nt0 + a) * 8 + g;
@@ -250,14 +333,6 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
       }
     }
   }
-  // ---- Qt = diag(D) Q, Kt = diag(D_C / D) K
-  const float Gl = G_s[GC - 1];
-  for (int idx = tid; idx < GC * GD; idx += 256) {
-    const int r = idx >> 7, i = idx & 127;
-    wsb[WS_QT + idx] = tf32r(Qs[r * LD128 + i] * __expf(G_s[r]));
-    wsb[WS_KT + idx] = tf32r(Ks[r * LD128 + i] * __expf(Gl - G_s[r]));
-  }
-  if (tid == 0) wsb[WS_DC] = __expf(Gl);
 }
 
 // ---------------------------------------------------------------------------------------------- kernel 2
@@ -454,16 +529,16 @@ extern "C" int spark_gdn_chunk_prefill(const void* proj, int ldp, const void* ab
                                        cudaStream_t s) {
   if (n_chunks <= 0) return 0;
   if (D != GD || Hv % Hk) return -5;
-  constexpr int SM1 = (3 * GC * LD128 + 2 * GC * LD64 + 2 * GC) * 4;
   constexpr int SM2 = (3 * GC * LD128 + GC * LD64 + GC * LD32 + GVS * LD128) * 4;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM1);
+    cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP_SMEM);
     cudaFuncSetAttribute(gdn_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM2);
     attr = true;
   }
-  gdn_chunk_prep_kernel<<<dim3(n_chunks, Hv), 256, SM1, s>>>((const __nv_bfloat16*)proj, ldp, (const __nv_bfloat16*)ab, ldab,
-                                                              conv_w, A_log, dt_bias, tail, seg, chunks, ws, Hk, Hv, eps);
+  gdn_chunk_prep_kernel<<<dim3(n_chunks, Hv), 256, PREP_SMEM, s>>>((const __nv_bfloat16*)proj, ldp, (const __nv_bfloat16*)ab, ldab,
+                                                              conv_w, A_log, dt_bias, tail, seg, chunks, ws, Hk, Hv, eps,
+                                                                  (reinterpret_cast<uintptr_t>(conv_w) & 15) == 0);
   gdn_chunk_state_kernel<<<dim3(GD / GVS, Hv, nseg), 128, SM2, s>>>(ws, seg, seg_chunk0, (const __nv_bfloat16*)proj, ldp, S,
                                                                     tail, o_raw, Hv * GD, Hk, Hv);
   gdn_chunk_out_kernel<<<dim3(n_chunks, Hv), 256, 0, s>>>(o_raw, Hv * GD, (const __nv_bfloat16*)proj, ldp, norm_w, seg, chunks,
