@@ -9,6 +9,7 @@
 // Reference: engine-rs/shim/qwen_moe.cu:10-92, dataflow.cu:370-572, ds41_ops.cu:375-421 (routers);
 // moe_exl3.cuh:141-231 (count/scan/fill), :1085 (slot-order combine).
 #include "../common/decode.cuh"
+#include <type_traits>
 
 namespace spark {
 
@@ -158,81 +159,70 @@ struct RouterArgs {
   int n_self; float* self_w;                 // identity experts: the last n_self outputs, their weight per row [R]
 };
 
-constexpr int ROUTER_RB = 16;
+constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16;
 
-template <int EPL>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ void router_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A CTA owns 8 gate columns, its 16 warps split K: a lane takes 8 consecutive k of its row(s) and of its column as 16-byte loads
+// straight into MMA fragments (the same order of k on both sides), up to eight of them in flight, and the warps' 16 x 8 partial sums
+// meet in shared memory in warp order.  What bounds it: two memory round trips and the chain of the choices, one warp per row.
+// (Before: the rows were staged in shared memory by every CTA and each column was 16 dot products on the FP32 units of one warp, two
+// rows' choices after one another: 4 rows of 2048 and 513 columns 13.7 -> 9.0 us, 16 rows 32 -> 13, 4 rows of the MXFP4 preset 37 -> 16.)
+template <int EPL, bool HI>                                 // HI: more than 8 rows
+__global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
-  extern __shared__ __align__(16) uint8_t smem_router[];
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem_router);     // [R][K]
+  __shared__ float part[ROUTER_WARPS][16][8];
   __shared__ int last_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int R = a.R, K = a.K;
-  // the gate matrix depends on no earlier launch: its first batch of loads is in flight before the dependency wait
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int R = a.R;
   const int NE = a.E + (a.shared_gate ? 1 : 0);
-  const int n0 = blockIdx.x * 8 + warp;                    // one gate column per warp
-  const uint4* w0 = reinterpret_cast<const uint4*>(a.Wg + static_cast<size_t>(n0 < NE ? n0 : 0) * a.ldw);
-  constexpr int BATCH = 8;                                 // weight loads in flight per lane
-  const int KV = K >> 3;
-  uint4 wa[BATCH];
+  const int n0 = blockIdx.x * 8;
+  const int KV = a.K >> 3;                                  // 16-byte vectors of a row; a step is four of them
+  constexpr int BATCH = HI ? 4 : 8;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const uint4* w = reinterpret_cast<const uint4*>(a.Wg + static_cast<size_t>(min(n0 + g, NE - 1)) * a.ldw) + t;
+  const uint4* xl = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(min(g, R - 1)) * a.ldx) + t;
+  const uint4* xh = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(min(g + 8, R - 1)) * a.ldx) + t;
+  // the gate matrix depends on no earlier launch: its first batch of loads is in flight before the dependency wait
+  uint4 wv[BATCH];
 #pragma unroll
   for (int u = 0; u < BATCH; ++u) {
-    const int kv = lane + 32 * u;
-    wa[u] = kv < KV ? __ldg(w0 + kv) : make_uint4(0u, 0u, 0u, 0u);
+    const int kv = (warp + u * ROUTER_WARPS) * 4;
+    wv[u] = kv + t < KV ? __ldg(w + kv) : zero;
   }
   pdl_wait();
   pdl_trigger();
-  const int KV8 = K >> 3;
-  for (int i = tid; i < R * KV8; i += 256) {
-    const int r = i / KV8, kv = i - r * KV8;
-    reinterpret_cast<uint4*>(xs)[i] = *reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(r) * a.ldx + kv * 8);
-  }
-  __syncthreads();
-  // ---- GEMV: this CTA's 8 gate columns (one per warp), all rows; one warp per output => fixed reduction order
-  if (n0 < NE) {
-    float acc0[ROUTER_RB];
+  {
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = warp; s0 * 4 < KV; s0 += ROUTER_WARPS * BATCH) {
+      uint4 lo[BATCH], hi[BATCH];
 #pragma unroll
-    for (int r = 0; r < ROUTER_RB; ++r) acc0[r] = 0.f;
-    for (int kv0 = lane; kv0 < KV; kv0 += 32 * BATCH) {
-      if (kv0 != lane) {
-#pragma unroll
-        for (int u = 0; u < BATCH; ++u) {
-          const int kv = kv0 + 32 * u;
-          wa[u] = kv < KV ? __ldg(w0 + kv) : make_uint4(0u, 0u, 0u, 0u);
-        }
+      for (int u = 0; u < BATCH; ++u) {
+        const int kv = (s0 + u * ROUTER_WARPS) * 4;
+        const bool in = kv + t < KV;
+        if (s0 != warp) wv[u] = in ? __ldg(w + kv) : zero;
+        lo[u] = in ? xl[kv] : zero;
+        hi[u] = HI && in ? xh[kv] : zero;
       }
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
-        const int kv = kv0 + 32 * u;
-        if (kv >= KV) break;
-        const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&wa[u]);
-        float fa[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 t0 = __bfloat1622float2(pa[i]);
-          fa[2 * i] = t0.x; fa[2 * i + 1] = t0.y;
-        }
-#pragma unroll
-        for (int r = 0; r < ROUTER_RB; ++r) {
-          if (r < R) {
-            const uint4 xv = *reinterpret_cast<const uint4*>(xs + static_cast<size_t>(r) * K + kv * 8);
-            const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&xv);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 t = __bfloat1622float2(px[i]);
-              acc0[r] = fmaf(fa[2 * i], t.x, acc0[r]); acc0[r] = fmaf(fa[2 * i + 1], t.y, acc0[r]);
-            }
-          }
-        }
+        router_mma(d, lo[u].x, hi[u].x, lo[u].y, hi[u].y, wv[u].x, wv[u].y);
+        router_mma(d, lo[u].z, hi[u].z, lo[u].w, hi[u].w, wv[u].z, wv[u].w);
       }
     }
+    *reinterpret_cast<float2*>(&part[warp][g][2 * t]) = make_float2(d[0], d[1]);
+    *reinterpret_cast<float2*>(&part[warp][g + 8][2 * t]) = make_float2(d[2], d[3]);
+  }
+  __syncthreads();
+  if (tid < 128) {
+    const int r = tid >> 3, c = tid & 7;
+    float v = 0.f;
 #pragma unroll
-    for (int r = 0; r < ROUTER_RB; ++r) {
-      if (r < R) {
-        const float s0 = warp_sum(acc0[r]);
-        if (lane == 0) a.logits[static_cast<size_t>(r) * a.ld + n0] = s0;
-      }
-    }
+    for (int i = 0; i < ROUTER_WARPS; ++i) v += part[i][r][c];
+    if (r < R && n0 + c < NE) a.logits[static_cast<size_t>(r) * a.ld + n0 + c] = v;
   }
   // ---- arrival: the last CTA to get here routes every row
   __syncthreads();
@@ -248,7 +238,7 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
   // EPL experts per lane (E <= 32 * EPL).  The k selection rounds are a serial chain, so each round is kept short (lane_best: a
   // serial compare chain in its place spent 5.8 us per group of rows).
   const int nj = (a.E + 31) >> 5;
-  for (int r = warp; r < R; r += 8) {
+  for (int r = warp; r < R; r += ROUTER_WARPS) {
     const float* lg = a.logits + static_cast<size_t>(r) * a.ld;
     float p[EPL], s[EPL];                                   // p: what the weights are made of; s: selection score
     float mx = -INFINITY;
@@ -662,20 +652,14 @@ extern "C" int spark_moe_router_topk(const void* x, int ldx, const void* Wg, int
   a.slots = slots; a.shared_expert = shared_expert; a.e_lo = e_lo; a.e_hi = e_hi; a.rank = rank; a.world = world < 1 ? 1 : world;
   a.wts = wts; a.ids = ids; a.pair_row = pair_row; a.sg = sg; a.counter = counter;
   const int NE = E + (shared_gate ? 1 : 0);
-  const size_t smem = static_cast<size_t>(R) * K * 2;
-  if (smem > 200 * 1024) return -6;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(moe_router_topk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_router_topk_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(moe_router_topk_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
-  }
-  const cudaError_t err = E <= 64
-      ? spark_launch_pdl(moe_router_topk_kernel<2>, dim3((NE + 7) / 8), dim3(256), smem, s, dim3(1, 1, 1), a)
-      : E <= 512
-      ? spark_launch_pdl(moe_router_topk_kernel<16>, dim3((NE + 7) / 8), dim3(256), smem, s, dim3(1, 1, 1), a)
-      : spark_launch_pdl(moe_router_topk_kernel<32>, dim3((NE + 7) / 8), dim3(256), smem, s, dim3(1, 1, 1), a);
+  // experts per lane: the narrowest form that holds E (a lane's work per choice grows with it)
+  auto pick = [&](auto hi) {
+    constexpr bool HI = decltype(hi)::value;
+    return E <= 64 ? moe_router_topk_kernel<2, HI> : E <= 256 ? moe_router_topk_kernel<8, HI>
+         : E <= 512 ? moe_router_topk_kernel<16, HI> : moe_router_topk_kernel<32, HI>;
+  };
+  void (*kern)(RouterArgs) = R > 8 ? pick(std::true_type{}) : pick(std::false_type{});
+  const cudaError_t err = spark_launch_pdl(kern, dim3((NE + 7) / 8), dim3(ROUTER_WARPS * 32), 0, s, dim3(1, 1, 1), a);
   return err == cudaSuccess ? 0 : -4;
 }
 
