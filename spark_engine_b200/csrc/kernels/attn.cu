@@ -21,8 +21,15 @@ struct AttnDims {
 };
 
 // ------------------------------------------------------------------------------------------ prep
-// grid (R, Hq + 2*Hkv + idx_heads + (idx_dim ? 1 : 0)); 128 threads; thread t owns dims t and t+128.
-__global__ void __launch_bounds__(128)
+// A job is one head of a row: job < Hq + 2*Hkv + idx_heads + (idx_dim ? 1 : 0).  W warps share a job, thread t of them owns dims
+// t + 32 W i.
+//   W = 4 (decode): a CTA per job, two dims a thread; the chain of one thread is the time.
+//   W = 1 (prompts): a warp per job, four of them in a CTA, no block barriers; 48 warps per SM, since the chain of loads, sums and
+//   sines is what takes the time (24 warps: 94 us).  128 threads per job were 92000 CTAs of a few hundred cycles for 3999 rows of 25
+//   heads: 91 -> 63 us.
+// The squares are added in the same order in both forms, so the same rows give the same bits.
+template <int W>
+__global__ void __launch_bounds__(128, W == 1 ? 12 : 1)
 attn_prep_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, AttnDims a,
                  const float* __restrict__ q_norm, const float* __restrict__ k_norm,
                  const float* __restrict__ iq_norm, const float* __restrict__ ik_norm,
@@ -34,12 +41,18 @@ attn_prep_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, AttnDims a,
                  void* __restrict__ kc, void* __restrict__ vc,                        // [tokens, Hkv, D]
                  float* __restrict__ ks, float* __restrict__ vs,                      // fp8 scales [tokens, Hkv]
                  float* __restrict__ qi_buf,                                          // [R, idx_heads, idx_dim]
-                 float* __restrict__ ik_raw, float* __restrict__ ik_pool) {
+                 float* __restrict__ ik_raw, float* __restrict__ ik_pool, int R, int jobs) {
+  constexpr int N = 8 / W, S = 32 * W;                       // dims of a thread and their distance
+  __shared__ float vals_s[4 / W][256];
   __shared__ float red[4];
-  __shared__ float vals[256];
   pdl_wait();
   pdl_trigger();
-  const int r = blockIdx.x, job = blockIdx.y, t = threadIdx.x;
+  const int warp = threadIdx.x >> 5, t = threadIdx.x & (S - 1);
+  const int id = W == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
+  if (id >= R * jobs) return;                                // whole warps (W = 1) or the whole CTA
+  const int r = id / jobs, job = id - r * jobs;
+  float* vals = vals_s[W == 1 ? warp : 0];
+  auto sync = [&]() { if (W == 1) __syncwarp(); else __syncthreads(); };
   const int qw = a.D * (a.gated ? 2 : 1);
   const int nq = a.Hq * qw, nkv = a.Hkv * a.D;
   const int p = pos[r];
@@ -57,94 +70,96 @@ attn_prep_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, AttnDims a,
   int rope = a.rope_dim, rp = p;
   const float* nw = nullptr;
   bool norm = false;
-  float x0 = 0.f, x1 = 0.f;
+  float x[N];
   if (kind == 4) {
     // raw key of this row; pooled key only when this row completes a block
-    for (int d = t; d < dim; d += 128) ik_raw[tok * dim + d] = __bfloat162float(row[off + d]);
+    for (int d = t; d < dim; d += S) ik_raw[tok * dim + d] = __bfloat162float(row[off + d]);
     if (row_pos0 != nullptr) return;          // tree rows: blocks are pooled when the accepted path is committed
     if ((p + 1) % a.block != 0) return;
     // mean of the block's raw keys BEFORE norm + rope at the block's first position
-    for (int d = t; d < dim; d += 128) {
-      float s = 0.f;
-      for (int b = 0; b < a.block; ++b) {
-        const int back = a.block - 1 - b;                 // rows p-back .. p
-        float v;
-        if (back <= row_j[r]) v = __bfloat162float(qkv[static_cast<size_t>(r - back) * ld + off + d]);   // same launch
-        else v = ik_raw[(tok - back) * dim + d];                                                          // earlier step
-        s += v;
-      }
-      vals[d] = s / a.block;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int d = t + S * i;
+      float sum = 0.f;
+      if (d < dim)
+        for (int b = 0; b < a.block; ++b) {
+          const int back = a.block - 1 - b;                 // rows p-back .. p
+          float v;
+          if (back <= row_j[r]) v = __bfloat162float(qkv[static_cast<size_t>(r - back) * ld + off + d]);   // same launch
+          else v = ik_raw[(tok - back) * dim + d];                                                          // earlier step
+          sum += v;
+        }
+      x[i] = d < dim ? sum / a.block : 0.f;
     }
-    __syncthreads();
-    x0 = t < dim ? vals[t] : 0.f; x1 = (t + 128) < dim ? vals[t + 128] : 0.f;
     norm = true; nw = ik_norm; rp = p + 1 - a.block; rope = min(a.rope_dim, dim);
   } else {
-    x0 = t < dim ? __bfloat162float(row[off + t]) : 0.f;
-    x1 = (t + 128) < dim ? __bfloat162float(row[off + t + 128]) : 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = t + S * i < dim ? __bfloat162float(row[off + t + S * i]) : 0.f;
     if (kind == 0) { norm = a.qk_norm; nw = q_norm; }
     if (kind == 1) { norm = a.qk_norm; nw = k_norm; }
     if (kind == 3) { norm = true; nw = iq_norm; rope = min(a.rope_dim, dim); }
     if (kind == 2) rope = 0;
   }
   if (norm) {
-    float ss = warp_sum(x0 * x0 + x1 * x1);
-    if ((t & 31) == 0) red[t >> 5] = ss;
-    __syncthreads();
-    ss = red[0] + red[1] + red[2] + red[3];
+    // pairs (d, d + 128), the 32 of a group, then the four groups
+    float ss = 0.f;
+    if (W == 1) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss += warp_sum(x[i % N] * x[i % N] + x[(i + 4) % N] * x[(i + 4) % N]);
+    } else {
+      const float v = warp_sum(x[0] * x[0] + x[1 % N] * x[1 % N]);
+      if ((t & 31) == 0) red[warp] = v;
+      __syncthreads();
+      ss = red[0] + red[1] + red[2] + red[3];
+    }
     const float rs = rsqrtf(ss / dim + a.eps);
-    if (t < dim) x0 = x0 * rs * (1.f + nw[t]);
-    if (t + 128 < dim) x1 = x1 * rs * (1.f + nw[t + 128]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) if (t + S * i < dim) x[i] = x[i] * rs * (1.f + nw[t + S * i]);
   }
-  __syncthreads();
-  vals[t] = x0; vals[t + 128] = x1;
-  __syncthreads();
   if (rope > 0) {
     const int half = rope / 2;
 #pragma unroll
-    for (int rep = 0; rep < 2; ++rep) {
-      const int d = t + rep * 128;
+    for (int i = 0; i < N; ++i) vals[t + S * i] = x[i];
+    sync();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int d = t + S * i;
       if (d < rope) {
-        const int i = d < half ? d : d - half;
-        const float ang = static_cast<float>(static_cast<double>(rp) * inv_freq[i]);
+        const int j = d < half ? d : d - half;
         float sn, cs;
-        sincosf(ang, &sn, &cs);
-        const float a1 = vals[i], a2 = vals[i + half];
-        const float o = d < half ? a1 * cs - a2 * sn : a2 * cs + a1 * sn;
-        if (rep == 0) x0 = o; else x1 = o;
+        sincosf(static_cast<float>(static_cast<double>(rp) * inv_freq[j]), &sn, &cs);
+        const float a1 = vals[j], a2 = vals[j + half];
+        x[i] = d < half ? a1 * cs - a2 * sn : a2 * cs + a1 * sn;
       }
     }
   }
   // ---- write
-  if (kind == 0) {
-    __nv_bfloat16* dst = qbuf + (static_cast<size_t>(r) * a.Hq + head) * a.D;
-    if (t < dim) dst[t] = __float2bfloat16(x0);
-    if (t + 128 < dim) dst[t + 128] = __float2bfloat16(x1);
-  } else if (kind == 1 || kind == 2) {
+  if ((kind == 1 || kind == 2) && a.fp8) {
     const size_t o = (static_cast<size_t>(tok) * a.Hkv + head) * a.D;
-    if (a.fp8) {
-      float am = warp_max(fmaxf(fabsf(x0), fabsf(x1)));
+    float am = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) am = fmaxf(am, fabsf(x[i]));
+    am = warp_max(am);
+    if (W != 1) {
       __syncthreads();
-      if ((t & 31) == 0) red[t >> 5] = am;
+      if ((t & 31) == 0) red[warp] = am;
       __syncthreads();
       am = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-      const float sc = fmaxf(am, 1e-8f) / 448.f;
-      __nv_fp8_e4m3* dst = reinterpret_cast<__nv_fp8_e4m3*>(kind == 1 ? kc : vc) + o;
-      if (t < dim) dst[t] = __nv_fp8_e4m3(x0 / sc);
-      if (t + 128 < dim) dst[t + 128] = __nv_fp8_e4m3(x1 / sc);
-      if (t == 0) (kind == 1 ? ks : vs)[static_cast<size_t>(tok) * a.Hkv + head] = sc;
-    } else {
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(kind == 1 ? kc : vc) + o;
-      if (t < dim) dst[t] = __float2bfloat16(x0);
-      if (t + 128 < dim) dst[t + 128] = __float2bfloat16(x1);
     }
-  } else if (kind == 3) {
-    float* dst = qi_buf + (static_cast<size_t>(r) * a.idx_heads + head) * dim;
-    if (t < dim) dst[t] = x0;
-    if (t + 128 < dim) dst[t + 128] = x1;
+    const float sc = fmaxf(am, 1e-8f) / 448.f;
+    __nv_fp8_e4m3* dst = reinterpret_cast<__nv_fp8_e4m3*>(kind == 1 ? kc : vc) + o;
+#pragma unroll
+    for (int i = 0; i < N; ++i) if (t + S * i < dim) dst[t + S * i] = __nv_fp8_e4m3(x[i] / sc);
+    if (t == 0) (kind == 1 ? ks : vs)[static_cast<size_t>(tok) * a.Hkv + head] = sc;
+  } else if (kind <= 2) {
+    __nv_bfloat16* dst = kind == 0 ? qbuf + (static_cast<size_t>(r) * a.Hq + head) * a.D
+                                   : reinterpret_cast<__nv_bfloat16*>(kind == 1 ? kc : vc) + (static_cast<size_t>(tok) * a.Hkv + head) * a.D;
+#pragma unroll
+    for (int i = 0; i < N; ++i) if (t + S * i < dim) dst[t + S * i] = __float2bfloat16(x[i]);
   } else {
-    float* dst = ik_pool + (tok / a.block) * dim;
-    if (t < dim) dst[t] = x0;
-    if (t + 128 < dim) dst[t + 128] = x1;
+    float* dst = kind == 3 ? qi_buf + (static_cast<size_t>(r) * a.idx_heads + head) * dim : ik_pool + (tok / a.block) * dim;
+#pragma unroll
+    for (int i = 0; i < N; ++i) if (t + S * i < dim) dst[t + S * i] = x[i];
   }
 }
 
@@ -513,10 +528,14 @@ extern "C" int spark_attn_prep(const void* qkv, int ld, int R, int Hq, int Hkv, 
   if (R <= 0) return 0;
   if (D > 256 || idx_dim > 256) return -5;
   AttnDims a{Hq, Hkv, D, rope_dim, gated, qk_norm, idx_heads, idx_dim, block, fp8, eps};
-  dim3 grid(R, Hq + 2 * Hkv + idx_heads + (idx_dim > 0 ? 1 : 0));
-  const cudaError_t err = spark_launch_pdl(attn_prep_kernel, grid, dim3(128), 0, s, dim3(1, 1, 1), (const __nv_bfloat16*)qkv, ld, a,
-                                           q_norm, k_norm, iq_norm, ik_norm, inv_freq, pos, row_kv, row_j, row_pos0, (__nv_bfloat16*)qbuf,
-                                           kc, vc, ks, vs, qi_buf, ik_raw, ik_pool);
+  const int jobs = Hq + 2 * Hkv + idx_heads + (idx_dim > 0 ? 1 : 0);
+  if (static_cast<long long>(R) * jobs > 0x7fffffffLL) return -5;
+  // W = 1 once its warps are four to a scheduler of the GPU
+  const bool many = R * jobs >= 148 * 16;
+  const dim3 grid(many ? (R * jobs + 3) / 4 : R * jobs);
+  const cudaError_t err = spark_launch_pdl(many ? attn_prep_kernel<1> : attn_prep_kernel<4>, grid, dim3(128), 0, s, dim3(1, 1, 1),
+                                           (const __nv_bfloat16*)qkv, ld, a, q_norm, k_norm, iq_norm, ik_norm, inv_freq, pos, row_kv, row_j,
+                                           row_pos0, (__nv_bfloat16*)qbuf, kc, vc, ks, vs, qi_buf, ik_raw, ik_pool, R, jobs);
   return err == cudaSuccess ? 0 : -4;
 }
 
