@@ -224,7 +224,6 @@ struct Mx4Args {
   void* C; int ldc; int out_f32;
   int* status;
   uint32_t w_tx_bytes;        // bytes one weight tile adds to the stage barrier's transaction count (packed size)
-  int burst;                  // k-blocks whose tile loads are issued together (1 .. stages / 2)
 };
 
 // SMALL: every item has <= 16 rows (decode pairs).  The operands are swapped: the weight tile is the 128-row M
@@ -254,7 +253,7 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tmem_full = empty_bar + STAGES;
   uint64_t* tmem_empty = tmem_full + MX_ACC_STAGES;
   uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(tmem_empty + MX_ACC_STAGES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_k = g.K / MX_BK;
   const int nt_n = g.N / MX_BN;
   const int n_items = min(*g.n_items, g.max_items);
@@ -275,105 +274,102 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t tmem_base = *tmem_base_ptr;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0; bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int it = t / nt_n, nt = t - it * nt_n;
-        const int4 item = g.items[it];
-        if (item.z < 0 || item.y <= 0) continue;                 // expert of another rank / empty item
-        if (SMALL && item.y > 16) { set_status(g.status, ST_BOUNDS, blockIdx.x, t, item.y); break; }
-        const bool small = SMALL || item.y <= 16;
-        const uint32_t a_bytes = small ? 16 * MX_BK : MX_A_BYTES;
-        // the tile loads can go out in bursts of `burst` k-blocks (adjacent 64-byte row pieces requested together);
-        // measured neutral on B200, so the default is 1
-        for (int kb0 = 0; kb0 < num_k && ok; kb0 += g.burst) {
-          const int nb = min(g.burst, num_k - kb0);
-          int st = stage; uint32_t ph = phase;
-          for (int j = 0; j < nb; ++j) {
-            if (!mbar_wait(&empty_bar[st], ph ^ 1)) {
-              set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, kb0 + j); ok = false; break;
-            }
-            if (++st == STAGES) { st = 0; ph ^= 1; }
-          }
-          if (!ok) break;
-          for (int j = 0; j < nb; ++j) {
-            const int kb = kb0 + j;
-            uint8_t* a_dst = smem + stage * Cfg::A_REGION;
-            uint8_t* b_dst = smem + Cfg::B_OFF + stage * MX_B_BYTES;
-            mbar_arrive_expect_tx(&full_bar[stage], a_bytes + g.w_tx_bytes);
-            tma_load_2d(a_dst, small ? &tmA16 : &tmA, &full_bar[stage], kb * MX_BK, item.x);
-            tma_load_2d(b_dst, &tmW, &full_bar[stage], kb * MX_BK, item.z * g.N + nt * MX_BN);
-            if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          }
+    int stage = 0; uint32_t phase = 0; bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const int it = t / nt_n, nt = t - it * nt_n;
+      const int4 item = g.items[it];
+      const int row0 = __shfl_sync(0xffffffffu, item.x, 0), rows = __shfl_sync(0xffffffffu, item.y, 0), expert = __shfl_sync(0xffffffffu, item.z, 0);
+      if (expert < 0 || rows <= 0) continue;                     // expert of another rank / empty item
+      if (SMALL && rows > 16) { set_status(g.status, ST_BOUNDS, blockIdx.x, t, rows); break; }
+      const bool small = SMALL || rows <= 16;
+      const uint32_t bytes = (small ? 16 * MX_BK : MX_A_BYTES) + g.w_tx_bytes;
+      const CUtensorMap* ta = small ? &tmA16 : &tmA;
+      const int wrow = expert * g.N + nt * MX_BN;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1));
+        if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, kb); break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&full_bar[stage], bytes);
+          tma_load_2d(smem + stage * Cfg::A_REGION, ta, &full_bar[stage], kb * MX_BK, row0);
+          tma_load_2d(smem + Cfg::B_OFF + stage * MX_B_BYTES, &tmW, &full_bar[stage], kb * MX_BK, wrow);
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 6) {
     // second producer: the two scale blocks of every stage, so that the tile loads and the scale copies are issued
     // by different threads
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0; bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int it = t / nt_n, nt = t - it * nt_n;
-        const int4 item = g.items[it];
-        if (item.z < 0 || item.y <= 0) continue;
-        if (SMALL && item.y > 16) break;
-        const uint8_t* sa = g.sfa + static_cast<size_t>(it) * num_k * MX_SF_BYTES;
-        const uint8_t* sw = g.sfw + static_cast<size_t>(item.z * nt_n + nt) * num_k * MX_SF_BYTES;
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
-            set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, -kb - 1); ok = false; break;
-          }
+    int stage = 0; uint32_t phase = 0; bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const int it = t / nt_n, nt = t - it * nt_n;
+      const int4 item = g.items[it];
+      const int rows = __shfl_sync(0xffffffffu, item.y, 0), expert = __shfl_sync(0xffffffffu, item.z, 0);
+      if (expert < 0 || rows <= 0) continue;
+      if (SMALL && rows > 16) break;
+      const uint8_t* sa = g.sfa + static_cast<size_t>(it) * num_k * MX_SF_BYTES;
+      const uint8_t* sw = g.sfw + static_cast<size_t>(expert * nt_n + nt) * num_k * MX_SF_BYTES;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1));
+        if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, -kb - 1); break; }
+        if (elect_one()) {
           uint8_t* sf_dst = smem + Cfg::SF_OFF + stage * 2 * MX_SF_BYTES;
           mbar_arrive_expect_tx(&full_bar[stage], 2 * MX_SF_BYTES);
           bulk_load(sf_dst, sa + static_cast<size_t>(kb) * MX_SF_BYTES, MX_SF_BYTES, &full_bar[stage]);
           bulk_load(sf_dst + MX_SF_BYTES, sw + static_cast<size_t>(kb) * MX_SF_BYTES, MX_SF_BYTES, &full_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // 128-row tiles: D[activation rows, weight rows], weights are operand B (format e2m1 in bits [10,13)).
-      // SMALL: operands swapped, D[weight rows, 16 activation rows]: the MMA is 128 x 16 x 32 instead of
-      // 128 x 128 x 32, an eighth of the tensor-pipe time per weight byte, which is what lets the decode shape run at
-      // memory speed (with the 128-wide form the tensor pipe, padded 1 row -> 128, was the limit at 0.4 us per stage).
-      const uint32_t idesc0 = SMALL ? (make_idesc_mx(MX_BN, 16) | (5u << 7)) : (make_idesc_mx(MX_BM, MX_BN) | (5u << 10));
-      int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int4 item = g.items[t / nt_n];
-        if (item.z < 0 || item.y <= 0) continue;
-        if (SMALL && item.y > 16) break;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1)) {
-          set_status(g.status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, t, acc); break;
-        }
+    // 128-row tiles: D[activation rows, weight rows], weights are operand B (format e2m1 in bits [10,13)).
+    // SMALL: operands swapped, D[weight rows, 16 activation rows]: the MMA is 128 x 16 x 32 instead of
+    // 128 x 128 x 32, an eighth of the tensor-pipe time per weight byte, which is what lets the decode shape run at
+    // memory speed (with the 128-wide form the tensor pipe, padded 1 row -> 128, was the limit at 0.4 us per stage).
+    // The whole warp walks the loop and one elected lane issues: addresses and descriptors are warp-uniform then and stay in
+    // uniform registers, where the instructions want them (in a branch of one lane every
+    // operand was moved over for every instruction: 720 cycles per block of 128 k, whatever the memory did).  The producers do the same.
+    // 24 pairs of an MXFP4 layer 57 -> 36 us per product, 2048 rows 757 -> 639.
+    const uint32_t idesc0 = SMALL ? (make_idesc_mx(MX_BN, 16) | (5u << 7)) : (make_idesc_mx(MX_BM, MX_BN) | (5u << 10));
+    const uint32_t s0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0), tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const int4 item = g.items[t / nt_n];
+      const int expert = __shfl_sync(0xffffffffu, item.z, 0), rows = __shfl_sync(0xffffffffu, item.y, 0);
+      if (expert < 0 || rows <= 0) continue;
+      if (SMALL && rows > 16) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1))) {
+        set_status(g.status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, t, acc); break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tm + acc * MX_BN;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase));
+        if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * MX_BN;
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase)) {
-            set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); ok = false; break;
-          }
-          tc_fence_after();
-          const uint32_t s0 = smem_u32(smem);
-          const uint64_t x_desc = make_smem_desc_sw128(s0 + stage * Cfg::A_REGION);            // activations
-          const uint64_t w_desc = make_smem_desc_sw128(s0 + Cfg::B_OFF + stage * MX_B_BYTES);  // weights
-          const uint64_t a_desc = SMALL ? w_desc : x_desc, b_desc = SMALL ? x_desc : w_desc;
-          const uint32_t sf_addr = s0 + Cfg::SF_OFF + stage * 2 * MX_SF_BYTES;                 // [activations | weights]
-          const uint32_t tsfa = tmem_base + MX_SF_COL0 + stage * 8, tsfb = tsfa + 4;
-          tmem_cp_32x128b_x4(tsfa, make_sf_desc(sf_addr + (SMALL ? MX_SF_BYTES : 0)));
-          tmem_cp_32x128b_x4(tsfb, make_sf_desc(sf_addr + (SMALL ? 0 : MX_SF_BYTES)));
+        const uint64_t x_desc = make_smem_desc_sw128(s0 + stage * Cfg::A_REGION);            // activations
+        const uint64_t w_desc = make_smem_desc_sw128(s0 + Cfg::B_OFF + stage * MX_B_BYTES);  // weights
+        const uint64_t a_desc = SMALL ? w_desc : x_desc, b_desc = SMALL ? x_desc : w_desc;
+        const uint32_t sf_addr = s0 + Cfg::SF_OFF + stage * 2 * MX_SF_BYTES;                 // [activations | weights]
+        const uint32_t tsfa = tm + MX_SF_COL0 + stage * 8, tsfb = tsfa + 4;
+        const uint64_t sfa_desc = make_sf_desc(sf_addr + (SMALL ? MX_SF_BYTES : 0)), sfb_desc = make_sf_desc(sf_addr + (SMALL ? 0 : MX_SF_BYTES));
+        if (elect_one()) {
+          tmem_cp_32x128b_x4(tsfa, sfa_desc);
+          tmem_cp_32x128b_x4(tsfb, sfb_desc);
 #pragma unroll
           for (int k = 0; k < MX_BK / 32; ++k) {
             const uint32_t idesc = idesc0 | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29);
             umma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, tsfa, tsfb, (kb | k) != 0);
           }
           umma_commit(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (kb == num_k - 1) umma_commit(&tmem_full[acc]);
         }
-        if (!ok) break;
-        umma_commit(&tmem_full[acc]);
-        if (++acc == MX_ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++acc == MX_ACC_STAGES) { acc = 0; acc_phase ^= 1; }
     }
   } else {
     const int quarter = warp & 3;
@@ -629,13 +625,7 @@ extern "C" int spark_moe_mxfp4(const void* A, int lda, int rows_a, const void* W
   if (r) return r - 10;
   // a 16U4_ALIGN16B copy completes the barrier with the packed bytes it read (64 per row), not the 128 it writes
   const uint32_t w_tx = MX_B_BYTES / 2;
-  static const int burst_env = [] { const char* e = getenv("SPARK_MX4_BURST"); return e ? atoi(e) : 0; }();   // tuning knob
-  int burst = burst_env > 0 ? burst_env : 1;
-  const int max_burst = (small ? Mx4Cfg<true>::STAGES : Mx4Cfg<false>::STAGES) / 2;
-  if (burst > max_burst) burst = max_burst;
-  if (burst < 1) burst = 1;
-  Mx4Args g{(const int4*)items, n_items, max_items, N, K, (const uint8_t*)sfa, (const uint8_t*)sfw, C, ldc, out_f32, status, w_tx,
-            burst};
+  Mx4Args g{(const int4*)items, n_items, max_items, N, K, (const uint8_t*)sfa, (const uint8_t*)sfw, C, ldc, out_f32, status, w_tx};
   static bool attr_done = false;
   if (!attr_done) {
     cudaFuncSetAttribute(moe_mxfp4_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<false>::SMEM);
