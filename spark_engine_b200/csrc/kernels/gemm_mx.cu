@@ -210,9 +210,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // core untouched: the tensor map type 16U4_ALIGN16B makes TMA expand 16 nibbles (8 bytes) into the 16-byte padded
 // slots that `tcgen05.mma.kind::mxf8f6f4` reads for a 4-bit operand, so a 128-k slice of a weight row is 128 bytes of
 // shared memory exactly like an fp8 row, and the descriptors of the fp8 kernel apply unchanged (B format = e2m1).
-// Items with <= 16 rows (decode: one row per (token, expert) pair) fetch a 16-row activation box instead of 128 rows;
-// the other rows of the tile are whatever shared memory held, which only reaches accumulator rows that are never
-// stored.  The A scale blocks are tile-local (row r of the item, not of the matrix): mx_sf_tile_blocks_kernel.
+// An item fetches only the 16-row pieces of the activation tile that it has.  The A scale blocks are tile-local (row r of the item, not of the matrix): mx_sf_tile_blocks_kernel.
 // Reference paths replaced: engine-rs/shim/ds41_mx.cu (mxfp4 expert GEMMs through dequantised tiles).
 struct Mx4Args {
   const int4* items;          // (first A row, rows, expert, first C row)
@@ -226,10 +224,8 @@ struct Mx4Args {
   uint32_t w_tx_bytes;        // bytes one weight tile adds to the stage barrier's transaction count (packed size)
 };
 
-// SMALL: every item has <= 16 rows (decode pairs).  The operands are swapped: the weight tile is the 128-row M
-// operand, the 16-row activation box the N operand, so the accumulator is [128 weight rows, 16 activation rows] and
-// the tensor pipe does an eighth of the work per weight byte.  A stage is 19 KB (2 KB activations, 16 KB weights,
-// two scale blocks) and ten stages fit.
+// SMALL: every item has <= 16 rows (decode pairs): a stage is 19 KB (2 KB activations, 16 KB weights, two scale blocks) and ten
+// stages fit.
 template <bool SMALL>
 struct Mx4Cfg {
   static constexpr int STAGES = SMALL ? 10 : MX_STAGES;
@@ -281,16 +277,17 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int row0 = __shfl_sync(0xffffffffu, item.x, 0), rows = __shfl_sync(0xffffffffu, item.y, 0), expert = __shfl_sync(0xffffffffu, item.z, 0);
       if (expert < 0 || rows <= 0) continue;                     // expert of another rank / empty item
       if (SMALL && rows > 16) { set_status(g.status, ST_BOUNDS, blockIdx.x, t, rows); break; }
-      const bool small = SMALL || rows <= 16;
-      const uint32_t bytes = (small ? 16 * MX_BK : MX_A_BYTES) + g.w_tx_bytes;
-      const CUtensorMap* ta = small ? &tmA16 : &tmA;
+      const int pieces = SMALL ? 1 : min((rows + 15) >> 4, 8);   // 16-row pieces of the activation tile that the item has
+      const uint32_t bytes = pieces * 16 * MX_BK + g.w_tx_bytes;
       const int wrow = expert * g.N + nt * MX_BN;
       for (int kb = 0; kb < num_k; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1));
         if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, kb); break; }
         if (elect_one()) {
           mbar_arrive_expect_tx(&full_bar[stage], bytes);
-          tma_load_2d(smem + stage * Cfg::A_REGION, ta, &full_bar[stage], kb * MX_BK, row0);
+          uint8_t* a_dst = smem + stage * Cfg::A_REGION;
+          if (!SMALL && pieces == 8) tma_load_2d(a_dst, &tmA, &full_bar[stage], kb * MX_BK, row0);
+          else for (int p = 0; p < pieces; ++p) tma_load_2d(a_dst + p * 16 * MX_BK, &tmA16, &full_bar[stage], kb * MX_BK, row0 + p * 16);
           tma_load_2d(smem + Cfg::B_OFF + stage * MX_B_BYTES, &tmW, &full_bar[stage], kb * MX_BK, wrow);
         }
         __syncwarp();
@@ -323,15 +320,12 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // 128-row tiles: D[activation rows, weight rows], weights are operand B (format e2m1 in bits [10,13)).
-    // SMALL: operands swapped, D[weight rows, 16 activation rows]: the MMA is 128 x 16 x 32 instead of
-    // 128 x 128 x 32, an eighth of the tensor-pipe time per weight byte, which is what lets the decode shape run at
-    // memory speed (with the 128-wide form the tensor pipe, padded 1 row -> 128, was the limit at 0.4 us per stage).
+    // The weights are the 128-row operand (format e2m1 in bits [7,10)), the rows of the item the other, rounded up to 16: decode pairs
+    // run at memory speed, and the 30 or 40 rows of an expert in a prompt do not pay for 128 (2048 rows: 639 -> 535 us per product).
     // The whole warp walks the loop and one elected lane issues: addresses and descriptors are warp-uniform then and stay in
     // uniform registers, where the instructions want them (in a branch of one lane every
     // operand was moved over for every instruction: 720 cycles per block of 128 k, whatever the memory did).  The producers do the same.
     // 24 pairs of an MXFP4 layer 57 -> 36 us per product, 2048 rows 757 -> 639.
-    const uint32_t idesc0 = SMALL ? (make_idesc_mx(MX_BN, 16) | (5u << 7)) : (make_idesc_mx(MX_BM, MX_BN) | (5u << 10));
     const uint32_t s0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0), tm = __shfl_sync(0xffffffffu, tmem_base, 0);
     int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
@@ -344,23 +338,23 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       tc_fence_after();
       const uint32_t d_tmem = tm + acc * MX_BN;
+      const uint32_t idesc0 = make_idesc_mx(MX_BN, SMALL ? 16 : min((rows + 15) & ~15, 128)) | (5u << 7);
       for (int kb = 0; kb < num_k; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase));
         if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); break; }
         tc_fence_after();
         const uint64_t x_desc = make_smem_desc_sw128(s0 + stage * Cfg::A_REGION);            // activations
         const uint64_t w_desc = make_smem_desc_sw128(s0 + Cfg::B_OFF + stage * MX_B_BYTES);  // weights
-        const uint64_t a_desc = SMALL ? w_desc : x_desc, b_desc = SMALL ? x_desc : w_desc;
         const uint32_t sf_addr = s0 + Cfg::SF_OFF + stage * 2 * MX_SF_BYTES;                 // [activations | weights]
         const uint32_t tsfa = tm + MX_SF_COL0 + stage * 8, tsfb = tsfa + 4;
-        const uint64_t sfa_desc = make_sf_desc(sf_addr + (SMALL ? MX_SF_BYTES : 0)), sfb_desc = make_sf_desc(sf_addr + (SMALL ? 0 : MX_SF_BYTES));
+        const uint64_t sfa_desc = make_sf_desc(sf_addr + MX_SF_BYTES), sfb_desc = make_sf_desc(sf_addr);
         if (elect_one()) {
           tmem_cp_32x128b_x4(tsfa, sfa_desc);
           tmem_cp_32x128b_x4(tsfb, sfb_desc);
 #pragma unroll
           for (int k = 0; k < MX_BK / 32; ++k) {
             const uint32_t idesc = idesc0 | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29);
-            umma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, tsfa, tsfb, (kb | k) != 0);
+            umma_mxf8(d_tmem, w_desc + 2 * k, x_desc + 2 * k, idesc, tsfa, tsfb, (kb | k) != 0);
           }
           umma_commit(&empty_bar[stage]);
           if (kb == num_k - 1) umma_commit(&tmem_full[acc]);
@@ -384,51 +378,19 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after();
       const int r = quarter * 32 + lane;
       const uint32_t t_addr = tmem_base + acc * MX_BN + (static_cast<uint32_t>(quarter * 32) << 16);
-      if (SMALL) {
-        // lane = weight row (output column), TMEM column j = activation row j of the item
+      // lane = weight row (output column), TMEM column j = activation row j of the item
+      const int col = nt * MX_BN + r;
+#pragma unroll 1
+      for (int c = 0; c < (SMALL ? 16 : item.y); c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32(t_addr, v);
+        tmem_ld_32x32(t_addr + c, v);
         tmem_ld_wait();
-        const int col = nt * MX_BN + r;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (j < item.y) {
-            const size_t o = (static_cast<size_t>(item.w) + j) * g.ldc + col;
+        for (int j = 0; j < (SMALL ? 16 : 32); ++j) {
+          if (c + j < item.y) {
+            const size_t o = (static_cast<size_t>(item.w) + c + j) * g.ldc + col;
             if (g.out_f32) reinterpret_cast<float*>(g.C)[o] = __uint_as_float(v[j]);
             else reinterpret_cast<__nv_bfloat16*>(g.C)[o] = __float2bfloat16(__uint_as_float(v[j]));
-          }
-        }
-      } else
-      // a warp whose 32 rows all lie past the item's rows has nothing to read
-      if (quarter * 32 < item.y) {
-#pragma unroll 1
-        for (int c = 0; c < MX_BN; c += 32) {
-          uint32_t v[32];
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait();
-          const int col = nt * MX_BN + c;
-          if (r < item.y) {
-            const size_t row = static_cast<size_t>(item.w) + r;
-            if (g.out_f32) {
-              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + row * g.ldc + col);
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                dst[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]),
-                                     __uint_as_float(v[4 * i + 3]));
-            } else {
-              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
-#pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                uint4 o;
-                __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-                __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
-                __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5]));
-                __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7]));
-                o.x = *reinterpret_cast<uint32_t*>(&p0); o.y = *reinterpret_cast<uint32_t*>(&p1);
-                o.z = *reinterpret_cast<uint32_t*>(&p2); o.w = *reinterpret_cast<uint32_t*>(&p3);
-                *reinterpret_cast<uint4*>(dst + i) = o;
-              }
-            }
           }
         }
       }
