@@ -9,9 +9,9 @@
 // term of a row uses the same reference), so most tiles never touch it.
 // The rows of a segment see the committed prefix of their sequence (already in the cache) plus the rows before them in the segment
 // (stored by the prep kernel of the same step).  One CTA owns a (row tile, head) from first key to last, so results are run-to-run
-// identical.  What bounds it: L2.  Every tile brings 64 KB of keys and values to 128 rows (D = 256), 2140 cycles at the 30 bytes per
-// cycle and SM that 148 of them get together; the softmax of a tile takes 900, its products 770.  4000 rows of 16 heads (2 for keys),
-// D = 256: 214 us, 612 TFLOP/s (64-row tiles on warp-level products: 828 us with block masks).
+// identical.  What bounds it: L2 and the softmax together: every tile brings 64 KB of keys and values to 128 rows (D = 256), and its
+// exponentials take one warp per scheduler 900 cycles.  4000 rows of 16 heads (2 for keys), D = 256: 165 us, 795 TFLOP/s (64-row
+// tiles on warp-level products: 828 us with block masks).
 // Serves: GQA / QSA layers (engine-rs/shim/qwen_qsa.cu attn paths; the reference runs prefill rows through the same per-row kernel
 // as decode).
 #include "../common/ptx.cuh"
@@ -105,7 +105,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* p_full = s_read + 1;
   uint64_t* o_full = p_full + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_full + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     if (!L::QT) tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
@@ -159,53 +159,53 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t id_s = make_idesc(1, 1, PF_BM, PF_BN), id_o = make_idesc(1, 1, PF_BM, D) | (1u << 16);
-      int slot = 0; uint32_t ph = 0;
-      bool ok = mbar_wait(q_full, 0);
-      if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -2);
-      const uint32_t qs = smem_u32(smem), rs = smem_u32(ring);
-      for (int j = -1; j < ntiles && ok; ++j) {
-        if (j + 1 < ntiles) {
-          // the scores have one buffer, free as soon as every warp has loaded those of tile j
-          if (!mbar_wait(&full[slot], ph) || (j >= 0 && !mbar_wait(s_read, j & 1))) {
-            set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
+    // (the whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers, where the instructions want
+    // them.  4000 rows of 16 heads of 256: 213 -> 165 us)
+    const uint32_t id_s = make_idesc(1, 1, PF_BM, PF_BN), id_o = make_idesc(1, 1, PF_BM, D) | (1u << 16);
+    const uint32_t qs = __shfl_sync(0xffffffffu, smem_u32(smem), 0), rs = qs + L::Q_BYTES, tm = __shfl_sync(0xffffffffu, tmem, 0);
+    int slot = 0; uint32_t ph = 0;
+    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0));
+    if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -2);
+    for (int j = -1; j < ntiles && ok; ++j) {
+      if (j + 1 < ntiles) {
+        // the scores have one buffer, free as soon as every warp has loaded those of tile j
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[slot], ph) && (j < 0 || mbar_wait(s_read, j & 1)));
+        if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j); break; }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int c = 0; c < CH; ++c) {
             const uint64_t kd = make_smem_desc_sw128(rs + slot * SLOT + c * KV_CHUNK);
             if (L::QT) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) pf_mma_ts(tmem + L::S_COL, tmem + L::Q_COL + c * 32 + k * 8, kd + 2 * k, id_s, (c | k) != 0);
+              for (int k = 0; k < 4; ++k) pf_mma_ts(tm + L::S_COL, tm + L::Q_COL + c * 32 + k * 8, kd + 2 * k, id_s, (c | k) != 0);
             } else {
               const uint64_t qd = make_smem_desc_sw128(qs + c * Q_CHUNK);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) umma_f16(tmem + L::S_COL, qd + 2 * k, kd + 2 * k, id_s, (c | k) != 0);
+              for (int k = 0; k < 4; ++k) umma_f16(tm + L::S_COL, qd + 2 * k, kd + 2 * k, id_s, (c | k) != 0);
             }
           }
           umma_commit(&empty[slot]);
           umma_commit(s_full);
-          if (++slot == SLOTS) { slot = 0; ph ^= 1; }
         }
-        if (j < 0) continue;
-        if (!mbar_wait(&full[slot], ph) || !mbar_wait(&p_full[j & 1], (j >> 1) & 1) ||
-            (j == ntiles - 1 && nkeys < ntiles * PF_BN && !mbar_wait(v_fixed, 0))) {
-          set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t p = tmem + L::P_COL + (j & 1) * 32;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          pf_mma_ts(tmem + O_COL, p + k * 8, pf_desc_nmajor(rs + slot * SLOT + k * 2048, KV_CHUNK), id_o, (j | k) != 0);
-        umma_commit(&empty[slot]);
-        umma_commit(&o_full[j & 1]);
+        __syncwarp();
         if (++slot == SLOTS) { slot = 0; ph ^= 1; }
       }
+      if (j < 0) continue;
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[slot], ph) && mbar_wait(&p_full[j & 1], (j >> 1) & 1) &&
+                                       (j < ntiles - 1 || nkeys == ntiles * PF_BN || mbar_wait(v_fixed, 0)));
+      if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j); break; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t p = tm + L::P_COL + (j & 1) * 32;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          pf_mma_ts(tm + O_COL, p + k * 8, pf_desc_nmajor(rs + slot * SLOT + k * 2048, KV_CHUNK), id_o, (j | k) != 0);
+        umma_commit(&empty[slot]);
+        umma_commit(&o_full[j & 1]);
+      }
+      __syncwarp();
+      if (++slot == SLOTS) { slot = 0; ph ^= 1; }
     }
   } else {
     // ------------------------------------------------------------ softmax, one query row per thread
