@@ -77,7 +77,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* tmem_full = empty_bar + MX_STAGES;
   uint64_t* tmem_empty = tmem_full + MX_ACC_STAGES;
   uint32_t* tmem_base_ptr = reinterpret_cast<uint32_t*>(tmem_empty + MX_ACC_STAGES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_k = g.K / MX_BK;
   const int mt_n = (g.M + MX_BM - 1) / MX_BM, nt_n = (g.N + MX_BN - 1) / MX_BN;
   const int num_tiles = mt_n * nt_n;
@@ -95,15 +95,15 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_ptr;
 
+  // (the whole warp walks the loops of the issuing roles, one elected lane issues: see moe_mxfp4_kernel.  2048 rows, two products of the shared expert: 85 -> 72 us)
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0; bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int mt = t / nt_n, nt = t % nt_n;
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
-            set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, kb); ok = false; break;
-          }
+    int stage = 0; uint32_t phase = 0; bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      const int mt = t / nt_n, nt = t % nt_n;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], phase ^ 1));
+        if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, kb); break; }
+        if (elect_one()) {
           uint8_t* a_dst = smem + stage * MX_STAGE_BYTES;
           uint8_t* b_dst = a_dst + MX_A_BYTES;
           uint8_t* sfa_dst = b_dst + MX_B_BYTES;
@@ -113,31 +113,33 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           bulk_load(sfa_dst, g.sfa + (static_cast<size_t>(mt) * num_k + kb) * MX_SF_BYTES, MX_SF_BYTES, &full_bar[stage]);
           bulk_load(sfa_dst + MX_SF_BYTES, g.sfb + (static_cast<size_t>(nt) * num_k + kb) * MX_SF_BYTES, MX_SF_BYTES,
                     &full_bar[stage]);
-          if (++stage == MX_STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == MX_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc0 = make_idesc_mx(MX_BM, MX_BN);
-      int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1)) {
-          set_status(g.status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, t, acc); break;
-        }
+    const uint32_t idesc0 = make_idesc_mx(MX_BM, MX_BN);
+    const uint32_t s0 = __shfl_sync(0xffffffffu, smem_u32(smem), 0), tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1))) {
+        set_status(g.status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, t, acc); break;
+      }
+      tc_fence_after();
+      const uint32_t d_tmem = tm + acc * MX_BN;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase));
+        if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * MX_BN;
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase)) {
-            set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); ok = false; break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * MX_STAGE_BYTES);
-          const uint64_t a_desc = make_smem_desc_sw128(a_addr);
-          const uint64_t b_desc = make_smem_desc_sw128(a_addr + MX_A_BYTES);
-          const uint32_t tsfa = tmem_base + MX_SF_COL0 + stage * 8, tsfb = tsfa + 4;
-          tmem_cp_32x128b_x4(tsfa, make_sf_desc(a_addr + MX_A_BYTES + MX_B_BYTES));
-          tmem_cp_32x128b_x4(tsfb, make_sf_desc(a_addr + MX_A_BYTES + MX_B_BYTES + MX_SF_BYTES));
+        const uint32_t a_addr = s0 + stage * MX_STAGE_BYTES;
+        const uint64_t a_desc = make_smem_desc_sw128(a_addr);
+        const uint64_t b_desc = make_smem_desc_sw128(a_addr + MX_A_BYTES);
+        const uint64_t sfa_desc = make_sf_desc(a_addr + MX_A_BYTES + MX_B_BYTES), sfb_desc = make_sf_desc(a_addr + MX_A_BYTES + MX_B_BYTES + MX_SF_BYTES);
+        const uint32_t tsfa = tm + MX_SF_COL0 + stage * 8, tsfb = tsfa + 4;
+        if (elect_one()) {
+          tmem_cp_32x128b_x4(tsfa, sfa_desc);
+          tmem_cp_32x128b_x4(tsfb, sfb_desc);
 #pragma unroll
           for (int k = 0; k < MX_BK / 32; ++k) {
             // 32 fp8 = 32 bytes along K inside the swizzled row: +2 in the encoded address; scale byte k of the block
@@ -145,11 +147,13 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             umma_mxf8(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, tsfa, tsfb, (kb | k) != 0);
           }
           umma_commit(&empty_bar[stage]);
-          if (++stage == MX_STAGES) { stage = 0; phase ^= 1; }
+          if (kb == num_k - 1) umma_commit(&tmem_full[acc]);
         }
-        umma_commit(&tmem_full[acc]);
-        if (++acc == MX_ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == MX_STAGES) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++acc == MX_ACC_STAGES) { acc = 0; acc_phase ^= 1; }
     }
   } else {
     const int quarter = warp & 3;
