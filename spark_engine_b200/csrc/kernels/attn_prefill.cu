@@ -1,8 +1,8 @@
 // Causal GQA attention for prefill segments (bf16 KV cache): streaming softmax on tcgen05.  One CTA = 128 query rows of one q head,
 // key/value tiles of 64 tokens.
-//   warp 0      TMA: the query tile, then key and value tiles into a ring of four slots in the order the products use them;
-//               values past the last key of a ragged tile are zeroed in shared memory (a masked probability of 0 times whatever
-//               the cache holds there would otherwise not be 0)
+//   warp 0      TMA: key and value tiles into a ring of four or six slots in the order the products use them (D = 64 / 128: the
+//               query tile before them).  A ragged last tile is brought in as boxes of eight rows and plain copies of the rest;
+//               its values past the last key are zeroed (a masked probability of 0 times whatever lies there would not be 0)
 //   warp 1      issues S = Q K^T one tile ahead of O += P V (P in tensor memory, V as an N-major operand straight from its rows)
 //   warps 2..5  softmax, one query row per thread: a row's 64 scores are one tensor-memory load, maximum and sum stay in the thread
 // The accumulator is rescaled only where a row's maximum has grown by more than 2^8 since its reference (the sums stay exact: every
@@ -34,7 +34,7 @@ template <int D> struct Pf {
 };
 
 struct PrefillArgs {
-  const __nv_bfloat16* q;                             // [R, Hq, D]
+  const __nv_bfloat16 *q, *k, *v;                     // [R, Hq, D], [tokens, Hkv, D]
   const long long* row_kv; const int* seg;            // cache row of a sequence's first token per row; [nseg][4]
   const __nv_bfloat16* qkv; int ld, gated;            // gate columns
   __nv_bfloat16* out;
@@ -81,7 +81,8 @@ __device__ __forceinline__ uint64_t pf_desc_nmajor(uint32_t addr, uint32_t chunk
 template <int D, bool MASK>
 __global__ void __launch_bounds__(PF_THREADS, D == 256 ? 1 : 2)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ PrefillArgs a) {
+                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmK8,
+                    const __grid_constant__ CUtensorMap tmV8, const __grid_constant__ PrefillArgs a) {
   using L = Pf<D>;
   constexpr int CH = D / 64, SLOT = L::SLOT, SLOTS = L::SLOTS, KV_CHUNK = PF_BN * 128, Q_CHUNK = PF_BM * 128;
   constexpr int COLS = L::COLS, O_COL = L::O_COL;
@@ -99,8 +100,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + SLOTS * SLOT);
   uint64_t* empty = full + SLOTS;
   uint64_t* q_full = empty + SLOTS;
-  uint64_t* v_fixed = q_full + 1;
-  uint64_t* s_full = v_fixed + 1;
+  uint64_t* s_full = q_full + 1;
   uint64_t* s_read = s_full + 1;
   uint64_t* p_full = s_read + 1;
   uint64_t* o_full = p_full + 2;
@@ -110,7 +110,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (!L::QT) tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
     for (int s = 0; s < SLOTS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    mbar_init(q_full, L::QT ? 4 : 1); mbar_init(v_fixed, 1); mbar_init(s_full, 1); mbar_init(s_read, 4);
+    mbar_init(q_full, L::QT ? 4 : 1); mbar_init(s_full, 1); mbar_init(s_read, 4);
     for (int s = 0; s < 2; ++s) { mbar_init(&p_full[s], 4); mbar_init(&o_full[s], 1); }
     fence_barrier_init();
   }
@@ -129,33 +129,40 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_arrive_expect_tx(q_full, PF_BM * D * 2);
       for (int c = 0; c < CH; ++c) tma_load_2d(smem + c * Q_CHUNK, &tmQ, q_full, h * D + c * 64, r0 + qt * PF_BM);
     }
-    int last_slot = 0; uint32_t last_ph = 0;
+    const int keep = nkeys - (ntiles - 1) * PF_BN, keep8 = keep & ~7;      // keys of the last tile, in groups of 8
     for (int i = 0; i < 2 * ntiles; ++i) {                    // K0 K1 V0 K2 V1 .. K(n-1) V(n-2) V(n-1)
       const bool is_v = i == 2 * ntiles - 1 || (i >= 2 && !(i & 1));
       const int j = i == 0 ? 0 : i == 2 * ntiles - 1 ? ntiles - 1 : is_v ? i / 2 - 1 : (i + 1) / 2;
       ok = __all_sync(0xffffffffu, mbar_wait(&empty[slot], ph ^ 1));
       if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, blockIdx.y, i); break; }
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&full[slot], SLOT);
-        for (int c = 0; c < CH; ++c)
-          tma_load_2d(ring + slot * SLOT + c * KV_CHUNK, is_v ? &tmV : &tmK, &full[slot], hk * D + c * 64, base + j * PF_BN);
-      }
-      __syncwarp();
-      last_slot = slot; last_ph = ph;
-      if (++slot == SLOTS) { slot = 0; ph ^= 1; }
-    }
-    const int keep = nkeys - (ntiles - 1) * PF_BN;
-    if (ok && keep < PF_BN) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[last_slot], last_ph));
-      if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -1);
-      if (ok) {
-        const int per = (PF_BN - keep) * 8;                   // 16-byte units of a chunk's rows past the last key
-        for (int u = lane; u < CH * per; u += 32)
-          *reinterpret_cast<uint4*>(ring + last_slot * SLOT + (u / per) * KV_CHUNK + keep * 128 + (u % per) * 16) = make_uint4(0u, 0u, 0u, 0u);
+      uint8_t* dst = ring + slot * SLOT;
+      if (j < ntiles - 1 || keep == PF_BN) {
+        if (lane == 0) {
+          mbar_arrive_expect_tx(&full[slot], SLOT);
+          for (int c = 0; c < CH; ++c) tma_load_2d(dst + c * KV_CHUNK, is_v ? &tmV : &tmK, &full[slot], hk * D + c * 64, base + j * PF_BN);
+        }
+      } else {
+        // rows keep8 .. keep as plain copies in the swizzle's order, value rows from keep on zero; unread key rows stay as they are
+        const __nv_bfloat16* src = is_v ? a.v : a.k;
+        const int per = ((is_v ? PF_BN : keep) - keep8) * 8;   // 16-byte units of a chunk
+        for (int u = lane; u < CH * per; u += 32) {
+          const int c = u / per, row = keep8 + (u - c * per) / 8, x = u & 7;
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          if (row < keep) v = __ldg(reinterpret_cast<const uint4*>(src + (static_cast<size_t>(base + j * PF_BN + row) * a.Hkv + hk) * D + c * 64) + x);
+          *reinterpret_cast<uint4*>(dst + c * KV_CHUNK + row * 128 + ((x ^ (row & 7)) * 16)) = v;
+        }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(v_fixed);
+        if (lane == 0) {
+          if (keep8 == 0) mbar_arrive(&full[slot]);
+          else mbar_arrive_expect_tx(&full[slot], CH * keep8 * 128);
+          for (int c = 0; c < CH; ++c)
+            for (int r = 0; r < keep8; r += 8)
+              tma_load_2d(dst + c * KV_CHUNK + r * 128, is_v ? &tmV8 : &tmK8, &full[slot], hk * D + c * 64, base + j * PF_BN + r);
+        }
       }
+      __syncwarp();
+      if (++slot == SLOTS) { slot = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -192,8 +199,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (++slot == SLOTS) { slot = 0; ph ^= 1; }
       }
       if (j < 0) continue;
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[slot], ph) && mbar_wait(&p_full[j & 1], (j >> 1) & 1) &&
-                                       (j < ntiles - 1 || nkeys == ntiles * PF_BN || mbar_wait(v_fixed, 0)));
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[slot], ph) && mbar_wait(&p_full[j & 1], (j >> 1) & 1));
       if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, j); break; }
       tc_fence_after();
       if (elect_one()) {
@@ -374,17 +380,18 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 }
 
 template <int D, bool MASK>
-static int launch_prefill(const void* qbuf, int R, const void* kc, const void* vc, long long tokens, int nseg, int max_rows,
-                          const PrefillArgs& a, cudaStream_t s) {
-  CUtensorMap tq, tk, tv;
+static int launch_prefill(int R, long long tokens, int nseg, int max_rows, const PrefillArgs& a, cudaStream_t s) {
+  CUtensorMap tq, tk, tv, tk8, tv8;
   const uint64_t wq = static_cast<uint64_t>(a.Hq) * D, wk = static_cast<uint64_t>(a.Hkv) * D;
-  if (int r = make_tmap_rows64(&tq, qbuf, R, wq, wq, PF_BM, 1)) return r;
-  if (int r = make_tmap_rows64(&tk, kc, tokens, wk, wk, PF_BN, 1)) return r;
-  if (int r = make_tmap_rows64(&tv, vc, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_rows64(&tq, a.q, R, wq, wq, PF_BM, 1)) return r;
+  if (int r = make_tmap_rows64(&tk, a.k, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_rows64(&tv, a.v, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_rows64(&tk8, a.k, tokens, wk, wk, 8, 1)) return r;
+  if (int r = make_tmap_rows64(&tv8, a.v, tokens, wk, wk, 8, 1)) return r;
   auto kern = attn_prefill_kernel<D, MASK>;
   static bool done = false;
   if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Pf<D>::SMEM); done = true; }
-  kern<<<dim3(a.Hq, (max_rows + PF_BM - 1) / PF_BM, nseg), PF_THREADS, Pf<D>::SMEM, s>>>(tq, tk, tv, a);
+  kern<<<dim3(a.Hq, (max_rows + PF_BM - 1) / PF_BM, nseg), PF_THREADS, Pf<D>::SMEM, s>>>(tq, tk, tv, tk8, tv8, a);
   return spark_launch_rc(__func__);
 }
 
@@ -412,25 +419,25 @@ sel_blockmask_kernel(const int* __restrict__ sel, const int* __restrict__ sel_n,
 using namespace spark;
 
 template <bool MASK>
-static int prefill(const void* qbuf, int R, const void* kc, const void* vc, long long tokens, int nseg, int max_rows, int D,
-                   const PrefillArgs& a, cudaStream_t s) {
+static int prefill(int R, long long tokens, int nseg, int max_rows, int D, const PrefillArgs& a, cudaStream_t s) {
   if (tokens <= 0 || tokens > 0x7fffffffLL || a.Hkv <= 0 || a.Hq % a.Hkv || (a.gated && (a.ld & 1))) return -5;
-  if (D == 256) return launch_prefill<256, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
-  if (D == 128) return launch_prefill<128, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
-  if (D == 64) return launch_prefill<64, MASK>(qbuf, R, kc, vc, tokens, nseg, max_rows, a, s);
+  if (D == 256) return launch_prefill<256, MASK>(R, tokens, nseg, max_rows, a, s);
+  if (D == 128) return launch_prefill<128, MASK>(R, tokens, nseg, max_rows, a, s);
+  if (D == 64) return launch_prefill<64, MASK>(R, tokens, nseg, max_rows, a, s);
   return -5;
 }
 
 // Dense causal attention over bf16 caches for whole segments.  seg: int [nseg][4] = slot, first row, rows, first position; R: rows of
-// qbuf; max_rows = longest segment; tokens: cache rows that may be touched (past the last key of every segment: what lies
-// between is read and masked, what lies beyond is not read).  head_dim 64, 128 or 256.
+// qbuf; max_rows = longest segment; tokens: rows of the caches.  No row past the last key of a segment is read (a cache that grows
+// on demand may not have it), and none of the bounds is the host's: seg and row_kv may change between replays of a captured launch.
+// head_dim 64, 128 or 256.
 extern "C" int spark_attn_prefill(const void* qbuf, const void* kc, const void* vc, const long long* row_kv, const int* seg,
                                   int nseg, int max_rows, const void* qkv, int ld, int gated, void* out, int Hq, int Hkv,
                                   int D, float scale, int R, long long tokens, int* status, cudaStream_t s) {
   if (nseg <= 0 || max_rows <= 0 || R <= 0) return 0;
-  const PrefillArgs a{(const __nv_bfloat16*)qbuf, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
+  const PrefillArgs a{(const __nv_bfloat16*)qbuf, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
                       nullptr, 0, status};
-  return prefill<false>(qbuf, R, kc, vc, tokens, nseg, max_rows, D, a, s);
+  return prefill<false>(R, tokens, nseg, max_rows, D, a, s);
 }
 
 // The same tiles for rows with a block-sparse selection (4-token blocks): sel / sel_n are the per-row token lists of the
@@ -442,7 +449,7 @@ extern "C" int spark_attn_prefill_masked(const void* qbuf, const void* kc, const
   if (nseg <= 0 || max_rows <= 0 || R <= 0) return 0;
   if (mw <= 0 || mw > 8192 || !sel || !sel_n || !bmask) return -5;
   sel_blockmask_kernel<<<R, 256, mw * 4, s>>>(sel, sel_n, sel_ld, bmask, mw);
-  const PrefillArgs a{(const __nv_bfloat16*)qbuf, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
+  const PrefillArgs a{(const __nv_bfloat16*)qbuf, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
                       bmask, mw, status};
-  return prefill<true>(qbuf, R, kc, vc, tokens, nseg, max_rows, D, a, s);
+  return prefill<true>(R, tokens, nseg, max_rows, D, a, s);
 }

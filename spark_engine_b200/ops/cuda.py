@@ -1285,12 +1285,6 @@ def tree_ancestor_masks(plan, device) -> torch.Tensor:
     return torch.from_numpy(m.view(np.int32)).to(device)
 
 
-def _keys_end(plan, seqs):
-    """First cache row behind every key of the plan: whole tiles may be read up to here (a cache that grows on demand is backed up
-    to its highest lease)."""
-    return max(seqs[s.slot].kv_base + s.pos0 + s.n for s in plan.segs)
-
-
 def attn_mixer(mixer, qkv, plan, seqs):
     c = mixer.c
     dev = qkv.device
@@ -1340,7 +1334,7 @@ def attn_mixer(mixer, qkv, plan, seqs):
         rc = lib().spark_attn_prefill(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
                                       max(s.n for s in plan.segs), P(qkv), qkv.stride(0), int(c.gated), P(out),
                                       c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), R,
-                                      _keys_end(plan, seqs), P(status_word(dev)), stream())
+                                      mixer.k.shape[0], P(status_word(dev)), stream())
         check(rc, "spark_attn_prefill")
         return out
     if (sel is not None and not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.block == 4
@@ -1355,7 +1349,7 @@ def attn_mixer(mixer, qkv, plan, seqs):
         rc = lib().spark_attn_prefill_masked(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
                                              max(s.n for s in plan.segs), P(qkv), qkv.stride(0), int(c.gated), P(out),
                                              c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), P(sel),
-                                             P(sel_n), sel_ld, R, P(bmask), mw, _keys_end(plan, seqs), P(status_word(dev)),
+                                             P(sel_n), sel_ld, R, P(bmask), mw, mixer.k.shape[0], P(status_word(dev)),
                                              stream())
         check(rc, "spark_attn_prefill_masked")
         return out

@@ -96,3 +96,36 @@ def test_repeats_bitwise():
     a, _ = _run(256, 4, 2, [(257, 100, 0)], gated=True, masked=True)
     b, _ = _run(256, 4, 2, [(257, 100, 0)], gated=True, masked=True)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("sparse", [0, 8])
+def test_captured_rows_follow_their_plan(sparse):
+    """A captured round of 32 and more rows per sequence replayed further along its sequence: the keys it reads follow the staged
+    positions (dense rows, and rows whose blocks are selected)."""
+    import dataclasses
+    from spark_engine_b200.config import tiny_hybrid
+    from spark_engine_b200.models.model import Model
+    from spark_engine_b200.models.plan import make_plan
+    from spark_engine_b200.models.weights import init_weights, to_device
+    from spark_engine_b200.serving.graphs import RoundGraph
+    cfg = tiny_hybrid()
+    cfg.n_layers, cfg.layer_types = 1, ["attn"]
+    cfg.attn = dataclasses.replace(cfg.attn, sparse_topk_blocks=sparse)
+    cfg.moe = dataclasses.replace(cfg.moe, dense_layers=1, dense_ffn=128)
+    W = to_device(init_weights(cfg, seed=0), DEV)
+    ids = torch.randint(0, cfg.vocab, (240,), generator=torch.Generator().manual_seed(1)).tolist()
+    n = 37
+
+    def model():
+        m = Model(cfg, W, device=DEV, dtype=torch.bfloat16, n_slots=1, kv_tokens=256)
+        m.forward(make_plan([(0, ids[:40], 0)], device=DEV))
+        return m
+    eager, m = model(), model()
+    graph = RoundGraph(m, [0], n, 256)
+    for p in range(40, 240 - n, n):
+        want = eager.forward(make_plan([(0, ids[p: p + n], p)], device=DEV)).float()
+        graph.stage([ids[p: p + n]], [p])
+        graph.run(commit=True)
+        torch.cuda.synchronize()
+        got = graph.logits.float()
+        assert ((got - want).norm() / want.norm()).item() < 2.0 ** -7, p
