@@ -5,13 +5,17 @@
 //               its values past the last key are zeroed (a masked probability of 0 times whatever lies there would not be 0)
 //   warp 1      issues S = Q K^T one tile ahead of O += P V (P in tensor memory, V as an N-major operand straight from its rows)
 //   warps 2..5  softmax, one query row per thread: a row's 64 scores are one tensor-memory load, maximum and sum stay in the thread
-// The accumulator is rescaled only where a row's maximum has grown by more than 2^8 since its reference (the sums stay exact: every
-// term of a row uses the same reference), so most tiles never touch it.
+//   all warps   the epilogue's gates and stores
+// Every weight is taken against the running maximum, so that the heaviest of a row is exactly 1 in bf16 (a reference that lags behind
+// the maximum would spare most of the rescaling, and rounds the heavy weights by up to 2^-8): the accumulator is rescaled in 32 bits
+// at every tile where a row of the warp has a new maximum.
 // The rows of a segment see the committed prefix of their sequence (already in the cache) plus the rows before them in the segment
 // (stored by the prep kernel of the same step).  One CTA owns a (row tile, head) from first key to last, so results are run-to-run
-// identical.  What bounds it: L2 and the softmax together: every tile brings 64 KB of keys and values to 128 rows (D = 256), and its
-// exponentials take one warp per scheduler 900 cycles.  4000 rows of 16 heads (2 for keys), D = 256: 165 us, 795 TFLOP/s (64-row
-// tiles on warp-level products: 828 us with block masks).
+// identical.  What bounds it: the softmax, whose exponentials and rescaling are the chain of one warp per scheduler, and L2, from
+// which every tile brings 64 KB of keys and values to 128 rows (D = 256).  3999 rows of 16 heads (2 for keys), D = 256, block masks:
+// 203 us, 645 TFLOP/s (64-row tiles on warp-level products: 828 us; weights up to 2^8 against a lagging reference, with approximate
+// divisions: 165 us).  The rescaling behind the exponentials instead of before them: 20 us less; the epilogue's divisions, chains
+// that only other warps hide, over eight warps instead of four: 40 us less.
 // Serves: GQA / QSA layers (engine-rs/shim/qwen_qsa.cu attn paths; the reference runs prefill rows through the same per-row kernel
 // as decode).
 #include "../common/ptx.cuh"
@@ -20,8 +24,7 @@ namespace spark {
 
 int make_tmap_rows64(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
 
-constexpr int PF_BM = 128, PF_BN = 64, PF_THREADS = 192;
-constexpr float PF_GROW = 8.f;          // log2 of how far a maximum may outgrow its reference
+constexpr int PF_BM = 128, PF_BN = 64, PF_WARPS = 8, PF_THREADS = PF_WARPS * 32;
 
 // D = 256: the queries are a tensor-memory operand (a product of 64 keys reads 2 KB of shared memory per step instead of 6: 74 -> 25
 // cycles of issue each) and the ring has the room; 64 / 128: 256 columns hold everything with the queries in shared memory, and two
@@ -61,7 +64,6 @@ __device__ __forceinline__ void pf_tmem_st_x32(uint32_t addr, const uint32_t (&r
         "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 __device__ __forceinline__ void pf_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ float pf_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ uint32_t pf_pack(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -85,7 +87,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const __grid_constant__ CUtensorMap tmV8, const __grid_constant__ PrefillArgs a) {
   using L = Pf<D>;
   constexpr int CH = D / 64, SLOT = L::SLOT, SLOTS = L::SLOTS, KV_CHUNK = PF_BN * 128, Q_CHUNK = PF_BM * 128;
-  constexpr int COLS = L::COLS, O_COL = L::O_COL;
+  constexpr int COLS = L::COLS, O_COL = L::O_COL, LX = D + 1;           // LX: floats of a row in the epilogue
   const int sg = blockIdx.z, h = blockIdx.x;
   const int qt = gridDim.y - 1 - blockIdx.y;                 // longest row tiles (most key tiles) are scheduled first
   const int r0 = a.seg[sg * 4 + 1], n = a.seg[sg * 4 + 2], pos0 = a.seg[sg * 4 + 3];
@@ -120,11 +122,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
 
+  bool ok = true;
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     const int hk = h / (a.Hq / a.Hkv);
     const int base = static_cast<int>(a.row_kv[r0]);
-    int slot = 0; uint32_t ph = 0; bool ok = true;
+    int slot = 0; uint32_t ph = 0;
     if (!L::QT && lane == 0) {
       mbar_arrive_expect_tx(q_full, PF_BM * D * 2);
       for (int c = 0; c < CH; ++c) tma_load_2d(smem + c * Q_CHUNK, &tmQ, q_full, h * D + c * 64, r0 + qt * PF_BM);
@@ -167,11 +170,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     // (the whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers, where the instructions want
-    // them.  4000 rows of 16 heads of 256: 213 -> 165 us)
+    // them: 48 us less for 4000 rows of 16 heads of 256)
     const uint32_t id_s = make_idesc(1, 1, PF_BM, PF_BN), id_o = make_idesc(1, 1, PF_BM, D) | (1u << 16);
     const uint32_t qs = __shfl_sync(0xffffffffu, smem_u32(smem), 0), rs = qs + L::Q_BYTES, tm = __shfl_sync(0xffffffffu, tmem, 0);
     int slot = 0; uint32_t ph = 0;
-    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0));
+    ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0));
     if (!ok) set_status(a.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, -2);
     for (int j = -1; j < ntiles && ok; ++j) {
       if (j + 1 < ntiles) {
@@ -213,7 +216,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       __syncwarp();
       if (++slot == SLOTS) { slot = 0; ph ^= 1; }
     }
-  } else {
+  } else if (warp < 6) {
     // ------------------------------------------------------------ softmax, one query row per thread
     const int q = warp & 3, row = q * 32 + lane;
     const uint32_t t_lane = tmem + (static_cast<uint32_t>(q * 32) << 16);
@@ -244,7 +247,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     float m = -INFINITY, l = 0.f;
     uint32_t word = MASK ? __ldg(bm) : 0u;
-    bool ok = true;
     for (int j = 0; j < ntiles; ++j) {
       uint32_t next = 0u;
       if (MASK && (j & 1) && j + 1 < ntiles) next = __ldg(bm + ((j + 1) >> 1));
@@ -283,32 +285,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
       for (int i = 8; i < 64; ++i) mx[i & 7] = fmaxf(mx[i & 7], s[i]);
       const float top = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7]))) * a.scale_log2;
-      // m stays the reference until a maximum outgrows it; m = -inf: this row has seen no key yet
-      const bool grow = top > m + PF_GROW;
-      if (__any_sync(0xffffffffu, grow)) {
-        const float c = grow ? pf_exp2(m - top) : 1.f;
-        if (grow) { m = top; l *= c; }
-        if (j > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1));
-          if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
-          tc_fence_after();
-#pragma unroll 1
-          for (int cc = 0; cc < D; cc += 32) {
-            uint32_t o[32];
-            tmem_ld_32x32(t_lane + O_COL + cc, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * c);
-            pf_tmem_st_x32(t_lane + O_COL + cc, o);
-          }
-        }
-      }
+      const bool grow = top > m;                               // m = -inf: this row has seen no key yet
+      const bool rescale = j > 0 && __any_sync(0xffffffffu, grow);
+      const float c = grow ? exp2f(m - top) : 1.f;
+      if (grow) { m = top; l *= c; }
       const float ref = m == -INFINITY ? 0.f : m;
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
       uint32_t p[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        const float e0 = pf_exp2(fmaf(s[2 * i], a.scale_log2, -ref)), e1 = pf_exp2(fmaf(s[2 * i + 1], a.scale_log2, -ref));
+        const float e0 = exp2f(fmaf(s[2 * i], a.scale_log2, -ref)), e1 = exp2f(fmaf(s[2 * i + 1], a.scale_log2, -ref));
         sum[i & 1] += e0; sum[2 + (i & 1)] += e1;
         p[i] = pf_pack(e0, e1);
       }
@@ -319,63 +305,84 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
       }
       pf_tmem_st_x32(t_lane + L::P_COL + (j & 1) * 32, p);
+      if (rescale) {                                           // behind the exponentials: the product before has finished by now
+        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1));
+        if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
+        tc_fence_after();
+#pragma unroll 1
+        for (int cc = 0; cc < D; cc += 64) {
+          uint32_t o[2][32];
+          tmem_ld_32x32(t_lane + O_COL + cc, o[0]);
+          tmem_ld_32x32(t_lane + O_COL + cc + 32, o[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            o[0][i] = __float_as_uint(__uint_as_float(o[0][i]) * c);
+            o[1][i] = __float_as_uint(__uint_as_float(o[1][i]) * c);
+          }
+          pf_tmem_st_x32(t_lane + O_COL + cc, o[0]);
+          pf_tmem_st_x32(t_lane + O_COL + cc + 32, o[1]);
+        }
+      }
       pf_tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[j & 1]);
     }
-    // ---- epilogue: normalise, gate, store
+    // ---- epilogue: normalise, through shared memory (queries, keys and values are used up), so that a row's columns are read and
+    // written together
     if (ok) {
       ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1));
       if (!ok) set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, ntiles);
     }
     if (ok) {
       tc_fence_after();
-      // through shared memory (queries, keys and values are used up), so that a row's columns are read and written together
-      constexpr int LX = D + 1, CW = D / 64;                   // 64-column pieces of a row: a lane has columns 2 lane, 2 lane + 1 of each
-      float* x = reinterpret_cast<float*>(smem) + q * (32 * LX);
+      float* x = reinterpret_cast<float*>(smem) + row * LX;
       const float inv = 1.f / l;
-      const int live = min(32, rows_valid - q * 32);
-      const size_t rw = static_cast<size_t>(r0 + qt * PF_BM + q * 32);
 #pragma unroll 1
       for (int cc = 0; cc < D; cc += 32) {
         uint32_t o[32];
         tmem_ld_32x32(t_lane + O_COL + cc, o);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) x[lane * LX + cc + i] = __uint_as_float(o[i]) * inv;
-      }
-      __syncwarp();
-      // eight rows' gates are asked for before the first is used
-#pragma unroll 1
-      for (int i0 = 0; i0 < live; i0 += 8) {
-        uint32_t gate[8][CW];
-        if (a.gated) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const __nv_bfloat16* gp = a.qkv + (rw + min(i0 + i, live - 1)) * a.ld + h * 2 * D + D + 2 * lane;
-#pragma unroll
-            for (int c = 0; c < CW; ++c) gate[i][c] = __ldg(reinterpret_cast<const uint32_t*>(gp + c * 64));
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          __nv_bfloat16* dst = a.out + ((rw + i0 + i) * a.Hq + h) * D + 2 * lane;
-#pragma unroll
-          for (int c = 0; c < CW; ++c) {
-            float v0 = x[(i0 + i) * LX + c * 64 + 2 * lane], v1 = x[(i0 + i) * LX + c * 64 + 2 * lane + 1];
-            if (a.gated) {
-              const float2 gt = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gate[i][c]));
-              v0 = __fdividef(v0, 1.f + __expf(-gt.x)); v1 = __fdividef(v1, 1.f + __expf(-gt.y));
-            }
-            if (i0 + i < live) *reinterpret_cast<uint32_t*>(dst + c * 64) = pf_pack(v0, v1);
-          }
-        }
+        for (int i = 0; i < 32; ++i) x[cc + i] = __uint_as_float(o[i]) * inv;
       }
     }
   }
   tc_fence_before();
-  __syncthreads();
+  if (__syncthreads_and(ok)) {
+    // ---- gate, store: eight rows of all eight warps at a time (a division is a chain of its own, which only other warps hide), the
+    // gates of a group asked for before the first is used
+    constexpr int CW = D / 64;                                 // 64-column pieces of a row: a lane has columns 2 lane, 2 lane + 1 of each
+    const float* x = reinterpret_cast<const float*>(smem);
+    const size_t rw = static_cast<size_t>(r0 + qt * PF_BM);
+#pragma unroll 1
+    for (int i0 = warp * 8; i0 < rows_valid; i0 += PF_WARPS * 8) {
+      uint32_t gate[8][CW];
+      if (a.gated) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const __nv_bfloat16* gp = a.qkv + (rw + min(i0 + i, rows_valid - 1)) * a.ld + h * 2 * D + D + 2 * lane;
+#pragma unroll
+          for (int c = 0; c < CW; ++c) gate[i][c] = __ldg(reinterpret_cast<const uint32_t*>(gp + c * 64));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i0 + i >= rows_valid) break;
+        __nv_bfloat16* dst = a.out + ((rw + i0 + i) * a.Hq + h) * D + 2 * lane;
+#pragma unroll
+        for (int c = 0; c < CW; ++c) {
+          float v0 = x[(i0 + i) * LX + c * 64 + 2 * lane], v1 = x[(i0 + i) * LX + c * 64 + 2 * lane + 1];
+          if (a.gated) {
+            const float2 gt = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gate[i][c]));
+            v0 = v0 / (1.f + __expf(-gt.x)); v1 = v1 / (1.f + __expf(-gt.y));
+          }
+          *reinterpret_cast<uint32_t*>(dst + c * 64) = pf_pack(v0, v1);
+        }
+      }
+    }
+  }
   if (warp == 1) { tc_fence_after(); tmem_dealloc<COLS>(tmem); }
 }
 

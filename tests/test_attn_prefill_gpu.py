@@ -129,3 +129,24 @@ def test_captured_rows_follow_their_plan(sparse):
         torch.cuda.synchronize()
         got = graph.logits.float()
         assert ((got - want).norm() / want.norm()).item() < 2.0 ** -7, p
+
+
+def test_heaviest_weight_is_exact():
+    """Two keys with the same value share a row's weight, the later one 2 to 2^8 times the earlier.  Each is the largest where it comes
+    up, so its weight is 1 there and the earlier sum is scaled in 32 bits: the result is that value.  (A weight of 2^x in bf16, as a
+    reference that lags behind the maximum gives it, moves the result by up to 2^-8 of it.)"""
+    from spark_engine_b200.ops import cuda as cu
+    P, D, n, p = cu.P, 64, 200, 128
+    q = torch.zeros(n, 1, D, device=DEV, dtype=torch.bfloat16)
+    q[:, 0, 0] = torch.linspace(1, 8, n, device=DEV).bfloat16()
+    k = torch.zeros(p + n, 1, D, device=DEV, dtype=torch.bfloat16)
+    k[1:, 0, 0] = -2000
+    k[64, 0, 0] = 5.5                                               # log2 of its weight over the first key's: 0.99 q
+    v = torch.zeros_like(k)
+    v[0, 0] = v[64, 0] = (1 + 127 / 128 - torch.arange(D, device=DEV) / 128).bfloat16()
+    out = torch.empty(n, D, device=DEV, dtype=torch.bfloat16)
+    seg = torch.tensor([[0, 0, n, p]], dtype=torch.int32, device=DEV)
+    row_kv = torch.zeros(n, dtype=torch.int64, device=DEV)
+    cu.check(cu.lib().spark_attn_prefill(P(q), P(k), P(v), P(row_kv), P(seg), 1, n, None, 0, 0, P(out), 1, 1, D, 0.125, n, p + n,
+                                         P(cu.status_word(torch.device(DEV))), cu.stream()), "dense")
+    assert torch.equal(out, v[0, 0].expand_as(out))
