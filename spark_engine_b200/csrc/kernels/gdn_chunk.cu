@@ -166,7 +166,7 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
         const int r = warp * 8 + i;
         float4 y = r < nv ? gdn_conv(x, i, w) : make_float4(0.f, 0.f, 0.f, 0.f);
         float f = 1.f;
-        if (part < 2) {
+        if (part < 2 && r < nv) {                           // rows past the end stay zero, whatever eps is
           const float ss = warp_sum(fmaf(y.w, y.w, fmaf(y.z, y.z, fmaf(y.y, y.y, y.x * y.x))));
           f = rsqrtf(ss + eps) * (part == 0 ? rsqrtf(static_cast<float>(GD)) : 1.f);
         }

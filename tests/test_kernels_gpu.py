@@ -269,6 +269,48 @@ def test_gdn_chunked_prefill_matches_sequential_kernel(lens):
     assert row_err.max() < 3e-2, row_err.max()
 
 
+def _gdn_both_forms(rows, eps=1e-6, fill=None, S0=True):
+    """(outputs, states) of the sequential and of the chunked form for one segment of `rows` random rows; fill(proj, w, nq) edits the
+    projections (columns q | k | v | z) and the weights."""
+    import dataclasses
+    from spark_engine_b200.config import ModelConfig, GdnConfig
+    from spark_engine_b200.models.model import GdnMixer
+    from spark_engine_b200.models.plan import make_plan
+    cfg = dataclasses.replace(ModelConfig(), gdn=GdnConfig(n_k_heads=1, n_v_heads=2, head_dim=128), norm_eps=eps)
+    c = cfg.gdn
+    g = torch.Generator(device=DEV).manual_seed(13)
+    nq, nv = c.n_k_heads * c.head_dim, c.n_v_heads * c.head_dim
+    w = {"conv": (torch.rand(2 * nq + nv, c.conv_k, device=DEV, generator=g) - 0.5),
+         "A_log": torch.log(torch.rand(c.n_v_heads, device=DEV, generator=g) * 7 + 1),
+         "dt_bias": torch.rand(c.n_v_heads, device=DEV, generator=g) * 2 - 1,
+         "norm": torch.rand(c.head_dim, device=DEV, generator=g) + 0.5}
+    proj = torch.randn(rows, 2 * nq + 2 * nv, device=DEV, generator=g).bfloat16()
+    ab = torch.randn(rows, 2 * c.n_v_heads, device=DEV, generator=g).bfloat16()
+    if fill:
+        fill(proj, ab, w, nq)
+    plan = make_plan([(0, [1] * rows, 5)], device=DEV)
+    outs = []
+    for chunked in (False, True):
+        m = GdnMixer(cfg, w, 1, DEV, torch.bfloat16)
+        if S0:
+            m.S.copy_(torch.randn(m.S.shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(14)) * 0.1)
+        cu().GDN_CHUNKED = chunked
+        try:
+            out = cu().gdn_mixer(m, proj, ab, plan, True)
+        finally:
+            cu().GDN_CHUNKED = True
+        torch.cuda.synchronize()
+        outs.append((out.double(), m.S.double()))
+    return outs
+
+
+def test_gdn_chunked_ragged_end_without_eps():
+    """Rows past the end of the last chunk are zero rows; with eps 0 they have no norm to divide by."""
+    (o0, S0), (o1, S1) = _gdn_both_forms(77, eps=0.0)
+    assert torch.isfinite(o1).all() and torch.isfinite(S1).all()
+    assert rel_err(o1, o0) < 1e-2 and rel_err(S1, S0) < 5e-3
+
+
 # ------------------------------------------------------------------------------ KDA
 @pytest.mark.parametrize("D", [32, 64, 128])
 def test_kda_kernel_matches_torch_recurrence(D):
