@@ -76,7 +76,10 @@ __device__ __forceinline__ void gdn_widen_rows(const uint2 (&u)[11], const float
   if (first < 0) {
 #pragma unroll
     for (int j = 0; j < 3; ++j)
-      if (first + j < 0) x[j] = *reinterpret_cast<const float4*>(hist + static_cast<size_t>(first + j + 3) * hist_ld);
+      if (first + j < 0) {                                   // (three rows of a segment: no vectors, the caller's tail may start anywhere)
+        const float* p = hist + static_cast<size_t>(first + j + 3) * hist_ld;
+        x[j] = make_float4(p[0], p[1], p[2], p[3]);
+      }
   }
 }
 // conv(k = 4) + SiLU of row i (x[i .. i + 3]); w[c]: taps of channel c

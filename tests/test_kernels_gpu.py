@@ -304,6 +304,27 @@ def _gdn_both_forms(rows, eps=1e-6, fill=None, S0=True):
     return outs
 
 
+def test_gdn_chunked_history_on_any_float():
+    """A history of earlier inputs that does not start on 16 bytes (views of a larger buffer) gives the bits of one that does."""
+    import dataclasses
+    from spark_engine_b200.config import ModelConfig, GdnConfig
+    from spark_engine_b200.models.model import GdnMixer
+    from spark_engine_b200.models.plan import make_plan
+    cfg = dataclasses.replace(ModelConfig(), gdn=GdnConfig(n_k_heads=1, n_v_heads=2, head_dim=128))
+    g = torch.Generator(device=DEV).manual_seed(15)
+    w = {"conv": torch.rand(512, 4, device=DEV, generator=g) - 0.5, "A_log": torch.zeros(2, device=DEV), "dt_bias": torch.zeros(2, device=DEV),
+         "norm": torch.ones(128, device=DEV)}
+    proj = torch.randn(70, 768, device=DEV, generator=g).bfloat16()
+    ab = torch.randn(70, 4, device=DEV, generator=g).bfloat16()
+    outs = []
+    for shift in (0, 1):
+        m = GdnMixer(cfg, w, 1, DEV, torch.bfloat16)
+        tail = torch.randn(m.tail.shape, device=DEV, generator=torch.Generator(device=DEV).manual_seed(16))
+        m.tail = torch.empty(tail.numel() + shift, device=DEV)[shift:].view(tail.shape).copy_(tail)
+        outs.append((cu().gdn_mixer(m, proj, ab, make_plan([(0, [1] * 70, 5)], device=DEV), True), m.S, m.tail))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 def test_gdn_chunked_ragged_end_without_eps():
     """Rows past the end of the last chunk are zero rows; with eps 0 they have no norm to divide by."""
     (o0, S0), (o1, S1) = _gdn_both_forms(77, eps=0.0)
