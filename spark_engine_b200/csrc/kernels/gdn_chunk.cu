@@ -44,7 +44,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], float a0, float a1, floa
                : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)),
                  "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
-__device__ __forceinline__ float silu(float x) { return __fdividef(x, 1.f + __expf(-x)); }      // rounded to TF32 next
+__device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
@@ -52,9 +52,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // ---------------------------------------------------------------------------------------------- kernel 1
 // grid (chunks, Hv); 256 threads.  Two CTAs share an SM (107 KB each): A and T take the place of Q once its products are through.
-// What bounds it: the chain of its phases, of which the convolution is the longest (a row of a warp is 95 instructions for four
-// channels), hidden only by the second CTA; 302 MB are written at 1.5 TB/s.  64 chunks of 32 heads: 544 -> 198 us (one CTA per SM,
-// one channel per lane with its rows loaded one after the other: 20 us for the convolution of a CTA).
+// What bounds it: the chain of its phases, of which the convolution with its SiLU is the longest, hidden only by the second CTA;
+// 302 MB are written at 1.2 TB/s.  64 chunks of 32 heads: 544 -> 245 us (one CTA per SM, one channel per lane with its rows loaded
+// one after the other: 20 us for the convolution of a CTA).  47 us of it are the IEEE divisions of the SiLU: an approximate one
+// gives 0 below -87.3, and values that small are numbers of the state.
 constexpr int SM_AT = GC * LD128, SM_AT_EXTRA = 2 * GC * LD64 - SM_AT;      // floats of A and T past the end of Q
 constexpr int PREP_SMEM = (3 * GC * LD128 + SM_AT_EXTRA + 3 * GC) * 4;
 
@@ -82,12 +83,12 @@ __device__ __forceinline__ void gdn_widen_rows(const uint2 (&u)[11], const float
       }
   }
 }
-// conv(k = 4) + SiLU of row i (x[i .. i + 3]); w[c]: taps of channel c
+// conv(k = 4) of row i (x[i .. i + 3]); w[c]: taps of channel c
 __device__ __forceinline__ float4 gdn_conv(const float4 (&x)[11], int i, const float4 (&w)[4]) {
-  return make_float4(silu(x[i].x * w[0].x + x[i + 1].x * w[0].y + x[i + 2].x * w[0].z + x[i + 3].x * w[0].w),
-                     silu(x[i].y * w[1].x + x[i + 1].y * w[1].y + x[i + 2].y * w[1].z + x[i + 3].y * w[1].w),
-                     silu(x[i].z * w[2].x + x[i + 1].z * w[2].y + x[i + 2].z * w[2].z + x[i + 3].z * w[2].w),
-                     silu(x[i].w * w[3].x + x[i + 1].w * w[3].y + x[i + 2].w * w[3].z + x[i + 3].w * w[3].w));
+  return make_float4(x[i].x * w[0].x + x[i + 1].x * w[0].y + x[i + 2].x * w[0].z + x[i + 3].x * w[0].w,
+                     x[i].y * w[1].x + x[i + 1].y * w[1].y + x[i + 2].y * w[1].z + x[i + 3].y * w[1].w,
+                     x[i].z * w[2].x + x[i + 1].z * w[2].y + x[i + 2].z * w[2].z + x[i + 3].z * w[2].w,
+                     x[i].w * w[3].x + x[i + 1].w * w[3].y + x[i + 2].w * w[3].z + x[i + 3].w * w[3].w);
 }
 __device__ __forceinline__ float4 scale_tf32(float4 v, float f) { return make_float4(tf32r(v.x * f), tf32r(v.y * f), tf32r(v.z * f), tf32r(v.w * f)); }
 
@@ -149,7 +150,8 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
     *reinterpret_cast<float2*>(D_s + lane * 2) = make_float2(__expf(G0), __expf(G1));
   }
   __syncthreads();
-  // ---- conv + SiLU + L2 norms -> shared memory (TF32), Qt = diag(D) Q and Kt = diag(D_C / D) K -> workspace
+  // ---- conv -> shared memory, then SiLU + L2 norms (TF32) in place, Qt = diag(D) Q and Kt = diag(D_C / D) K -> workspace.  Every lane
+  // goes over what it wrote itself, as a short loop: 96 IEEE divisions unrolled behind the convolution spilled (64 chunks of 32 heads: 257 us)
   {
     const float Gl = G_s[GC - 1];
     float4 w[4];
@@ -165,19 +167,26 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
       }
       float* dst = (part == 0 ? Qs : part == 1 ? Ks : Vs) + warp * 8 * LD128 + lane * 4;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = warp * 8 + i;
-        float4 y = r < nv ? gdn_conv(x, i, w) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(dst + i * LD128) = gdn_conv(x, i, w);
+    }
+#pragma unroll 4
+    for (int i = 0; i < 24; ++i) {
+      const int part = i >> 3, r = warp * 8 + (i & 7);
+      float4* at = reinterpret_cast<float4*>((part == 0 ? Qs : part == 1 ? Ks : Vs) + r * LD128 + lane * 4);
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);           // rows past the end stay zero, whatever eps is
+      if (r < nv) {
+        y = *at;
+        y = make_float4(silu(y.x), silu(y.y), silu(y.z), silu(y.w));
         float f = 1.f;
-        if (part < 2 && r < nv) {                           // rows past the end stay zero, whatever eps is
+        if (part < 2) {
           const float ss = warp_sum(fmaf(y.w, y.w, fmaf(y.z, y.z, fmaf(y.y, y.y, y.x * y.x))));
           f = rsqrtf(ss + eps) * (part == 0 ? rsqrtf(static_cast<float>(GD)) : 1.f);
         }
         y = scale_tf32(y, f);
-        *reinterpret_cast<float4*>(dst + i * LD128) = y;
-        if (part < 2)
-          *reinterpret_cast<float4*>(wsb + (part == 0 ? WS_QT : WS_KT) + r * GD + lane * 4) = scale_tf32(y, part == 0 ? D_s[r] : __expf(Gl - G_s[r]));
       }
+      *at = y;
+      if (part < 2)
+        *reinterpret_cast<float4*>(wsb + (part == 0 ? WS_QT : WS_KT) + r * GD + lane * 4) = scale_tf32(y, part == 0 ? D_s[r] : __expf(Gl - G_s[r]));
     }
     if (tid == 0) wsb[WS_DC] = __expf(Gl);
   }

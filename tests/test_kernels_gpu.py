@@ -325,6 +325,17 @@ def test_gdn_chunked_history_on_any_float():
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
+def test_gdn_chunked_silu_of_very_negative_values():
+    """Values whose SiLU is near the smallest normal number (1 + e^87.5 is beyond what an approximate division takes) reach the state."""
+    def fill(proj, ab, w, nq):
+        w["conv"][2 * nq:] = torch.tensor([0.0, 0.0, 0.0, 1.0], device=DEV)
+        proj[:, 2 * nq: 2 * nq + 256] = -87.5
+    (_, S0), (_, S1) = _gdn_both_forms(64, fill=fill, S0=False)
+    assert S0.norm() > 0
+    # a term below the smallest normal number (1.2e-38 beside a state of about 1e-37) may count as 0
+    assert ((S1 - S0).norm() / S0.norm()).item() < 0.1
+
+
 def test_gdn_chunked_ragged_end_without_eps():
     """Rows past the end of the last chunk are zero rows; with eps 0 they have no norm to divide by."""
     (o0, S0), (o1, S1) = _gdn_both_forms(77, eps=0.0)
