@@ -159,70 +159,73 @@ struct RouterArgs {
   int n_self; float* self_w;                 // identity experts: the last n_self outputs, their weight per row [R]
 };
 
-constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16;
+constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16, ROUTER_COLS = 4;
 
-__device__ __forceinline__ void router_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// A CTA owns 8 gate columns, its 16 warps split K: a lane takes 8 consecutive k of its row(s) and of its column as 16-byte loads
-// straight into MMA fragments (the same order of k on both sides), up to eight of them in flight, and the warps' 16 x 8 partial sums
-// meet in shared memory in warp order.  What bounds it: two memory round trips and the chain of the choices, one warp per row.
-// (Before: the rows were staged in shared memory by every CTA and each column was 16 dot products on the FP32 units of one warp, two
-// rows' choices after one another: 4 rows of 2048 and 513 columns 13.7 -> 9.0 us, 16 rows 32 -> 13, 4 rows of the MXFP4 preset 37 -> 16.)
-template <int EPL, bool HI>                                 // HI: more than 8 rows
+// A CTA owns four gate columns, a warp one of them for every fourth row (NR of them).  A lane adds the products of every 32nd 16-byte
+// vector in one 32-bit chain per row, the lanes' sums meet by shuffles: the order of a row's sum depends on neither R nor NR.  The
+// loads are 16 bytes, straight from memory, a batch of a row's and a column's vectors in flight (the rows of a CTA stay in L1).
+// What bounds it: a memory round trip per batch and the chain of the choices, one warp per row.  4 rows of 2048 and 513 columns 13.7 ->
+// 8.4 us, 16 rows 32 -> 16.7, 4 rows of the MXFP4 preset 37 -> 17 (before: a warp per column for all rows, the rows staged in shared
+// memory, two rows' choices after one another).  Tensor cores in place of the FP32 units (9.3, 13, 16 us) add 16 products at a time
+// with fewer bits: the logits' error grew 1.2 to 15 times over K = 256 .. 7168.
+template <int EPL, int NR>                                  // NR: rows of a warp (R <= 4 NR)
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
-  __shared__ float part[ROUTER_WARPS][16][8];
   __shared__ int last_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int R = a.R;
   const int NE = a.E + (a.shared_gate ? 1 : 0);
-  const int n0 = blockIdx.x * 8;
-  const int KV = a.K >> 3;                                  // 16-byte vectors of a row; a step is four of them
-  constexpr int BATCH = HI ? 4 : 8;
+  const int n = blockIdx.x * ROUTER_COLS + (warp & 3), r0 = warp >> 2;
+  const int KV = a.K >> 3;                                  // 16-byte vectors of a row
+  constexpr int BATCH = NR == 1 ? 8 : NR == 4 && EPL == 32 ? 2 : 4;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  const uint4* w = reinterpret_cast<const uint4*>(a.Wg + static_cast<size_t>(min(n0 + g, NE - 1)) * a.ldw) + t;
-  const uint4* xl = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(min(g, R - 1)) * a.ldx) + t;
-  const uint4* xh = reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(min(g + 8, R - 1)) * a.ldx) + t;
+  const uint4* w = reinterpret_cast<const uint4*>(a.Wg + static_cast<size_t>(min(n, NE - 1)) * a.ldw);
   // the gate matrix depends on no earlier launch: its first batch of loads is in flight before the dependency wait
   uint4 wv[BATCH];
 #pragma unroll
   for (int u = 0; u < BATCH; ++u) {
-    const int kv = (warp + u * ROUTER_WARPS) * 4;
-    wv[u] = kv + t < KV ? __ldg(w + kv) : zero;
+    const int kv = lane + 32 * u;
+    wv[u] = kv < KV ? __ldg(w + kv) : zero;
   }
   pdl_wait();
   pdl_trigger();
-  {
-    float d[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int s0 = warp; s0 * 4 < KV; s0 += ROUTER_WARPS * BATCH) {
-      uint4 lo[BATCH], hi[BATCH];
+  if (n < NE && r0 < R) {
+    float acc[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) acc[i] = 0.f;
+    for (int k0 = lane; k0 < KV; k0 += 32 * BATCH) {
+      uint4 xv[NR][BATCH];
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
-        const int kv = (s0 + u * ROUTER_WARPS) * 4;
-        const bool in = kv + t < KV;
-        if (s0 != warp) wv[u] = in ? __ldg(w + kv) : zero;
-        lo[u] = in ? xl[kv] : zero;
-        hi[u] = HI && in ? xh[kv] : zero;
+        const int kv = k0 + 32 * u;
+        if (k0 != lane) wv[u] = kv < KV ? __ldg(w + kv) : zero;
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          xv[i][u] = kv < KV ? reinterpret_cast<const uint4*>(a.x + static_cast<size_t>(min(r0 + 4 * i, R - 1)) * a.ldx)[kv] : zero;
       }
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
-        router_mma(d, lo[u].x, hi[u].x, lo[u].y, hi[u].y, wv[u].x, wv[u].y);
-        router_mma(d, lo[u].z, hi[u].z, lo[u].w, hi[u].w, wv[u].z, wv[u].w);
+        if (k0 + 32 * u >= KV) break;
+        const __nv_bfloat162* pw = reinterpret_cast<const __nv_bfloat162*>(&wv[u]);
+        float2 f[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = __bfloat1622float2(pw[j]);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+          const __nv_bfloat162* px = reinterpret_cast<const __nv_bfloat162*>(&xv[i][u]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 t = __bfloat1622float2(px[j]);
+            acc[i] = fmaf(f[j].x, t.x, acc[i]); acc[i] = fmaf(f[j].y, t.y, acc[i]);
+          }
+        }
       }
     }
-    *reinterpret_cast<float2*>(&part[warp][g][2 * t]) = make_float2(d[0], d[1]);
-    *reinterpret_cast<float2*>(&part[warp][g + 8][2 * t]) = make_float2(d[2], d[3]);
-  }
-  __syncthreads();
-  if (tid < 128) {
-    const int r = tid >> 3, c = tid & 7;
-    float v = 0.f;
 #pragma unroll
-    for (int i = 0; i < ROUTER_WARPS; ++i) v += part[i][r][c];
-    if (r < R && n0 + c < NE) a.logits[static_cast<size_t>(r) * a.ld + n0 + c] = v;
+    for (int i = 0; i < NR; ++i) {
+      const float v = warp_sum(acc[i]);
+      if (lane == 0 && r0 + 4 * i < R) a.logits[static_cast<size_t>(r0 + 4 * i) * a.ld + n] = v;
+    }
   }
   // ---- arrival: the last CTA to get here routes every row
   __syncthreads();
@@ -653,13 +656,14 @@ extern "C" int spark_moe_router_topk(const void* x, int ldx, const void* Wg, int
   a.wts = wts; a.ids = ids; a.pair_row = pair_row; a.sg = sg; a.counter = counter;
   const int NE = E + (shared_gate ? 1 : 0);
   // experts per lane: the narrowest form that holds E (a lane's work per choice grows with it)
-  auto pick = [&](auto hi) {
-    constexpr bool HI = decltype(hi)::value;
-    return E <= 64 ? moe_router_topk_kernel<2, HI> : E <= 256 ? moe_router_topk_kernel<8, HI>
-         : E <= 512 ? moe_router_topk_kernel<16, HI> : moe_router_topk_kernel<32, HI>;
+  auto pick = [&](auto rows) {
+    constexpr int NR = decltype(rows)::value;
+    return E <= 64 ? moe_router_topk_kernel<2, NR> : E <= 256 ? moe_router_topk_kernel<8, NR>
+         : E <= 512 ? moe_router_topk_kernel<16, NR> : moe_router_topk_kernel<32, NR>;
   };
-  void (*kern)(RouterArgs) = R > 8 ? pick(std::true_type{}) : pick(std::false_type{});
-  const cudaError_t err = spark_launch_pdl(kern, dim3((NE + 7) / 8), dim3(ROUTER_WARPS * 32), 0, s, dim3(1, 1, 1), a);
+  void (*kern)(RouterArgs) = R <= 4 ? pick(std::integral_constant<int, 1>{}) : R <= 8 ? pick(std::integral_constant<int, 2>{})
+                                    : pick(std::integral_constant<int, 4>{});
+  const cudaError_t err = spark_launch_pdl(kern, dim3((NE + ROUTER_COLS - 1) / ROUTER_COLS), dim3(ROUTER_WARPS * 32), 0, s, dim3(1, 1, 1), a);
   return err == cudaSuccess ? 0 : -4;
 }
 

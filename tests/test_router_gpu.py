@@ -35,3 +35,33 @@ def test_logits_and_choice(R, K, E, k):
     cu.check(cu.lib().spark_moe_router_topk(P(x[R - 1:]), K, P(w), K, P(alone), ld, 1, K, E, k, 0, None, 1.0, 1, k, E, 0, E, 0, 1, P(wts), P(ids),
                                             P(row), P(sg), P(counter), 0, None, cu.stream()), "router")
     assert torch.equal(alone[0, : E + 1], logits[R - 1, : E + 1])
+
+
+@pytest.mark.parametrize("R", [1, 4, 5, 9, 16])
+@pytest.mark.parametrize("K,E", [(8, 3), (2048, 512), (4104, 61), (6152, 513)])
+def test_logits_are_32_bit_chains(R, K, E):
+    """A logit is the sum the rest of the engine takes for a row: a lane's products in one 32-bit chain, the lanes pairwise.  (A product
+    of two bf16 numbers is exact in 32 bits, so the chain can be followed with plain additions.)"""
+    from spark_engine_b200.ops import cuda as cu
+    P, g = cu.P, torch.Generator(device=DEV).manual_seed(K + R)
+    x = (torch.randn(R, K, device=DEV, generator=g).abs() + 0.5).bfloat16()
+    w = torch.rand(E + 1, K, device=DEV, generator=g).bfloat16()
+    ld = (E + 8) // 8 * 8
+    logits = torch.empty(R, ld, device=DEV)
+    counter = torch.zeros(4, dtype=torch.int32, device=DEV)
+    wts, ids = torch.empty(R, 1, device=DEV), torch.empty(R, 1, dtype=torch.int32, device=DEV)
+    row, sg = torch.empty(R, 1, dtype=torch.int32, device=DEV), torch.empty(R, device=DEV)
+    cu.check(cu.lib().spark_moe_router_topk(P(x), K, P(w), K, P(logits), ld, R, K, E, 1, 0, None, 1.0, 1, 1, E, 0, E, 0, 1, P(wts), P(ids),
+                                            P(row), P(sg), P(counter), 0, None, cu.stream()), "router")
+    steps = -(-K // 256)
+    prod = torch.zeros(R, E + 1, steps * 256, device=DEV)
+    prod[..., :K] = x.float().unsqueeze(1) * w.float()
+    prod = prod.view(R, E + 1, steps, 32, 8)
+    acc = torch.zeros(R, E + 1, 32, device=DEV)
+    for s in range(steps):
+        for j in range(8):
+            acc = acc + prod[:, :, s, :, j]
+    while acc.shape[-1] > 1:
+        h = acc.shape[-1] // 2
+        acc = acc[..., :h] + acc[..., h:]
+    assert torch.equal(logits[:, : E + 1], acc[..., 0])
