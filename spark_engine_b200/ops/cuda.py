@@ -483,7 +483,8 @@ def exl3_tc(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, glu: Opti
     Pn, K = xh.shape
     n = w.n // 2 if glu is not None else w.n
     y = torch.empty(Pn, n, dtype=torch.float16 if glu is not None else torch.float32 if out_f32 else torch.bfloat16, device=xh.device)
-    rc = lib().spark_exl3_tc(P(xh), xh.stride(0), Pn, P(w.trellis), P(w.svh), (K // 16) * (w.n // 16) * 32, w.n,
+    t = w.trellis if P(w.trellis) % 16 == 0 else w.trellis.clone()      # the kernel's bulk copies start on 16 bytes
+    rc = lib().spark_exl3_tc(P(xh), xh.stride(0), Pn, P(t), P(w.svh), (K // 16) * (w.n // 16) * 32, w.n,
                              P(glu.suh) if glu is not None else None, n, P(tiles), P(ntile), max_tiles, P(y), n, int(out_f32), K, w.n,
                              int(glu is not None), float(limit), 0 if w.kind == "mul1" else 1, P(status_word(xh.device)), stream())
     check(rc, "spark_exl3_tc")

@@ -77,3 +77,13 @@ def test_gathered_input_rows():
     e = ids.view(-1)[perm.long()].clamp_min(0).long()
     ref = _had(x[perm.long() // k].double() * w.suh[e].double())
     assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -11                      # fp16 rounding of the result
+
+
+def test_trellis_on_any_word():
+    """Experts whose packed words start on 4 bytes only (a view of a larger buffer) give the bits of ones on 16."""
+    cu, w, ids, tiles, ntile, max_tiles, g = _setup([17, 40], 256, 384, "mul1")
+    x = torch.randn(len(ids), 256, device=DEV, generator=g).half()
+    y = cu.exl3_tc(x, w, tiles, ntile, max_tiles)
+    buf = torch.empty(w.trellis.numel() + 2, dtype=w.trellis.dtype, device=DEV)
+    moved = Q.Exl3Weight(buf[2:].view(w.trellis.shape).copy_(w.trellis), w.suh, w.svh, 4, w.kind)
+    assert torch.equal(cu.exl3_tc(x, moved, tiles, ntile, max_tiles), y)
