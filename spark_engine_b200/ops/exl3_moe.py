@@ -17,7 +17,15 @@ from . import cuda as cu
 
 
 EXL3_MOE_FUSED = os.environ.get("SPARK_EXL3_MOE_FUSED", "1") == "1"
-F32_MAX_ROWS_PER_EXPERT = 48   # average rows per expert up to which the down rows stay fp32 until they are combined
+# Average rows per expert up to which the down rows stay fp32 until they are combined; beyond, the second half of their bytes is what
+# a prompt would pay for precision that the bf16 result does not keep.  fp32 / bf16, us of a sublayer of 512 experts of 2048 x 512, top
+# 10: 1021 rows 632 / 628, 2048 rows 741 / 735 (here 48 per expert are 2457 rows), 4096 rows 1125 / 1106, 8192 rows 2080 / 2046.
+F32_MAX_ROWS_PER_EXPERT = 48
+
+
+def down_rows_f32(pairs: int, c) -> bool:
+    """`pairs`: routed pairs of all ranks, so the experts of all ranks are what they spread over."""
+    return pairs <= F32_MAX_ROWS_PER_EXPERT * c.n_experts
 
 
 def exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c):
@@ -28,7 +36,7 @@ def exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c):
     xh = cu.exl3_had_gather(h, wgu.suh, perm, ids, H)
     if EXL3_MOE_FUSED and wgu.bits == 4 and wd.bits == 4:
         xh2 = cu.exl3_tc(xh, wgu, tiles, ntile, max_tiles, glu=wd, limit=c.swiglu_limit)
-        return cu.exl3_tc(xh2, wd, tiles, ntile, max_tiles, out_f32=xh.shape[0] <= F32_MAX_ROWS_PER_EXPERT * E)
+        return cu.exl3_tc(xh2, wd, tiles, ntile, max_tiles, out_f32=down_rows_f32(xh.shape[0], c))
     # rows past this rank's pairs are filler (perm 0): their expert id may be -1 (non-local) -> clamp, they are
     # never part of a tile and never combined
     row_expert = ids.view(-1)[perm.long()].clamp_min(0).to(torch.int32).contiguous()

@@ -87,3 +87,31 @@ def test_trellis_on_any_word():
     buf = torch.empty(w.trellis.numel() + 2, dtype=w.trellis.dtype, device=DEV)
     moved = Q.Exl3Weight(buf[2:].view(w.trellis.shape).copy_(w.trellis), w.suh, w.svh, 4, w.kind)
     assert torch.equal(cu.exl3_tc(x, moved, tiles, ntile, max_tiles), y)
+
+
+@pytest.mark.parametrize("R,dtype", [(96, torch.float32), (97, torch.bfloat16)])
+@pytest.mark.parametrize("local", [8, 4])
+def test_down_rows_on_both_sides_of_the_format(R, dtype, local):
+    """The down rows are fp32 up to 48 pairs per expert of the model (8 experts, top 4: 96 rows), on a rank that holds half of the
+    experts as on one that holds all; either way they are the products of their experts."""
+    from spark_engine_b200.config import MoeConfig
+    from spark_engine_b200.ops import exl3_moe
+    from spark_engine_b200.ops import cuda as cu
+    g = torch.Generator(device=DEV).manual_seed(R)
+    E, k, H, F = 8, 4, 256, 128
+    c = MoeConfig(n_experts=E, top_k=k, ffn=F)
+    wgu, wd = Q.random_exl3(2 * F, H, 4, local, 0.05, 1, DEV), Q.random_exl3(H, F, 4, local, 0.05, 2, DEV)
+    h = torch.randn(R, H, device=DEV, generator=g).bfloat16()
+    ids = torch.rand(R, E, device=DEV, generator=g).topk(k, -1).indices.int()
+    ids = torch.where(ids < local, ids, -1)                        # the others live on another rank
+    perm, inv, offs, tiles, ntile, max_tiles = cu.moe_sort(ids.view(-1), local)
+    y = exl3_moe.exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
+    assert y.dtype == dtype and cu.read_status(torch.device(DEV))[0] == 0
+    for e in range(local):
+        pairs = (ids.view(-1) == e).nonzero()[:, 0]
+        x = _had(h[pairs // k].double() * wgu.suh[e].double()).half()
+        a, u = _product(x, wgu, e).chunk(2, -1)
+        z = _had(torch.nn.functional.silu(a) * u * wd.suh[e].double())
+        ref = _product(z, wd, e)
+        err = ((y[inv[pairs].long()].double() - ref).norm() / ref.norm()).item()
+        assert err < 2.0 ** -7.5, (e, err)                        # roundings of the gated rows (three in bf16, one in fp16) and of the result
