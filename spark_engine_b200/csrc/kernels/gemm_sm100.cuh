@@ -135,8 +135,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int s0 = tc.a_row0 / g.ag_rows, s1 = min(g.ag_world - 1, (tc.a_row0 + GEMM_BM - 1) / g.ag_rows);
         for (int src = s0; src <= s1 && ok; ++src) {
           if (src == g.ag_rank || (ag_seen >> src) & 1u) continue;
-          CommCtx cc; cc.wait_ns = g.ag_wait_ns; cc.status = g.status;
-          ok = __all_sync(0xffffffffu, wait_flag(cc, g.ag_flags + src, ag_seq, src));
+          if (lane == 0) {                  // one system-scope poll a CTA; the others take its answer (and what it acquired) below
+            CommCtx cc; cc.wait_ns = g.ag_wait_ns; cc.status = g.status;
+            ok = wait_flag(cc, g.ag_flags + src, ag_seq, src);
+          }
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          __syncwarp();
           if (!ok) break;
           ag_seen |= 1u << src;
           asm volatile("fence.proxy.async;" ::: "memory");   // peer's generic-proxy stores -> our TMA reads
