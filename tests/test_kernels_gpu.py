@@ -304,6 +304,21 @@ def _gdn_both_forms(rows, eps=1e-6, fill=None, S0=True):
     return outs
 
 
+@pytest.mark.parametrize("rows", [64, 200])
+@pytest.mark.parametrize("noise", [0.0, 0.05, 0.5])
+def test_gdn_chunked_correlated_keys(rows, noise):
+    """Keys that are nearly the same, written with strength near 1 and hardly forgotten: I + A is close to a full triangle of ones,
+    where the inverse lives on cancellation between its blocks."""
+    def fill(proj, ab, w, nq):
+        g = torch.Generator(device=DEV).manual_seed(17)
+        base = torch.randn(1, 2 * nq, device=DEV, generator=g) + 1
+        proj[:, : 2 * nq] = (base + noise * torch.randn(rows, 2 * nq, device=DEV, generator=g)).bfloat16()
+        ab[:, :2] = 6.0
+        w["A_log"].fill_(-6.0)
+    (o0, S0), (o1, S1) = _gdn_both_forms(rows, fill=fill)
+    assert rel_err(o1, o0) < 1e-2 and rel_err(S1, S0) < 5e-3
+
+
 def test_gdn_chunked_history_on_any_float():
     """A history of earlier inputs that does not start on 16 bytes (views of a larger buffer) gives the bits of one that does."""
     import dataclasses

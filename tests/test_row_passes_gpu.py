@@ -136,5 +136,14 @@ def test_route(E, k, kind, R):
         assert torch.allclose(wts.double(), w, rtol=1e-4, atol=1e-6)
         if kind != 5:
             assert torch.allclose(sw.double(), (w * (ref >= E - n_self)).sum(-1), rtol=1e-4, atol=1e-6)
+    else:                                                          # the scores are rounded, so near-ties may fall either way: the weights
+        num = torch.gather(p, 1, full)                             # of the experts that were chosen, from p without the bias
+        if not own.any():
+            assert torch.allclose(wts.double(), num / num.sum(-1, keepdim=True).clamp_min(1e-20) * 1.5, rtol=1e-4, atol=1e-6)
+        else:                                                      # an identity expert's number is not in `ids`: ratios of the others
+            a, b = torch.where(own, 0.0, wts.double()), torch.where(own, 0.0, num)
+            assert torch.allclose(a * b.sum(-1, keepdim=True), b * a.sum(-1, keepdim=True), rtol=1e-4, atol=1e-6)
+    if kind != 4:                                                  # what the other experts leave of the whole is the identity experts'
+        assert torch.allclose(sw.double(), 1.5 - torch.where(own, 0.0, wts.double()).sum(-1), rtol=1e-4, atol=1e-5)
     assert torch.equal(row, torch.arange(R, device=DEV, dtype=torch.int32).unsqueeze(1).expand(R, k))
     assert torch.allclose(sg, torch.sigmoid(x[:, E]), rtol=1e-5, atol=1e-6)
