@@ -22,7 +22,7 @@
 
 namespace spark {
 
-int make_tmap_rows64(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
+int make_tmap_bf16(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
 
 constexpr int PF_BM = 128, PF_BN = 64, PF_WARPS = 8, PF_THREADS = PF_WARPS * 32;
 
@@ -46,24 +46,6 @@ struct PrefillArgs {
   int* status;
 };
 
-__device__ __forceinline__ void pf_mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void pf_tmem_st_x32(uint32_t addr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
-        "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
-}
-__device__ __forceinline__ void pf_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t pf_pack(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -188,7 +170,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const uint64_t kd = make_smem_desc_sw128(rs + slot * SLOT + c * KV_CHUNK);
             if (L::QT) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) pf_mma_ts(tm + L::S_COL, tm + L::Q_COL + c * 32 + k * 8, kd + 2 * k, id_s, (c | k) != 0);
+              for (int k = 0; k < 4; ++k) umma_f16_ts(tm + L::S_COL, tm + L::Q_COL + c * 32 + k * 8, kd + 2 * k, id_s, (c | k) != 0);
             } else {
               const uint64_t qd = make_smem_desc_sw128(qs + c * Q_CHUNK);
 #pragma unroll
@@ -209,7 +191,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint32_t p = tm + L::P_COL + (j & 1) * 32;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          pf_mma_ts(tm + O_COL, p + k * 8, pf_desc_nmajor(rs + slot * SLOT + k * 2048, KV_CHUNK), id_o, (j | k) != 0);
+          umma_f16_ts(tm + O_COL, p + k * 8, pf_desc_nmajor(rs + slot * SLOT + k * 2048, KV_CHUNK), id_o, (j | k) != 0);
         umma_commit(&empty[slot]);
         umma_commit(&o_full[j & 1]);
       }
@@ -232,9 +214,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint4 v = __ldg(qp + c / 4 + i);
           w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
         }
-        pf_tmem_st_x32(t_lane + L::Q_COL + c, w);
+        tmem_st_32x32(t_lane + L::Q_COL + c, w);
       }
-      pf_tmem_st_wait();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(q_full);
@@ -304,7 +286,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         ok = __all_sync(0xffffffffu, mbar_wait(&o_full[j & 1], ((j - 2) >> 1) & 1));
         if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
       }
-      pf_tmem_st_x32(t_lane + L::P_COL + (j & 1) * 32, p);
+      tmem_st_32x32(t_lane + L::P_COL + (j & 1) * 32, p);
       if (rescale) {                                           // behind the exponentials: the product before has finished by now
         ok = __all_sync(0xffffffffu, mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1));
         if (!ok) { set_status(a.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, j); break; }
@@ -320,11 +302,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             o[0][i] = __float_as_uint(__uint_as_float(o[0][i]) * c);
             o[1][i] = __float_as_uint(__uint_as_float(o[1][i]) * c);
           }
-          pf_tmem_st_x32(t_lane + O_COL + cc, o[0]);
-          pf_tmem_st_x32(t_lane + O_COL + cc + 32, o[1]);
+          tmem_st_32x32(t_lane + O_COL + cc, o[0]);
+          tmem_st_32x32(t_lane + O_COL + cc + 32, o[1]);
         }
       }
-      pf_tmem_st_wait();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[j & 1]);
@@ -390,11 +372,11 @@ template <int D, bool MASK>
 static int launch_prefill(int R, long long tokens, int nseg, int max_rows, const PrefillArgs& a, cudaStream_t s) {
   CUtensorMap tq, tk, tv, tk8, tv8;
   const uint64_t wq = static_cast<uint64_t>(a.Hq) * D, wk = static_cast<uint64_t>(a.Hkv) * D;
-  if (int r = make_tmap_rows64(&tq, a.q, R, wq, wq, PF_BM, 1)) return r;
-  if (int r = make_tmap_rows64(&tk, a.k, tokens, wk, wk, PF_BN, 1)) return r;
-  if (int r = make_tmap_rows64(&tv, a.v, tokens, wk, wk, PF_BN, 1)) return r;
-  if (int r = make_tmap_rows64(&tk8, a.k, tokens, wk, wk, 8, 1)) return r;
-  if (int r = make_tmap_rows64(&tv8, a.v, tokens, wk, wk, 8, 1)) return r;
+  if (int r = make_tmap_bf16(&tq, a.q, R, wq, wq, PF_BM, 1)) return r;
+  if (int r = make_tmap_bf16(&tk, a.k, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_bf16(&tv, a.v, tokens, wk, wk, PF_BN, 1)) return r;
+  if (int r = make_tmap_bf16(&tk8, a.k, tokens, wk, wk, 8, 1)) return r;
+  if (int r = make_tmap_bf16(&tv8, a.v, tokens, wk, wk, 8, 1)) return r;
   auto kern = attn_prefill_kernel<D, MASK>;
   static bool done = false;
   if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Pf<D>::SMEM); done = true; }

@@ -20,7 +20,7 @@
 
 namespace spark {
 
-int make_tmap_rows64(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
+int make_tmap_bf16(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt);
 
 struct Exl3TcArgs {
   const uint32_t* trellis; long long t_stride;        // [E][K/16][N/16][32] words
@@ -37,33 +37,6 @@ constexpr int TC_B_BYTES = 128 * 128, TC_T_BYTES = 4 * 16 * 128, TC_STAGE = TC_B
 constexpr int TC_XP = 2 * 16 * 256 * 4;               // epilogue exchange: two buffers of 16 rows x 256 columns
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE + TC_XP + 256 + 1024;
 constexpr int TC_A_COLS = 64, TC_A_BUFS = 4, TC_D_COLS = 256;
-
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void umma_f16_ta(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_st_x16(uint32_t addr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld_x16(uint32_t addr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(addr) : "memory");
-}
 
 // Accumulator halves an item takes, the same sequence in the MMA and the epilogue role: an item of <= 64 rows takes the next
 // half, a larger one both.
@@ -177,8 +150,8 @@ exl3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            umma_f16_ta(d0, ta + k * 16, bd + 2 * k, idesc, (s | k) != 0);
-            umma_f16_ta(d1, ta + k * 16 + 8, bd + 2 * k, idesc, (s | k) != 0);
+            umma_f16_ts(d0, ta + k * 16, bd + 2 * k, idesc, (s | k) != 0);
+            umma_f16_ts(d1, ta + k * 16 + 8, bd + 2 * k, idesc, (s | k) != 0);
           }
           umma_commit(&empty[st]);
           umma_commit(&a_empty[ab]);
@@ -231,8 +204,8 @@ exl3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
       }
       for (int c = 0; c < it.n; c += 16) {
         uint32_t v0[16], v1[16];
-        tmem_ld_x16(d0 + c, v0);
-        tmem_ld_x16(d1 + c, v1);
+        tmem_ld_32x16(d0 + c, v0);
+        tmem_ld_32x16(d1 + c, v1);
         tmem_ld_wait();
         if (c + 16 >= it.n) {                                 // last columns read: the accumulator may be overwritten
           tc_fence_before();
@@ -310,7 +283,7 @@ exl3_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
         ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[ab], aph ^ 1));
         if (!ok) { set_status(a.status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, t, s); break; }
         tc_fence_after();
-        tmem_st_x16(ta + ab * TC_A_COLS, r);
+        tmem_st_32x16(ta + ab * TC_A_COLS, r);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -353,7 +326,7 @@ extern "C" int spark_exl3_tc(const void* xh, int ldx, int P, const void* trellis
   if ((K & 127) || (N & 127) || K <= 0 || N <= 0 || (ldx & 7) || (ldy & 3) || (glu && (N & 255))) return -5;
   if (reinterpret_cast<uintptr_t>(trellis) & 15) return -5;
   CUtensorMap tm;
-  if (int r = make_tmap_rows64(&tm, xh, P, K, ldx, 32, 0)) return r;
+  if (int r = make_tmap_bf16(&tm, xh, P, K, ldx, 32, 0)) return r;
   Exl3TcArgs a;
   a.trellis = (const uint32_t*)trellis; a.t_stride = t_stride_words; a.svh = (const __half*)svh; a.svh_stride = svh_stride;
   a.suh2 = (const __half*)suh2; a.suh2_stride = suh2_stride; a.tiles = (const int4*)tiles; a.ntile = ntile;

@@ -37,10 +37,6 @@ int make_tmap_bf16(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, 
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-int make_tmap_rows64(CUtensorMap* m, const void* base, uint64_t rows, uint64_t K, uint64_t ld, int box_rows, int fmt) {
-  return make_tmap_bf16(m, base, rows, K, ld, box_rows, fmt);
-}
-
 static int num_sms() {
   static int n = 0;
   if (!n) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
