@@ -157,7 +157,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {         // whole 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; one thread issues.
+// D[tmem] (+)= A[smem desc] * B[smem desc]; one lane issues (an elected one of a whole warp keeps the operands in uniform registers).
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(

@@ -73,8 +73,7 @@ __global__ void exl3_reconstruct_bits_kernel(const uint32_t* __restrict__ trelli
 // y[r, :] = had128(x[r, :] * scale[:]) (pre) or had128(x[r, :]) * scale[:] (post); 128-blocks along the row.
 // Eight lanes per 128-block, four blocks per warp: a lane moves 16 consecutive elements as 16-byte vectors.  With one block per
 // warp (four elements a lane, five shuffle stages, an index division per 128 elements) the pass was bound by issue and shuffles:
-// 4096 rows of 12288
-// and of 2048 columns out (fp32 -> bf16) 99 -> 74 us, 4096 rows in (bf16 -> fp16) 21 -> 13 us.
+// 4096 rows of 12288 and of 2048 columns out (fp32 -> bf16) 96 -> 75 us, 4096 rows in (bf16 -> fp16) 21 -> 13 us.
 __device__ __forceinline__ void ld16(const float* p, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

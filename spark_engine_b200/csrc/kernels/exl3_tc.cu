@@ -13,8 +13,11 @@
 // run the epilogue (TMEM -> shared memory -> output Hadamard per row, one warp per 128-block).  Items of <= 64 rows use half of
 // the accumulator columns each, so that one item's epilogue overlaps the next one's products.
 //
-// What bounds it: the decode.  A word of 8 weights costs about 35 instructions, of which 8 multiplies and 8 byte sums go through
-// the half-rate FMA-heavy pipe and 15 through the half-rate ALU pipe; the MMAs of an item hide behind it up to 128 rows.
+// What bounds it: the decode takes half of the time or less.  A word of 8 weights costs about 35 instructions, of which 8 multiplies
+// and 8 byte sums go through the half-rate FMA-heavy pipe and 15 through the half-rate ALU pipe: 194 us of issue for 512 experts of
+// 2048 x 512, once, of the 271 + 147 measured at 1021 rows.  The rest is each decoder's chain per 64 k (wait, load, decode, wait, store,
+// wait, arrive; four warps a scheduler in step).  8192 rows decode twice, 390 us of 861 + 550: items of more than 64 rows take both
+// accumulator halves, so that nothing runs beside their epilogue, in which four warps transform a row at a time.
 // Reference: engine-rs/shim/moe_exl3.cuh:521-1233 (gemm_grouped / gux / gu2 kernels, mma.sync m16n8k16).
 #include "exl3_common.cuh"
 

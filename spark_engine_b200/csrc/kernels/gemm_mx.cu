@@ -2,12 +2,13 @@
 // 32 elements along K for every row of A and of B (MXFP8), accumulated in fp32 in TMEM.  The scales are applied by the
 // tensor core itself (`tcgen05.mma.kind::mxf8f6f4.block_scale`): no dequantised copy of the weights ever exists.
 //
-// Same skeleton as the bf16 GEMM (persistent CTAs, warp 0 = TMA producer, warp 1 = one-thread MMA issuer, warps 2..5 =
-// epilogue, 128-byte-swizzled K-major tiles, two TMEM accumulator stages), plus the scale-factor path:
+// Same skeleton as the bf16 GEMM (persistent CTAs, warp 0 = TMA producer, warp 1 = MMA issuer, both as whole warps of which one
+// elected lane issues, warps 2..5 = epilogue, 128-byte-swizzled K-major tiles, two TMEM accumulator stages), plus the
+// scale-factor path:
 //   * scales live in global memory in the layout the tensor core wants, one 512-byte block per (128 rows, 128 k):
 //     byte (row % 32) * 16 + (row / 32) * 4 + (k / 32) % 4  (act_quant / weight preparation write this directly);
 //   * the producer fetches the block of A and of B with a bulk copy onto the stage's full barrier;
-//   * the MMA thread copies both blocks to tensor memory (`tcgen05.cp.32x128b.warpx4`: 32 rows x 16 bytes, replicated
+//   * the MMA warp copies both blocks to tensor memory (`tcgen05.cp.32x128b.warpx4`: 32 rows x 16 bytes, replicated
 //     to the four lane quadrants) and issues four K=32 MMAs per stage whose descriptors select scale byte 0..3.
 // Tile 128 x 128 x 128 bytes of K; TMEM: 2 x 128 accumulator columns + 8 scale columns per stage.
 // Every wait is bounded (status word + normal teardown).  Reference paths replaced: engine-rs/shim/ds41_mx.cu

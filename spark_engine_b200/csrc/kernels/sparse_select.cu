@@ -530,7 +530,10 @@ extern "C" int spark_topk_select(const float* score, int ld, const int* pos, int
                                  int sel_ld, int* sel_n, cudaStream_t s, int window) {
   if (R <= 0) return 0;
   if (sel_ld < k * block + block + window || window < 0) return -5;
-  // 256 threads once eight such CTAs per SM have rows, and a few rounds of 1024 candidates cover a row (ld: blocks of the longest)
+  // 256 threads once two such CTAs per SM have rows, and a few rounds of 1024 candidates cover a row (ld: blocks of the longest).
+  // 1024 / 256 threads, us: 148 rows of 1000 7.3 / 5.8, of 4096 7.7 / 13.5; 296 rows of 1000 9.7 / 6.3, of 2000 10.0 / 9.5, of 4096
+  // 10.6 / 14.8; 592 rows of 4096 19.6 / 20.5; 1000 rows of 1000 29 / 12, of 8192 65 / 62; 4096 rows of 1000 110 / 33, of 8192 250 / 194.
+  // (So a few hundred rows of more than 2000 pay 4 us, and 4096 rows of 12000, which stay with 1024, would take 272 instead of 342.)
   if (R >= 2 * 148 && ld <= 8192) topk_select_kernel<256><<<R, 256, 0, s>>>(score, ld, pos, block, k, window, sel, sel_ld, sel_n);
   else topk_select_kernel<1024><<<R, 1024, 0, s>>>(score, ld, pos, block, k, window, sel, sel_ld, sel_n);
   return spark_launch_rc(__func__);

@@ -1,9 +1,10 @@
 """Device ops for the micro-scaled weight formats (FP8 128x128-block dense weights, MXFP4 experts).
 
-Decode / verify rows (<= 16) and MoE (expert,row) pairs stream the packed weights through the tensor-core
-GEMV of `csrc/kernels/mx.cu`; prefill-size batches convert the weights to bf16 once per call and run the
-tcgen05 GEMM (dense) or the grouped tcgen05 GEMM over the ragged expert tile list.  Activation
-quantisers (FP8 1x128, MXFP8 1x32) are exposed for the block-scaled paths and the FP8 KV / latent stores.
+Decode / verify rows (<= 16) of dense weights stream the packed weights through the tensor-core GEMV of `csrc/kernels/mx.cu`.
+Longer batches of MXFP8 weights quantise the activations to MXFP8 and run the block-scaled tcgen05 GEMM, MXFP4 experts the grouped
+one (`gemm_mx.cu`) for decode pairs and prompts alike: neither decodes a copy of the weights.  FP8-block and dense MXFP4 weights
+are converted to bf16 once per call for longer batches; experts of other widths or formats take the warp-level kernel or that
+conversion.  Activation quantisers (FP8 1x128, MXFP8 1x32) are exposed for the block-scaled paths and the FP8 KV / latent stores.
 Reference: engine-rs/shim/ds41_mx.cu (fp8_gemv_mx, up_mx/down_mx, up_gemm/down_gemm, act_quant),
 fp8.cu / fp8ws.cu, engine-rs/src/ds41/load.rs:116-160.
 """
