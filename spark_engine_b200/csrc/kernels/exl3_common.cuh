@@ -62,6 +62,14 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// the same from zero
+__device__ __forceinline__ void mma_f16_16816_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // 128-point Walsh-Hadamard (unnormalised) held by one warp: lane l owns elements 4l..4l+3.
 __device__ __forceinline__ void fwht128_warp(float (&v)[4], int lane) {
   float a = v[0] + v[1], b = v[0] - v[1], c = v[2] + v[3], d = v[2] - v[3];
@@ -80,18 +88,36 @@ __device__ __forceinline__ void fwht128_warp(float (&v)[4], int lane) {
 // The same transform of one 128-block by eight lanes: lane l & 7 owns elements 16 (l & 7) .. + 15.  Strides 1 .. 8 stay in the lane
 // and only three cross lanes, 0.38 shuffles per element instead of 0.63; a stage is one shuffle and one exact fused multiply-add
 // (by +-1).  Same pairs in the same order as fwht128_warp, so the same bits.
+// Pairs of elements go through packed 32-bit additions and multiply-adds (one instruction each, rounded like single ones).
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
 __device__ __forceinline__ void fwht128_oct(float (&v)[16], int lane) {
+  const uint64_t minus = f2_pack(-1.f, -1.f);
+  uint64_t p[8];
 #pragma unroll
-  for (int st = 1; st < 16; st <<= 1)
+  for (int i = 0; i < 8; ++i) p[i] = f2_pack(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (!(i & st)) { const float a = v[i], b = v[i | st]; v[i] = a + b; v[i | st] = a - b; }
+  for (int st = 1; st < 8; st <<= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (!(i & st)) { const uint64_t a = p[i], b = p[i | st]; p[i] = f2_add(a, b); p[i | st] = f2_fma(b, minus, a); }
 #pragma unroll
   for (int m = 1; m < 8; m <<= 1) {
     const float sg = (lane & m) ? -1.f : 1.f;
+    const uint64_t sg2 = f2_pack(sg, sg);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = fmaf(sg, v[i], __shfl_xor_sync(0xffffffffu, v[i], m));
+    for (int i = 0; i < 8; ++i) {
+      float a, b;
+      f2_unpack(p[i], a, b);
+      p[i] = f2_fma(sg2, p[i], f2_pack(__shfl_xor_sync(0xffffffffu, a, m), __shfl_xor_sync(0xffffffffu, b, m)));
+    }
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f2_unpack(p[i], v[2 * i], v[2 * i + 1]);
 }
 
 }  // namespace spark

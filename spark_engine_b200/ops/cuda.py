@@ -392,21 +392,28 @@ def dense_linear(x: torch.Tensor, w: torch.Tensor, out_f32: bool = False, out=No
 
 
 # ----------------------------------------------------------------------------- EXL3
-def _pick_slices(K: int, items: int = 1) -> int:
-    """K-slices per 128-column strip = CTAs of one cluster (<= 8): aim at 256-deep slices so that one
-    batch of loads per warp covers the whole slice.  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS force the count for
-    single-matrix / per-pair launches."""
+EXL3_CTAS = 5 * 148                # CTAs of the EXL3 GEMV that run at a time
+
+
+def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> int:
+    """K-slices per 128-column strip = CTAs of one cluster (<= 8).  Rows of one matrix (summed slice by slice, so that S may
+    depend on K and N only): as many as run at a time.  `pairs` of a row and an expert (summed in chunks of 256, whatever S is): the same for all
+    `items`, and further while a slice keeps 1024 k and two waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048 24.5 / 16.3 / 12.7 / 11.6, 40 pairs 33.7 / 29.1 /
+    29.4 / 34.0, 160 pairs 85 / 86 / 96 / 120; 40 pairs of 2048 x 512 17.6 / 21.0 / 28.9; 16 pairs of 3072 x 4096 - / 62.7 / 58.8 / 61.7; one row
+    of 12288 x 2048 15.1 / 12.8 / 10.6 / 11.7.  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS force the count for single-matrix / per-pair launches."""
     blocks = K // 128
-    forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if items > 1 else "SPARK_EXL3_S", "0"))
+    forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if pairs else "SPARK_EXL3_S", "0"))
     if forced and blocks % forced == 0:
         return forced
-    best = 1
+    unit = 2 if pairs and blocks % 2 == 0 else 1
+    strips = N // 128 * (items if pairs else 1)
+    best = 0
     for s in range(1, 9):
-        if blocks % s == 0 and K // s >= 128:
+        if blocks % (s * unit) or K // s > 2048:
+            continue
+        if not best or strips * s <= EXL3_CTAS or (pairs and K // s >= 1024 and strips * s <= 2.2 * EXL3_CTAS):
             best = s
-            if K // s <= 256:
-                break
-    return best
+    return best or 1
 
 
 def exl3_gemv(x, w: Exl3Weight, items=1, rows_per_item=None, pair_expert=None, pair_row=None, act=0, limit=0.0,
@@ -419,7 +426,7 @@ def exl3_gemv(x, w: Exl3Weight, items=1, rows_per_item=None, pair_expert=None, p
     if dbg.CHECK:
         dbg.check_index("exl3_gemv pair_expert", pair_expert, 0, w.trellis.shape[0] if w.experts else 1, allow=-1, count=items)
         dbg.check_index("exl3_gemv pair_row", pair_row, 0, x.shape[0], count=items)
-    S = _pick_slices(K, items)
+    S = _pick_slices(K, items, N, pair_expert is not None and rows_per_item == 1)
     dev = x.device
     y = torch.empty(items * rows_per_item, N, dtype=torch.float32 if out_f32 else torch.bfloat16, device=dev)
     tw = (K // 16) * (N // 16) * 32

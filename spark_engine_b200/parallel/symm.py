@@ -264,7 +264,7 @@ class FusedAllReduce:
         R = x.shape[0]
         out = torch.empty(R, self.N, dtype=out_dtype, device=x.device)
         ar = self._args(R, None, res, norm_w, eps, out)
-        S = cu._pick_slices(w.k)
+        S = cu._pick_slices(w.k, N=w.n)
         rc = cu.lib().spark_exl3_gemv(cu.P(x), x.stride(0), cu.P(w.trellis), cu.P(w.suh), cu.P(w.svh), 0, 0, 0, None,
                                       self.N, 0, None, None, 1, R, w.k, w.n, S, act, float(limit),
                                       0 if w.kind == "mul1" else 1, cu.stream(), C.addressof(ar), 0)
