@@ -429,15 +429,15 @@ extern "C" int spark_attn_prefill(const void* qbuf, const void* kc, const void* 
   return prefill<false>(R, tokens, nseg, max_rows, D, a, s);
 }
 
-// The same tiles for rows with a block-sparse selection (4-token blocks): sel / sel_n are the per-row token lists of the
-// selection kernels (R rows, plan order), bmask a scratch of R * mw words with mw >= ceil(max context / 128).
+// The same tiles for rows with a block-sparse selection (4-token blocks): bmask [R, mw] has a bit per block (mw >= ceil(max context / 128)),
+// as spark_topk_mask leaves it; with sel / sel_n (per-row token lists, plan order) it is scratch and made from them.
 extern "C" int spark_attn_prefill_masked(const void* qbuf, const void* kc, const void* vc, const long long* row_kv,
                                          const int* seg, int nseg, int max_rows, const void* qkv, int ld, int gated, void* out,
                                          int Hq, int Hkv, int D, float scale, const int* sel, const int* sel_n, int sel_ld,
                                          int R, unsigned* bmask, int mw, long long tokens, int* status, cudaStream_t s) {
   if (nseg <= 0 || max_rows <= 0 || R <= 0) return 0;
-  if (mw <= 0 || mw > 8192 || !sel || !sel_n || !bmask) return -5;
-  sel_blockmask_kernel<<<R, 256, mw * 4, s>>>(sel, sel_n, sel_ld, bmask, mw);
+  if (mw <= 0 || mw > 8192 || (sel && !sel_n) || !bmask) return -5;
+  if (sel) sel_blockmask_kernel<<<R, 256, mw * 4, s>>>(sel, sel_n, sel_ld, bmask, mw);
   const PrefillArgs a{(const __nv_bfloat16*)qbuf, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, row_kv, seg, (const __nv_bfloat16*)qkv, ld, gated, (__nv_bfloat16*)out, Hq, Hkv, scale * 1.4426950408889634f,
                       bmask, mw, status};
   return prefill<true>(R, tokens, nseg, max_rows, D, a, s);

@@ -9,34 +9,70 @@
 // are >= 0, so their bit patterns sort like unsigned integers), one CTA per row.
 // Reference: engine-rs/shim/qwen_qsa.cu:903-1076 (score_kernel, select_kernel), topk_select.cuh,
 // dataflow.cu:159-336 (dsa_score*), dsa_index.cu:225 (dsa_topk_rows).
-#include "../common/ptx.cuh"
+#include "../common/decode.cuh"
 
 namespace spark {
 
-// grid (ceil(nb_max/8), R), 256 threads: warp w of CTA x scores block x*8+w.  idx_dim <= 128 (4 dims per lane).
+// grid (ceil(nb_max / 32), R), 256 threads: a warp scores four blocks.  idx_dim <= 128: a lane has four dimensions.  Four blocks by four
+// heads are sixteen sums over the lanes, which are folded together: each step halves the sums a lane carries, 16 shuffles where sixteen
+// butterflies take 80, the same pairs in the same order.  What bounds it: the chain position -> keys -> queries -> folds (a warp per block:
+// two waves of CTAs, 8.7 us for 4 rows of 4000 blocks, 4 heads of 128).  vec: rows of `pool` and `qi` start on 16 bytes.
+constexpr int IDX_B = 4;
+
+__device__ __forceinline__ float4 idx_ld4(const float* p, int lane, int Dm, int vec) {
+  const int i = lane * 4;
+  if (vec) return i < Dm ? __ldg(reinterpret_cast<const float4*>(p + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(i < Dm ? p[i] : 0.f, i + 1 < Dm ? p[i + 1] : 0.f, i + 2 < Dm ? p[i + 2] : 0.f, i + 3 < Dm ? p[i + 3] : 0.f);
+}
+
 __global__ void __launch_bounds__(256)
 idx_score_kernel(const float* __restrict__ qi, int H, int Dm, const float* __restrict__ pool, const long long* __restrict__ row_kv,
                  const int* __restrict__ pos, int block, const float* __restrict__ head_w, float scale,
-                 float* __restrict__ score, int ld) {
+                 float* __restrict__ score, int ld, int vec) {
+  pdl_wait();
+  pdl_trigger();
   const int r = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * 8 + warp;
+  const int b0 = (blockIdx.x * 8 + warp) * IDX_B;
   const int vis = (pos[r] + 1) / block;
-  if (b >= vis) return;
-  const float* kc = pool + (row_kv[r] / block + b) * Dm;
-  float k[4];
+  if (b0 >= vis) return;
+  const float* kc = pool + (row_kv[r] / block + b0) * Dm;
+  float4 k[IDX_B];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) k[j] = (lane * 4 + j) < Dm ? kc[lane * 4 + j] : 0.f;
-  float acc = 0.f;
-  for (int h = 0; h < H; ++h) {
-    const float* q = qi + (static_cast<size_t>(r) * H + h) * Dm;
-    float d = 0.f;
+  for (int i = 0; i < IDX_B; ++i) k[i] = idx_ld4(kc + static_cast<size_t>(min(i, vis - 1 - b0)) * Dm, lane, Dm, vec);
+  float acc = 0.f;                                            // of block lane >> 3
+  for (int h0 = 0; h0 < H; h0 += 4) {
+    float4 q[4];
+    float w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) if (lane * 4 + j < Dm) d = fmaf(q[lane * 4 + j], k[j], d);
-    d = warp_sum(d);
-    d = fmaxf(d, 0.f) * scale;
-    acc += head_w ? head_w[static_cast<size_t>(r) * H + h] * d : d;
+    for (int j = 0; j < 4; ++j) {
+      const size_t at = static_cast<size_t>(r) * H + min(h0 + j, H - 1);
+      q[j] = idx_ld4(qi + at * Dm, lane, Dm, vec);
+      w[j] = head_w ? head_w[at] : 1.f;
+    }
+    float d[16];                                              // block i, head h0 + j at 4 i + j
+#pragma unroll
+    for (int v = 0; v < 16; ++v) {
+      const float4 a = q[v & 3], b = k[v >> 2];
+      d[v] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, 0.f))));
+    }
+#pragma unroll
+    for (int o = 16, m = 8; m >= 1; o >>= 1, m >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int v = 0; v < m; ++v) {
+        const float keep = up ? d[v + m] : d[v], give = up ? d[v] : d[v + m];
+        d[v] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
+    const float sum = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);       // sum v is on lanes 2 v and 2 v + 1
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float s = fmaxf(__shfl_sync(0xffffffffu, sum, (lane & 24) + 2 * j), 0.f) * scale;
+      if (h0 + j < H) acc += head_w ? w[j] * s : s;
+    }
   }
-  if (lane == 0) score[static_cast<size_t>(r) * ld + b] = acc;
+  const int b = b0 + (lane >> 3);
+  if ((lane & 7) == 0 && b < vis) score[static_cast<size_t>(r) * ld + b] = acc;
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -77,7 +113,7 @@ idx_score_mma_kernel(const float* __restrict__ qi, int H, int Dm, const float* _
   float* Ss = Ks + 2 * IS_N * LQ;                                    // [64][65]
   const int sg = blockIdx.y, rpc = IS_M / H;
   const int r0 = seg[sg * 4 + 1], n = seg[sg * 4 + 2], pos0 = seg[sg * 4 + 3];
-  const int q0 = blockIdx.x * rpc;                                   // first row of this CTA inside the segment
+  const int q0 = (gridDim.x - 1 - blockIdx.x) * rpc;                 // first row of this CTA inside the segment, longest contexts first
   if (q0 >= n) return;
   const int rows_valid = min(rpc, n - q0);
   const int nb = (pos0 + q0 + rows_valid) / block;                   // blocks visible to the CTA's last row
@@ -116,6 +152,7 @@ idx_score_mma_kernel(const float* __restrict__ qi, int H, int Dm, const float* _
     float s[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) { s[i][0] = 0.f; s[i][1] = 0.f; s[i][2] = 0.f; s[i][3] = 0.f; }
+#pragma unroll 4
     for (int ks = 0; ks < Dm / 8; ++ks) {
       uint32_t ah[4], al[4];
       is_split(Qs[m_lo * LQ + ks * 8 + t], ah[0], al[0]);
@@ -185,19 +222,30 @@ __device__ __forceinline__ uint32_t order_key(uint32_t b) {
 // memory and the emission has two block scans; the digit of a pass is found by one warp's scan over the bins (one thread walking
 // them was most of the time).  Four rows of 4000 candidates: 27.7 -> 7.2 us.  NT = 256: prompts, where many rows of up to a few
 // thousand candidates share an SM: 3999 rows of up to 1000, 145 -> 22 us.
-template <int NT>
+// MASK: the same blocks (of 4 tokens) as a bit each, mw words per row in `sel`, for the tiles of prompt attention: eight lanes fill a
+// word (a token list per row, turned into bits by a kernel of its own, took 22 + 25 us for 3999 rows of up to 1000).
+template <int NT, bool MASK>
 __global__ void __launch_bounds__(NT)
 topk_select_kernel(const float* __restrict__ score, int ld, const int* __restrict__ pos, int block, int k, int window,
-                   int* __restrict__ sel, int sel_ld, int* __restrict__ sel_n) {
+                   int* __restrict__ sel, int sel_ld, int* __restrict__ sel_n, int mw) {
   __shared__ int s_straddle;
   __shared__ int hist[256];
   __shared__ int warp_tot[NT / 32];
   __shared__ uint32_t s_prefix;
   __shared__ int s_need;
   const int r = blockIdx.x, t = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   const int p = pos[r];
   const int vis = (p + 1) / block;
-  int* out = sel + static_cast<size_t>(r) * sel_ld;
+  if (MASK && vis <= k) {                          // every token is visible
+    for (int i = t; i < mw; i += NT) {
+      const int n = (p >> 2) + 1 - i * 32;         // bits of this word
+      sel[static_cast<size_t>(r) * mw + i] = n >= 32 ? -1 : n > 0 ? static_cast<int>((1u << n) - 1u) : 0;
+    }
+    return;
+  }
+  int* out = sel + static_cast<size_t>(r) * (MASK ? mw : sel_ld);
   if (vis <= k) {                                  // every token is visible
     for (int i = t; i <= p; i += NT) out[i] = i;
     if (t == 0) sel_n[r] = p + 1;
@@ -255,8 +303,8 @@ topk_select_kernel(const float* __restrict__ score, int ld, const int* __restric
   if (t == 0) s_straddle = 0;
   __syncthreads();
   int n_out = 0, eq_taken = 0;
-  for (int base = 0; base < vis; base += NT * 4) {
-    if (!once) load(base);
+  for (int base = 0; base < (MASK ? mw * 32 : vis); base += NT * 4) {
+    if (!once || (MASK && base)) load(base);
     const int i0 = base + t * 4;
     int eq = 0;
 #pragma unroll
@@ -275,6 +323,16 @@ topk_select_kernel(const float* __restrict__ score, int ld, const int* __restric
       if ((i + 1) * block <= lo) full |= 1u << j;
       else if (i == sb && lo > sb * block) s_straddle = 1;
     }
+    if (MASK) {
+      eq_taken += tot_eq;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) full |= (i0 + j >= sb && i0 + j <= p >> 2 ? 1u : 0u) << j;       // the always-visible range
+      unsigned word = full << ((t & 7) * 4);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
+      if ((t & 7) == 0 && i0 >> 5 < mw) out[i0 >> 5] = static_cast<int>(word);
+      continue;
+    }
     int tot_take;
     int o = n_out + block_excl_scan<NT>(__popc(full), warp_tot, tot_take);
 #pragma unroll
@@ -288,6 +346,7 @@ topk_select_kernel(const float* __restrict__ score, int ld, const int* __restric
     n_out += tot_take;
     eq_taken += tot_eq;
   }
+  if (MASK) return;
   __syncthreads();
   int cnt = n_out * block;
   if (s_straddle) {
@@ -507,8 +566,10 @@ extern "C" int spark_idx_score(const float* qi, int R, int H, int Dm, const floa
                                int nb_max, cudaStream_t s) {
   if (R <= 0 || nb_max <= 0) return 0;
   if (Dm > 128) return -5;
-  idx_score_kernel<<<dim3((nb_max + 7) / 8, R), 256, 0, s>>>(qi, H, Dm, pool, row_kv, pos, block, head_w, scale, score, ld);
-  return spark_launch_rc(__func__);
+  const int vec = (Dm & 3) == 0 && ((reinterpret_cast<uintptr_t>(qi) | reinterpret_cast<uintptr_t>(pool)) & 15) == 0;
+  const cudaError_t err = spark_launch_pdl(idx_score_kernel, dim3((nb_max + 8 * IDX_B - 1) / (8 * IDX_B), R), dim3(256), 0, s, dim3(1, 1, 1),
+                                           qi, H, Dm, pool, row_kv, pos, block, head_w, scale, score, ld, vec);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 // Prefill rows (whole segments): tensor-core scoring.  H a power of two <= 64, Dm % 8 == 0, Dm <= 128.
@@ -534,9 +595,21 @@ extern "C" int spark_topk_select(const float* score, int ld, const int* pos, int
   // 1024 / 256 threads, us: 148 rows of 1000 7.3 / 5.8, of 4096 7.7 / 13.5; 296 rows of 1000 9.7 / 6.3, of 2000 10.0 / 9.5, of 4096
   // 10.6 / 14.8; 592 rows of 4096 19.6 / 20.5; 1000 rows of 1000 29 / 12, of 8192 65 / 62; 4096 rows of 1000 110 / 33, of 8192 250 / 194.
   // (So a few hundred rows of more than 2000 pay 4 us, and 4096 rows of 12000, which stay with 1024, would take 272 instead of 342.)
-  if (R >= 2 * 148 && ld <= 8192) topk_select_kernel<256><<<R, 256, 0, s>>>(score, ld, pos, block, k, window, sel, sel_ld, sel_n);
-  else topk_select_kernel<1024><<<R, 1024, 0, s>>>(score, ld, pos, block, k, window, sel, sel_ld, sel_n);
-  return spark_launch_rc(__func__);
+  const bool many = R >= 2 * 148 && ld <= 8192;
+  const cudaError_t err = spark_launch_pdl(many ? topk_select_kernel<256, false> : topk_select_kernel<1024, false>, dim3(R),
+                                           dim3(many ? 256 : 1024), 0, s, dim3(1, 1, 1), score, ld, pos, block, k, window, sel, sel_ld, sel_n, 0);
+  return err == cudaSuccess ? 0 : -4;
+}
+
+// The selected blocks of 4 tokens (and the blocks of the always-visible range) as bits: bmask [R, mw], mw * 128 tokens of a row.
+extern "C" int spark_topk_mask(const float* score, int ld, const int* pos, int R, int k, unsigned* bmask, int mw, cudaStream_t s, int window) {
+  if (R <= 0) return 0;
+  if (mw <= 0 || window < 0) return -5;
+  const bool many = R >= 2 * 148 && ld <= 8192;
+  const cudaError_t err = spark_launch_pdl(many ? topk_select_kernel<256, true> : topk_select_kernel<1024, true>, dim3(R),
+                                           dim3(many ? 256 : 1024), 0, s, dim3(1, 1, 1), score, ld, pos, 4, k, window,
+                                           reinterpret_cast<int*>(bmask), 0, static_cast<int*>(nullptr), mw);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 // Multi-CTA exact selection: `ctas` CTAs per row (<= 64); work: int32 [R * (3 * 2048 + 3 * ctas)] scratch.

@@ -1330,13 +1330,10 @@ def attn_mixer(mixer, qkv, plan, seqs):
     sel = sel_n = None
     sel_ld = 0
     max_ctx = d["max_ctx"]
-    if sparse and max_ctx > c.sparse_topk_blocks * c.block:
-        from . import sparse as sp
-        sel, sel_n = sp.select_blocks(mixer, qi, plan, d)
-        sel_ld = sel.shape[1]
-        max_ctx = sel_ld
-    if (sel is None and not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.head_dim in (64, 128, 256)
-            and min(s.n for s in plan.segs) >= ATTN_PREFILL_MIN_ROWS):
+    selects = sparse and max_ctx > c.sparse_topk_blocks * c.block
+    tiles = (not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.head_dim in (64, 128, 256)
+             and min(s.n for s in plan.segs) >= ATTN_PREFILL_MIN_ROWS)
+    if tiles and not selects:
         # whole segments, dense context: streaming softmax on tcgen05 (one CTA per 128 rows of a head)
         out = torch.empty(R, c.n_q_heads * c.head_dim, dtype=torch.bfloat16, device=dev)
         rc = lib().spark_attn_prefill(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
@@ -1345,22 +1342,25 @@ def attn_mixer(mixer, qkv, plan, seqs):
                                       mixer.k.shape[0], P(status_word(dev)), stream())
         check(rc, "spark_attn_prefill")
         return out
-    if (sel is not None and not tree and not mixer.fp8 and ATTN_PREFILL_KERNEL and c.block == 4
-            and c.head_dim in (64, 128, 256) and min(s.n for s in plan.segs) >= ATTN_PREFILL_MIN_ROWS
-            and max(s.pos0 + s.n // 2 for s in plan.segs) <= ATTN_MASKED_MAX_KEYS):
+    if tiles and c.block == 4 and max(s.pos0 + s.n // 2 for s in plan.segs) <= ATTN_MASKED_MAX_KEYS:
         # block-sparse rows on a context of a few thousand tokens: the dense tiles with the unselected blocks masked
         # (128 rows share every key tile) beat one gathering CTA per row, which is bound by L2 bandwidth
-        mw = (d["max_ctx"] + 127) // 128
-        bmask = scratch("attn_block_mask", R * mw, torch.int32, dev)
+        from . import sparse as sp
+        mw = (max_ctx + 127) // 128
+        bmask = sp.select_block_mask(mixer, qi, plan, d, scratch("attn_block_mask", R * mw, torch.int32, dev), mw)
         out = torch.empty(R, c.n_q_heads * c.head_dim, dtype=torch.bfloat16, device=dev)
-        add_launches(1)
         rc = lib().spark_attn_prefill_masked(P(qbuf), P(mixer.k), P(mixer.v), P(d["row_kv"]), P(d["seg"]), len(plan.segs),
                                              max(s.n for s in plan.segs), P(qkv), qkv.stride(0), int(c.gated), P(out),
-                                             c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), P(sel),
-                                             P(sel_n), sel_ld, R, P(bmask), mw, mixer.k.shape[0], P(status_word(dev)),
+                                             c.n_q_heads, c.n_kv_heads, c.head_dim, 1.0 / math.sqrt(c.head_dim), None,
+                                             None, 0, R, P(bmask), mw, mixer.k.shape[0], P(status_word(dev)),
                                              stream())
         check(rc, "spark_attn_prefill_masked")
         return out
+    if selects:
+        from . import sparse as sp
+        sel, sel_n = sp.select_blocks(mixer, qi, plan, d)
+        sel_ld = sel.shape[1]
+        max_ctx = sel_ld
     nsplit, chunks = (max_ctx + ATT_TS - 1) // ATT_TS, 1
     if R >= 64 and c.head_dim in (64, 128, 256) and c.n_q_heads // c.n_kv_heads <= 16:
         # prefill-size batches have rows enough to fill the GPU: one CTA walks a row's whole context with a running

@@ -23,6 +23,8 @@ def _dll():
         dll.spark_idx_score_mma.restype = i32
         dll.spark_topk_select.argtypes = [vp, i32, vp, i32, i32, i32, vp, i32, vp, vp, i32]
         dll.spark_topk_select.restype = i32
+        dll.spark_topk_mask.argtypes = [vp, i32, vp, i32, i32, vp, i32, vp, i32]
+        dll.spark_topk_mask.restype = i32
         dll.spark_topk_select_mc.argtypes = [vp, i32, vp, i32, i32, i32, vp, i32, vp, vp, i32, i32, vp]
         dll.spark_topk_select_mc.restype = i32
         _bound = True
@@ -33,16 +35,12 @@ SCORE_MMA = os.environ.get("SPARK_IDX_SCORE_MMA", "1") == "1"
 SCORE_MMA_MIN_ROWS = 64
 
 
-def select_tokens(qi, pool, row_kv, pos32, block, topk, max_ctx, head_w=None, scale=None, window=0, segs=None):
-    """qi [R,H,Dm] fp32 indexer queries; pool [*, Dm] fp32 pooled keys (block b of a sequence at row_kv/block + b).
-    `window` > 0 keeps the last `window` positions visible as well.  `segs` = (segment table int32 [nseg, 4], nseg,
-    longest segment) when the rows are whole segments at consecutive positions: prefill-size batches are then scored
-    on tensor cores.  Returns (sel [R, topk*block + block + window] int32 token indices, sel_n [R])."""
+def block_scores(qi, pool, row_kv, pos32, block, max_ctx, head_w=None, scale=None, segs=None):
+    """Indexer scores [R, max(1, max_ctx // block)] fp32 of the complete blocks (scratch); arguments as in `select_tokens`."""
     R, H, Dm = qi.shape
-    dev = qi.device
     nb_max = max(1, max_ctx // block)
-    score = cu.scratch("idx_score", R * nb_max, torch.float32, dev)
-    cu.add_launches(2)
+    score = cu.scratch("idx_score", R * nb_max, torch.float32, qi.device)
+    cu.add_launches(2)                          # with the selection that follows
     sc = float(scale if scale is not None else 1.0 / math.sqrt(Dm))
     if (SCORE_MMA and segs is not None and R >= SCORE_MMA_MIN_ROWS and 1 <= H <= 64 and H & (H - 1) == 0
             and Dm % 8 == 0 and 8 <= Dm <= 128):
@@ -54,8 +52,16 @@ def select_tokens(qi, pool, row_kv, pos32, block, topk, max_ctx, head_w=None, sc
         rc = _dll().spark_idx_score(cu.P(qi), R, H, Dm, cu.P(pool), cu.P(row_kv), cu.P(pos32), block, cu.P(head_w), sc,
                                     cu.P(score), nb_max, nb_max, cu.stream())
         cu.check(rc, "spark_idx_score")
-    sel, sel_n = topk_select(score, nb_max, pos32, block, topk, window)
-    return sel, sel_n
+    return score, nb_max
+
+
+def select_tokens(qi, pool, row_kv, pos32, block, topk, max_ctx, head_w=None, scale=None, window=0, segs=None):
+    """qi [R,H,Dm] fp32 indexer queries; pool [*, Dm] fp32 pooled keys (block b of a sequence at row_kv/block + b).
+    `window` > 0 keeps the last `window` positions visible as well.  `segs` = (segment table int32 [nseg, 4], nseg,
+    longest segment) when the rows are whole segments at consecutive positions: prefill-size batches are then scored
+    on tensor cores.  Returns (sel [R, topk*block + block + window] int32 token indices, sel_n [R])."""
+    score, nb_max = block_scores(qi, pool, row_kv, pos32, block, max_ctx, head_w, scale, segs)
+    return topk_select(score, nb_max, pos32, block, topk, window)
 
 
 MC_MIN_CANDIDATES = int(os.environ.get("SPARK_TOPK_MC_MIN", "32768"))
@@ -85,7 +91,19 @@ def topk_select(score, nb_max, pos32, block, topk, window=0, ctas=None):
     return sel, sel_n
 
 
+def _segs(plan, d):
+    return None if plan.is_tree else (d["seg"], len(plan.segs), max(s.n for s in plan.segs))
+
+
 def select_blocks(mixer, qi, plan, d):
     c = mixer.c
-    segs = None if plan.is_tree else (d["seg"], len(plan.segs), max(s.n for s in plan.segs))
-    return select_tokens(qi, mixer.ik_pool, d["row_kv"], d["pos32"], c.block, c.sparse_topk_blocks, d["max_ctx"], segs=segs)
+    return select_tokens(qi, mixer.ik_pool, d["row_kv"], d["pos32"], c.block, c.sparse_topk_blocks, d["max_ctx"], segs=_segs(plan, d))
+
+
+def select_block_mask(mixer, qi, plan, d, bmask, mw):
+    """The blocks (of 4 tokens) of `select_blocks` as bits: `bmask` int32 [R * mw]."""
+    c = mixer.c
+    score, nb_max = block_scores(qi, mixer.ik_pool, d["row_kv"], d["pos32"], c.block, d["max_ctx"], segs=_segs(plan, d))
+    rc = _dll().spark_topk_mask(cu.P(score), nb_max, cu.P(d["pos32"]), qi.shape[0], c.sparse_topk_blocks, cu.P(bmask), mw, cu.stream(), 0)
+    cu.check(rc, "spark_topk_mask")
+    return bmask
