@@ -20,6 +20,8 @@ split_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ p
   // change a bit of the result).
   extern __shared__ float wts[];                        // [hpc][nsplit]: exp(m_s - M) / l
   __shared__ int live_s;                                // splits that hold visible tokens
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x == 0) live_s = 0;
   __syncthreads();
   const int r = blockIdx.x, h0 = blockIdx.y * hpc;
@@ -87,10 +89,10 @@ static inline int launch_split_merge(const float* part_o, const float* part_ml, 
   if (hpc * nsplit * 4 > 48 * 1024) return -6;
   const int L4 = L >> 2;
   const int threads = hpc * L4 >= 256 ? 256 : ((hpc * L4 + 31) / 32 * 32);   // whole warps
-  split_merge_kernel<<<dim3(R, (H + hpc - 1) / hpc), threads, hpc * nsplit * 4, s>>>(part_o, part_ml, nsplit, sink, H, L, hpc,
-                                                                                  (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, ldg,
-                                                                                  rows, out_by_row, ldo ? ldo : H * L, out_scale);
-  return 0;
+  const cudaError_t err = spark_launch_pdl(split_merge_kernel, dim3(R, (H + hpc - 1) / hpc), dim3(threads), hpc * nsplit * 4, s, dim3(1, 1, 1),
+                                           part_o, part_ml, nsplit, sink, H, L, hpc, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, ldg, rows,
+                                           out_by_row, ldo ? ldo : H * L, out_scale);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace spark

@@ -118,6 +118,102 @@ gemv_bf16_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat
   }
 }
 
+// Strided items of short contractions (per-head matrices: K of a few hundred): a lane group of LPC lanes owns a column, a lane four columns,
+// whose first loads are all in flight before the rows are staged (and before the dependency wait, where the tables allow it).  The sums
+// are those of gemv_bf16_kernel: a lane's chain over every LPC-th vector, the lanes folded as a butterfly.  What bounds it: one memory
+// round trip and the launch.  64 heads of [512, 128] and of [128, 512], 4 rows: 17 us each with two columns per warp (2048 CTAs of one
+// vector per lane on half of the lanes).
+constexpr int GEMV_IT_COLS = 4, GEMV_IT_U = 2;
+
+template <int RB, int LPC, typename TO>
+__global__ void __launch_bounds__(GEMV_WARPS * 32)
+gemv_items_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ W, long long expert_stride, int ldw,
+                  TO* __restrict__ y, int ldy, int R, int N, int K, const int* __restrict__ pair_expert, int pairs_early,
+                  long long x_item_stride, long long y_item_stride, const OutAct oact) {
+  extern __shared__ __align__(16) uint8_t smem_gemv[];
+  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem_gemv);     // [RB][K]
+  constexpr int G = 32 / LPC;
+  const int item = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane % LPC;
+  const int n0 = (blockIdx.x * GEMV_WARPS + warp) * GEMV_IT_COLS * G + lane / LPC;      // column c of this lane: n0 + c * G
+  const int KV = K >> 3;
+  if (pair_expert && !pairs_early) pdl_wait();
+  const int e = pair_expert ? pair_expert[item] : 0;
+  if (e < 0) { if (pairs_early) pdl_wait(); return; }                  // pair of an expert that lives on another rank
+  const __nv_bfloat16* Wb = W + e * expert_stride;
+  uint4 wv[GEMV_IT_U][GEMV_IT_COLS];
+  auto load = [&](int kv0) {
+#pragma unroll
+    for (int u = 0; u < GEMV_IT_U; ++u)
+#pragma unroll
+      for (int c = 0; c < GEMV_IT_COLS; ++c) {
+        const int kv = kv0 + u * LPC;
+        wv[u][c] = kv < KV ? __ldg(reinterpret_cast<const uint4*>(Wb + static_cast<size_t>(min(n0 + c * G, N - 1)) * ldw) + kv) : make_uint4(0u, 0u, 0u, 0u);
+      }
+  };
+  load(l);
+  if (!pair_expert || pairs_early) pdl_wait();
+  x += item * x_item_stride;
+  y += item * y_item_stride;
+  for (int i = threadIdx.x; i < R * KV; i += GEMV_WARPS * 32) {
+    const int r = i / KV, kv = i - r * KV;
+    *reinterpret_cast<uint4*>(xs + r * K + kv * 8) = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * ldx + kv * 8);
+  }
+  __syncthreads();
+  float acc[RB][GEMV_IT_COLS];
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int c = 0; c < GEMV_IT_COLS; ++c) acc[r][c] = 0.f;
+  for (int kv0 = l; kv0 < KV; kv0 += LPC * GEMV_IT_U) {
+    if (kv0 != l) load(kv0);
+#pragma unroll
+    for (int u = 0; u < GEMV_IT_U; ++u) {
+      const int kv = kv0 + u * LPC;
+      if (kv < KV) {
+        float w[GEMV_IT_COLS][8];
+#pragma unroll
+        for (int c = 0; c < GEMV_IT_COLS; ++c) unpack8(wv[u][c], w[c]);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          if (r >= R) break;
+          float xv[8];
+          unpack8(*reinterpret_cast<const uint4*>(xs + r * K + kv * 8), xv);
+#pragma unroll
+          for (int c = 0; c < GEMV_IT_COLS; ++c)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[r][c] = fmaf(w[c][i], xv[i], acc[r][c]);
+        }
+      }
+    }
+  }
+  pdl_trigger();
+  const int oc = item * oact.batch_cols;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    if (r >= R) break;
+#pragma unroll
+    for (int c = 0; c < GEMV_IT_COLS; ++c) {
+      float v = acc[r][c];
+#pragma unroll
+      for (int o = LPC / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      const int n = n0 + c * G;
+      if (l == 0 && n < N) y[static_cast<size_t>(r) * ldy + n] = static_cast<TO>(out_act(oact, v, r, oc + n));
+    }
+  }
+}
+
+template <int RB, typename TO>
+static int launch_gemv_items(const void* x, int ldx, const void* W, long long es, int ldw, void* y, int ldy, int items, int rows, int N, int K,
+                             const int* pe, int early, const OutAct& oact, cudaStream_t s, long long xis, long long yis) {
+  const bool half = K <= 16 * 8;                      // a column's vectors fit 16 lanes
+  const int per = GEMV_WARPS * GEMV_IT_COLS * (half ? 2 : 1);
+  const cudaError_t err = spark_launch_pdl(half ? gemv_items_kernel<RB, 16, TO> : gemv_items_kernel<RB, 32, TO>, dim3((N + per - 1) / per, items),
+                                           dim3(GEMV_WARPS * 32), RB * K * 2, s, dim3(1, 1, 1), (const __nv_bfloat16*)x, ldx,
+                                           (const __nv_bfloat16*)W, es, ldw, (TO*)y, ldy, rows, N, K, pe, early, xis, yis, oact);
+  return err == cudaSuccess ? 0 : -4;
+}
+constexpr int GEMV_ITEMS_MAX_K = 1024;               // 32 KB for 16 rows; longer contractions keep eight vectors per lane in flight
+
 template <int RB, typename TO>
 static int launch_gemv(const void* x, int ldx, const void* W, long long es, int ldw, void* y, int ldy, int items,
                        int rows, int N, int K, const int* pe, const int* pr, int act, const GluAct& glu, const OutAct& oact, cudaStream_t s,
@@ -189,8 +285,8 @@ gemv_wide_mma_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bf
   };
   const uint4 *w0, *w1;
   int n0 = rows_of(0, w0, w1);
+  if (n0 < N) load(w0, w1, kb);                          // in flight while the launch before ends and the rows are staged
   pdl_wait();
-  if (n0 < N) load(w0, w1, kb);                          // in flight while the rows are staged
   // rows past R are left as they are: an MMA column only ever reaches its own row's outputs, which are not stored
   const int KV8 = K >> 3;
   for (int i0 = threadIdx.x; i0 < R * KV8; i0 += 2 * GEMV_WARPS * 32) {
@@ -420,13 +516,27 @@ extern "C" int spark_gemv_bf16(const void* x, int ldx, const void* W, long long 
 // Strided items: item i multiplies rows x + i * x_item_stride + r * ldx (r < rows_per_item) by expert
 // pair_expert[i] (or W itself) and writes y + i * y_item_stride + r * ldy.  Used for per-head projections of
 // [rows, heads, dim] tensors: every head's matrix is streamed once for all rows.  Strides in elements; the item
-// offsets must keep x 16-byte aligned.
+// offsets must keep x 16-byte aligned.  pairs_early: pair_expert was written at least two launches back, so the weights may be asked for
+// before the dependency wait.
 extern "C" int spark_gemv_bf16_items(const void* x, int ldx, long long x_item_stride, const void* W, long long expert_stride,
                                      int ldw, void* y, int ldy, long long y_item_stride, int items, int rows_per_item, int N,
-                                     int K, const int* pair_expert, int out_f32, const OutAct* out, cudaStream_t s) {
+                                     int K, const int* pair_expert, int out_f32, const OutAct* out, cudaStream_t s, int pairs_early) {
   const OutAct oact = out ? *out : OutAct{};
   if (items <= 0 || rows_per_item <= 0) return 0;
   if (K % 8 || rows_per_item > 16 || (x_item_stride & 7) || (ldx & 7) || (x_item_stride | y_item_stride) == 0) return -5;
+  if (K <= GEMV_ITEMS_MAX_K) {
+#define SPARK_GEMV_SHORT(RB)                                                                                         \
+  if (rows_per_item <= RB)                                                                                           \
+    return out_f32 ? launch_gemv_items<RB, float>(x, ldx, W, expert_stride, ldw, y, ldy, items, rows_per_item, N, K, pair_expert, pairs_early,  \
+                                                  oact, s, x_item_stride, y_item_stride)                             \
+                   : launch_gemv_items<RB, __nv_bfloat16>(x, ldx, W, expert_stride, ldw, y, ldy, items, rows_per_item, N, K, pair_expert,       \
+                                                          pairs_early, oact, s, x_item_stride, y_item_stride);
+    SPARK_GEMV_SHORT(1)
+    SPARK_GEMV_SHORT(4)
+    SPARK_GEMV_SHORT(8)
+    SPARK_GEMV_SHORT(16)
+#undef SPARK_GEMV_SHORT
+  }
 #define SPARK_GEMV_ITEMS(RB)                                                                                         \
   if (rows_per_item <= RB)                                                                                           \
     return out_f32 ? launch_gemv<RB, float>(x, ldx, W, expert_stride, ldw, y, ldy, items, rows_per_item, N, K,       \

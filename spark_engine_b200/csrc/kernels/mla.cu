@@ -56,7 +56,8 @@ __device__ __forceinline__ void idx_key_gate(const __nv_bfloat16* a, int o1, int
   gate = d < Dm ? __bfloat162float(a[o1 + Dm + d]) : 0.f;
 }
 
-// grid R; 128 threads.  a: [R, q_lora + kv_lora + rope + 2*idx_dim + idx_heads] bf16.
+// grid (R, 3); 128 threads: the query activation, the latent row, the indexer state of a row.  a: [R, q_lora + kv_lora + rope + 2*idx_dim +
+// idx_heads] bf16.  Bound by its chain of reductions: the three after one another took 7.6 us for 4 rows.
 __global__ void __launch_bounds__(128)
 mla_prep_kernel(const __nv_bfloat16* __restrict__ a, int lda, MlaDims dm, const float* __restrict__ q_norm,
                 const float* __restrict__ kv_norm, const float* __restrict__ ln_w, const float* __restrict__ ln_b,
@@ -67,24 +68,31 @@ mla_prep_kernel(const __nv_bfloat16* __restrict__ a, int lda, MlaDims dm, const 
                 const int* __restrict__ row_pos0, int lat_fp8) {
   __shared__ float red[4];
   __shared__ int tmax[4];
-  const int r = blockIdx.x, t = threadIdx.x;
+  const int r = blockIdx.x, part = blockIdx.y, t = threadIdx.x;
+  pdl_wait();
+  pdl_trigger();
   const __nv_bfloat16* ar = a + static_cast<size_t>(r) * lda;
   const int p = pos[r];
   // rows of a verification tree (row_pos0 given) are rotated at their depth position p but stored at the slot of
   // their node, first in-flight slot + node index; their pools are finished when the accepted path is compacted
   const long long tok = row_kv[r] + (row_pos0 ? row_pos0[r] + row_j[r] : p);
   const int KW = dm.kv_lora + dm.rope;
-  // q low-rank activation
-  float ss = 0.f;
-  for (int i = t; i < dm.q_lora; i += 128) { const float x = __bfloat162float(ar[i]); ss = fmaf(x, x, ss); }
-  float rs = rsqrtf(block_sum_128(ss, red) / dm.q_lora + dm.eps);
-  for (int i = t; i < dm.q_lora; i += 128)
-    cq[static_cast<size_t>(r) * dm.q_lora + i] = __float2bfloat16(__bfloat162float(ar[i]) * rs * q_norm[i]);
-  // latent row
+  if (part == 0) {                                             // q low-rank activation
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = t; i < dm.q_lora; i += 128) { const float x = __bfloat162float(ar[i]); ss = fmaf(x, x, ss); }
+    const float rs = rsqrtf(block_sum_128(ss, red) / dm.q_lora + dm.eps);
+#pragma unroll 4
+    for (int i = t; i < dm.q_lora; i += 128)
+      cq[static_cast<size_t>(r) * dm.q_lora + i] = __float2bfloat16(__bfloat162float(ar[i]) * rs * q_norm[i]);
+    return;
+  }
+  if (part == 1) {                                             // latent row
   const __nv_bfloat16* akv = ar + dm.q_lora;
-  ss = 0.f;
+  float ss = 0.f;
+#pragma unroll 4
   for (int i = t; i < dm.kv_lora; i += 128) { const float x = __bfloat162float(akv[i]); ss = fmaf(x, x, ss); }
-  rs = rsqrtf(block_sum_128(ss, red) / dm.kv_lora + dm.eps);
+  const float rs = rsqrtf(block_sum_128(ss, red) / dm.kv_lora + dm.eps);
   __nv_bfloat16* lrow = lat + tok * KW;
   if (lat_fp8) {
     const int nt8 = max(1, dm.kv_lora >> 7), tw = dm.kv_lora / nt8;
@@ -115,6 +123,8 @@ mla_prep_kernel(const __nv_bfloat16* __restrict__ a, int lda, MlaDims dm, const 
     sincosf(ang, &sn, &cs);
     lrow[dm.kv_lora + i] = __float2bfloat16(x1 * cs - x2 * sn);
     lrow[dm.kv_lora + half + i] = __float2bfloat16(x2 * cs + x1 * sn);
+  }
+  return;
   }
   // indexer state
   const int o1 = dm.q_lora + KW, Dm = dm.idx_dim;
@@ -152,6 +162,8 @@ __global__ void mla_qrope_kernel(const __nv_bfloat16* __restrict__ qb, int ldq, 
                                  const double* __restrict__ inv_freq, const int* __restrict__ pos,
                                  __nv_bfloat16* __restrict__ q_full, int H) {
   const int r = blockIdx.x, h = blockIdx.y, i = threadIdx.x, half = rope >> 1;
+  pdl_wait();
+  pdl_trigger();
   if (i >= half) return;
   const __nv_bfloat16* q = qb + static_cast<size_t>(r) * ldq + h * (D + rope) + D;
   const float x1 = __bfloat162float(q[i]), x2 = __bfloat162float(q[half + i]);
@@ -183,10 +195,12 @@ __device__ __forceinline__ void mla_mma(float (&c)[4], const uint32_t (&a)[4], u
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// grid (R, ceil(nsplit / spc)); 256 threads; a CTA walks `spc` consecutive splits.  HM = 16-head MMA tiles (H <= 16*HM).  KW = kv_lora + rope (multiple of 16),
+// grid (R, ceil(nsplit / spc)); NW warps (16 where a CTA has 64 heads and an SM to itself, else 8); a CTA walks `spc` consecutive splits.  HM = 16-head MMA tiles (H <= 16*HM).  KW = kv_lora + rope (multiple of 16),
 // L = kv_lora (multiple of 16).
+template <int HM> constexpr int mla_warps() { return HM == 4 ? 16 : 8; }
+
 template <int HM, bool SPLITP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(mla_warps<HM>() * 32)
 mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
                   const __nv_bfloat16* __restrict__ lat,         // [tokens, KW]
                   const int* __restrict__ pos, const long long* __restrict__ row_kv, const int* __restrict__ sel,
@@ -196,6 +210,9 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
                   const int* __restrict__ row_pos0, const int* __restrict__ row_j, const int* __restrict__ anc,
                   int lat_fp8, MlaPages pg) {
   extern __shared__ __align__(16) uint8_t smem_mla[];
+  constexpr int NW = mla_warps<HM>(), NT = NW * 32, HG = NW / 8, HMG = HM / HG;      // HG groups of eight warps split the head tiles
+  pdl_wait();
+  pdl_trigger();
   const int LDK = KW + 8;
   __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(smem_mla);          // [HM*16][LDK]
   __nv_bfloat16* Ls = Qs + HM * 16 * LDK;                                   // [64][LDK]
@@ -216,7 +233,7 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
   const int* pages = pg.table ? pg.table + static_cast<size_t>(pg.row_slot[pr]) * pg.ld : nullptr;
   const int VPR = KW >> 3;
   // the row's queries (all heads) are staged once and serve every split this CTA walks through
-  for (int i = tid; i < HM * 16 * VPR; i += 256) {
+  for (int i = tid; i < HM * 16 * VPR; i += NT) {
     const int h = i / VPR, v = i - h * VPR;
     if (h < H) mla_cp16(Qs + h * LDK + v * 8, q_full + (static_cast<size_t>(r) * H + h) * KW + v * 8);
     else *reinterpret_cast<uint4*>(Qs + h * LDK + v * 8) = make_uint4(0u, 0u, 0u, 0u);
@@ -225,7 +242,7 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
   const int t0 = sp * MLA_TS;
   const size_t pb = (static_cast<size_t>(r) * H) * nsplit + sp;
   if (t0 >= n_ctx) {                                           // empty split: neutral partial
-    for (int h = tid; h < H; h += 256) {
+    for (int h = tid; h < H; h += NT) {
       part_ml[(pb + static_cast<size_t>(h) * nsplit) * 2] = -INFINITY;
       part_ml[(pb + static_cast<size_t>(h) * nsplit) * 2 + 1] = 0.f;
     }
@@ -237,7 +254,7 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
   if (tid < MLA_TS) stok[tid] = tid < nt ? (sel ? sel[static_cast<size_t>(r) * sel_ld + t0 + tid] : t0 + tid) : -1;
   __syncthreads();
   if (!lat_fp8) {
-    for (int i = tid; i < MLA_TS * VPR; i += 256) {
+    for (int i = tid; i < MLA_TS * VPR; i += NT) {
       const int k = i / VPR, v = i - k * VPR;
       if (stok[k] >= 0) mla_cp16(Ls + k * LDK + v * 8, lat + (base + stok[k]) * KW + v * 8);
       else *reinterpret_cast<uint4*>(Ls + k * LDK + v * 8) = make_uint4(0u, 0u, 0u, 0u);
@@ -250,14 +267,14 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
     // tail into registers before any lane writes
     const int RB = L + 16 + 2 * (KW - L), CH = RB >> 4;
     const uint8_t* lat8 = reinterpret_cast<const uint8_t*>(lat);
-    for (int i = tid; i < MLA_TS * CH; i += 256) {
+    for (int i = tid; i < MLA_TS * CH; i += NT) {
       const int k = i / CH, v = i - k * CH;
       if (stok[k] >= 0) mla_cp16(reinterpret_cast<uint8_t*>(Ls + k * LDK) + L + v * 16, lat8 + (base + stok[k]) * RB + v * 16);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const int nt8 = max(1, L >> 7), tw = L / nt8, rch = (KW - L) >> 3;
-    for (int k = warp; k < MLA_TS; k += 8) {
+    for (int k = warp; k < MLA_TS; k += NW) {
       uint8_t* rowb = reinterpret_cast<uint8_t*>(Ls + k * LDK);
       if (stok[k] < 0) {
         for (int v = lane; v < VPR; v += 32) *reinterpret_cast<uint4*>(rowb + v * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -291,35 +308,36 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
   }
   // ---- phase 1: S[h][tok] for this warp's 8 tokens, all head tiles
   {
-    float s[HM][4];
+    const int tw8 = warp & 7, m0 = (warp >> 3) * HMG;
+    float s[HMG][4];
 #pragma unroll
-    for (int m = 0; m < HM; ++m) { s[m][0] = 0.f; s[m][1] = 0.f; s[m][2] = 0.f; s[m][3] = 0.f; }
+    for (int m = 0; m < HMG; ++m) { s[m][0] = 0.f; s[m][1] = 0.f; s[m][2] = 0.f; s[m][3] = 0.f; }
     for (int ks = 0; ks < KW / 16; ks += 2) {
-      // B: tokens 8*warp..+7; matrices (k0..7), (k8..15) of step ks and of step ks+1
+      // B: tokens 8 * tw8 ..+7; matrices (k0..7), (k8..15) of step ks and of step ks+1
       uint32_t b[4];
       const bool two = ks + 1 < KW / 16;
-      mla_ldsm4(b, Ls + (warp * 8 + (lane & 7)) * LDK + ks * 16 + (two ? (lane >> 3) * 8 : ((lane >> 3) & 1) * 8));
+      mla_ldsm4(b, Ls + (tw8 * 8 + (lane & 7)) * LDK + ks * 16 + (two ? (lane >> 3) * 8 : ((lane >> 3) & 1) * 8));
 #pragma unroll
-      for (int m = 0; m < HM; ++m) {
+      for (int m = 0; m < HMG; ++m) {
         uint32_t a[4];
-        mla_ldsm4(a, Qs + (m * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + ks * 16 + (lane >> 4) * 8);
+        mla_ldsm4(a, Qs + ((m0 + m) * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + ks * 16 + (lane >> 4) * 8);
         mla_mma(s[m], a, b[0], b[1]);
         if (two) {
-          mla_ldsm4(a, Qs + (m * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + (ks + 1) * 16 + (lane >> 4) * 8);
+          mla_ldsm4(a, Qs + ((m0 + m) * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + (ks + 1) * 16 + (lane >> 4) * 8);
           mla_mma(s[m], a, b[2], b[3]);
         }
       }
     }
 #pragma unroll
-    for (int m = 0; m < HM; ++m) {
-      const int c = warp * 8 + 2 * t;
-      Ss[(m * 16 + g) * 65 + c] = s[m][0] * scale; Ss[(m * 16 + g) * 65 + c + 1] = s[m][1] * scale;
-      Ss[(m * 16 + g + 8) * 65 + c] = s[m][2] * scale; Ss[(m * 16 + g + 8) * 65 + c + 1] = s[m][3] * scale;
+    for (int m = 0; m < HMG; ++m) {
+      const int c = tw8 * 8 + 2 * t, h = (m0 + m) * 16 + g;
+      Ss[h * 65 + c] = s[m][0] * scale; Ss[h * 65 + c + 1] = s[m][1] * scale;
+      Ss[(h + 8) * 65 + c] = s[m][2] * scale; Ss[(h + 8) * 65 + c + 1] = s[m][3] * scale;
     }
   }
   __syncthreads();
   // ---- phase 2: per-head softmax statistics over the split; P (bf16) for the second product
-  for (int h = warp; h < HM * 16; h += 8) {
+  for (int h = warp; h < HM * 16; h += NW) {
     bool v0 = lane < nt, v1 = lane + 32 < nt;
     if (tree) {
       const int k0 = t0 + lane - tp0, k1 = k0 + 32;
@@ -344,7 +362,7 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
   }
   __syncthreads();
   // ---- phase 3: O[h][d] = sum_tok P[h][tok] lat[tok][d]; column pairs (16 wide) round-robin over the warps
-  for (int np = warp; np < L / 16; np += 8) {
+  for (int np = warp; np < L / 16; np += NW) {
     float o[HM][2][4];
 #pragma unroll
     for (int m = 0; m < HM; ++m)
@@ -403,18 +421,19 @@ extern "C" int spark_mla_prep(const void* a, int lda, int R, int q_lora, int kv_
   if (idx_dim > 128 || idx_heads > 128 || pool_sz > 8 || pool_sz < 1 || (rope & 1)) return -5;
   if (lat_fp8 && !mla_fp8_ok(kv_lora, rope)) return -5;
   MlaDims dm{q_lora, kv_lora, rope, idx_dim, idx_heads, pool_sz, eps};
-  mla_prep_kernel<<<R, 128, 0, s>>>((const __nv_bfloat16*)a, lda, dm, q_norm, kv_norm, ln_w, ln_b, ape, inv_freq, pos, row_kv,
-                                    row_j, (__nv_bfloat16*)cq, (__nv_bfloat16*)lat, ik, ig, pool, hw, row_pos0, lat_fp8);
-  return spark_launch_rc(__func__);
+  const cudaError_t err = spark_launch_pdl(mla_prep_kernel, dim3(R, 3), dim3(128), 0, s, dim3(1, 1, 1), (const __nv_bfloat16*)a, lda, dm, q_norm,
+                                           kv_norm, ln_w, ln_b, ape, inv_freq, pos, row_kv, row_j, (__nv_bfloat16*)cq, (__nv_bfloat16*)lat,
+                                           ik, ig, pool, hw, row_pos0, lat_fp8);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int spark_mla_qrope(const void* qb, int ldq, int R, int H, int D, int rope, int kv_lora, const double* inv_freq,
                                const int* pos, void* q_full, cudaStream_t s) {
   if (R <= 0 || rope <= 0) return 0;
   if (rope > 512) return -5;
-  mla_qrope_kernel<<<dim3(R, H), (rope / 2 + 31) / 32 * 32, 0, s>>>((const __nv_bfloat16*)qb, ldq, D, rope, kv_lora, inv_freq, pos,
-                                                                    (__nv_bfloat16*)q_full, H);
-  return spark_launch_rc(__func__);
+  const cudaError_t err = spark_launch_pdl(mla_qrope_kernel, dim3(R, H), dim3((rope / 2 + 31) / 32 * 32), 0, s, dim3(1, 1, 1),
+                                           (const __nv_bfloat16*)qb, ldq, D, rope, kv_lora, inv_freq, pos, (__nv_bfloat16*)q_full, H);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 namespace spark {
@@ -427,9 +446,10 @@ static int launch_mla_decode(dim3 grid, int smem, cudaStream_t s, const void* q_
   auto kern = mla_decode_kernel<HM, SPLITP>;
   static bool done = false;
   if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); done = true; }
-  kern<<<grid, 256, smem, s>>>((const __nv_bfloat16*)q_full, (const __nv_bfloat16*)lat, pos, row_kv, sel, sel_n, sel_ld, part_o,
-                               part_ml, H, KW, L, scale, nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg);
-  return 0;
+  const cudaError_t err = spark_launch_pdl(kern, grid, dim3(mla_warps<HM>() * 32), smem, s, dim3(1, 1, 1), (const __nv_bfloat16*)q_full,
+                                           (const __nv_bfloat16*)lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, L, scale,
+                                           nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 static int mla_attn(const void* q_full, const void* lat, const int* pos, const long long* row_kv, const int* sel,
@@ -447,13 +467,14 @@ static int mla_attn(const void* q_full, const void* lat, const int* pos, const l
   // few rows (decode): one split per CTA for parallelism; many rows (prefill): a CTA per row walks all its splits
   const int spc = R >= 128 ? nsplit : (R >= 32 ? 4 : 1);
   const dim3 grid(R, (nsplit + spc - 1) / spc);
+  int rc;
 #define SPARK_MLA_DEC(HMV, SPV)                                                                                            \
-  launch_mla_decode<HMV, SPV>(grid, smem, s, q_full, lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, kv_lora, \
+  rc = launch_mla_decode<HMV, SPV>(grid, smem, s, q_full, lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, kv_lora, \
                               scale, nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg)
   if (splitp) { if (HM == 1) SPARK_MLA_DEC(1, true); else if (HM == 2) SPARK_MLA_DEC(2, true); else SPARK_MLA_DEC(4, true); }
   else { if (HM == 1) SPARK_MLA_DEC(1, false); else if (HM == 2) SPARK_MLA_DEC(2, false); else SPARK_MLA_DEC(4, false); }
 #undef SPARK_MLA_DEC
-  const int rc = launch_split_merge(part_o, part_ml, nsplit, sink, R, H, kv_lora, out, gate, ldg, pg.rows, 0, s);
+  if (!rc) rc = launch_split_merge(part_o, part_ml, nsplit, sink, R, H, kv_lora, out, gate, ldg, pg.rows, 0, s);
   if (rc) return rc;
   return spark_launch_rc("spark_mla_attn");
 }

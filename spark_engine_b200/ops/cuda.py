@@ -30,7 +30,7 @@ _SIGS = {
     "spark_gemm_simt": [vp, i32, i64, vp, i32, i64, vp, i32, i64, i32, i32, i32, i32, i32, i32, vp, vp],
     "spark_gemm_simt_grouped": [vp, i32, vp, i32, i64, vp, i32, i32, i32, vp, vp, i32, vp, i32, i32, i32, vp, vp],
     "spark_gemv_bf16": [vp, i32, vp, i64, i32, vp, i32, i32, i32, i32, i32, vp, vp, i32, vp, i32, vp, vp, vp],
-    "spark_gemv_bf16_items": [vp, i32, i64, vp, i64, i32, vp, i32, i64, i32, i32, i32, i32, vp, i32, vp, vp],
+    "spark_gemv_bf16_items": [vp, i32, i64, vp, i64, i32, vp, i32, i64, i32, i32, i32, i32, vp, i32, vp, vp, i32],
     "spark_add_rmsnorm": [vp, i32, vp, vp, vp, i32, i32, f32, i32, vp],
     "spark_rmsnorm_bf16": [vp, vp, vp, i32, i32, f32, i32, vp],
     "spark_embed": [vp, vp, vp, i32, i32, vp, i32, vp],
@@ -331,13 +331,14 @@ def gemv_bf16(x, w, items=1, rows_per_item=None, pair_expert=None, pair_row=None
 
 
 def gemv_bf16_items(x, ldx, x_item_stride, w, expert_stride, ldw, y, ldy, y_item_stride, items, rows_per_item, n, k,
-                    pair_expert, oact=None):
+                    pair_expert, oact=None, pairs_early=False):
     """Per-item GEMV over strided slices: item i multiplies rows x[i * x_item_stride + r * ldx] (r < rows_per_item) by
-    matrix pair_expert[i] of `w` and writes y[i * y_item_stride + r * ldy].  Strides in elements."""
+    matrix pair_expert[i] of `w` and writes y[i * y_item_stride + r * ldy].  Strides in elements.  `pairs_early`: see `exl3_gemv`."""
     if dbg.CHECK:
         dbg.check_index("gemv_bf16_items pair_expert", pair_expert, 0, w.shape[0], count=items)
     rc = lib().spark_gemv_bf16_items(P(x), ldx, x_item_stride, P(w), expert_stride, ldw, P(y), ldy, y_item_stride, items,
-                                     rows_per_item, n, k, P(pair_expert), int(y.dtype == torch.float32), _act(oact), stream())
+                                     rows_per_item, n, k, P(pair_expert), int(y.dtype == torch.float32), _act(oact), stream(),
+                                     int(pairs_early))
     check(rc, "spark_gemv_bf16_items")
     return y
 
@@ -1232,9 +1233,9 @@ def mla_mixer(mixer, h, plan, seqs):
         if key not in md:
             md[key] = torch.arange(H, dtype=torch.int32, device=dev)
         heads = md[key]
-        qn = qb[:, :nq].contiguous()
+        qn = qb if qb.stride(0) % 8 == 0 else qb[:, :nq].contiguous()
         # absorb W_uk: one item per head over all rows (the head's [L, D] matrix is streamed once for the round)
-        gemv_bf16_items(qn, H * (D + Rr), D + Rr, md["w_ukT"], L * D, D, q_full, H * KW, KW, H, R, L, D, heads)
+        gemv_bf16_items(qn, qn.stride(0), D + Rr, md["w_ukT"], L * D, D, q_full, H * KW, KW, H, R, L, D, heads, pairs_early=True)
     else:
         q_full[..., :L] = torch.einsum("thd,hld->thl", qb[:, :nq].view(R, H, D + Rr)[..., :D], md["w_ukT"])
     if Rr:
@@ -1262,7 +1263,8 @@ def mla_mixer(mixer, h, plan, seqs):
     check(rc, "spark_mla_attn")
     if decode:
         out = torch.empty(R, H * D, dtype=torch.bfloat16, device=dev)
-        return gemv_bf16_items(out_lat, H * L, L, md["w_uv"], D * L, L, out, H * D, D, H, R, D, L, md[("mla_heads", H)])
+        return gemv_bf16_items(out_lat, H * L, L, md["w_uv"], D * L, L, out, H * D, D, H, R, D, L, md[("mla_heads", H)],
+                               pairs_early=True)
     return torch.einsum("thl,hdl->thd", out_lat, md["w_uv"]).reshape(R, H * D)
 
 
