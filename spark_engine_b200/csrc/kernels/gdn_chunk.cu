@@ -13,7 +13,7 @@
 //                            W = T diag(beta D) K,  Ut = T diag(beta) V,  Qt = diag(D) Q,  Kt = diag(D_C/D) K
 //   kernel 2 (v-slice, head, segment), sequential over the chunks of one sequence, S kept in registers:
 //                            U = Ut - W S0^T;  O = Qt S0^T + P U;  S <- D_C S + U^T Kt
-//                            (the Dv rows of S are independent, so a head is split over 4 CTAs of 32 rows)
+//                            (the Dv rows of S are independent, so a head is split over 2 CTAs of 64 rows)
 //   kernel 3 (chunk, head):  RMSNorm(o) * w * sigmoid(z) -> bf16
 // All decay ratios are exp() of non-positive numbers: nothing can overflow.  Operands are rounded to tf32
 // (10-bit mantissa) once, when they are written; sums are fp32.  Decode and verify rows keep using the
@@ -27,11 +27,15 @@ constexpr int GC = 64;            // chunk length
 constexpr int GD = 128;           // head dim (k and v)
 constexpr int LD128 = 136;        // smem row stride of 128-wide arrays (8 mod 32: conflict-free fragment loads)
 constexpr int LD64 = 72;
-constexpr int LD32 = 40;
-constexpr int GVS = 32;           // value rows of S per CTA in the state pass
-// workspace per (chunk, head), floats
-constexpr int WS_W = 0, WS_UT = GC * GD, WS_QT = 2 * GC * GD, WS_KT = 3 * GC * GD, WS_P = 4 * GC * GD,
+constexpr int GVS = 64;           // value rows of S per CTA in the state pass
+// Workspace per (chunk, head), floats: the shared-memory images of the state pass's operands, so that plain bulk copies bring them in.
+// K-major rows of 32 floats (128 bytes, 128-byte swizzle): [Qt; W] as four tiles of 128 rows, Kt^T as two of 128, P as two of 64;
+// Ut per slice of GVS value columns as [column / 4][row][4].
+constexpr int WS_QW = 0, WS_UT = 2 * GC * GD, WS_KT = 3 * GC * GD, WS_P = 4 * GC * GD,
               WS_DC = 4 * GC * GD + GC * GC, WS_STRIDE = 4 * GC * GD + GC * GC + 64;
+// float of row r, column k in tiles of `rows` rows
+__device__ __forceinline__ int ws_at(int rows, int r, int k) { return (k >> 5) * rows * 32 + r * 32 + ((((k >> 2) ^ r) & 7) << 2) + (k & 3); }
+__device__ __forceinline__ int ws_ut(int r, int v) { return (v >> 2) * GC * 4 + r * 4 + (v & 3); }
 
 __device__ __forceinline__ float tf32r(float x) {
   uint32_t r;
@@ -185,12 +189,23 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
         y = scale_tf32(y, f);
       }
       *at = y;
-      if (part < 2)
-        *reinterpret_cast<float4*>(wsb + (part == 0 ? WS_QT : WS_KT) + r * GD + lane * 4) = scale_tf32(y, part == 0 ? D_s[r] : __expf(Gl - G_s[r]));
+      if (part == 0) *reinterpret_cast<float4*>(wsb + WS_QW + ws_at(2 * GC, r, lane * 4)) = scale_tf32(y, D_s[r]);
     }
     if (tid == 0) wsb[WS_DC] = __expf(Gl);
   }
   __syncthreads();
+  {
+    // Kt^T: a thread moves four rows of a channel; two lanes fill a 32-byte sector
+    const float Gl = G_s[GC - 1];
+#pragma unroll 2
+    for (int i = tid; i < GD * (GC / 4); i += 256) {
+      const int k = (i >> 1) & (GD - 1), r = ((i >> 8) * 2 + (i & 1)) * 4;
+      const float* kp = Ks + r * LD128 + k;
+      *reinterpret_cast<float4*>(wsb + WS_KT + ws_at(GD, k, r)) =
+          make_float4(tf32r(kp[0] * __expf(Gl - G_s[r])), tf32r(kp[LD128] * __expf(Gl - G_s[r + 1])),
+                      tf32r(kp[2 * LD128] * __expf(Gl - G_s[r + 2])), tf32r(kp[3 * LD128] * __expf(Gl - G_s[r + 3])));
+    }
+  }
 
   const int g = lane >> 2, t = lane & 3;
   // ---- K K^T and Q K^T (lower triangle only): warp -> m-tile (warp&3), n-tiles 4*(warp>>2) .. +4
@@ -238,7 +253,7 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
           }
         }
         *reinterpret_cast<float2*>(As + row * LD64 + col) = make_float2(av[0], av[1]);
-        *reinterpret_cast<float2*>(Pg + row * GC + col) = make_float2(pv[0], pv[1]);
+        *reinterpret_cast<float2*>(Pg + ws_at(GC, row, col)) = make_float2(pv[0], pv[1]);
       }
     }
   }
@@ -334,166 +349,249 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
           mma_tf32(acc[a], a0, a1, a2, a3, bb[0], bb[4 * LD128]);
         }
       }
-      float* Og = wsb + (which == 0 ? WS_W : WS_UT);
+      float* Og = wsb + (which == 0 ? WS_QW : WS_UT);
 #pragma unroll
       for (int a = 0; a < 8; ++a) {
         const int col = (nt0 + a) * 8 + 2 * t, row = mt * 16 + g;
         float2 lo = make_float2(acc[a][0], acc[a][1]), hi = make_float2(acc[a][2], acc[a][3]);
         if (which == 0) { lo.x = tf32r(lo.x); lo.y = tf32r(lo.y); hi.x = tf32r(hi.x); hi.y = tf32r(hi.y); }
-        *reinterpret_cast<float2*>(Og + row * GD + col) = lo;
-        *reinterpret_cast<float2*>(Og + (row + 8) * GD + col) = hi;
+        *reinterpret_cast<float2*>(Og + (which == 0 ? ws_at(2 * GC, GC + row, col) : ws_ut(row, col))) = lo;
+        *reinterpret_cast<float2*>(Og + (which == 0 ? ws_at(2 * GC, GC + row + 8, col) : ws_ut(row + 8, col))) = hi;
       }
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------------- kernel 2
-// grid (4, Hv, nseg); 128 threads; sequential over the chunks of one segment
-__global__ void __launch_bounds__(128)
+// grid (2, Hv, nseg); sequential over the chunks of one segment, 64 value rows of S per CTA.  Products on tcgen05 (kind::tf32), the state
+// in registers:
+//   [O; X] = [Qt; W] S^T          M = 128 rows, N = 64 values, K = 128          D1 (two buffers)
+//   U      = Ut - X                by the warps that own the lanes of X
+//   D3     = Kt^T U                M = 128 keys, N = 64, K = 64                  then S^T <- D_C S^T + D3 in registers
+//   O     += P U                   the M = 128 operand's rows past P's 64 are whatever follows it: they end in X's lanes, which are read
+// Warp 0 brings the operands in, tiles of 16 KB through a ring of 11 (eight per chunk); warp 1 issues; eight warps (two per lane quarter,
+// 32 value columns each) keep S, write it and U as K-major operands and store O.
+// What bounds it: the chain state -> product -> U -> product of a chunk, and the 128 KB per chunk that a CTA pulls from L2.
+// 64 chunks of 32 heads: 293 us with warp-level TF32 products and the operands copied between them (four CTAs of 32 values a head).
+constexpr int ST_SLOTS = 11, ST_SLOT = 16384, ST_THREADS = 10 * 32;
+constexpr int ST_B1 = GVS * GD * 4, ST_B2 = GVS * GC * 4;
+constexpr int ST_SMEM = ST_SLOTS * ST_SLOT + ST_B1 + ST_B2 + 256 + 1024;
+static_assert(ST_SMEM <= 232448, "shared memory of the state pass");
+
+__global__ void __launch_bounds__(ST_THREADS, 1)
 gdn_chunk_state_kernel(const float* __restrict__ ws, const int* __restrict__ seg, const int* __restrict__ seg_chunk0,
                        const __nv_bfloat16* __restrict__ proj, int ldp, float* __restrict__ S, float* __restrict__ tail,
-                       float* __restrict__ o_raw, int ldo, int Hk, int Hv) {
-  extern __shared__ __align__(16) float sm[];
-  float* Wsm = sm;                          // [64][136]
-  float* Qsm = Wsm + GC * LD128;
-  float* Ksm = Qsm + GC * LD128;
-  float* Psm = Ksm + GC * LD128;            // [64][72]
-  float* Usm = Psm + GC * LD64;             // [64][40]  Ut, then U
-  float* Ssm = Usm + GC * LD32;             // [32][136]
+                       float* __restrict__ o_raw, int ldo, int Hk, int Hv, int* __restrict__ status) {
+  extern __shared__ uint8_t smem_raw[];
   const int vs = blockIdx.x, h = blockIdx.y, sg = blockIdx.z;
   const int ci0 = seg_chunk0[sg];
   if (ci0 < 0) return;
-  const int slot = seg[sg * 4], r0 = seg[sg * 4 + 1], n = seg[sg * 4 + 2];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* B1 = smem + ST_SLOTS * ST_SLOT;                   // S^T as [64 values][128 keys]: four tiles of 64 rows
+  uint8_t* B2 = B1 + ST_B1;                                  // U^T as [64 values][64 rows]: two tiles of 64 rows
+  uint64_t* full = reinterpret_cast<uint64_t*>(B2 + ST_B2);
+  uint64_t* empty = full + ST_SLOTS;
+  uint64_t* s_ready = empty + ST_SLOTS;
+  uint64_t* x_full = s_ready + 1;
+  uint64_t* u_ready = x_full + 1;
+  uint64_t* s_full = u_ready + 1;
+  uint64_t* o_full = s_full + 1;                             // [2]: its waiters may be a chunk behind
+  uint64_t* o_read = o_full + 2;                             // [2]
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_read + 2);
+  const int slot_id = seg[sg * 4], r0 = seg[sg * 4 + 1], n = seg[sg * 4 + 2];
   const int nch = (n + GC - 1) / GC;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int v0 = vs * GVS;
-  // S accumulator fragments: warp -> v rows 16*(warp&1).., k columns 64*(warp>>1)..
-  const int smt = warp & 1, sng = warp >> 1;
-  float sacc[8][4];
-  float* Sg = S + ((static_cast<size_t>(slot) * Hv + h) * GD + v0) * GD;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int col = sng * 64 + a * 8 + 2 * t, row = smt * 16 + g;
-    const float2 lo = *reinterpret_cast<const float2*>(Sg + row * GD + col);
-    const float2 hi = *reinterpret_cast<const float2*>(Sg + (row + 8) * GD + col);
-    sacc[a][0] = lo.x; sacc[a][1] = lo.y; sacc[a][2] = hi.x; sacc[a][3] = hi.y;
-    Ssm[row * LD128 + col] = tf32r(lo.x); Ssm[row * LD128 + col + 1] = tf32r(lo.y);
-    Ssm[(row + 8) * LD128 + col] = tf32r(hi.x); Ssm[(row + 8) * LD128 + col + 1] = tf32r(hi.y);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < ST_SLOTS; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    mbar_init(s_ready, 8); mbar_init(x_full, 1); mbar_init(u_ready, 4); mbar_init(s_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&o_full[i], 1); mbar_init(&o_read[i], 4); }
+    fence_barrier_init();
   }
-  for (int c = 0; c < nch; ++c) {
-    const float* wsb = ws + (static_cast<size_t>(ci0 + c) * Hv + h) * WS_STRIDE;
-    // ---- stage this chunk's operands
-    for (int idx = tid; idx < GC * GD / 4; idx += 128) {
-      const int r = idx >> 5, c4 = (idx & 31) * 4;
-      cp_async16(Wsm + r * LD128 + c4, wsb + WS_W + r * GD + c4);
-      cp_async16(Qsm + r * LD128 + c4, wsb + WS_QT + r * GD + c4);
-      cp_async16(Ksm + r * LD128 + c4, wsb + WS_KT + r * GD + c4);
-    }
-    for (int idx = tid; idx < GC * GC / 4; idx += 128) {
-      const int r = idx >> 4, c4 = (idx & 15) * 4;
-      cp_async16(Psm + r * LD64 + c4, wsb + WS_P + r * GC + c4);
-    }
-    for (int idx = tid; idx < GC * GVS / 4; idx += 128) {
-      const int r = idx >> 3, c4 = (idx & 7) * 4;
-      cp_async16(Usm + r * LD32 + c4, wsb + WS_UT + r * GD + v0 + c4);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const float dc = wsb[WS_DC];
-    // ---- X = W S0^T and O = Qt S0^T: warp -> token rows 16*warp.., 4 n-tiles (32 v columns), 16 k-steps
-    float xacc[4][4], oacc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) { xacc[a][b] = 0.f; oacc[a][b] = 0.f; }
-    {
-      const float* wa = Wsm + (warp * 16 + g) * LD128 + t;
-      const float* qa = Qsm + (warp * 16 + g) * LD128 + t;
-#pragma unroll 4
-      for (int ks = 0; ks < GD / 8; ++ks) {
-        const float w0 = wa[ks * 8], w1 = wa[8 * LD128 + ks * 8], w2 = wa[ks * 8 + 4], w3 = wa[8 * LD128 + ks * 8 + 4];
-        const float q0 = qa[ks * 8], q1 = qa[8 * LD128 + ks * 8], q2 = qa[ks * 8 + 4], q3 = qa[8 * LD128 + ks * 8 + 4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const float* sb = Ssm + (a * 8 + g) * LD128 + ks * 8 + t;
-          const float b0 = sb[0], b1 = sb[4];
-          mma_tf32(xacc[a], w0, w1, w2, w3, b0, b1);
-          mma_tf32(oacc[a], q0, q1, q2, q3, b0, b1);
+  if (warp == 1) { tmem_alloc<256>(tmem_ptr); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_ptr;
+  constexpr uint32_t D3 = 128;                               // D1 buffers at columns 0 and 64
+  const float* wsh = ws + (static_cast<size_t>(ci0) * Hv + h) * WS_STRIDE;
+  const size_t ws_step = static_cast<size_t>(Hv) * WS_STRIDE;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer: a chunk is [Qt; W] x 4, Ut, Kt^T x 2, P
+    int sl = 0; uint32_t ph = 0; bool ok = true;
+    for (int c = 0; c < nch && ok; ++c) {
+      const float* w = wsh + c * ws_step;
+      for (int i = 0; i < 8; ++i) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty[sl], ph ^ 1));
+        if (!ok) { set_status(status, ST_TIMEOUT_MBAR_EMPTY, blockIdx.x, blockIdx.y, c); break; }
+        if (elect_one()) {
+          const float* src = i < 4 ? w + WS_QW + i * 4096 : i == 4 ? w + WS_UT + vs * GVS * GC : i < 7 ? w + WS_KT + (i - 5) * 4096 : w + WS_P;
+          mbar_arrive_expect_tx(&full[sl], ST_SLOT);
+          bulk_load(smem + sl * ST_SLOT, src, ST_SLOT, &full[sl]);
         }
+        __syncwarp();
+        if (++sl == ST_SLOTS) { sl = 0; ph ^= 1; }
       }
     }
-    // ---- U = Ut - X (each element is read and written by the same thread)
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    const uint32_t idesc = make_idesc(2, 2, 128, GVS);
+    const uint32_t sb = __shfl_sync(0xffffffffu, smem_u32(smem), 0), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t b1 = sb + ST_SLOTS * ST_SLOT, b2 = b1 + ST_B1;
+    int sl = 0; uint32_t ph = 0; bool ok = true;
+    auto next = [&]() { if (++sl == ST_SLOTS) { sl = 0; ph ^= 1; } };
+    for (int c = 0; c < nch && ok; ++c) {
+      const uint32_t d1 = tm + (c & 1) * GVS;
+      ok = __all_sync(0xffffffffu, mbar_wait(s_ready, c & 1) && (c < 2 || mbar_wait(&o_read[c & 1], ((c >> 1) & 1) ^ 1)));
+      if (!ok) { set_status(status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, blockIdx.y, c); break; }
+      for (int i = 0; i < 4 && ok; ++i) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[sl], ph));
+        tc_fence_after();
+        if (ok && elect_one()) {
+          const uint64_t ad = make_smem_desc_sw128(sb + sl * ST_SLOT), bd = make_smem_desc_sw128(b1 + i * (GVS * 128));
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int col = a * 8 + 2 * t, row = warp * 16 + g;
-      float* u0 = Usm + row * LD32 + col;
-      float* u1 = Usm + (row + 8) * LD32 + col;
-      u0[0] = tf32r(u0[0] - xacc[a][0]); u0[1] = tf32r(u0[1] - xacc[a][1]);
-      u1[0] = tf32r(u1[0] - xacc[a][2]); u1[1] = tf32r(u1[1] - xacc[a][3]);
-    }
-    __syncthreads();
-    // ---- O += P U (P is lower triangular: k-steps up to this warp's diagonal block)
-    {
-      const float* pa = Psm + (warp * 16 + g) * LD64 + t;
-      for (int ks = 0; ks < 2 * (warp + 1); ++ks) {
-        const float p0 = pa[ks * 8], p1 = pa[8 * LD64 + ks * 8], p2 = pa[ks * 8 + 4], p3 = pa[8 * LD64 + ks * 8 + 4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const float* ub = Usm + (ks * 8 + t) * LD32 + a * 8 + g;
-          mma_tf32(oacc[a], p0, p1, p2, p3, ub[0], ub[4 * LD32]);
+          for (int k = 0; k < 4; ++k) umma_tf32(d1, ad + 2 * k, bd + 2 * k, idesc, (i | k) != 0);
+          umma_commit(&empty[sl]);
+          if (i == 3) umma_commit(x_full);
         }
+        __syncwarp();
+        next();
       }
-      const int nvr = min(GC, n - c * GC);
+      if (!ok) { set_status(status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, c); break; }
+      const int ut = sl;                                     // freed with P's tile: U is written, so Ut is read
+      next();
+      ok = __all_sync(0xffffffffu, mbar_wait(u_ready, c & 1));
+      if (!ok) { set_status(status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, c); break; }
+      for (int i = 0; i < 2 && ok; ++i) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[sl], ph));
+        tc_fence_after();
+        if (ok && elect_one()) {
+          const uint64_t ad = make_smem_desc_sw128(sb + sl * ST_SLOT), bd = make_smem_desc_sw128(b2 + i * (GVS * 128));
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int col = h * GD + v0 + a * 8 + 2 * t, row = warp * 16 + g;
-        if (row < nvr)
-          *reinterpret_cast<float2*>(o_raw + static_cast<size_t>(r0 + c * GC + row) * ldo + col) = make_float2(oacc[a][0], oacc[a][1]);
-        if (row + 8 < nvr)
-          *reinterpret_cast<float2*>(o_raw + static_cast<size_t>(r0 + c * GC + row + 8) * ldo + col) = make_float2(oacc[a][2], oacc[a][3]);
+          for (int k = 0; k < 4; ++k) umma_tf32(tm + D3, ad + 2 * k, bd + 2 * k, idesc, (i | k) != 0);
+          umma_commit(&empty[sl]);
+          if (i == 1) umma_commit(s_full);
+        }
+        __syncwarp();
+        next();
+      }
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(&full[sl], ph));
+      if (!ok) { set_status(status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, c); break; }
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint64_t ad = make_smem_desc_sw128(sb + sl * ST_SLOT + i * (GC * 128)), bd = make_smem_desc_sw128(b2 + i * (GVS * 128));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_tf32(d1, ad + 2 * k, bd + 2 * k, idesc, 1);
+        }
+        umma_commit(&empty[sl]);
+        umma_commit(&empty[ut]);
+        umma_commit(&o_full[c & 1]);
+      }
+      __syncwarp();
+      next();
+    }
+  } else {
+    // ------------------------------------------------------------ state, U and O: lanes 32 q .. of tensor memory, value columns 32 hc ..
+    const int q = warp & 3, hc = (warp - 2) >> 2;
+    const int row = q * 32 + lane, v0 = vs * GVS + hc * 32;
+    const uint32_t t_lane = tmem + (static_cast<uint32_t>(q * 32) << 16) + hc * 32;
+    float* Sg = S + ((static_cast<size_t>(slot_id) * Hv + h) * GD + v0) * GD + row;       // value v0 + i: Sg[i * GD]
+    // this thread's float of value row i of an operand tile of 64 rows: key `row` of S^T, row `row - 64` of U^T
+    uint8_t* s_tile = B1 + q * (GVS * 128) + hc * 32 * 128 + (lane & 3) * 4;
+    uint8_t* u_tile = B2 + (q & 1) * (GVS * 128) + hc * 32 * 128 + (lane & 3) * 4;
+    float s[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) s[i] = Sg[i * GD];
+    bool ok = true;
+    auto store_o = [&](int c) {                              // lanes of O: rows of chunk c
+      if (!mbar_wait(&o_full[c & 1], (c >> 1) & 1)) return false;
+      tc_fence_after();
+      uint32_t o[32];
+      tmem_ld_32x32(t_lane + (c & 1) * GVS, o);
+      tmem_ld_wait();
+      tc_fence_before();
+      if (c * GC + row < n) {
+        float4* dst = reinterpret_cast<float4*>(o_raw + static_cast<size_t>(r0 + c * GC + row) * ldo + h * GD + v0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          dst[i] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]), __uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3]));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_read[c & 1]);
+      return true;
+    };
+    float dc = 1.f;
+    for (int c = 0; c <= nch; ++c) {
+      const float dc_next = c < nch ? __ldg(wsh + c * ws_step + WS_DC) : 1.f;
+      if (c > 0) {
+        ok = __all_sync(0xffffffffu, mbar_wait(s_full, (c - 1) & 1));
+        if (!ok) { set_status(status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, c); break; }
+        tc_fence_after();
+        uint32_t d[32];
+        tmem_ld_32x32(t_lane + D3, d);
+        tmem_ld_wait();
+        tc_fence_before();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) s[i] = fmaf(dc, s[i], __uint_as_float(d[i]));
+      }
+      dc = dc_next;
+      if (c < nch) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) *reinterpret_cast<float*>(s_tile + i * 128 + ((((lane >> 2) ^ i) & 7) << 4)) = tf32r(s[i]);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_ready);
+      }
+      if (q < 2) {
+        if (c > 0) {
+          ok = __all_sync(0xffffffffu, store_o(c - 1));
+          if (!ok) { set_status(status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, blockIdx.y, c); break; }
+        }
+      } else if (c < nch) {
+        const int use = 8 * c + 4, sl = use % ST_SLOTS;
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[sl], (use / ST_SLOTS) & 1) && mbar_wait(x_full, c & 1));
+        if (!ok) { set_status(status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, blockIdx.y, c); break; }
+        tc_fence_after();
+        uint32_t x[32];
+        tmem_ld_32x32(t_lane + (c & 1) * GVS, x);
+        const float4* ut = reinterpret_cast<const float4*>(smem + sl * ST_SLOT) + hc * 8 * GC + row - GC;
+        float4 u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] = ut[i * GC];
+        tmem_ld_wait();
+        tc_fence_before();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float uv = i % 4 == 0 ? u[i / 4].x : i % 4 == 1 ? u[i / 4].y : i % 4 == 2 ? u[i / 4].z : u[i / 4].w;
+          *reinterpret_cast<float*>(u_tile + i * 128 + ((((lane >> 2) ^ i) & 7) << 4)) = tf32r(uv - __uint_as_float(x[i]));
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(u_ready);
       }
     }
-    // ---- S <- D_C S + U^T Kt: A[m = v][k = j] = U[j][v], B[k = j][n] = Kt[j][n]
+    if (ok) {
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+      for (int i = 0; i < 32; ++i) Sg[i * GD] = s[i];
+    }
+    if (vs == 0 && hc == 0) {          // conv history for the next call: raw inputs of the last three positions
+      const int hk = h / (Hv / Hk), i = row;
+      float* tl = tail + (static_cast<size_t>(slot_id) * 3 * Hv + h) * 3 * GD;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) sacc[a][b] *= dc;
-    for (int ks = 0; ks < GC / 8; ++ks) {
-      const float* ua = Usm + (ks * 8 + t) * LD32 + smt * 16 + g;
-      const float a0 = ua[0], a1 = ua[8], a2 = ua[4 * LD32], a3 = ua[4 * LD32 + 8];
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const float* kb = Ksm + (ks * 8 + t) * LD128 + sng * 64 + a * 8 + g;
-        mma_tf32(sacc[a], a0, a1, a2, a3, kb[0], kb[4 * LD128]);
+      for (int j = 0; j < 3; ++j) {
+        const __nv_bfloat16* pr = proj + static_cast<size_t>(r0 + n - 3 + j) * ldp;
+        float* tj = tl + static_cast<size_t>(j) * Hv * 3 * GD;
+        tj[i] = __bfloat162float(pr[hk * GD + i]);
+        tj[GD + i] = __bfloat162float(pr[Hk * GD + hk * GD + i]);
+        tj[2 * GD + i] = __bfloat162float(pr[2 * Hk * GD + h * GD + i]);
       }
     }
-    __syncthreads();            // every warp is done with the old S and with this chunk's operands
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int col = sng * 64 + a * 8 + 2 * t, row = smt * 16 + g;
-      Ssm[row * LD128 + col] = tf32r(sacc[a][0]); Ssm[row * LD128 + col + 1] = tf32r(sacc[a][1]);
-      Ssm[(row + 8) * LD128 + col] = tf32r(sacc[a][2]); Ssm[(row + 8) * LD128 + col + 1] = tf32r(sacc[a][3]);
-    }
-    __syncthreads();
   }
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int col = sng * 64 + a * 8 + 2 * t, row = smt * 16 + g;
-    *reinterpret_cast<float2*>(Sg + row * GD + col) = make_float2(sacc[a][0], sacc[a][1]);
-    *reinterpret_cast<float2*>(Sg + (row + 8) * GD + col) = make_float2(sacc[a][2], sacc[a][3]);
-  }
-  if (vs == 0) {          // conv history for the next call: raw inputs of the last three positions
-    const int hk = h / (Hv / Hk), i = tid;
-    float* tl = tail + (static_cast<size_t>(slot) * 3 * Hv + h) * 3 * GD;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const __nv_bfloat16* pr = proj + static_cast<size_t>(r0 + n - 3 + j) * ldp;
-      float* tj = tl + static_cast<size_t>(j) * Hv * 3 * GD;
-      tj[i] = __bfloat162float(pr[hk * GD + i]);
-      tj[GD + i] = __bfloat162float(pr[Hk * GD + hk * GD + i]);
-      tj[2 * GD + i] = __bfloat162float(pr[2 * Hk * GD + h * GD + i]);
-    }
-  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc<256>(tmem); }
 }
 
 // ---------------------------------------------------------------------------------------------- kernel 3
@@ -538,21 +636,20 @@ extern "C" int spark_gdn_chunk_prefill(const void* proj, int ldp, const void* ab
                                        const float* A_log, const float* dt_bias, const float* norm_w, float* S, float* tail,
                                        const int* seg, int nseg, const int* chunks, int n_chunks, const int* seg_chunk0,
                                        float* ws, float* o_raw, void* out, int ldo, int Hk, int Hv, int D, float eps,
-                                       cudaStream_t s) {
+                                       int* status, cudaStream_t s) {
   if (n_chunks <= 0) return 0;
-  if (D != GD || Hv % Hk) return -5;
-  constexpr int SM2 = (3 * GC * LD128 + GC * LD64 + GC * LD32 + GVS * LD128) * 4;
+  if (D != GD || Hv % Hk || ((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(o_raw)) & 15)) return -5;
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREP_SMEM);
-    cudaFuncSetAttribute(gdn_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM2);
+    cudaFuncSetAttribute(gdn_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM);
     attr = true;
   }
   gdn_chunk_prep_kernel<<<dim3(n_chunks, Hv), 256, PREP_SMEM, s>>>((const __nv_bfloat16*)proj, ldp, (const __nv_bfloat16*)ab, ldab,
                                                               conv_w, A_log, dt_bias, tail, seg, chunks, ws, Hk, Hv, eps,
                                                                   (reinterpret_cast<uintptr_t>(conv_w) & 15) == 0);
-  gdn_chunk_state_kernel<<<dim3(GD / GVS, Hv, nseg), 128, SM2, s>>>(ws, seg, seg_chunk0, (const __nv_bfloat16*)proj, ldp, S,
-                                                                    tail, o_raw, Hv * GD, Hk, Hv);
+  gdn_chunk_state_kernel<<<dim3(GD / GVS, Hv, nseg), ST_THREADS, ST_SMEM, s>>>(ws, seg, seg_chunk0, (const __nv_bfloat16*)proj, ldp, S,
+                                                                              tail, o_raw, Hv * GD, Hk, Hv, status);
   gdn_chunk_out_kernel<<<dim3(n_chunks, Hv), 256, 0, s>>>(o_raw, Hv * GD, (const __nv_bfloat16*)proj, ldp, norm_w, seg, chunks,
                                                           (__nv_bfloat16*)out, ldo, Hk, Hv, eps);
   return spark_launch_rc(__func__);

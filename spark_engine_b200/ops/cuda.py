@@ -65,7 +65,7 @@ _SIGS = {
     "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp],
     "spark_exl3_had_gather": [vp, i32, vp, vp, i32, vp, i64, vp, i32, i32, i32, vp],
     "spark_gdn_chunk_prefill": [vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32,
-                                i32, f32, vp],
+                                i32, f32, vp, vp],
     "spark_attn_prep": [vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp, vp, vp, vp,
                         vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
     "spark_attn_decode": [vp, vp, vp, vp, vp, i32, vp, vp, vp, vp, i32, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32,
@@ -1013,7 +1013,7 @@ def _gdn_chunk_prefill(mixer, proj, ab, plan, d, out):
     rc = dll.spark_gdn_chunk_prefill(P(proj), proj.stride(0), P(ab), ab.stride(0), P(w["conv"]), P(w["A_log"]),
                                      P(w["dt_bias"]), P(w["norm"]), P(mixer.S), P(mixer.tail), P(d["seg"]), len(plan.segs),
                                      P(chunks), nch, P(first), P(ws), P(o_raw), P(out), out.stride(0), c.n_k_heads,
-                                     c.n_v_heads, c.head_dim, float(mixer.cfg.norm_eps), stream())
+                                     c.n_v_heads, c.head_dim, float(mixer.cfg.norm_eps), P(status_word(dev)), stream())
     check(rc, "spark_gdn_chunk_prefill")
     return out
 
