@@ -72,7 +72,10 @@ extern "C" int spark_gemm_bf16(const void* A, const void* B, void* C, int M, int
   GemmArgs g{};
   g.M = M; g.N = N; g.K = K; g.status = status; g.ab_fmt = fmt;
   const int mt = (M + GEMM_BM - 1) / GEMM_BM;
-  if (N > 128) {
+  // 256 columns per tile unless 128 are less time by whole waves: few tiles leave SMs idle, and a ragged N pays for the columns it does not
+  // have (1021 rows of 1024 / 513 columns, 8192 rows of 513)
+  const int w256 = (mt * ((N + 255) / 256) + num_sms() - 1) / num_sms() * 256, w128 = (mt * ((N + 127) / 128) + num_sms() - 1) / num_sms() * 128;
+  if (N > 128 && w256 <= w128 + w128 / 4) {
     g.num_n_tiles = (N + 255) / 256; g.num_tiles = mt * g.num_n_tiles;
     int grid = g.num_tiles < num_sms() ? g.num_tiles : num_sms();
     if (out_f32) return launch<256, EpiStoreF32, false>(tA, tB, g, EpiStoreF32{(float*)C, ldc, N}, grid, stream);

@@ -63,6 +63,7 @@ _SIGS = {
     "spark_attn_prefill_masked": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp, vp, i32, i32, vp,
                                   i32, i64, vp, vp],
     "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp],
+    "spark_gemm_exl3": [vp, i32, vp, vp, vp, i32, i32, i32, i32, vp, vp],
     "spark_exl3_had_gather": [vp, i32, vp, vp, i32, vp, i64, vp, i32, i32, i32, vp],
     "spark_gdn_chunk_prefill": [vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32,
                                 i32, f32, vp, vp],
@@ -500,6 +501,16 @@ def exl3_tc(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, glu: Opti
 
 
 EXL3_RESIDENT_MAX_BYTES = int(os.environ.get("SPARK_EXL3_RESIDENT_MB", "4096")) << 20
+def gemm_exl3(xh, wt, svh):
+    """had128(xh [M, K] @ wt [N, K]^T) * svh [N] -> bf16 [M, N] (fp16 operands, the transform in the product's epilogue)."""
+    M, K = xh.shape
+    N = wt.shape[0]
+    y = torch.empty(M, N, dtype=torch.bfloat16, device=xh.device)
+    rc = lib().spark_gemm_exl3(P(xh), xh.stride(0), P(wt), P(svh), P(y), N, M, N, K, P(status_word(xh.device)), stream())
+    check(rc, "spark_gemm_exl3")
+    return y
+
+
 _exl3_resident_bytes = 0
 
 
@@ -526,8 +537,7 @@ def exl3_linear(x, w: Exl3Weight):
     wt = _exl3_resident(w) if (x.shape[0] <= 16 and not w.experts) else None
     if wt is None:
         wt = exl3_reconstruct(w, scratch("exl3_recon", w.n * w.k, torch.float16, x.device)[: w.n * w.k].view(w.n, w.k))
-    acc = gemm_bf16(xh, wt, out_f32=True, fmt=0)
-    return exl3_had_rows(acc, w.svh, post=True)
+    return gemm_exl3(xh, wt, w.svh)
 
 
 def quant_linear(x, w: QuantWeight):
@@ -758,7 +768,10 @@ def moe_route(h, w, c, e_lo=0, e_hi=None, self_w=None):
     """`self_w` fp32 [R]: gets the weight of a row's identity experts."""
     R = h.shape[0]
     dev = h.device
-    logits = dense_linear(h, w["gate"], out_f32=True)
+    # (rows of the logits start on 16 bytes: 513 columns of 8192 rows, stored one by one, were 110 us of product)
+    n = w["gate"].shape[0]
+    padded = torch.empty(R, (n + 3) // 4 * 4, dtype=torch.float32, device=dev) if R > 16 else None
+    logits = dense_linear(h, w["gate"], out_f32=True, out=None if padded is None else padded[:, :n])
     wts = torch.empty(R, c.top_k, dtype=torch.float32, device=dev)
     ids = torch.empty(R, c.top_k, dtype=torch.int32, device=dev)
     prow = torch.empty(R, c.top_k, dtype=torch.int32, device=dev)
