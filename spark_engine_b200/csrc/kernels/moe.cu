@@ -168,12 +168,13 @@ constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16, ROUTER_COLS = 4;
 // 8.4 us, 16 rows 32 -> 16.7, 4 rows of the MXFP4 preset 37 -> 17 (before: a warp per column for all rows, the rows staged in shared
 // memory, two rows' choices after one another).  Tensor cores in place of the FP32 units (9.3, 13, 16 us) add 16 products at a time
 // with fewer bits: the logits' error grew 1.2 to 15 times over K = 256 .. 7168.
-template <int EPL, int NR>                                  // NR: rows of a warp (R <= 4 NR)
+// KIND: 0, 1 and 2 alone, 3 the others (the kernel is fetched anew in every layer: what a kind does not run costs instruction misses)
+template <int EPL, int NR, int KIND>                        // NR: rows of a warp (R <= 4 NR)
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
   __shared__ int last_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int R = a.R;
+  const int R = a.R, kind = KIND == 3 ? a.kind : KIND;
   const int NE = a.E + (a.shared_gate ? 1 : 0);
   const int n = blockIdx.x * ROUTER_COLS + (warp & 3), r0 = warp >> 2;
   const int KV = a.K >> 3;                                  // 16-byte vectors of a row
@@ -223,7 +224,10 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
     }
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-      const float v = warp_sum(acc[i]);
+      float v = warp_sum(acc[i]);
+      // kinds whose score is a function of the logit alone are scored here, on every SM, and not by the last CTA
+      if (n < a.E && kind == 1) v = 1.f / (1.f + expf(-v));
+      if (n < a.E && kind == 2) v = sqrtf(v > 20.f ? v : log1pf(expf(v)));
       if (lane == 0 && r0 + 4 * i < R) a.logits[static_cast<size_t>(r0 + 4 * i) * a.ld + n] = v;
     }
   }
@@ -249,19 +253,19 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
     for (int j = 0; j < EPL; ++j) {
       const int e = lane + 32 * j;
       p[j] = (j < nj && e < a.E) ? __ldcg(lg + e) : -INFINITY;
-      if (a.kind == 5 && a.bias && j < nj && e < a.E) p[j] += a.bias[e];
+      if (kind == 5 && a.bias && j < nj && e < a.E) p[j] += a.bias[e];
       s[j] = p[j];
       mx = fmaxf(mx, p[j]);
     }
-    if (a.kind == 4) {
+    if (kind == 4) {
       // ranked by the logits, only the k winners' sigmoids are formed
-    } else if (a.kind == 5) {
+    } else if (kind == 5) {
       mx = warp_max(mx);
-    } else if (a.kind == 0) {
+    } else if (kind == 0) {
       // softmax -> top-k -> renormalise: the softmax denominator cancels, so experts are ranked by their logits and
       // only the k winners are exponentiated
       mx = warp_max(mx);
-    } else if (a.kind == 3) {
+    } else if (kind == 3) {
       // the bias is added to the probabilities, so the ranking needs the denominator
       mx = warp_max(mx);
       float sum = 0.f;
@@ -282,11 +286,8 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
 #pragma unroll
       for (int j = 0; j < EPL; ++j) {
         const int e = lane + 32 * j;
-        if (j < nj && e < a.E) {
-          const float v = p[j];
-          p[j] = a.kind == 1 ? 1.f / (1.f + expf(-v)) : sqrtf(v > 20.f ? v : log1pf(expf(v)));
-          s[j] = p[j] + (a.bias ? a.bias[e] : 0.f);
-        } else { p[j] = 0.f; s[j] = -INFINITY; }
+        if (j < nj && e < a.E) s[j] = p[j] + (a.bias ? a.bias[e] : 0.f);
+        else { p[j] = 0.f; s[j] = -INFINITY; }
       }
     }
     float selp = 0.f; int seli = -1;                        // lane k keeps slot k's weight numerator and expert
@@ -305,16 +306,16 @@ moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
       if (wi == cand && wi != 0x7fffffff) {                 // this lane owns the winner
 #pragma unroll
         for (int j = 0; j < EPL; ++j) if (j == bj) { bp = p[j]; s[j] = -INFINITY; }
-        if (a.kind == 0) bp = __expf(bp - mx);
-        if (a.kind == 5) bp = expf(bp - mx);
-        if (a.kind == 4) bp = 1.f / (1.f + expf(-bp));
+        if (kind == 0) bp = __expf(bp - mx);
+        if (kind == 5) bp = expf(bp - mx);
+        if (kind == 4) bp = 1.f / (1.f + expf(-bp));
         lane_best(s, best, bj);
       }
       const float wp = __shfl_sync(0xffffffffu, bp, wi & 31);
       if (lane == k) { selp = wp; seli = wi; }
       tot += wp;                                            // slot order, identical on every lane
     }
-    tot = a.kind == 4 ? 1.f : fmaxf(tot, 1e-20f);
+    tot = kind == 4 ? 1.f : fmaxf(tot, 1e-20f);
     if (a.self_w) {
       float own = 0.f;
       for (int k = 0; k < a.top_k; ++k) {                   // slot order, as the combine adds the others
@@ -407,40 +408,8 @@ moe_combine_norm_kernel(const float* __restrict__ y, const float* __restrict__ w
 }
 
 // ---------------------------------------------------------------------------------- counting sort
-// One CTA.  ids [P] expert per pair (P = R*top_k).  Outputs: perm[P] (pair index in expert order),
-// offsets[E+1], tile_list[int4] of <=128-row tiles {row0, row_end, expert, 0}, tile_count.
-__global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ perm, int* __restrict__ inv_perm,
-                int* __restrict__ offsets, int4* __restrict__ tile_list, int* __restrict__ tile_count) {
-  extern __shared__ int sh[];          // counts[E], starts[E+1]
-  int* cnt = sh; int* start = sh + E;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < P; i += blockDim.x) if (ids[i] >= 0) atomicAdd(&cnt[ids[i]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0, nt = 0;
-    for (int e = 0; e < E; ++e) {
-      start[e] = acc; offsets[e] = acc;
-      for (int r0 = 0; r0 < cnt[e]; r0 += 128) tile_list[nt++] = make_int4(acc + r0, acc + cnt[e], e, 0);
-      acc += cnt[e];
-    }
-    start[E] = acc; offsets[E] = acc; *tile_count = nt;
-  }
-  __syncthreads();
-  // stable placement: pair i goes to start[e] + (number of earlier pairs with the same expert)
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    const int e = ids[i];
-    if (e < 0) { if (inv_perm) inv_perm[i] = -1; continue; }   // not a local expert
-    int rank = 0;
-    for (int j = 0; j < i; ++j) rank += (ids[j] == e);     // P is small on the decode path
-    perm[start[e] + rank] = i;
-    if (inv_perm) inv_perm[i] = start[e] + rank;
-  }
-}
-
-// Prefill-size stable sort: rank of pair i inside its expert = exclusive count over earlier pairs.
-// Two passes over blocks of pairs with per-block histograms (deterministic, int atomics only in smem).
+// ids [P] expert per pair (P = R * top_k) -> perm [P] (pair index in expert order), offsets [E + 1], list of row tiles, its length.
+// Stable: rank of pair i inside its expert = exclusive count over earlier pairs.  Two passes over blocks of pairs with per-block histograms (deterministic, int atomics only in smem).
 __global__ void moe_hist_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ block_hist) {
   extern __shared__ int sh[];
   for (int e = threadIdx.x; e < E; e += blockDim.x) sh[e] = 0;
@@ -455,7 +424,7 @@ __global__ void moe_hist_kernel(const int* __restrict__ ids, int P, int E, int* 
 // own tiles; a single thread walking the 512 experts took 72 us per layer of a prefill chunk.
 __global__ void __launch_bounds__(1024)
 moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restrict__ offsets,
-                int4* __restrict__ tile_list, int* __restrict__ tile_count) {
+                int4* __restrict__ tile_list, int* __restrict__ tile_count, int tile_rows) {
   extern __shared__ int tot[];                         // [E]
   __shared__ int sa[1024], sb[1024];
   const int e = threadIdx.x;
@@ -476,7 +445,7 @@ moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restric
     tot[e] = acc;
     mine = acc;
   }
-  const int my_tiles = (mine + 127) / 128;
+  const int my_tiles = (mine + tile_rows - 1) / tile_rows;
   sa[e] = mine; sb[e] = my_tiles;
   __syncthreads();
   for (int st = 1; st < 1024; st <<= 1) {               // inclusive scans of rows and of tiles
@@ -488,7 +457,12 @@ moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restric
   if (e < E) {
     const int off = sa[e] - mine, t0 = sb[e] - my_tiles;
     offsets[e] = off;
-    for (int i = 0; i < my_tiles; ++i) tile_list[t0 + i] = make_int4(off + i * 128, off + mine, e, 0);
+    if (tile_rows == 128) {                              // the consumer cuts a tile at the expert's end
+      for (int i = 0; i < my_tiles; ++i) tile_list[t0 + i] = make_int4(off + i * 128, off + mine, e, 0);
+    } else if (my_tiles) {                               // even split
+      const int q = mine / my_tiles, more = mine % my_tiles;
+      for (int i = 0; i < my_tiles; ++i) tile_list[t0 + i] = make_int4(off + i * q + min(i, more), off + mine, e, q + (i < more));
+    }
     if (e == E - 1) { offsets[E] = sa[e]; *tile_count = sb[e]; }
   }
 }
@@ -510,24 +484,25 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, int P, int E, cons
 
 // ---------------------------------------------------------------------------------- combine
 // res[R,H] += sum_slot w[r,slot] * y[pair_pos(r,slot), :] (+ sg[r] * shared[r,:]).  y fp32 or bf16.
-// A thread owns V consecutive columns (one 16-byte load of y per slot; V = 1 where H or an address does not allow it) and asks for
-// four slots before it adds them, in slot order.  Bound by reading y: 8192 rows of 2048, ten bf16 slots, took 224 us with one
-// column per thread and take 110 (3.4 TB/s); 2048 rows of 4096, eight fp32 slots, 91 -> 49.
-template <int V, typename T> __device__ __forceinline__ void ldv(const T* p, float (&v)[V]) {
-  if (V * sizeof(T) == 16) {
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
-    if (sizeof(T) == 4) {
-      v[0] = __uint_as_float(r.x); v[1 % V] = __uint_as_float(r.y); v[2 % V] = __uint_as_float(r.z); v[3 % V] = __uint_as_float(r.w);
-    } else {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
-#pragma unroll
-      for (int i = 0; i < V / 2; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < V; ++i) v[i] = static_cast<float>(p[i]);
-  }
+// A thread owns V consecutive columns (one 16-byte load of y per slot; V = 1 where H or an address does not allow it).  The row's slots
+// are looked up once per CTA, and a thread's loads of eight slots are issued before the first is widened (a load and its widening in one
+// branch per slot waited for every slot by itself).  Added in slot order.  Bound by reading y: 8192 rows of 2048, ten bf16 slots, took
+// 224 us with one column per thread and 110 with a vector; 2048 rows of 4096, eight fp32 slots, 91 and 49.
+template <int V, typename T> struct CombVec { typedef T type; };
+template <> struct CombVec<4, float> { typedef uint4 type; };
+template <> struct CombVec<8, __nv_bfloat16> { typedef uint4 type; };
+__device__ __forceinline__ void comb_widen(const uint4& r, float (&v)[4]) {
+  v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2] = __uint_as_float(r.z); v[3] = __uint_as_float(r.w);
 }
+__device__ __forceinline__ void comb_widen(const uint4& r, float (&v)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
+__device__ __forceinline__ void comb_widen(const float& r, float (&v)[1]) { v[0] = r; }
+__device__ __forceinline__ void comb_widen(const __nv_bfloat16& r, float (&v)[1]) { v[0] = __bfloat162float(r); }
+
+constexpr int COMB_SLOTS = 32, COMB_U = 8;
 
 template <typename TY, int V>
 __global__ void __launch_bounds__(256)
@@ -535,51 +510,67 @@ moe_combine_kernel(float* __restrict__ res, const TY* __restrict__ y, const int*
                    const float* __restrict__ wts, int top_k, const __nv_bfloat16* __restrict__ shared,
                    const float* __restrict__ sg, int H, __nv_bfloat16* __restrict__ out_bf16,
                    const int* __restrict__ pair_expert) {
+  typedef typename CombVec<V, TY>::type Raw;
+  __shared__ int row_s[COMB_SLOTS];                           // row of y, -1: the expert lives on another rank
+  __shared__ float w_s[COMB_SLOTS];
   const int r = blockIdx.x;
   const float gate = shared && sg ? sg[r] : 1.f;
-  for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * V; i < H; i += gridDim.y * blockDim.x * V) {
-    float acc[V];
+  const int i = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+  float acc[V];
 #pragma unroll
-    for (int j = 0; j < V; ++j) acc[j] = 0.f;
-    for (int k0 = 0; k0 < top_k; k0 += 4) {
-      float v[4][V], w[4];
-      bool live[4];
+  for (int j = 0; j < V; ++j) acc[j] = 0.f;
+  for (int s0 = 0; s0 < top_k; s0 += COMB_SLOTS) {
+    const int n = min(top_k - s0, COMB_SLOTS);
+    if (s0) __syncthreads();
+    if (threadIdx.x < n) {
+      const int pi = r * top_k + s0 + threadIdx.x;
+      row_s[threadIdx.x] = pair_expert && pair_expert[pi] < 0 ? -1 : (inv_perm ? inv_perm[pi] : pi);
+      w_s[threadIdx.x] = wts[pi];
+    }
+    __syncthreads();
+    if (i >= H) continue;
+    for (int k0 = 0; k0 < n; k0 += COMB_U) {
+      Raw raw[COMB_U];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int pi = r * top_k + min(k0 + u, top_k - 1);
-        live[u] = k0 + u < top_k && !(pair_expert && pair_expert[pi] < 0);       // else: no slot, or the expert lives on another rank
-        const int row = inv_perm ? inv_perm[pi] : pi;
-        w[u] = wts[pi];
-        if (live[u]) ldv<V>(y + static_cast<size_t>(row) * H + i, v[u]);
+      for (int u = 0; u < COMB_U; ++u) {
+        const int row = k0 + u < n ? row_s[k0 + u] : -1;
+        if (row >= 0) raw[u] = __ldg(reinterpret_cast<const Raw*>(y + static_cast<size_t>(row) * H + i));
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (live[u]) {
+      for (int u = 0; u < COMB_U; ++u)
+        if (k0 + u < n && row_s[k0 + u] >= 0) {
+          float v[V];
+          comb_widen(raw[u], v);
 #pragma unroll
-          for (int j = 0; j < V; ++j) acc[j] = fmaf(w[u], v[u][j], acc[j]);
+          for (int j = 0; j < V; ++j) acc[j] = fmaf(w_s[k0 + u], v[j], acc[j]);
         }
     }
-    const size_t o = static_cast<size_t>(r) * H + i;
-    if (shared) {
+  }
+  if (i >= H) return;
+  const size_t o = static_cast<size_t>(r) * H + i;
+  if (shared) {
+    uint32_t sw[(V + 1) / 2];                                 // V consecutive elements, as one load
+    if (V == 8) { const uint4 t = *reinterpret_cast<const uint4*>(shared + o); sw[0] = t.x; sw[1 % ((V + 1) / 2)] = t.y; sw[2 % ((V + 1) / 2)] = t.z; sw[3 % ((V + 1) / 2)] = t.w; }
+    else if (V == 4) { const uint2 t = *reinterpret_cast<const uint2*>(shared + o); sw[0] = t.x; sw[1 % ((V + 1) / 2)] = t.y; }
+    else sw[0] = reinterpret_cast<const uint16_t*>(shared)[o];
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const float s = __bfloat162float(shared[o + j]);
-        acc[j] += sg ? gate * s : s;
-      }
+    for (int j = 0; j < V; ++j) {
+      const float s = __uint_as_float(j & 1 ? sw[j >> 1] & 0xffff0000u : sw[j >> 1] << 16);
+      acc[j] += sg ? gate * s : s;
     }
-    if (res) {
+  }
+  if (res) {
 #pragma unroll
-      for (int j = 0; j < V; ++j) res[o + j] += acc[j];
-    }
-    if (out_bf16) {
-      if (V == 1) {
-        out_bf16[o] = __float2bfloat16(acc[0]);
-      } else {
+    for (int j = 0; j < V; ++j) res[o + j] += acc[j];
+  }
+  if (out_bf16) {
+    if (V == 1) {
+      out_bf16[o] = __float2bfloat16(acc[0]);
+    } else {
 #pragma unroll
-        for (int j = 0; j < V; j += 4) {
-          const __nv_bfloat162 b0 = __floats2bfloat162_rn(acc[j % V], acc[(j + 1) % V]), b1 = __floats2bfloat162_rn(acc[(j + 2) % V], acc[(j + 3) % V]);
-          *reinterpret_cast<uint2*>(out_bf16 + o + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
-        }
+      for (int j = 0; j < V; j += 4) {
+        const __nv_bfloat162 b0 = __floats2bfloat162_rn(acc[j % V], acc[(j + 1) % V]), b1 = __floats2bfloat162_rn(acc[(j + 2) % V], acc[(j + 3) % V]);
+        *reinterpret_cast<uint2*>(out_bf16 + o + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
       }
     }
   }
@@ -609,18 +600,15 @@ extern "C" int spark_moe_route(const float* logits, int ld, int R, int E, int to
 }
 
 // Scratch `block_hist` must hold ceil(P/256) * E ints when P > 2048.
+// tile_rows 128: tiles {row, end of the expert, expert, 0} of up to 128 rows; another number: even tiles {row, end, expert, rows} of up to that.
 extern "C" int spark_moe_sort(const int* ids, int P, int E, int* perm, int* inv_perm, int* offsets, void* tile_list,
-                              int* tile_count, int* block_hist, cudaStream_t s) {
+                              int* tile_count, int* block_hist, cudaStream_t s, int tile_rows) {
   if (P <= 0) return 0;
-  if (E > 1024) return -5;                     // one thread per expert in the scan
-  if (P <= 2048) {
-    moe_sort_kernel<<<1, 1024, (2 * E + 1) * sizeof(int), s>>>(ids, P, E, perm, inv_perm, offsets, (int4*)tile_list, tile_count);
-  } else {
-    const int nb = (P + 255) / 256;
-    moe_hist_kernel<<<nb, 256, E * sizeof(int), s>>>(ids, P, E, block_hist);
-    moe_scan_kernel<<<1, 1024, E * sizeof(int), s>>>(block_hist, nb, E, offsets, (int4*)tile_list, tile_count);
-    moe_place_kernel<<<nb, 256, 256 * sizeof(int), s>>>(ids, P, E, block_hist, offsets, perm, inv_perm);
-  }
+  if (E > 1024 || tile_rows < 16 || tile_rows > 192) return -5;                     // one thread per expert in the scan
+  const int nb = (P + 255) / 256;
+  moe_hist_kernel<<<nb, 256, E * sizeof(int), s>>>(ids, P, E, block_hist);
+  moe_scan_kernel<<<1, 1024, E * sizeof(int), s>>>(block_hist, nb, E, offsets, (int4*)tile_list, tile_count, tile_rows);
+  moe_place_kernel<<<nb, 256, 256 * sizeof(int), s>>>(ids, P, E, block_hist, offsets, perm, inv_perm);
   return spark_launch_rc(__func__);
 }
 
@@ -628,7 +616,7 @@ extern "C" int spark_moe_combine(float* res, const void* y, int y_f32, const int
                                  int top_k, const void* shared, const float* sg, int H, void* out_bf16, cudaStream_t s,
                                  const int* pair_expert) {
   if (R <= 0) return 0;
-  const bool wide = H % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out_bf16)) & 15) == 0;
+  const bool wide = H % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out_bf16) | reinterpret_cast<uintptr_t>(shared)) & 15) == 0;
 #define SPARK_CMB(T, V) launch_combine<T, V>(res, y, inv_perm, wts, R, top_k, shared, sg, H, out_bf16, pair_expert, s)
   if (y_f32) { if (wide) SPARK_CMB(float, 4); else SPARK_CMB(float, 1); }
   else { if (wide) SPARK_CMB(__nv_bfloat16, 8); else SPARK_CMB(__nv_bfloat16, 1); }
@@ -656,13 +644,17 @@ extern "C" int spark_moe_router_topk(const void* x, int ldx, const void* Wg, int
   a.wts = wts; a.ids = ids; a.pair_row = pair_row; a.sg = sg; a.counter = counter;
   const int NE = E + (shared_gate ? 1 : 0);
   // experts per lane: the narrowest form that holds E (a lane's work per choice grows with it)
-  auto pick = [&](auto rows) {
-    constexpr int NR = decltype(rows)::value;
-    return E <= 64 ? moe_router_topk_kernel<2, NR> : E <= 256 ? moe_router_topk_kernel<8, NR>
-         : E <= 512 ? moe_router_topk_kernel<16, NR> : moe_router_topk_kernel<32, NR>;
+  auto pick = [&](auto rows, auto knd) {
+    constexpr int NR = decltype(rows)::value, KD = decltype(knd)::value;
+    return E <= 64 ? moe_router_topk_kernel<2, NR, KD> : E <= 256 ? moe_router_topk_kernel<8, NR, KD>
+         : E <= 512 ? moe_router_topk_kernel<16, NR, KD> : moe_router_topk_kernel<32, NR, KD>;
   };
-  void (*kern)(RouterArgs) = R <= 4 ? pick(std::integral_constant<int, 1>{}) : R <= 8 ? pick(std::integral_constant<int, 2>{})
-                                    : pick(std::integral_constant<int, 4>{});
+  auto of = [&](auto knd) {
+    return R <= 4 ? pick(std::integral_constant<int, 1>{}, knd) : R <= 8 ? pick(std::integral_constant<int, 2>{}, knd)
+                  : pick(std::integral_constant<int, 4>{}, knd);
+  };
+  void (*kern)(RouterArgs) = kind == 0 ? of(std::integral_constant<int, 0>{}) : kind == 1 ? of(std::integral_constant<int, 1>{})
+                           : kind == 2 ? of(std::integral_constant<int, 2>{}) : of(std::integral_constant<int, 3>{});
   const cudaError_t err = spark_launch_pdl(kern, dim3((NE + ROUTER_COLS - 1) / ROUTER_COLS), dim3(ROUTER_WARPS * 32), 0, s, dim3(1, 1, 1), a);
   return err == cudaSuccess ? 0 : -4;
 }

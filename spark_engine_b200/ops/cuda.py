@@ -72,7 +72,7 @@ _SIGS = {
     "spark_attn_decode": [vp, vp, vp, vp, vp, i32, vp, vp, vp, vp, i32, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32,
                           f32, vp, vp, vp, vp, vp, i32],
     "spark_moe_route": [vp, i32, i32, i32, i32, i32, vp, f32, i32, vp, vp, vp, vp, vp, i32, i32, i32, vp],
-    "spark_moe_sort": [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp],
+    "spark_moe_sort": [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32],
     "spark_moe_combine": [vp, vp, i32, vp, vp, i32, i32, vp, vp, i32, vp, vp, vp],
     "spark_exl3_gemv": [vp, i32, vp, vp, vp, i64, i64, i64, vp, i32, i32, vp, vp, i32, i32, i32, i32, i32, i32,
                         f32, i32, vp, vp, i32],
@@ -795,18 +795,19 @@ def _expert_gemv(x, w, pairs, pair_expert, pair_row, act, limit, out_f32, pairs_
                      limit=limit, out_f32=out_f32, expert_stride=N * K, n=N, k=K)
 
 
-def moe_sort(ids, E):
+def moe_sort(ids, E, tile_rows=128):
+    """`tile_rows`: 128, or another number for the even tiles that `exl3_tc` (up to 192) and `moe_mxfp4_tc` (up to 128) alone take."""
     Pn = ids.numel()
     dev = ids.device
     dbg.check_index("moe_sort expert ids", ids, 0, E, allow=-1)
     perm = torch.zeros(Pn, dtype=torch.int32, device=dev)      # entries past the local pairs stay valid indices
     inv = torch.empty(Pn, dtype=torch.int32, device=dev)
     offs = torch.empty(E + 1, dtype=torch.int32, device=dev)
-    max_tiles = (Pn + 127) // 128 + E
+    max_tiles = (Pn + tile_rows - 1) // tile_rows + E
     tiles = torch.empty(max_tiles, 4, dtype=torch.int32, device=dev)
     ntile = torch.empty(1, dtype=torch.int32, device=dev)
     hist = scratch("moe_hist", ((Pn + 255) // 256) * E, torch.int32, dev)
-    rc = lib().spark_moe_sort(P(ids), Pn, E, P(perm), P(inv), P(offs), P(tiles), P(ntile), P(hist), stream())
+    rc = lib().spark_moe_sort(P(ids), Pn, E, P(perm), P(inv), P(offs), P(tiles), P(ntile), P(hist), stream(), tile_rows)
     check(rc, "spark_moe_sort")
     return perm, inv, offs, tiles, ntile, max_tiles
 
