@@ -62,7 +62,7 @@ _SIGS = {
     "spark_attn_prefill": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, i32, i64, vp, vp],
     "spark_attn_prefill_masked": [vp, vp, vp, vp, vp, i32, i32, vp, i32, i32, vp, i32, i32, i32, f32, vp, vp, i32, i32, vp,
                                   i32, i64, vp, vp],
-    "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp],
+    "spark_exl3_tc": [vp, i32, i32, vp, vp, i64, i64, vp, i64, vp, vp, i32, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32],
     "spark_gemm_exl3": [vp, i32, vp, vp, vp, i32, i32, i32, i32, vp, vp],
     "spark_exl3_had_gather": [vp, i32, vp, vp, i32, vp, i64, vp, i32, i32, i32, vp],
     "spark_gdn_chunk_prefill": [vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32,
@@ -400,9 +400,9 @@ EXL3_CTAS = 5 * 148                # CTAs of the EXL3 GEMV that run at a time
 def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> int:
     """K-slices per 128-column strip = CTAs of one cluster (<= 8).  Rows of one matrix (summed slice by slice, so that S may
     depend on K and N only): as many as run at a time.  `pairs` of a row and an expert (summed in chunks of 256, whatever S is): the same for all
-    `items`, and further while a slice keeps 1024 k and two waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048 24.5 / 16.3 / 12.7 / 11.6, 40 pairs 33.7 / 29.1 /
-    29.4 / 34.0, 160 pairs 85 / 86 / 96 / 120; 40 pairs of 2048 x 512 17.6 / 21.0 / 28.9; 16 pairs of 3072 x 4096 - / 62.7 / 58.8 / 61.7; one row
-    of 12288 x 2048 15.1 / 12.8 / 10.6 / 11.7.  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS force the count for single-matrix / per-pair launches."""
+    `items`, and further while a slice keeps 1024 k and two waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048 19.0 / 14.8 / 12.6 / 11.5, 40 pairs 32.4 / 27.8 /
+    29.0 / 33.4, 160 pairs 82 / 85 / 96 / 119; 40 pairs of 2048 x 512 17.2 / 21.1 / 30.3; 16 pairs of 3072 x 4096 - / 58.7 / 54.9 / 61.5; one row
+    of 12288 x 2048 12.9 / 12.2 / 10.4 / 11.8.  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS force the count for single-matrix / per-pair launches."""
     blocks = K // 128
     forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if pairs else "SPARK_EXL3_S", "0"))
     if forced and blocks % forced == 0:
@@ -486,21 +486,26 @@ def exl3_had_gather(x, scale, perm, ids, expert_stride):
     return y
 
 
-def exl3_tc(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, glu: Optional[Exl3Weight] = None, limit=0.0):
+def exl3_tc(xh, w: Exl3Weight, tiles, ntile, max_tiles, out_f32=False, glu: Optional[Exl3Weight] = None, limit=0.0,
+            tile_rows=128):
     """Rows in expert order (fp16, input transform applied) x expert trellises on tcgen05 -> [P, N], output transform applied.
-    `glu`: w is [gate | up]; the result is the fp16 input [P, F] of the product with `glu` (gated, its input transform applied)."""
+    `glu`: w is [gate | up]; the result is the fp16 input [P, F] of the product with `glu` (gated, its input transform applied).
+    `tile_rows`: what `tiles` was made with."""
     Pn, K = xh.shape
     n = w.n // 2 if glu is not None else w.n
     y = torch.empty(Pn, n, dtype=torch.float16 if glu is not None else torch.float32 if out_f32 else torch.bfloat16, device=xh.device)
     t = w.trellis if P(w.trellis) % 16 == 0 else w.trellis.clone()      # the kernel's bulk copies start on 16 bytes
     rc = lib().spark_exl3_tc(P(xh), xh.stride(0), Pn, P(t), P(w.svh), (K // 16) * (w.n // 16) * 32, w.n,
                              P(glu.suh) if glu is not None else None, n, P(tiles), P(ntile), max_tiles, P(y), n, int(out_f32), K, w.n,
-                             int(glu is not None), float(limit), 0 if w.kind == "mul1" else 1, P(status_word(xh.device)), stream())
+                             int(glu is not None), float(limit), 0 if w.kind == "mul1" else 1, P(status_word(xh.device)), stream(),
+                             int(tile_rows > 96))
     check(rc, "spark_exl3_tc")
     return y
 
 
 EXL3_RESIDENT_MAX_BYTES = int(os.environ.get("SPARK_EXL3_RESIDENT_MB", "4096")) << 20
+
+
 def gemm_exl3(xh, wt, svh):
     """had128(xh [M, K] @ wt [N, K]^T) * svh [N] -> bf16 [M, N] (fp16 operands, the transform in the product's epilogue)."""
     M, K = xh.shape
@@ -957,11 +962,12 @@ def moe(h, w, c, defer: bool = False):
         y = _expert_gemv(gu, wd, Pn, pe, None, 1, c.swiglu_limit, True)            # [P, H] fp32
         inv = None
     else:
-        perm, inv, offs, tiles, ntile, max_tiles = moe_sort(ids.view(-1), (ep[1] - ep[0]) if ep else c.n_experts)
+        from . import exl3_moe
+        tile_rows = exl3_moe.tile_rows(wgu, wd, Pn, c.n_experts) if isinstance(wgu, Exl3Weight) else 128
+        perm, inv, offs, tiles, ntile, max_tiles = moe_sort(ids.view(-1), (ep[1] - ep[0]) if ep else c.n_experts, tile_rows)
         gathered = lambda: gather_rows(h, torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32))
         if isinstance(wgu, Exl3Weight):
-            from .exl3_moe import exl3_grouped_experts
-            y = exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
+            y = exl3_moe.exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows)
         elif isinstance(wgu, QuantWeight):
             from . import mx
             y = mx.grouped_experts(gathered(), wgu, wd, ids, perm, tiles, ntile, max_tiles, c)

@@ -1,7 +1,7 @@
 """Prompt-size MoE over EXL3 experts.
 
 4 bits per weight: the rows go through the input transform of their expert in expert order (one gathering pass), then two
-grouped tcgen05 products decode each expert's packed trellis once per <= 128 of its rows into tensor memory (`exl3_tc.cu`); the
+grouped tcgen05 products decode each expert's packed trellis once per <= 192 of its rows into tensor memory (`exl3_tc.cu`); the
 gate / up product's epilogue applies the activation and the down product's input transform, the down product's the output
 transform.  Other bit widths: all experts' trellises reconstructed to fp16 K-major matrices in one launch, grouped tcgen05 GEMM
 over the same tile list, transforms as passes of their own.  The reference runs this with mma.sync grouped kernels that decode
@@ -28,15 +28,25 @@ def down_rows_f32(pairs: int, c) -> bool:
     return pairs <= F32_MAX_ROWS_PER_EXPERT * c.n_experts
 
 
-def exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c):
+def _fused(wgu, wd) -> bool:
+    return EXL3_MOE_FUSED and wgu.bits == 4 and wd.bits == 4
+
+
+def tile_rows(wgu, wd, pairs: int, n_experts: int) -> int:
+    """Rows of a tile for the products of these experts: 96 (two items' accumulators side by side) while an expert has up to 48 rows
+    on average, beyond 192 (an expert is decoded once, its rows are read out by the decoders)."""
+    return 128 if not _fused(wgu, wd) else 96 if pairs <= 48 * n_experts else 192
+
+
+def exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows=128):
     dev = h.device
     E = wgu.trellis.shape[0]
     H, F2 = wgu.k, wgu.n
     F = F2 // 2
     xh = cu.exl3_had_gather(h, wgu.suh, perm, ids, H)
-    if EXL3_MOE_FUSED and wgu.bits == 4 and wd.bits == 4:
-        xh2 = cu.exl3_tc(xh, wgu, tiles, ntile, max_tiles, glu=wd, limit=c.swiglu_limit)
-        return cu.exl3_tc(xh2, wd, tiles, ntile, max_tiles, out_f32=down_rows_f32(xh.shape[0], c))
+    if _fused(wgu, wd):
+        xh2 = cu.exl3_tc(xh, wgu, tiles, ntile, max_tiles, glu=wd, limit=c.swiglu_limit, tile_rows=tile_rows)
+        return cu.exl3_tc(xh2, wd, tiles, ntile, max_tiles, out_f32=down_rows_f32(xh.shape[0], c), tile_rows=tile_rows)
     # rows past this rank's pairs are filler (perm 0): their expert id may be -1 (non-local) -> clamp, they are
     # never part of a tile and never combined
     row_expert = ids.view(-1)[perm.long()].clamp_min(0).to(torch.int32).contiguous()

@@ -1,0 +1,171 @@
+"""Edges of the kernels of prompts and decode rounds: even row tiles, paired EXL3 products, block masks, per-head products, EXL3 pairs."""
+import pytest
+import torch
+
+from spark_engine_b200.quant import formats as Q
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _gen(seed):
+    return torch.Generator(device=DEV).manual_seed(seed)
+
+
+def _had(x):
+    return (x.view(*x.shape[:-1], -1, 128) @ Q.hadamard128().double().to(x.device)).view(x.shape)
+
+
+def _ids(sizes, seed):
+    ids = torch.tensor([e for e, n in enumerate(sizes) for _ in range(n)], dtype=torch.int32, device=DEV)
+    return ids, ids[torch.randperm(len(ids), device=DEV, generator=_gen(seed))].contiguous()
+
+
+@pytest.mark.parametrize("rows", [64, 96, 192])
+@pytest.mark.parametrize("sizes", [[1], [63, 64, 65, 0, 128, 129], [191, 192, 193, 384, 385, 0, 2500], [3] * 300])
+def test_even_tiles_cover_every_row_once(sizes, rows):
+    from spark_engine_b200.ops import cuda as cu
+    ids, shuffled = _ids(sizes, 1)
+    perm, inv, offs, tiles, ntile, max_tiles = cu.moe_sort(shuffled, len(sizes), rows)
+    t = tiles[: ntile.item()].tolist()
+    assert len(t) == sum(-(-n // rows) for n in sizes) <= max_tiles
+    assert sorted(r for row, _, _, n in t for r in range(row, row + n)) == list(range(len(ids)))
+    for row, end, e, n in t:
+        assert 0 < n <= rows and offs[e] <= row and row + n <= end == offs[e + 1]
+    assert torch.equal(shuffled[perm.long()], ids)
+
+
+@pytest.mark.parametrize("rows", [96, 192])
+@pytest.mark.parametrize("sizes,K,N", [([96, 97, 0, 16], 256, 256), ([191, 192, 193, 1], 128, 384), ([400, 20], 1024, 128)])
+def test_exl3_tc_even_tiles(sizes, K, N, rows):
+    from spark_engine_b200.ops import cuda as cu
+    w = Q.random_exl3(N, K, 4, len(sizes), 0.05, 2, DEV)
+    wd = Q.random_exl3(128, 128, 4, len(sizes), 0.05, 3, DEV)
+    ids, shuffled = _ids(sizes, 1)
+    x = torch.randn(len(ids), K, device=DEV, generator=_gen(5)).half()
+    _, _, _, t128, n128, m128 = cu.moe_sort(shuffled, len(sizes))
+    _, _, _, tiles, ntile, max_tiles = cu.moe_sort(shuffled, len(sizes), rows)
+    y = cu.exl3_tc(x, w, tiles, ntile, max_tiles, out_f32=True, tile_rows=rows)
+    assert torch.equal(y, cu.exl3_tc(x, w, t128, n128, m128, out_f32=True))          # a row's sum does not know its tile
+    if N == 256:
+        assert torch.equal(cu.exl3_tc(x, w, tiles, ntile, max_tiles, glu=wd, tile_rows=rows), cu.exl3_tc(x, w, t128, n128, m128, glu=wd))
+    assert cu.read_status(torch.device(DEV))[0] == 0
+    for e in ids.unique().tolist():
+        r = ids == e
+        ref = _had(x[r].double() @ Q.exl3_inner(w.trellis[e], w.kind).double()) * w.svh[e].double()
+        assert ((y[r].double() - ref).norm() / ref.norm()).item() < (K + 128) * 2.0 ** -23
+
+
+@pytest.mark.parametrize("K", [128, 192 * 2, 1024])
+def test_exl3_tc_many_items_of_both_kinds_per_cta(K):
+    """Items that take half of the accumulators and items that take all, in changing order, several per CTA."""
+    from spark_engine_b200.ops import cuda as cu
+    sizes = [(i * 73) % 230 for i in range(300)]
+    w = Q.random_exl3(512, K, 4, len(sizes), 0.05, 2, DEV)
+    _, shuffled = _ids(sizes, 1)
+    x = torch.randn(len(shuffled), K, device=DEV, generator=_gen(5)).half()
+    _, _, _, t128, n128, m128 = cu.moe_sort(shuffled, len(sizes))
+    y = cu.exl3_tc(x, w, t128, n128, m128)
+    assert torch.equal(cu.exl3_tc(x, w, t128, n128, m128, tile_rows=96), y)              # all items read out by the epilogue warps
+    for rows in (96, 192):
+        _, _, _, tiles, ntile, max_tiles = cu.moe_sort(shuffled, len(sizes), rows)
+        assert torch.equal(cu.exl3_tc(x, w, tiles, ntile, max_tiles, tile_rows=rows), y)
+    assert cu.read_status(torch.device(DEV))[0] == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 128, 128), (256, 384, 256), (257, 1024, 2048), (1021, 2048, 512), (2500, 2176, 384)])
+def test_paired_exl3_product(M, N, K):
+    """Both tile widths, ragged rows, a last tile of half its columns."""
+    from spark_engine_b200.ops import cuda as cu
+    w = Q.random_exl3(N, K, 4, 0, 0.05, M, DEV)
+    xh = torch.randn(M, K, device=DEV, generator=_gen(M)).half()
+    wt = cu.exl3_reconstruct(w)
+    y = cu.gemm_exl3(xh, wt, w.svh)
+    assert torch.equal(y, cu.gemm_exl3(xh, wt, w.svh)) and cu.read_status(torch.device(DEV))[0] == 0
+    ref = _had(xh.double() @ wt.double().t()) * w.svh.double()
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -9                 # bf16 rounding of the result
+    assert torch.equal(y, cu.exl3_had_rows(cu.gemm_bf16(xh, wt, out_f32=True, fmt=0), w.svh, post=True))
+
+
+@pytest.mark.parametrize("R,pos0,k", [(40, 100, 8), (64, 4000, 512), (300, 0, 16), (5, 17000, 512)])
+def test_block_mask_is_the_token_list(R, pos0, k):
+    from spark_engine_b200.ops import cuda as cu, sparse as sp
+    pos = torch.arange(pos0, pos0 + R, dtype=torch.int32, device=DEV)
+    ctx = pos0 + R
+    nb, mw = max(1, ctx // 4), (ctx + 127) // 128
+    score = torch.randint(0, 50, (R, nb), device=DEV, generator=_gen(R)).float()       # ties
+    sel, sel_n = sp.topk_select(score, nb, pos, 4, k)
+    mask = torch.full((R, mw), -1, dtype=torch.int32, device=DEV)
+    cu.check(sp._dll().spark_topk_mask(cu.P(score), nb, cu.P(pos), R, k, cu.P(mask), mw, cu.stream(), 0), "spark_topk_mask")
+    for r in range(R):
+        want = torch.zeros(mw * 32, dtype=torch.bool, device=DEV)
+        want[(sel[r, : sel_n[r]] // 4).long()] = True
+        got = (mask[r].view(mw, 1) >> torch.arange(32, device=DEV, dtype=torch.int32) & 1).bool().view(-1)
+        assert torch.equal(got, want), r
+
+
+@pytest.mark.parametrize("H,Dm", [(1, 8), (3, 66), (4, 128), (5, 127)])
+def test_decode_block_scores(H, Dm):
+    from spark_engine_b200.ops import sparse as sp
+    g = _gen(H)
+    pos = torch.tensor([3, 200, 517], dtype=torch.int32, device=DEV)
+    pool = torch.randn(3 * 130, Dm, device=DEV, generator=g)
+    qi, hw = torch.randn(3, H, Dm, device=DEV, generator=g), torch.randn(3, H, device=DEV, generator=g)
+    row_kv = torch.tensor([0, 520, 1040], dtype=torch.int64, device=DEV)
+    for w in (None, hw):
+        score, nb = sp.block_scores(qi, pool, row_kv, pos, 4, 518, head_w=w)
+        for r in range(3):
+            vis = (int(pos[r]) + 1) // 4
+            d = (qi[r].double() @ pool[130 * r: 130 * r + vis].double().t()).relu() / Dm ** 0.5
+            ref = (d if w is None else d * w[r].double().unsqueeze(1)).sum(0)
+            assert torch.allclose(score.view(-1)[r * nb: r * nb + vis].double(), ref, rtol=0, atol=(Dm + H) * 2.0 ** -23 * H * 4 * Dm ** 0.5)
+
+
+@pytest.mark.parametrize("rows,n,k", [(1, 5, 8), (3, 130, 128), (4, 512, 136), (8, 64, 512), (16, 33, 1024), (2, 16, 1032)])
+def test_per_head_products(rows, n, k):
+    from spark_engine_b200.ops import cuda as cu
+    g, H = _gen(n), 6
+    x = torch.randn(rows, H, k + 8, device=DEV, generator=g).bfloat16()
+    w = torch.randn(H, n, k, device=DEV, generator=g).bfloat16()
+    heads = torch.tensor([5, 0, -1, 2, 1, 4], dtype=torch.int32, device=DEV)
+    for early in (False, True):
+        y = torch.zeros(rows, H, n, dtype=torch.float32, device=DEV)
+        cu.gemv_bf16_items(x, H * (k + 8), k + 8, w, n * k, k, y, H * n, n, H, rows, n, k, heads, pairs_early=early)
+        for i, e in enumerate(heads.tolist()):
+            ref = x[:, i, :k].double() @ w[e].double().t() if e >= 0 else torch.zeros(rows, n, device=DEV, dtype=torch.float64)
+            assert torch.allclose(y[:, i].double(), ref, rtol=0, atol=k * 2.0 ** -24 * 8 * k ** 0.5), (i, early)
+
+
+@pytest.mark.parametrize("K,N,act", [(512, 256, 1), (2048, 384, 0), (1536, 128, 1), (640, 256, 0)])
+def test_exl3_pairs_do_not_depend_on_their_number(K, N, act):
+    """Few pairs take more slices than many: the bits of a pair are the same."""
+    from spark_engine_b200.ops import cuda as cu
+    E, many = 12, 900
+    w = Q.random_exl3(N, K, 4, E, 0.05, 4, DEV)
+    x = torch.randn(many, 2 * K if act else K, device=DEV, generator=_gen(K)).bfloat16()
+    e = torch.randint(0, E, (many,), device=DEV, generator=_gen(N), dtype=torch.int32)
+    run = lambda n: cu.exl3_gemv(x[:n], w, items=n, rows_per_item=1, pair_expert=e[:n].contiguous(), act=act, out_f32=True)
+    y = run(many)
+    for n in (1, 2, 40, 200):
+        assert torch.equal(run(n), y[:n]), n
+    h = x[:40].double()
+    if act:
+        h = torch.nn.functional.silu(h[:, :K]) * h[:, K:]
+    for i in range(40):
+        j = e[i].item()
+        xh = _had(h[i: i + 1] * w.suh[j].double()).half().double()
+        ref = _had(xh @ Q.exl3_inner(w.trellis[j], w.kind).double()) * w.svh[j].double()
+        assert ((y[i].double() - ref).norm() / ref.norm()).item() < 2.0 ** -10          # fp16 rounding of the transformed rows
+
+
+def test_mxfp4_tiles_of_64_rows():
+    from spark_engine_b200.ops import cuda as cu, mx
+    E, N, K = 5, 256, 512
+    ids, shuffled = _ids([64, 65, 0, 1, 200], 3)
+    w = Q.random_mxfp4(N, K, E, 0.05, 3, DEV)
+    x = torch.randn(len(ids), K, device=DEV, generator=_gen(8)).bfloat16()
+    got = []
+    for rows in (64, 128):
+        _, _, _, tiles, ntile, max_tiles = cu.moe_sort(shuffled, E, rows)
+        got.append(mx.moe_mxfp4_tc(x, w, len(ids), max_tiles, tiles=tiles, ntile=ntile, out_f32=True, tile_rows=rows))
+    assert torch.equal(*got) and cu.read_status(torch.device(DEV))[0] == 0
