@@ -13,7 +13,7 @@
 // Tile 128 x 128 x 128 bytes of K; TMEM: 2 x 128 accumulator columns + 8 scale columns per stage.
 // Every wait is bounded (status word + normal teardown).  Reference paths replaced: engine-rs/shim/ds41_mx.cu
 // fp8_gemm_mx* (warp-level block-scaled mma.sync), fp8.cu / fp8pf.cu (wmma + scale promotion).
-#include "../common/ptx.cuh"
+#include "../common/decode.cuh"
 #include <cstdlib>
 #include <mutex>
 
@@ -225,25 +225,28 @@ struct Mx4Args {
   uint32_t w_tx_bytes;        // bytes one weight tile adds to the stage barrier's transaction count (packed size)
 };
 
-// SMALL: every item has <= 16 rows (decode pairs): a stage is 19 KB (2 KB activations, 16 KB weights, two scale blocks) and ten
-// stages fit.
-template <bool SMALL>
+// ROWS: the most rows of an item.  16: decode pairs, a stage is 19 KB (2 KB activations, 16 KB weights, two scale blocks) and ten stages fit.
+// 64: prompts of a few dozen rows per expert, 25 KB, nine stages; 128: 33 KB, six.  The packed bytes in flight per SM are what the weight
+// stream runs on: 40 KB of them (five stages of 128 rows) reach 4.9 TB/s, 72 KB (nine of 64) 5.6: 1065 -> 933 us for both products of 2048
+// rows, six experts each of 384 of [4096 -> 2 x 2048 -> 4096].
+template <int ROWS>
 struct Mx4Cfg {
-  static constexpr int STAGES = SMALL ? 10 : MX_STAGES;
-  static constexpr int A_REGION = SMALL ? 16 * MX_BK : MX_A_BYTES;
+  static constexpr int STAGES = ROWS == 16 ? 10 : ROWS == 64 ? 9 : 6;
+  static constexpr int A_REGION = ROWS * MX_BK;
   static constexpr int B_OFF = STAGES * A_REGION;
   static constexpr int SF_OFF = B_OFF + STAGES * MX_B_BYTES;
   static constexpr int BAR_OFF = SF_OFF + STAGES * 2 * MX_SF_BYTES;
   static constexpr int SMEM = BAR_OFF + 256 + 1024;
+  static_assert(SMEM <= 232448 && MX_SF_COL0 + STAGES * 8 <= MX_TMEM_COLS, "shared memory, scale columns");
 };
 
-template <bool SMALL>
+template <int ROWS>
 __global__ void __launch_bounds__(MX4_THREADS, 1)
 moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA16,
                  const __grid_constant__ CUtensorMap tmW, Mx4Args g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  using Cfg = Mx4Cfg<SMALL>;
+  using Cfg = Mx4Cfg<ROWS>;
   constexpr int STAGES = Cfg::STAGES;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::BAR_OFF);
   uint64_t* empty_bar = full_bar + STAGES;
@@ -253,8 +256,6 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_k = g.K / MX_BK;
   const int nt_n = g.N / MX_BN;
-  const int n_items = min(*g.n_items, g.max_items);
-  const int num_tiles = n_items * nt_n;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -269,6 +270,10 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_ptr;
+  pdl_wait();                                                    // (barriers and tensor memory are set up beside the kernel before)
+  pdl_trigger();
+  const int n_items = min(*g.n_items, g.max_items);
+  const int num_tiles = n_items * nt_n;
 
   if (warp == 0) {
     int stage = 0; uint32_t phase = 0; bool ok = true;
@@ -277,8 +282,8 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int4 item = g.items[it];
       const int row0 = __shfl_sync(0xffffffffu, item.x, 0), rows = __shfl_sync(0xffffffffu, item.y, 0), expert = __shfl_sync(0xffffffffu, item.z, 0);
       if (expert < 0 || rows <= 0) continue;                     // expert of another rank / empty item
-      if (SMALL && rows > 16) { set_status(g.status, ST_BOUNDS, blockIdx.x, t, rows); break; }
-      const int pieces = SMALL ? 1 : min((rows + 15) >> 4, 8);   // 16-row pieces of the activation tile that the item has
+      if (rows > ROWS) { set_status(g.status, ST_BOUNDS, blockIdx.x, t, rows); break; }
+      const int pieces = ROWS == 16 ? 1 : (rows + 15) >> 4;   // 16-row pieces of the activation tile that the item has
       const uint32_t bytes = pieces * 16 * MX_BK + g.w_tx_bytes;
       const int wrow = expert * g.N + nt * MX_BN;
       for (int kb = 0; kb < num_k; ++kb) {
@@ -287,7 +292,7 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (elect_one()) {
           mbar_arrive_expect_tx(&full_bar[stage], bytes);
           uint8_t* a_dst = smem + stage * Cfg::A_REGION;
-          if (!SMALL && pieces == 8) tma_load_2d(a_dst, &tmA, &full_bar[stage], kb * MX_BK, row0);
+          if (pieces * 16 == 128) tma_load_2d(a_dst, &tmA, &full_bar[stage], kb * MX_BK, row0);
           else for (int p = 0; p < pieces; ++p) tma_load_2d(a_dst + p * 16 * MX_BK, &tmA16, &full_bar[stage], kb * MX_BK, row0 + p * 16);
           tma_load_2d(smem + Cfg::B_OFF + stage * MX_B_BYTES, &tmW, &full_bar[stage], kb * MX_BK, wrow);
         }
@@ -304,7 +309,7 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int4 item = g.items[it];
       const int rows = __shfl_sync(0xffffffffu, item.y, 0), expert = __shfl_sync(0xffffffffu, item.z, 0);
       if (expert < 0 || rows <= 0) continue;
-      if (SMALL && rows > 16) break;
+      if (rows > ROWS) break;
       const uint8_t* sa = g.sfa + static_cast<size_t>(it) * num_k * MX_SF_BYTES;
       const uint8_t* sw = g.sfw + static_cast<size_t>(expert * nt_n + nt) * num_k * MX_SF_BYTES;
       for (int kb = 0; kb < num_k; ++kb) {
@@ -333,13 +338,13 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int4 item = g.items[t / nt_n];
       const int expert = __shfl_sync(0xffffffffu, item.z, 0), rows = __shfl_sync(0xffffffffu, item.y, 0);
       if (expert < 0 || rows <= 0) continue;
-      if (SMALL && rows > 16) break;
+      if (rows > ROWS) break;
       if (!__all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1))) {
         set_status(g.status, ST_TIMEOUT_TMEM_EMPTY, blockIdx.x, t, acc); break;
       }
       tc_fence_after();
       const uint32_t d_tmem = tm + acc * MX_BN;
-      const uint32_t idesc0 = make_idesc_mx(MX_BN, SMALL ? 16 : min((rows + 15) & ~15, 128)) | (5u << 7);
+      const uint32_t idesc0 = make_idesc_mx(MX_BN, ROWS == 16 ? 16 : (rows + 15) & ~15) | (5u << 7);
       for (int kb = 0; kb < num_k; ++kb) {
         ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase));
         if (!ok) { set_status(g.status, ST_TIMEOUT_MBAR_FULL, blockIdx.x, t, kb); break; }
@@ -373,6 +378,7 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int it = t / nt_n, nt = t - it * nt_n;
       const int4 item = g.items[it];
       if (item.z < 0 || item.y <= 0) continue;
+      if (item.y > ROWS) break;
       if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[acc], acc_phase))) {
         set_status(g.status, ST_TIMEOUT_TMEM_FULL, blockIdx.x, t, acc); break;
       }
@@ -382,12 +388,12 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // lane = weight row (output column), TMEM column j = activation row j of the item
       const int col = nt * MX_BN + r;
 #pragma unroll 1
-      for (int c = 0; c < (SMALL ? 16 : item.y); c += 32) {
+      for (int c = 0; c < (ROWS == 16 ? 16 : item.y); c += 32) {
         uint32_t v[32];
         tmem_ld_32x32(t_addr + c, v);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < (SMALL ? 16 : 32); ++j) {
+        for (int j = 0; j < (ROWS == 16 ? 16 : 32); ++j) {
           if (c + j < item.y) {
             const size_t o = (static_cast<size_t>(item.w) + c + j) * g.ldc + col;
             if (g.out_f32) reinterpret_cast<float*>(g.C)[o] = __uint_as_float(v[j]);
@@ -406,7 +412,7 @@ moe_mxfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) { tc_fence_after(); tmem_dealloc<MX_TMEM_COLS>(tmem_base); }
 }
 
-// Work items of the grouped kernel.  mode 0: from the expert-sorted tile list (first row, end row, expert): one item
+// Work items of the grouped kernel.  mode 0: from the expert-sorted tile list (first row, end row, expert, rows or 0: up to 128): one item
 // per tile, C rows = A rows.  mode 1: one item per (token, expert) pair: A row = pair_row[p] (or p), C row = p.
 __global__ void mx4_items_kernel(int mode, const int4* __restrict__ tiles, const int* __restrict__ ntile,
                                  const int* __restrict__ pair_expert, const int* __restrict__ pair_row, int pairs,
@@ -419,7 +425,7 @@ __global__ void mx4_items_kernel(int mode, const int4* __restrict__ tiles, const
   if (i < n) {
     if (mode == 0) {
       const int4 td = tiles[i];
-      it = make_int4(td.x, min(128, td.y - td.x), td.z, td.x);
+      it = make_int4(td.x, td.w ? td.w : min(128, td.y - td.x), td.z, td.x);
     } else {
       it = make_int4(pair_row ? pair_row[i] : i, 1, pair_expert[i], i);
     }
@@ -452,14 +458,16 @@ __global__ void mx_sf_tile_blocks_kernel(const uint8_t* __restrict__ sf, const i
 __global__ void mx4_prep_kernel(int mode, const int4* __restrict__ tiles, const int* __restrict__ ntile,
                                 const int* __restrict__ pair_expert, const int* __restrict__ pair_row, int pairs,
                                 int max_items, const uint8_t* __restrict__ sf, int kblocks32, int4* __restrict__ items,
-                                int* __restrict__ n_items, uint8_t* __restrict__ out) {
+                                int* __restrict__ n_items, uint8_t* __restrict__ out, int words) {
+  pdl_wait();
+  pdl_trigger();
   const int i = blockIdx.x;
   const int n = mode == 0 ? min(*ntile, max_items) : min(pairs, max_items);
   int4 item = make_int4(0, 0, -1, 0);
   if (i < n) {
     if (mode == 0) {
       const int4 td = tiles[i];
-      item = make_int4(td.x, min(128, td.y - td.x), td.z, td.x);
+      item = make_int4(td.x, td.w ? td.w : min(128, td.y - td.x), td.z, td.x);
     } else {
       item = make_int4(pair_row ? pair_row[i] : i, 1, pair_expert[i], i);
     }
@@ -470,6 +478,15 @@ __global__ void mx4_prep_kernel(int mode, const int4* __restrict__ tiles, const 
   }
   if (i >= n) return;
   const int kb128 = kblocks32 >> 2;
+  if (words) {                                                   // the four scales of a row and block are one word on both sides
+    for (int j = threadIdx.x; j < kb128 * 128; j += blockDim.x) {
+      const int kt = j >> 7, r = (j & 3) * 32 + ((j >> 2) & 31);
+      uint32_t v = 0u;
+      if (item.z >= 0 && r < item.y) v = reinterpret_cast<const uint32_t*>(sf)[static_cast<size_t>(item.x + r) * kb128 + kt];
+      reinterpret_cast<uint32_t*>(out)[static_cast<size_t>(i) * kb128 * 128 + j] = v;
+    }
+    return;
+  }
   for (int j = threadIdx.x; j < kb128 * 512; j += blockDim.x) {
     const int kt = j >> 9, within = j & 511;
     const int r32 = within >> 4, q = (within >> 2) & 3, kk = within & 3;
@@ -566,18 +583,21 @@ extern "C" int spark_mx4_prep(int mode, const void* tiles, const int* ntile, con
                               cudaStream_t stream) {
   if (max_items <= 0 || kblocks32 <= 0) return 0;
   if (kblocks32 % 4) return -5;
-  mx4_prep_kernel<<<max_items, 256, 0, stream>>>(mode, (const int4*)tiles, ntile, pair_expert, pair_row, pairs, max_items,
-                                                 (const uint8_t*)sf, kblocks32, (int4*)items, n_items, (uint8_t*)out);
-  return spark_launch_rc(__func__);
+  const cudaError_t err = spark_launch_pdl(mx4_prep_kernel, dim3(max_items), dim3(256), 0, stream, dim3(1, 1, 1), mode, (const int4*)tiles, ntile,
+                                           pair_expert, pair_row, pairs, max_items, (const uint8_t*)sf, kblocks32, (int4*)items, n_items,
+                                           (uint8_t*)out, ((reinterpret_cast<uintptr_t>(sf) | reinterpret_cast<uintptr_t>(out)) & 3) == 0 ? 1 : 0);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 // A e4m3 [rows_a, K] (row stride lda bytes); W packed e2m1 [E * N, K / 2]; sfa item-local blocks
 // (spark_mx_sf_tile_blocks), sfw blocks of the flattened [E * N, K / 32] scales (spark_mx_sf_to_blocks);
-// C [*, ldc] bf16 or fp32.  N % 128 == 0, K % 128 == 0.  small != 0: every item has <= 16 rows (ten-stage variant).
+// C [*, ldc] bf16 or fp32.  N % 128 == 0, K % 128 == 0.  item_rows: the most rows of an item, 16, 64 or 128
+// (longer ones: an error in the status word).
 extern "C" int spark_moe_mxfp4(const void* A, int lda, int rows_a, const void* W, const void* sfa, const void* sfw,
                                const void* items, const int* n_items, int max_items, int E, int N, int K, void* C, int ldc,
-                               int out_f32, int small, int* status, cudaStream_t stream) {
+                               int out_f32, int item_rows, int* status, cudaStream_t stream) {
   if (max_items <= 0 || rows_a <= 0) return 0;
+  if (item_rows != 16 && item_rows != 64 && item_rows != 128) return -5;
   if (K % MX_BK || N % MX_BN || (ldc & 7) || (reinterpret_cast<uintptr_t>(C) & 15)) return -5;
   CUtensorMap tA, tA16, tW;
   int r = make_tmap_u8(&tA, A, rows_a, K, lda);
@@ -589,19 +609,20 @@ extern "C" int spark_moe_mxfp4(const void* A, int lda, int rows_a, const void* W
   // a 16U4_ALIGN16B copy completes the barrier with the packed bytes it read (64 per row), not the 128 it writes
   const uint32_t w_tx = MX_B_BYTES / 2;
   Mx4Args g{(const int4*)items, n_items, max_items, N, K, (const uint8_t*)sfa, (const uint8_t*)sfw, C, ldc, out_f32, status, w_tx};
+  void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, Mx4Args) = item_rows == 16 ? moe_mxfp4_kernel<16> : item_rows == 64 ? moe_mxfp4_kernel<64> : moe_mxfp4_kernel<128>;
+  const int smem = item_rows == 16 ? Mx4Cfg<16>::SMEM : item_rows == 64 ? Mx4Cfg<64>::SMEM : Mx4Cfg<128>::SMEM;
   static bool attr_done = false;
   if (!attr_done) {
-    cudaFuncSetAttribute(moe_mxfp4_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<false>::SMEM);
-    cudaFuncSetAttribute(moe_mxfp4_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<true>::SMEM);
+    cudaFuncSetAttribute(moe_mxfp4_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<16>::SMEM);
+    cudaFuncSetAttribute(moe_mxfp4_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<64>::SMEM);
+    cudaFuncSetAttribute(moe_mxfp4_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mx4Cfg<128>::SMEM);
     attr_done = true;
   }
   static int sms = 0;
   if (!sms) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   const long long tiles = static_cast<long long>(max_items) * (N / MX_BN);
   const int grid = tiles < sms ? static_cast<int>(tiles) : sms;
-  if (small) moe_mxfp4_kernel<true><<<grid, MX4_THREADS, Mx4Cfg<true>::SMEM, stream>>>(tA, tA16, tW, g);
-  else moe_mxfp4_kernel<false><<<grid, MX4_THREADS, Mx4Cfg<false>::SMEM, stream>>>(tA, tA16, tW, g);
-  return spark_launch_rc(__func__);
+  return spark_launch_pdl(kern, dim3(grid), dim3(MX4_THREADS), smem, stream, dim3(1, 1, 1), tA, tA16, tW, g) == cudaSuccess ? 0 : -4;
 }
 
 // A e4m3 [M,K] (row stride lda bytes), B e4m3 [N,K]; sfa / sfb in block layout (spark_mx_sf_to_blocks); K % 128 == 0.

@@ -23,7 +23,7 @@
 #include <cstdint>
 #include <cstdlib>
 
-#include "../common/ptx.cuh"
+#include "../common/decode.cuh"
 
 #ifndef SPARK_FP4_CVT
 #define SPARK_FP4_CVT 0            // 1: E2M1 through the hardware conversion instruction, 0: integer-pipe decode
@@ -98,9 +98,9 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   __half* xs = reinterpret_cast<__half*>(smem_mx);              // [RB][XS]
   float* red = reinterpret_cast<float*>(smem_mx + static_cast<size_t>(RB) * XS * 2);   // [2][warps][16][16]
   const int item = blockIdx.y;
+  if (pair_expert) pdl_wait();                                 // (a single matrix is asked for before the dependency wait)
   if (pair_expert && pair_expert[item] < 0) return;            // pair of an expert that lives on another rank
   const int e = pair_expert ? pair_expert[item] : 0;
-  const int xr0 = pair_row ? pair_row[item] : item * rows_per_item;
   const int R = rows_per_item;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * MXV_COLS * cgroups;
@@ -230,6 +230,9 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   };
 
   load(wl0, wh0, sl0, sh0, 0);            // the first weights are in flight while the rows are staged
+  if (!pair_expert) pdl_wait();
+  pdl_trigger();
+  const int xr0 = pair_row ? pair_row[item] : item * rows_per_item;
   if (xvec) {
     // 16-byte loads, four in flight per thread: the rows are staged in about one memory latency
     const int K8 = K >> 3, chunks = RB * K8;
@@ -335,10 +338,10 @@ static int launch_mx_gemv(const void* x, int ldx, const void* W, const void* sc,
     if (!set_for) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); set_for = 1; }
   }
   dim3 grid(ngroups / cgroups, items);
-  kern<<<grid, MXV_WARPS * 32, smem, s>>>((const __nv_bfloat16*)x, ldx, (const uint8_t*)W, sc, wes, ses, (TO*)y, ldy, rows,
-                                          N, K, pe, pr, act, limit, cgroups,
-                                          xvec_ok && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ldx & 7) == 0 ? 1 : 0);
-  return spark_launch_rc(__func__);
+  const cudaError_t err = spark_launch_pdl(kern, grid, dim3(MXV_WARPS * 32), smem, s, dim3(1, 1, 1), (const __nv_bfloat16*)x, ldx,
+                                           (const uint8_t*)W, sc, wes, ses, (TO*)y, ldy, rows, N, K, pe, pr, act, limit, cgroups,
+                                           xvec_ok && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ldx & 7) == 0 ? 1 : 0);
+  return err == cudaSuccess ? 0 : -4;
 }
 
 template <int FMT, typename TO>
@@ -422,11 +425,15 @@ template <int BLOCK, typename TI, int PER>
 __global__ void __launch_bounds__(256)
 act_quant_kernel(const TI* __restrict__ x, int ldx, uint8_t* __restrict__ q, void* __restrict__ scales, int R,
                  int K, int pow2, int act, float limit, int vec) {
-  const int pr = K / PER;                                    // lanes of a row (a multiple of BLOCK / PER)
-  const long long id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, total = static_cast<long long>(R) * pr;
-  if (id - (threadIdx.x & 31) >= total) return;              // whole warps leave: the others shuffle
-  const bool live = id < total;
-  const int r = live ? static_cast<int>(id / pr) : R - 1, k = live ? static_cast<int>(id - static_cast<long long>(r) * pr) * PER : 0;
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t pr = K / PER;                               // lanes of a row (a multiple of BLOCK / PER)
+  const long long wide_id = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, total = static_cast<long long>(R) * pr;
+  if (wide_id - (threadIdx.x & 31) >= total) return;         // whole warps leave: the others shuffle
+  const bool live = wide_id < total;
+  // (a 64-bit division is longer than the rest of the index arithmetic: only where the lanes do not fit 32 bits)
+  const uint32_t row = total <= 0x7fffffffLL ? static_cast<uint32_t>(wide_id) / pr : static_cast<uint32_t>(wide_id / pr);
+  const int r = live ? static_cast<int>(row) : R - 1, k = live ? static_cast<int>(wide_id - static_cast<long long>(row) * pr) * PER : 0;
   const TI* xr = x + static_cast<size_t>(r) * ldx + k;
   constexpr int LANES = BLOCK / PER;                          // lanes of a block
   float v[PER];
@@ -460,9 +467,10 @@ act_quant_kernel(const TI* __restrict__ x, int ldx, uint8_t* __restrict__ q, voi
   const float inv = 1.f / sc;
   uint32_t w[(PER + 3) / 4] = {};
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const float s = fminf(fmaxf(p2 ? v[j] * inv : v[j] / sc, -448.f), 448.f);
-    w[j >> 2] |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(s, __NV_SATFINITE, __NV_E4M3)) << (8 * (j & 3));
+  for (int j = 0; j < PER; j += 2) {                         // (a conversion takes two)
+    const float2 s = make_float2(fminf(fmaxf(p2 ? v[j] * inv : v[j] / sc, -448.f), 448.f),
+                                 fminf(fmaxf(p2 ? v[j + 1] * inv : v[j + 1] / sc, -448.f), 448.f));
+    w[j >> 2] |= static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(s, __NV_SATFINITE, __NV_E4M3)) << (8 * (j & 3));
   }
   uint8_t* dst = q + static_cast<size_t>(r) * K + k;
   if (!vec) {
@@ -476,13 +484,13 @@ act_quant_kernel(const TI* __restrict__ x, int ldx, uint8_t* __restrict__ q, voi
 }
 
 template <int BLOCK, typename TI>
-static void launch_act_quant(const void* x, int ldx, uint8_t* q, void* scales, int R, int K, int pow2, int act, float limit, cudaStream_t s) {
+static int launch_act_quant(const void* x, int ldx, uint8_t* q, void* scales, int R, int K, int pow2, int act, float limit, cudaStream_t s) {
   // eight elements a lane once that still is a warp for every scheduler of the GPU
   const int vec = ((reinterpret_cast<uintptr_t>(x) & 15) | (static_cast<size_t>(ldx) * sizeof(TI) & 15) | (reinterpret_cast<uintptr_t>(q) & 7)) == 0;
   const bool many = static_cast<long long>(R) * K >= 148LL * 4 * 32 * 8;
   const unsigned blocks = static_cast<unsigned>((static_cast<long long>(R) * (K / (many || BLOCK == 128 ? 8 : 2)) + 255) / 256);
-  if (many || BLOCK == 128) act_quant_kernel<BLOCK, TI, 8><<<blocks, 256, 0, s>>>((const TI*)x, ldx, q, scales, R, K, pow2, act, limit, vec);
-  else act_quant_kernel<BLOCK, TI, BLOCK == 128 ? 8 : 2><<<blocks, 256, 0, s>>>((const TI*)x, ldx, q, scales, R, K, pow2, act, limit, vec);
+  return spark_launch_pdl(many || BLOCK == 128 ? act_quant_kernel<BLOCK, TI, 8> : act_quant_kernel<BLOCK, TI, BLOCK == 128 ? 8 : 2>, dim3(blocks),
+                          dim3(256), 0, s, dim3(1, 1, 1), (const TI*)x, ldx, q, scales, R, K, pow2, act, limit, vec) == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace spark
@@ -521,10 +529,9 @@ extern "C" int spark_act_quant(const void* x, int ldx, int in_f32, void* q, void
   if (R <= 0) return 0;
   if ((block != 128 && block != 32) || K % block) return -5;
 #define SPARK_AQ(B, T) launch_act_quant<B, T>(x, ldx, (uint8_t*)q, scales, R, K, pow2, act, limit, s)
-  if (block == 128) { if (in_f32) SPARK_AQ(128, float); else SPARK_AQ(128, __nv_bfloat16); }
-  else { if (in_f32) SPARK_AQ(32, float); else SPARK_AQ(32, __nv_bfloat16); }
+  if (block == 128) return in_f32 ? SPARK_AQ(128, float) : SPARK_AQ(128, __nv_bfloat16);
+  return in_f32 ? SPARK_AQ(32, float) : SPARK_AQ(32, __nv_bfloat16);
 #undef SPARK_AQ
-  return spark_launch_rc(__func__);
 }
 
 // ------------------------------------------------------------------------------------------ grouped MXFP4 GEMM

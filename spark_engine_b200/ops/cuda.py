@@ -962,17 +962,16 @@ def moe(h, w, c, defer: bool = False):
         y = _expert_gemv(gu, wd, Pn, pe, None, 1, c.swiglu_limit, True)            # [P, H] fp32
         inv = None
     else:
-        from . import exl3_moe
-        tile_rows = exl3_moe.tile_rows(wgu, wd, Pn, c.n_experts) if isinstance(wgu, Exl3Weight) else 128
+        from . import exl3_moe, mx
+        tile_rows = (exl3_moe.tile_rows(wgu, wd, Pn, c.n_experts) if isinstance(wgu, Exl3Weight)
+                     else mx.tile_rows(wgu, Pn, c.n_experts) if isinstance(wgu, QuantWeight) else 128)
         perm, inv, offs, tiles, ntile, max_tiles = moe_sort(ids.view(-1), (ep[1] - ep[0]) if ep else c.n_experts, tile_rows)
-        gathered = lambda: gather_rows(h, torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32))
         if isinstance(wgu, Exl3Weight):
             y = exl3_moe.exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows)
         elif isinstance(wgu, QuantWeight):
-            from . import mx
-            y = mx.grouped_experts(gathered(), wgu, wd, ids, perm, tiles, ntile, max_tiles, c)
+            y = mx.grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows)
         else:
-            a = gathered()
+            a = gather_rows(h, torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32))
             E, F2, K = wgu.shape
             act = grouped_gemm(a, wgu.view(E * F2, K), tiles, ntile, max_tiles, E, F2, F2 // 2, 1, c.swiglu_limit)
             y = grouped_gemm(act, wd.view(E * H, F2 // 2), tiles, ntile, max_tiles, E, H, H, 0)

@@ -153,13 +153,14 @@ MX_MOE_TC = os.environ.get("SPARK_MX_MOE_TC", "1") == "1"
 
 
 def moe_mxfp4_tc(x, w: Mxfp4Weight, out_rows, max_items, tiles=None, ntile=None, pair_expert=None, pair_row=None,
-                 act=0, limit=0.0, out_f32=False):
+                 act=0, limit=0.0, out_f32=False, tile_rows=128, quantised=None):
     """Grouped expert GEMM on the block-scaled tcgen05 path: MXFP8 activations (quantised here, SwiGLU of a
     [gate | up] input first when act=1) x packed MXFP4 experts, the nibbles expanded by TMA on the way to shared
-    memory.  Work items come from the expert-sorted tile list (prefill) or from (token, expert) pairs (decode)."""
+    memory.  Work items come from the expert-sorted tile list (prefill; `tile_rows`: the most rows of a tile, 64 or 128) or from
+    (token, expert) pairs (decode).  `quantised`: the rows of `x` as `act_quant` gives them, where the caller has them."""
     dev = x.device
     E, N, K = w.packed.shape[0], w.n, w.k
-    a_q, a_sf = act_quant(x, block=32, act=act, limit=limit)
+    a_q, a_sf = quantised or act_quant(x, block=32, act=act, limit=limit)
     items = torch.empty(max_items, 4, dtype=torch.int32, device=dev)
     n_items = torch.empty(1, dtype=torch.int32, device=dev)
     mode = 0 if tiles is not None else 1
@@ -173,7 +174,7 @@ def moe_mxfp4_tc(x, w: Mxfp4Weight, out_rows, max_items, tiles=None, ntile=None,
         wb = w._sf_blocks = sf_blocks(w.scales.reshape(E * N, K // 32))
     c = torch.empty(out_rows, N, dtype=torch.float32 if out_f32 else torch.bfloat16, device=dev)
     rc = _lib().spark_moe_mxfp4(cu.P(a_q), a_q.stride(0), a_q.shape[0], cu.P(w.packed), cu.P(sfa), cu.P(wb), cu.P(items),
-                                cu.P(n_items), max_items, E, N, K, cu.P(c), N, int(out_f32), int(mode == 1),
+                                cu.P(n_items), max_items, E, N, K, cu.P(c), N, int(out_f32), 16 if mode == 1 else tile_rows,
                                 cu.P(cu.status_word(dev)), cu.stream())
     cu.check(rc, "spark_moe_mxfp4")
     return c
@@ -223,15 +224,38 @@ def mx_mgemm(x, w: Mxfp4Weight, tiles, ntile, max_tiles, act=0, limit=0.0, out_f
     return y
 
 
-def grouped_experts(a, wgu, wd, ids, perm, tiles, ntile, max_tiles, c):
-    """Rows in expert order through gate/up (+SwiGLU) and down; returns fp32 [P, H]."""
+def _on_tensor_cores(wgu) -> bool:
+    return MX_MOE_TC and isinstance(wgu, Mxfp4Weight) and wgu.n % 256 == 0 and wgu.k % 128 == 0
+
+
+def tile_rows(wgu, pairs, n_experts) -> int:
+    """Rows of a tile for these experts: 64 (more of the weight stream in flight) while an expert has up to 40 rows on average, so
+    that few experts are read twice."""
+    return 64 if _on_tensor_cores(wgu) and pairs <= 40 * n_experts else 128
+
+
+def _quantised_rows(h, rows):
+    """`act_quant` of h[rows]: every row of h is quantised once and its bytes are gathered (rows of the routed pairs repeat; a row's
+    codes and scales are its own).  2048 rows of 4096, six experts each: 56 -> 20 us with the gather."""
+    q, sf = act_quant(h, block=32)
+    R, K = h.shape
+    q = cu.gather_rows(q.view(torch.bfloat16), rows).view(torch.float8_e4m3fn)
+    sf = cu.gather_rows(sf.view(torch.bfloat16), rows).view(torch.uint8) if K % 512 == 0 else sf.index_select(0, rows)
+    return q, sf
+
+
+def grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows=128):
+    """The routed pairs of rows `h`, in expert order (`perm`), through gate/up (+SwiGLU) and down; returns fp32 [P, H]."""
     E, F2, H = wgu.packed.shape[0] if isinstance(wgu, Mxfp4Weight) else wgu.q.shape[0], wgu.n, wgu.k
-    dev = a.device
-    if MX_MOE_TC and isinstance(wgu, Mxfp4Weight) and F2 % 256 == 0 and H % 128 == 0:
+    dev = h.device
+    rows = torch.div(perm, c.top_k, rounding_mode="floor").to(torch.int32)
+    if _on_tensor_cores(wgu):
         # block-scaled tensor-core path: MXFP8 activations x packed MXFP4 experts, no decoded copy of the weights
-        Pn = a.shape[0]
-        gu = moe_mxfp4_tc(cu._as_bf16(a).contiguous(), wgu, Pn, max_tiles, tiles=tiles, ntile=ntile)
-        return moe_mxfp4_tc(gu, wd, Pn, max_tiles, tiles=tiles, ntile=ntile, act=1, limit=c.swiglu_limit, out_f32=True)
+        Pn = perm.shape[0]
+        h = cu._as_bf16(h).contiguous()
+        gu = moe_mxfp4_tc(h, wgu, Pn, max_tiles, tiles=tiles, ntile=ntile, tile_rows=tile_rows, quantised=_quantised_rows(h, rows))
+        return moe_mxfp4_tc(gu, wd, Pn, max_tiles, tiles=tiles, ntile=ntile, act=1, limit=c.swiglu_limit, out_f32=True, tile_rows=tile_rows)
+    a = cu.gather_rows(h, rows)
     if MX_MOE_FUSED and isinstance(wgu, Mxfp4Weight) and F2 % 128 == 0 and H % 128 == 0 and a.shape[0] <= 512 * E:
         # packed experts straight into the MMA: the weights cross HBM once, SwiGLU is applied while the down
         # projection stages its input
