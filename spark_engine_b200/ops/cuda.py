@@ -250,7 +250,10 @@ def clear_status(device):
 
 def scratch(name: str, numel: int, dtype, device, zero: bool = False) -> torch.Tensor:
     """Persistent scratch keyed by name (grows, never shrinks): fixed addresses for graph replay."""
-    key = (name, dtype, str(device))
+    d = torch.device(device)
+    if d.type == "cuda" and d.index is None:                                  # "cuda" and "cuda:0" are one buffer
+        d = torch.device("cuda", torch.cuda.current_device())
+    key = (name, dtype, str(d))
     t = _scratch.get(key)
     if t is None or t.numel() < numel:
         if t is not None:
