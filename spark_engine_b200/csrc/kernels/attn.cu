@@ -322,7 +322,8 @@ attn_decode_tc_kernel(const __grid_constant__ AttnDecodeArgs a) {
   int* stok = reinterpret_cast<int*>(Ps + ATT_ROWS * 72);                           // [64]
   float* ksc = reinterpret_cast<float*>(stok + ATT_TS);                             // [64]
   float* vsc = ksc + ATT_TS;                                                        // [64]
-  // FP8: key bytes land where the bf16 values will be, value bytes behind everything (with both behind it one CTA fitted an SM at D = 256)
+  // FP8: key bytes land where the bf16 values will be, value bytes behind everything (with both behind it one CTA fitted an SM
+  // at D = 256, and 264 of them were two waves: 15.8 us, 9.8 now)
   uint8_t* k_stage = reinterpret_cast<uint8_t*>(Vs);                                // [64][D]
   uint8_t* v_stage = reinterpret_cast<uint8_t*>(vsc + ATT_TS);                      // [64][D]
   __shared__ float m_run[ATT_ROWS], l_run[ATT_ROWS], alpha[ATT_ROWS];
@@ -497,7 +498,8 @@ static size_t attn_decode_tc_smem() {
 
 // grid (R, Hq); a thread per dimension (whole warps, <= 256).  Splits merged in ascending order: their weights are formed once, by a
 // thread each, and eight partial rows are in flight per thread.  What bounds it: three memory round trips (statistics, partial rows,
-// store).  With every thread walking the statistics twice, one load after the other: 11.3 us for 4 rows of 16 heads of 256, 33 splits.
+// store).  4 rows of 16 heads of 256, 33 splits: 6.7 us (11.3
+// with every thread walking the statistics twice, one load after the other).
 constexpr int MERGE_T = 256;
 
 __global__ void __launch_bounds__(MERGE_T)

@@ -165,9 +165,9 @@ constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16, ROUTER_COLS = 4;
 // vector in one 32-bit chain per row, the lanes' sums meet by shuffles: the order of a row's sum depends on neither R nor NR.  The
 // loads are 16 bytes, straight from memory, a batch of a row's and a column's vectors in flight (the rows of a CTA stay in L1).
 // What bounds it: a memory round trip per batch and the chain of the choices, one warp per row.  4 rows of 2048 and 513 columns 13.7 ->
-// 8.4 us, 16 rows 32 -> 16.7, 4 rows of the MXFP4 preset 37 -> 17 (before: a warp per column for all rows, the rows staged in shared
-// memory, two rows' choices after one another).  Tensor cores in place of the FP32 units (9.3, 13, 16 us) add 16 products at a time
-// with fewer bits: the logits' error grew 1.2 to 15 times over K = 256 .. 7168.
+// 7.5 us, 16 rows 32 -> 15.2, 4 rows of the MXFP4 preset 37 -> 13.6 (before: a warp per column for all rows, the rows staged in shared
+// memory, two rows' choices after one another, one kernel for all kinds).  Tensor cores in place of the FP32 units (9.3, 13, 16 us) add
+// 16 products at a time with fewer bits: the logits' error grew 1.2 to 15 times over K = 256 .. 7168.
 // KIND: 0, 1 and 2 alone, 3 the others (the kernel is fetched anew in every layer: what a kind does not run costs instruction misses)
 template <int EPL, int NR, int KIND>                        // NR: rows of a warp (R <= 4 NR)
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
@@ -486,8 +486,8 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, int P, int E, cons
 // res[R,H] += sum_slot w[r,slot] * y[pair_pos(r,slot), :] (+ sg[r] * shared[r,:]).  y fp32 or bf16.
 // A thread owns V consecutive columns (one 16-byte load of y per slot; V = 1 where H or an address does not allow it).  The row's slots
 // are looked up once per CTA, and a thread's loads of eight slots are issued before the first is widened (a load and its widening in one
-// branch per slot waited for every slot by itself).  Added in slot order.  Bound by reading y: 8192 rows of 2048, ten bf16 slots, took
-// 224 us with one column per thread and 110 with a vector; 2048 rows of 4096, eight fp32 slots, 91 and 49.
+// branch per slot waited for every slot by itself).  Added in slot order.  Bound by reading y: 8192 rows of 2048, ten bf16 slots, 82 us
+// (110 with a wait per slot, 224 with one column per thread); 2048 rows of 4096, six fp32 slots, 42 (49, 91).
 template <int V, typename T> struct CombVec { typedef T type; };
 template <> struct CombVec<4, float> { typedef uint4 type; };
 template <> struct CombVec<8, __nv_bfloat16> { typedef uint4 type; };

@@ -15,8 +15,8 @@ namespace spark {
 
 // grid (ceil(nb_max / 32), R), 256 threads: a warp scores four blocks.  idx_dim <= 128: a lane has four dimensions.  Four blocks by four
 // heads are sixteen sums over the lanes, which are folded together: each step halves the sums a lane carries, 16 shuffles where sixteen
-// butterflies take 80, the same pairs in the same order.  What bounds it: the chain position -> keys -> queries -> folds (a warp per block:
-// two waves of CTAs, 8.7 us for 4 rows of 4000 blocks, 4 heads of 128).  vec: rows of `pool` and `qi` start on 16 bytes.
+// butterflies take 80, the same pairs in the same order.  What bounds it: the chain position -> keys -> queries -> folds (4 rows of 4000
+// blocks, 4 heads of 128: 4.1 us; a warp per block, two waves of CTAs: 8.7).  vec: rows of `pool` and `qi` start on 16 bytes.
 constexpr int IDX_B = 4;
 
 __device__ __forceinline__ float4 idx_ld4(const float* p, int lane, int Dm, int vec) {
@@ -81,7 +81,8 @@ idx_score_kernel(const float* __restrict__ qi, int H, int Dm, const float* __res
 // with cp.async (double buffered), S = Q K^T runs as 3xTF32 (every operand split into a TF32 head and a TF32 remainder,
 // three m16n8k8 MMAs per product: fp32-grade scores, so a row selects the same blocks whether it is scored here or by
 // the decode kernel), then relu x scale x head weight goes through shared memory where the H heads of a row are summed
-// in head order.  Blocks beyond a row's visible range get values nobody reads.
+// in head order.  Blocks beyond a row's visible range get values nobody reads.  Bound by the latency of the fragments' loads and splits: four
+// k-steps in flight and the longest contexts first, 3999 rows of 4 heads: 129 -> 89 us (16 warps of half the columns: 88).
 // Reference: engine-rs/shim/ds41_attn.cu:447-824, dataflow.cu:159-336 (tensor-core indexer scoring for prefill rows).
 constexpr int IS_M = 64, IS_N = 64;
 
@@ -223,7 +224,7 @@ __device__ __forceinline__ uint32_t order_key(uint32_t b) {
 // them was most of the time).  Four rows of 4000 candidates: 27.7 -> 7.2 us.  NT = 256: prompts, where many rows of up to a few
 // thousand candidates share an SM: 3999 rows of up to 1000, 145 -> 22 us.
 // MASK: the same blocks (of 4 tokens) as a bit each, mw words per row in `sel`, for the tiles of prompt attention: eight lanes fill a
-// word (a token list per row, turned into bits by a kernel of its own, took 22 + 25 us for 3999 rows of up to 1000).
+// word (3999 rows of up to 1000: 17 us; a token list per row, turned into bits by a kernel of its own, 22 + 25).
 template <int NT, bool MASK>
 __global__ void __launch_bounds__(NT)
 topk_select_kernel(const float* __restrict__ score, int ld, const int* __restrict__ pos, int block, int k, int window,
