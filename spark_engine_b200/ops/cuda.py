@@ -410,15 +410,18 @@ def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> i
     forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if pairs else "SPARK_EXL3_S", "0"))
     if forced and blocks % forced == 0:
         return forced
-    unit = 2 if pairs and blocks % 2 == 0 else 1
     strips = N // 128 * (items if pairs else 1)
-    best = 0
-    for s in range(1, 9):
-        if blocks % (s * unit) or K // s > 2048:
-            continue
-        if not best or strips * s <= EXL3_CTAS or (pairs and K // s >= 1024 and strips * s <= 2.2 * EXL3_CTAS):
-            best = s
-    return best or 1
+    # (pairs: counts that leave whole chunks, of 256 where any count does, else of 128 for all counts of this K)
+    for unit in ((2, 1) if pairs else (1,)):
+        best = 0
+        for s in range(1, 9):
+            if blocks % (s * unit) or K // s > 2048:
+                continue
+            if not best or strips * s <= EXL3_CTAS or (pairs and K // s >= 1024 and strips * s <= 2.2 * EXL3_CTAS):
+                best = s
+        if best:
+            return best
+    return 1
 
 
 def exl3_gemv(x, w: Exl3Weight, items=1, rows_per_item=None, pair_expert=None, pair_row=None, act=0, limit=0.0,
