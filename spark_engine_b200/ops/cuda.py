@@ -1236,7 +1236,9 @@ def mla_mixer(mixer, h, plan, seqs):
         inv = (c.rope_theta ** (-torch.arange(half, dtype=torch.float64) * 2 / max(Rr, 1))).to(dev)
         mixer._dev = {"inv": inv, "w_ukT": mixer.w_uk.transpose(1, 2).contiguous().to(torch.bfloat16),
                       "w_uv": mixer.w_uv.contiguous().to(torch.bfloat16),
-                      "ape": w["ape"].float().contiguous()}
+                      "ape": w["ape"].float().contiguous(),
+                      # (here, launches before the per-head products, which read it ahead of their dependency wait)
+                      "heads": torch.arange(H, dtype=torch.int32, device=dev)}
     md = mixer._dev
     if dbg.CHECK:
         _check_cache_rows("mla_mixer", d, tree, mixer.lat.shape[0])
@@ -1254,13 +1256,9 @@ def mla_mixer(mixer, h, plan, seqs):
     q_full = torch.empty(R, H, KW, dtype=torch.bfloat16, device=dev)
     decode = R * H <= 4096 and R <= 16
     if decode:
-        key = ("mla_heads", H)
-        if key not in md:
-            md[key] = torch.arange(H, dtype=torch.int32, device=dev)
-        heads = md[key]
         qn = qb if qb.stride(0) % 8 == 0 else qb[:, :nq].contiguous()
         # absorb W_uk: one item per head over all rows (the head's [L, D] matrix is streamed once for the round)
-        gemv_bf16_items(qn, qn.stride(0), D + Rr, md["w_ukT"], L * D, D, q_full, H * KW, KW, H, R, L, D, heads, pairs_early=True)
+        gemv_bf16_items(qn, qn.stride(0), D + Rr, md["w_ukT"], L * D, D, q_full, H * KW, KW, H, R, L, D, md["heads"], pairs_early=True)
     else:
         q_full[..., :L] = torch.einsum("thd,hld->thl", qb[:, :nq].view(R, H, D + Rr)[..., :D], md["w_ukT"])
     if Rr:
@@ -1288,7 +1286,7 @@ def mla_mixer(mixer, h, plan, seqs):
     check(rc, "spark_mla_attn")
     if decode:
         out = torch.empty(R, H * D, dtype=torch.bfloat16, device=dev)
-        return gemv_bf16_items(out_lat, H * L, L, md["w_uv"], D * L, L, out, H * D, D, H, R, D, L, md[("mla_heads", H)],
+        return gemv_bf16_items(out_lat, H * L, L, md["w_uv"], D * L, L, out, H * D, D, H, R, D, L, md["heads"],
                                pairs_early=True)
     return torch.einsum("thl,hdl->thd", out_lat, md["w_uv"]).reshape(R, H * D)
 
