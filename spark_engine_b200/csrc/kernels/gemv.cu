@@ -136,7 +136,7 @@ gemv_items_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloa
   const int item = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane % LPC;
   const int n0 = (blockIdx.x * GEMV_WARPS + warp) * GEMV_IT_COLS * G + lane / LPC;      // column c of this lane: n0 + c * G
   const int KV = K >> 3;
-  if (pair_expert && !pairs_early) pdl_wait();
+  if (!pairs_early) pdl_wait();
   const int e = pair_expert ? pair_expert[item] : 0;
   if (e < 0) { if (pairs_early) pdl_wait(); return; }                  // pair of an expert that lives on another rank
   const __nv_bfloat16* Wb = W + e * expert_stride;
@@ -151,7 +151,7 @@ gemv_items_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloa
       }
   };
   load(l);
-  if (!pair_expert || pairs_early) pdl_wait();
+  if (pairs_early) pdl_wait();
   x += item * x_item_stride;
   y += item * y_item_stride;
   for (int i = threadIdx.x; i < R * KV; i += GEMV_WARPS * 32) {
@@ -285,8 +285,8 @@ gemv_wide_mma_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bf
   };
   const uint4 *w0, *w1;
   int n0 = rows_of(0, w0, w1);
-  if (n0 < N) load(w0, w1, kb);                          // in flight while the launch before ends and the rows are staged
-  pdl_wait();
+  pdl_wait();                                            // (W too may come from the launch before: expansions on first use)
+  if (n0 < N) load(w0, w1, kb);                          // in flight while the rows are staged
   // rows past R are left as they are: an MMA column only ever reaches its own row's outputs, which are not stored
   const int KV8 = K >> 3;
   for (int i0 = threadIdx.x; i0 < R * KV8; i0 += 2 * GEMV_WARPS * 32) {
@@ -516,7 +516,7 @@ extern "C" int spark_gemv_bf16(const void* x, int ldx, const void* W, long long 
 // Strided items: item i multiplies rows x + i * x_item_stride + r * ldx (r < rows_per_item) by expert
 // pair_expert[i] (or W itself) and writes y + i * y_item_stride + r * ldy.  Used for per-head projections of
 // [rows, heads, dim] tensors: every head's matrix is streamed once for all rows.  Strides in elements; the item
-// offsets must keep x 16-byte aligned.  pairs_early: pair_expert was written at least two launches back, so the weights may be asked for
+// offsets must keep x 16-byte aligned.  pairs_early: pair_expert and W were written at least two launches back, so both may be read
 // before the dependency wait.
 extern "C" int spark_gemv_bf16_items(const void* x, int ldx, long long x_item_stride, const void* W, long long expert_stride,
                                      int ldw, void* y, int ldy, long long y_item_stride, int items, int rows_per_item, int N,

@@ -98,7 +98,7 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   __half* xs = reinterpret_cast<__half*>(smem_mx);              // [RB][XS]
   float* red = reinterpret_cast<float*>(smem_mx + static_cast<size_t>(RB) * XS * 2);   // [2][warps][16][16]
   const int item = blockIdx.y;
-  if (pair_expert) pdl_wait();                                 // (a single matrix is asked for before the dependency wait)
+  pdl_wait();
   if (pair_expert && pair_expert[item] < 0) return;            // pair of an expert that lives on another rank
   const int e = pair_expert ? pair_expert[item] : 0;
   const int R = rows_per_item;
@@ -230,7 +230,6 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   };
 
   load(wl0, wh0, sl0, sh0, 0);            // the first weights are in flight while the rows are staged
-  if (!pair_expert) pdl_wait();
   pdl_trigger();
   const int xr0 = pair_row ? pair_row[item] : item * rows_per_item;
   if (xvec) {

@@ -337,7 +337,8 @@ def gemv_bf16(x, w, items=1, rows_per_item=None, pair_expert=None, pair_row=None
 def gemv_bf16_items(x, ldx, x_item_stride, w, expert_stride, ldw, y, ldy, y_item_stride, items, rows_per_item, n, k,
                     pair_expert, oact=None, pairs_early=False):
     """Per-item GEMV over strided slices: item i multiplies rows x[i * x_item_stride + r * ldx] (r < rows_per_item) by
-    matrix pair_expert[i] of `w` and writes y[i * y_item_stride + r * ldy].  Strides in elements.  `pairs_early`: see `exl3_gemv`."""
+    matrix pair_expert[i] of `w` and writes y[i * y_item_stride + r * ldy].  Strides in elements.
+    `pairs_early`: `w` and `pair_expert` were written at least two launches back, so the kernel may read both before its dependency wait."""
     if dbg.CHECK:
         dbg.check_index("gemv_bf16_items pair_expert", pair_expert, 0, w.shape[0], count=items)
     rc = lib().spark_gemv_bf16_items(P(x), ldx, x_item_stride, P(w), expert_stride, ldw, P(y), ldy, y_item_stride, items,
@@ -427,7 +428,8 @@ def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> i
 def exl3_gemv(x, w: Exl3Weight, items=1, rows_per_item=None, pair_expert=None, pair_row=None, act=0, limit=0.0,
               out_f32=False, pairs_early: bool = False):
     """`pairs_early`: the pair tables were written at least two launches back, so the kernel may read them and issue
-    its weight loads before it waits for its predecessor (programmatic dependent launch)."""
+    its weight loads before it waits for its predecessor (programmatic dependent launch).  Without a pair table the
+    weights are asked for before that wait in any case: they are older than the launch before."""
     assert w.bits == 4, "the GEMV kernel handles 4 bpw"
     rows_per_item = rows_per_item if rows_per_item is not None else x.shape[0]
     K, N = w.k, w.n

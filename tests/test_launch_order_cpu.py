@@ -1,8 +1,12 @@
 """What kernels may read before their dependency wait: tables that are at least two launches old (shown on the CPU, launches recorded)."""
+import os
+import re
 from types import SimpleNamespace
 
+import pytest
 import torch
 
+from spark_engine_b200 import build
 from spark_engine_b200.models.plan import make_plan
 from spark_engine_b200.ops import cuda as cu
 
@@ -48,3 +52,14 @@ def test_head_table_of_latent_attention_is_two_launches_old(monkeypatch):
         at, t = made[table]
         assert torch.equal(t, arange(H, dtype=torch.int32))
         assert not early or i - at >= 2, (i, at)
+
+
+@pytest.mark.parametrize("source,kernel", [("gemv.cu", "gemv_bf16_kernel"), ("gemv.cu", "gemv_wide_mma_kernel"), ("gemv.cu", "gemv_long_mma_kernel"),
+                                           ("mx.cu", "mx_gemv_kernel")])
+def test_single_matrices_are_asked_for_after_the_dependency_wait(source, kernel):
+    """Their weights may come from the launch directly before (expansions on first use), and no argument says otherwise."""
+    with open(os.path.join(build.CSRC, "kernels", source)) as f:
+        body = f.read().split(f"\n{kernel}(", 1)[1].split("\n}\n", 1)[0]
+    wait = re.search(r"^  pdl_wait\(\);", body, re.M)
+    first = re.search(r"^  (?!auto)[^/\n]*\bload\(", body, re.M) or re.search(r"__ldg\(", body)
+    assert wait and first and wait.start() < first.start()
