@@ -403,20 +403,26 @@ EXL3_CTAS = 5 * 148                # CTAs of the EXL3 GEMV that run at a time
 
 def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> int:
     """K-slices per 128-column strip = CTAs of one cluster (<= 8).  Rows of one matrix (summed slice by slice, so that S may
-    depend on K and N only): as many as run at a time.  `pairs` of a row and an expert (summed in chunks of 256, whatever S is): the same for all
-    `items`, and further while a slice keeps 1024 k and two waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048 19.0 / 14.8 / 12.6 / 11.5, 40 pairs 32.4 / 27.8 /
-    29.0 / 33.4, 160 pairs 82 / 85 / 96 / 119; 40 pairs of 2048 x 512 17.2 / 21.1 / 30.3; 16 pairs of 3072 x 4096 - / 58.7 / 54.9 / 61.5; one row
-    of 12288 x 2048 12.9 / 12.2 / 10.4 / 11.8.  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS force the count for single-matrix / per-pair launches."""
+    depend on K and N only): as many as run at a time, and as keep the chains as short as slices of 256 had them (65536 x 2048, one / two
+    slices: error against 64 bits 6.8e-7 / 3.7e-7, 38.8 / 34.9 us).  `pairs` of a row and an expert (summed in chunks of 256, whatever S is):
+    the same for all `items`, and further while a slice keeps 1024 k and 2.2 waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048
+    14.0 / 13.3 / 11.3 / 10.5, 40 pairs 32.7 / 28.1 / 29.1 / 33.3, 160 pairs 82 / 85 / 96 / 118; 40 pairs of 2048 x 512 16.4 / 20.1; 16 pairs of
+    3072 x 4096, 2.08 waves at four - / 58.6 / 56.1 / 61.5, 12 of 4096 x 4096, 2.08 too - / 57.6 / 54.3 / 60.9, 32 of 2048 x 3072, 2.08 at three
+    52.0 with two, 57.4 with three; 24 of 4096 x 4096 98.9 with two, 102.7 with four (4.2 waves).  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS
+    force the count for single-matrix / per-pair launches."""
     blocks = K // 128
     forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if pairs else "SPARK_EXL3_S", "0"))
     if forced and blocks % forced == 0:
         return forced
     strips = N // 128 * (items if pairs else 1)
+    # rows: a chain of products (every fourth k-tile of a slice) no longer than the 16 of a slice of 256
+    counts = [s for s in range(1, 9) if blocks % s == 0]
+    least = 1 if pairs else -(-next((s for s in counts if K // s <= 256), counts[-1]) // 4)
     # (pairs: counts that leave whole chunks, of 256 where any count does, else of 128 for all counts of this K)
     for unit in ((2, 1) if pairs else (1,)):
         best = 0
-        for s in range(1, 9):
-            if blocks % (s * unit) or K // s > 2048:
+        for s in counts:
+            if blocks % (s * unit) or K // s > 2048 or s < least:
                 continue
             if not best or strips * s <= EXL3_CTAS or (pairs and K // s >= 1024 and strips * s <= 2.2 * EXL3_CTAS):
                 best = s

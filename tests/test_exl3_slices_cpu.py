@@ -23,3 +23,13 @@ def test_chunks_of_a_pair_do_not_depend_on_the_number_of_pairs():
         if any(_legal(K, s) for s in range(1, 9)):
             lengths = [K // cu._pick_slices(K, items, N, True) for N in (128, 1024, 4096) for items in (1, 3, 16, 40, 160, 256, 1000)]
             assert len({256 if k % 256 == 0 else 128 for k in lengths}) == 1, K
+
+
+def test_chains_of_rows_are_no_longer_than_those_of_slices_of_256():
+    """Four warps share a slice of one matrix, every fourth tile of 16 k each: the chain's length is what its rounding grows with."""
+    for K in range(128, 8 * 2048 + 1, 128):
+        legal = [s for s in range(1, 9) if _legal(K, s)]
+        if legal:
+            short = next((s for s in legal if K // s <= 256), legal[-1])
+            for N in (128, 2048, 12288, 65536, 151936):
+                assert K // cu._pick_slices(K, 1, N) // 64 <= K // short // 16, (K, N)
