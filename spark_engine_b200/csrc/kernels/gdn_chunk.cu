@@ -368,7 +368,8 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
 //   [O; X] = [Qt; W] S^T          M = 128 rows, N = 64 values, K = 128          D1 (two buffers)
 //   U      = Ut - X                by the warps that own the lanes of X
 //   D3     = Kt^T U                M = 128 keys, N = 64, K = 64                  then S^T <- D_C S^T + D3 in registers
-//   O     += P U                   the M = 128 operand's rows past P's 64 are whatever follows it: they end in X's lanes, which are read
+//   O     += P U                   the M = 128 operand's rows past P's 64 are whatever follows it: their lanes are off, as are those of
+//                                  the blocks of 16 rows in front of a step's rows of U (P is 0 there, and 0 times a NaN is none)
 // Warp 0 brings the operands in, tiles of 16 KB through a ring of 11 (eight per chunk); warp 1 issues; eight warps (two per lane quarter,
 // 32 value columns each) keep S, write it and U as K-major operands and store O.
 // What bounds it: the chain state -> product -> U -> product of a chunk, and the 128 KB per chunk that a CTA pulls from L2.
@@ -484,7 +485,10 @@ gdn_chunk_state_kernel(const float* __restrict__ ws, const int* __restrict__ seg
         for (int i = 0; i < 2; ++i) {
           const uint64_t ad = make_smem_desc_sw128(sb + sl * ST_SLOT + i * (GC * 128)), bd = make_smem_desc_sw128(b2 + i * (GVS * 128));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_tf32(d1, ad + 2 * k, bd + 2 * k, idesc, 1);
+          for (int k = 0; k < 4; ++k) {
+            const int b = 2 * i + (k >> 1);                    // rows 16 b .. of U: lanes from 16 b on, and none past P's 64
+            umma_tf32_add_lanes(d1, ad + 2 * k, bd + 2 * k, idesc, b == 0 ? 0u : b == 1 ? 0xffffu : ~0u, b == 3 ? 0xffffu : 0u, ~0u);
+          }
         }
         umma_commit(&empty[sl]);
         umma_commit(&empty[ut]);

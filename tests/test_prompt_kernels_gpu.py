@@ -175,3 +175,29 @@ def test_mxfp4_tiles_of_64_rows():
 def test_exl3_pairs_of_lengths_in_chunks_of_128(K, N, act):
     """No count of slices leaves these lengths whole chunks of 256."""
     test_exl3_pairs_do_not_depend_on_their_number(K, N, act)
+
+
+@pytest.mark.parametrize("at", [16, 40, 63, 107])
+def test_chunked_delta_rule_in_front_of_a_row_of_nan(at):
+    """Rows of earlier blocks than a row of NaN do not see it, as with products of 16 rows (P's blocks above the diagonal are 0, and not
+    multiplied).  A chunk's blocks are rows 0, 16 and 32 on: the inverse of its last 32 rows is one product."""
+    import dataclasses
+    from spark_engine_b200.config import ModelConfig, GdnConfig
+    from spark_engine_b200.models.model import GdnMixer
+    from spark_engine_b200.models.plan import make_plan
+    from spark_engine_b200.ops import cuda as cu
+    cfg = dataclasses.replace(ModelConfig(), gdn=GdnConfig(n_k_heads=1, n_v_heads=2, head_dim=128))
+    g = _gen(15)
+    w = {"conv": torch.rand(512, 4, device=DEV, generator=g) - 0.5, "A_log": torch.zeros(2, device=DEV), "dt_bias": torch.zeros(2, device=DEV),
+         "norm": torch.ones(128, device=DEV)}
+    proj = torch.randn(130, 768, device=DEV, generator=g).bfloat16()
+    ab = torch.randn(130, 4, device=DEV, generator=g).bfloat16()
+    outs = []
+    for bad in (False, True):
+        if bad:
+            proj[at] = float("nan")
+        m = GdnMixer(cfg, w, 1, DEV, torch.bfloat16)
+        outs.append(cu.gdn_mixer(m, proj, ab, make_plan([(0, [1] * 130, 5)], device=DEV), True))
+    assert cu.read_status(torch.device(DEV))[0] == 0
+    whole = at // 64 * 64 + (0, 16, 32, 32)[at % 64 // 16]
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:whole], outs[1][:whole]) and torch.isnan(outs[1][at:]).any(1).all()
