@@ -241,11 +241,13 @@ static int launch_gemm_exl3(const CUtensorMap& tA, const CUtensorMap& tB, const 
 
 using namespace spark;
 
-// xh fp16 [M, K] (row stride lda), W fp16 [N, K], svh fp16 [N], C bf16 [M, N] (row stride ldc, a multiple of 4).  N and K multiples of 128.
+// xh fp16 [M, K] (row stride lda), W fp16 [N, K], svh fp16 [N], C bf16 [M, N] (row stride ldc, a multiple of 4).  N and K multiples of 128; svh
+// and C start on 8 bytes.
 extern "C" int spark_gemm_exl3(const void* xh, int lda, const void* W, const void* svh, void* C, int ldc, int M, int N, int K, int* status,
                                cudaStream_t s) {
   if (M <= 0) return 0;
   if (N <= 0 || K <= 0 || (N & 127) || (K & 127) || (ldc & 3)) return -5;
+  if ((reinterpret_cast<uintptr_t>(svh) | reinterpret_cast<uintptr_t>(C)) & 7) return -5;
   static int sms = 0;
   if (!sms) { int dev; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   const int mt = (M + 2 * GX_BM - 1) / (2 * GX_BM);

@@ -525,6 +525,7 @@ def gemm_exl3(xh, wt, svh):
     M, K = xh.shape
     N = wt.shape[0]
     y = torch.empty(M, N, dtype=torch.bfloat16, device=xh.device)
+    svh = svh if P(svh) % 8 == 0 else svh.clone()                           # the epilogue reads four scales at a time
     rc = lib().spark_gemm_exl3(P(xh), xh.stride(0), P(wt), P(svh), P(y), N, M, N, K, P(status_word(xh.device)), stream())
     check(rc, "spark_gemm_exl3")
     return y

@@ -201,3 +201,13 @@ def test_chunked_delta_rule_in_front_of_a_row_of_nan(at):
     assert cu.read_status(torch.device(DEV))[0] == 0
     whole = at // 64 * 64 + (0, 16, 32, 32)[at % 64 // 16]
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:whole], outs[1][:whole]) and torch.isnan(outs[1][at:]).any(1).all()
+
+
+def test_exl3_scales_on_any_element():
+    """Output scales that start on 2 bytes (a view into a larger buffer) give the bits of aligned ones."""
+    from spark_engine_b200.ops import cuda as cu
+    w = Q.random_exl3(256, 128, 4, 0, 0.05, 3, DEV)
+    x = torch.randn(140, 128, device=DEV, generator=_gen(3)).bfloat16()
+    y = cu.exl3_linear(x, w)
+    w.svh = torch.cat((w.svh[:1], w.svh))[1:]
+    assert w.svh.data_ptr() % 8 == 2 and torch.equal(cu.exl3_linear(x, w), y)
