@@ -557,6 +557,13 @@ def exl3_linear(x, w: Exl3Weight):
     wt = _exl3_resident(w) if (x.shape[0] <= 16 and not w.experts) else None
     if wt is None:
         wt = exl3_reconstruct(w, scratch("exl3_recon", w.n * w.k, torch.float16, x.device)[: w.n * w.k].view(w.n, w.k))
+    # few rows of wide matrices wait for the weights, and one CTA per tile brings them in steadier than a pair, half of whose rows are not
+    # there.  us, one CTA and a transform pass / pairs: resident fp16 weights 4 rows of 2048 x 4096 17.7 / 18 to 22, 1 row of 2048 x 65536
+    # 73 / 85, 16 rows of 4096 x 12288 29 / 34, 16 of 4096 x 2048 23.6 / 20.3; expanded ones 25 rows of 2048 x 4096 22.8 / 27.4, 32 rows 22.6 /
+    # 20.9; 64 rows of 2048 x 9216 30.6 / 28.3, of 12288 36.8 / 38.5; 192 rows 49.7 / 40.8.  The bits are the same
+    M, N = xh.shape[0], w.n
+    if (M < 32 and N >= 4096) or (M <= 128 and N > 9216):
+        return exl3_had_rows(gemm_bf16(xh, wt, out_f32=True, fmt=0), w.svh, post=True)
     return gemm_exl3(xh, wt, w.svh)
 
 

@@ -211,3 +211,14 @@ def test_exl3_scales_on_any_element():
     y = cu.exl3_linear(x, w)
     w.svh = torch.cat((w.svh[:1], w.svh))[1:]
     assert w.svh.data_ptr() % 8 == 2 and torch.equal(cu.exl3_linear(x, w), y)
+
+
+@pytest.mark.parametrize("M,N,pairs", [(31, 4096, 0), (32, 4096, 1), (31, 3968, 1), (128, 9216, 1), (128, 9344, 0), (129, 9344, 1)])
+def test_exl3_rows_take_pairs_or_a_pass(monkeypatch, M, N, pairs):
+    from spark_engine_b200.ops import cuda as cu
+    w = Q.random_exl3(N, 128, 4, 0, 0.05, M, DEV)
+    x = torch.randn(M, 128, device=DEV, generator=_gen(M)).bfloat16()
+    calls, gemm = [], cu.gemm_exl3
+    monkeypatch.setattr(cu, "gemm_exl3", lambda *a: calls.append(1) or gemm(*a))
+    y = cu.exl3_linear(x, w)
+    assert len(calls) == pairs and torch.equal(y, gemm(cu.exl3_had_rows(x, w.suh, post=False), cu.exl3_reconstruct(w), w.svh))
