@@ -73,9 +73,15 @@ extern "C" int spark_gemm_bf16(const void* A, const void* B, void* C, int M, int
   g.M = M; g.N = N; g.K = K; g.status = status; g.ab_fmt = fmt;
   const int mt = (M + GEMM_BM - 1) / GEMM_BM;
   // 256 columns per tile unless 128 are less time by whole waves: few tiles leave SMs idle, and a ragged N pays for the columns it does not
-  // have (1021 rows of 1024 / 513 columns, 8192 rows of 513)
+  // have (1021 rows of 1024 / 513 columns, 8192 rows of 513).  Where row tiles read more of a large matrix again than L2 holds, 256 stay the
+  // better ones (us, 256 / 128: 300 rows of 4096 x 16384 64 / 70, 400 of 4096 x 12288 61 / 63.5, 256 of 4096 x 24576 74 / 77.5; but 256 rows
+  // of 2048 x 24576 43 / 39.5, 700 of 4096 x 9216 63 / 60); and where fewer than 32 rows are short (17 rows of 2048 x 12288 20.4 / 22.8, 31 with
+  // the matrix in L2 15.4 / 17.6; but 17 of 4096 x 12288 31.6 / 23.5, 64 of 2048 x 12288 21.5 / 15.7)
   const int w256 = (mt * ((N + 255) / 256) + num_sms() - 1) / num_sms() * 256, w128 = (mt * ((N + 127) / 128) + num_sms() - 1) / num_sms() * 128;
-  if (N > 128 && w256 <= w128 + w128 / 4) {
+  const long long w_bytes = static_cast<long long>(N) * K * 2;
+  const bool again = w_bytes >= (80LL << 20) && (mt - 1) * w_bytes >= (128LL << 20);
+  const bool few = M < 32 && K <= 2048 && N >= 9216;
+  if (N > 128 && (again || few || w256 <= w128 + w128 / 4)) {
     g.num_n_tiles = (N + 255) / 256; g.num_tiles = mt * g.num_n_tiles;
     int grid = g.num_tiles < num_sms() ? g.num_tiles : num_sms();
     if (out_f32) return launch<256, EpiStoreF32, false>(tA, tB, g, EpiStoreF32{(float*)C, ldc, N}, grid, stream);

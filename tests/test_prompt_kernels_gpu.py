@@ -222,3 +222,13 @@ def test_exl3_rows_take_pairs_or_a_pass(monkeypatch, M, N, pairs):
     monkeypatch.setattr(cu, "gemm_exl3", lambda *a: calls.append(1) or gemm(*a))
     y = cu.exl3_linear(x, w)
     assert len(calls) == pairs and torch.equal(y, gemm(cu.exl3_had_rows(x, w.suh, post=False), cu.exl3_reconstruct(w), w.svh))
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 24576, 2048), (257, 16384, 4096), (150, 9216, 128), (257, 641, 128)])
+def test_rows_of_a_product_do_not_depend_on_the_tile_width(M, N, K):
+    """Few rows, matrices that L2 keeps and that it does not, against rows in batches of 128 (other tile widths)."""
+    from spark_engine_b200.ops import cuda as cu
+    x = torch.randn(M, K, device=DEV, generator=_gen(M)).bfloat16()
+    w = torch.randn(N, K, device=DEV, generator=_gen(N)).bfloat16()
+    for f32 in (False, True):
+        assert torch.equal(cu.gemm_bf16(x, w, f32), torch.cat([cu.gemm_bf16(x[i: i + 128], w, f32) for i in range(0, M, 128)]))
