@@ -232,3 +232,17 @@ def test_rows_of_a_product_do_not_depend_on_the_tile_width(M, N, K):
     w = torch.randn(N, K, device=DEV, generator=_gen(N)).bfloat16()
     for f32 in (False, True):
         assert torch.equal(cu.gemm_bf16(x, w, f32), torch.cat([cu.gemm_bf16(x[i: i + 128], w, f32) for i in range(0, M, 128)]))
+
+
+@pytest.mark.parametrize("limit", [0.0, 3.0])
+@pytest.mark.parametrize("K,N", [(128, 128), (512, 256), (1152, 128), (2048, 1024)])
+def test_exl3_gated_rows_do_not_depend_on_their_number(K, N, limit):
+    """Few blocks are gated and transformed a warp each, many by eight lanes each: the bits of a row are the same, from rows on any alignment."""
+    from spark_engine_b200.ops import cuda as cu
+    w = Q.random_exl3(N, K, 4, 0, 0.05, 4, DEV)
+    x = 2 * torch.randn(16, 2 * K + 8, device=DEV, generator=_gen(K))
+    for shift in (0, 4, 1):
+        h = x.bfloat16()[:, shift: shift + 2 * K]
+        y = cu.exl3_gemv(h, w, act=1, limit=limit, out_f32=True)
+        for n in (1, 2, 5, 9):
+            assert torch.equal(cu.exl3_gemv(h[:n], w, act=1, limit=limit, out_f32=True), y[:n]), (shift, n)
