@@ -246,3 +246,25 @@ def test_exl3_gated_rows_do_not_depend_on_their_number(K, N, limit):
         y = cu.exl3_gemv(h, w, act=1, limit=limit, out_f32=True)
         for n in (1, 2, 5, 9):
             assert torch.equal(cu.exl3_gemv(h[:n], w, act=1, limit=limit, out_f32=True), y[:n]), (shift, n)
+
+
+@pytest.mark.parametrize("H", [64, 1028, 2050])
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 33])
+def test_combine_of_few_and_many_slots(H, k):
+    """Slots looked up by every thread and through the row's table; vectors and single columns; pairs of experts on other ranks."""
+    from spark_engine_b200.ops import cuda as cu
+    P, R, g = cu.P, 5, _gen(H + k)
+    w, sg = torch.rand(R, k, device=DEV, generator=g), torch.rand(R, device=DEV, generator=g)
+    inv = torch.randperm(R * k, device=DEV, generator=g).int()
+    pe = torch.randint(-1, 2, (R * k,), device=DEV, generator=g, dtype=torch.int32)
+    shared, res0 = torch.randn(R, H, device=DEV, generator=g).bfloat16(), torch.randn(R, H, device=DEV, generator=g)
+    for dtype in (torch.float32, torch.bfloat16):
+        y = torch.randn(R * k, H, device=DEV, generator=g).to(dtype)
+        res, out = res0.clone(), torch.empty(R, H, device=DEV, dtype=torch.bfloat16)
+        cu.check(cu.lib().spark_moe_combine(P(res), P(y), int(dtype == torch.float32), P(inv), P(w), R, k, P(shared), P(sg), H, P(out), cu.stream(),
+                                            P(pe)), "spark_moe_combine")
+        terms = (y[inv.long()].double() * (w.view(-1, 1) * (pe >= 0).view(-1, 1)).double()).view(R, k, H)
+        ref = terms.sum(1) + sg.double().unsqueeze(1) * shared.double()
+        size = terms.abs().sum(1) + (sg.unsqueeze(1) * shared).double().abs()
+        assert ((res.double() - res0.double() - ref).abs() <= (k + 2) * 2.0 ** -24 * (size + res0.double().abs())).all()
+        assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (k + 2) * 2.0 ** -24 * size).all()
