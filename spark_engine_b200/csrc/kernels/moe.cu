@@ -3,7 +3,7 @@
 //                  router kinds (softmax-renorm, sigmoid+bias x scale, sqrt-softplus+bias x scale);
 //                  also emits the (row, expert) pair table the grouped GEMV/GEMM kernels consume.
 //   moe_sort     : stable counting sort of the (row, slot) pairs by expert -> permuted row list, expert
-//                  offsets and the <=128-row tile list of the grouped tcgen05 GEMM (int atomics only,
+//                  offsets and the tile list (16 to 192 rows) of the grouped tcgen05 GEMMs (int atomics only,
 //                  order inside an expert = ascending pair index, so the result is deterministic).
 //   moe_combine  : residual += sum over slots (slot order) of weight * expert output (+ gated shared).
 // Reference: engine-rs/shim/qwen_moe.cu:10-92, dataflow.cu:370-572, ds41_ops.cu:375-421 (routers);
@@ -419,43 +419,23 @@ __global__ void moe_hist_kernel(const int* __restrict__ ids, int P, int E, int* 
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) block_hist[static_cast<size_t>(blockIdx.x) * E + e] = sh[e];
 }
-// one CTA: exclusive scan over blocks per expert, expert offsets, tile list.  Every step is parallel over the experts
-// (two block-wide scans: rows per expert -> offsets, tiles per expert -> first tile), each expert's thread writes its
-// own tiles; a single thread walking the 512 experts took 72 us per layer of a prefill chunk.
-__global__ void __launch_bounds__(1024)
-moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restrict__ offsets,
-                int4* __restrict__ tile_list, int* __restrict__ tile_count, int tile_rows) {
-  extern __shared__ int tot[];                         // [E]
-  __shared__ int sa[1024], sb[1024];
+// Offsets and row tiles of experts with `mine` rows each, a thread per expert (two scans over the CTA: rows -> offsets, tiles -> first tile);
+// each writes its own tiles (one thread walking 512 experts took 72 us).  Returns the expert's first row.  sa, sb: [blockDim.x].
+template <int NT>                                      // threads of the CTA, 0: blockDim.x
+__device__ __forceinline__ int moe_tiles(int mine, int E, int tile_rows, int* sa, int* sb, int* __restrict__ offsets, int4* __restrict__ tile_list,
+                                         int* __restrict__ tile_count) {
   const int e = threadIdx.x;
-  int mine = 0;
-  if (e < E) {
-    int acc = 0;
-    // sixteen counts are asked for before the first is overwritten (one at a time: 40 us for the 320 blocks of 8192 rows, top 10)
-    for (int b0 = 0; b0 < nblocks; b0 += 16) {
-      int c[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) c[u] = b0 + u < nblocks ? block_hist[static_cast<size_t>(b0 + u) * E + e] : 0;
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        if (b0 + u < nblocks) block_hist[static_cast<size_t>(b0 + u) * E + e] = acc;
-        acc += c[u];
-      }
-    }
-    tot[e] = acc;
-    mine = acc;
-  }
   const int my_tiles = (mine + tile_rows - 1) / tile_rows;
   sa[e] = mine; sb[e] = my_tiles;
   __syncthreads();
-  for (int st = 1; st < 1024; st <<= 1) {               // inclusive scans of rows and of tiles
+  for (int st = 1; st < (NT ? NT : blockDim.x); st <<= 1) {         // inclusive scans of rows and of tiles
     const int a = e >= st ? sa[e - st] : 0, b = e >= st ? sb[e - st] : 0;
     __syncthreads();
     sa[e] += a; sb[e] += b;
     __syncthreads();
   }
+  const int off = sa[e] - mine, t0 = sb[e] - my_tiles;
   if (e < E) {
-    const int off = sa[e] - mine, t0 = sb[e] - my_tiles;
     offsets[e] = off;
     if (tile_rows == 128) {                              // the consumer cuts a tile at the expert's end
       for (int i = 0; i < my_tiles; ++i) tile_list[t0 + i] = make_int4(off + i * 128, off + mine, e, 0);
@@ -465,6 +445,63 @@ moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restric
     }
     if (e == E - 1) { offsets[E] = sa[e]; *tile_count = sb[e]; }
   }
+  return off;
+}
+
+// Few pairs and experts in one launch, a thread per pair and per expert.  us, three launches / this: 257 pairs of 8 or 256
+// experts 8.1 / 4.5, 512 8.1 / 6.8, 640 8.1 / 8.3 (a thread's rank is a walk over the pairs before it)
+constexpr int SORT_ONE = 640;
+
+__global__ void __launch_bounds__(SORT_ONE)
+moe_sort_one_kernel(const int* __restrict__ ids, int P, int E, int* __restrict__ perm, int* __restrict__ inv_perm, int* __restrict__ offsets,
+                    int4* __restrict__ tile_list, int* __restrict__ tile_count, int tile_rows) {
+  __shared__ int sa[SORT_ONE], sb[SORT_ONE], first[SORT_ONE];
+  __shared__ __align__(16) int sid[SORT_ONE];
+  const int i = threadIdx.x, e = i < P ? ids[i] : -1;
+  sid[i] = e;
+  first[i] = 0;
+  __syncthreads();
+  if (e >= 0) atomicAdd(&first[e], 1);
+  __syncthreads();
+  const int mine = first[i];                             // threads past E: none
+  const int off = moe_tiles<0>(mine, E, tile_rows, sa, sb, offsets, tile_list, tile_count);
+  first[i] = off;
+  __syncthreads();
+  if (i >= P) return;
+  if (e < 0) { if (inv_perm) inv_perm[i] = -1; return; }
+  int dst = first[e];
+  int j = 0;                                             // earlier pairs of the expert
+#pragma unroll 4
+  for (; j + 4 <= i; j += 4) {
+    const int4 v = *reinterpret_cast<const int4*>(sid + j);
+    dst += (v.x == e) + (v.y == e) + (v.z == e) + (v.w == e);
+  }
+  for (; j < i; ++j) dst += sid[j] == e;
+  perm[dst] = i;
+  if (inv_perm) inv_perm[i] = dst;
+}
+
+// one CTA: exclusive scan over blocks per expert, offsets, tile list
+__global__ void __launch_bounds__(1024)
+moe_scan_kernel(int* __restrict__ block_hist, int nblocks, int E, int* __restrict__ offsets,
+                int4* __restrict__ tile_list, int* __restrict__ tile_count, int tile_rows) {
+  __shared__ int sa[1024], sb[1024];
+  const int e = threadIdx.x;
+  int mine = 0;
+  if (e < E) {
+    // sixteen counts are asked for before the first is overwritten (one at a time: 40 us for the 320 blocks of 8192 rows, top 10)
+    for (int b0 = 0; b0 < nblocks; b0 += 16) {
+      int c[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) c[u] = b0 + u < nblocks ? block_hist[static_cast<size_t>(b0 + u) * E + e] : 0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        if (b0 + u < nblocks) block_hist[static_cast<size_t>(b0 + u) * E + e] = mine;
+        mine += c[u];
+      }
+    }
+  }
+  moe_tiles<1024>(mine, E, tile_rows, sa, sb, offsets, tile_list, tile_count);
 }
 __global__ void moe_place_kernel(const int* __restrict__ ids, int P, int E, const int* __restrict__ block_hist,
                                  const int* __restrict__ offsets, int* __restrict__ perm, int* __restrict__ inv_perm) {
@@ -658,15 +695,20 @@ extern "C" int spark_moe_route(const float* logits, int ld, int R, int E, int to
   return spark_launch_rc(__func__);
 }
 
-// Scratch `block_hist` must hold ceil(P/256) * E ints when P > 2048.
+// Scratch `block_hist` must hold ceil(P/256) * E ints.
 // tile_rows 128: tiles {row, end of the expert, expert, 0} of up to 128 rows; another number: even tiles {row, end, expert, rows} of up to that.
 extern "C" int spark_moe_sort(const int* ids, int P, int E, int* perm, int* inv_perm, int* offsets, void* tile_list,
                               int* tile_count, int* block_hist, cudaStream_t s, int tile_rows) {
   if (P <= 0) return 0;
   if (E > 1024 || tile_rows < 16 || tile_rows > 192) return -5;                     // one thread per expert in the scan
+  if (P <= SORT_ONE && E <= SORT_ONE) {
+    const int n = ((P > E ? P : E) + 31) / 32 * 32;
+    moe_sort_one_kernel<<<1, n, 0, s>>>(ids, P, E, perm, inv_perm, offsets, (int4*)tile_list, tile_count, tile_rows);
+    return spark_launch_rc(__func__);
+  }
   const int nb = (P + 255) / 256;
   moe_hist_kernel<<<nb, 256, E * sizeof(int), s>>>(ids, P, E, block_hist);
-  moe_scan_kernel<<<1, 1024, E * sizeof(int), s>>>(block_hist, nb, E, offsets, (int4*)tile_list, tile_count, tile_rows);
+  moe_scan_kernel<<<1, 1024, 0, s>>>(block_hist, nb, E, offsets, (int4*)tile_list, tile_count, tile_rows);
   moe_place_kernel<<<nb, 256, 256 * sizeof(int), s>>>(ids, P, E, block_hist, offsets, perm, inv_perm);
   return spark_launch_rc(__func__);
 }

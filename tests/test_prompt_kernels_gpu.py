@@ -268,3 +268,22 @@ def test_combine_of_few_and_many_slots(H, k):
         size = terms.abs().sum(1) + (sg.unsqueeze(1) * shared).double().abs()
         assert ((res.double() - res0.double() - ref).abs() <= (k + 2) * 2.0 ** -24 * (size + res0.double().abs())).all()
         assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (k + 2) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("E", [1, 7, 640, 641])
+@pytest.mark.parametrize("P", [1, 33, 640, 641])
+def test_sort_of_few_pairs(E, P):
+    """One launch and three: stable order, pairs of other ranks (-1) left out."""
+    from spark_engine_b200.ops import cuda as cu
+    ids = torch.randint(-1, E, (P,), dtype=torch.int32, generator=torch.Generator().manual_seed(P))
+    perm, inv, offs, tiles, ntile, _ = cu.moe_sort(ids.to(DEV), E, 64)
+    local = (ids >= 0).nonzero()[:, 0]
+    order = local[torch.sort(ids[local], stable=True).indices]
+    n = torch.bincount(ids[local].long(), minlength=E)
+    want = torch.full((P,), -1, dtype=torch.int32)
+    want[order] = torch.arange(len(order), dtype=torch.int32)
+    assert torch.equal(perm[: len(order)].cpu().long(), order) and torch.equal(inv.cpu(), want)
+    assert torch.equal(offs.cpu().long(), torch.cat((torch.zeros(1, dtype=torch.int64), n.cumsum(0))))
+    t = tiles[: ntile.item()].tolist()
+    assert [e for _, _, e, _ in t] == [e for e in range(E) for _ in range(-(-int(n[e]) // 64))]
+    assert sorted(r for row, _, _, m in t for r in range(row, row + m)) == list(range(len(order)))
