@@ -107,10 +107,10 @@ __device__ __forceinline__ void exl3_fwht128_scaled(float (&v)[4], float2 s0, fl
     }
 }
 
-template <int CB, int NB, int WARPS>       // NB: blocks of 8 activation rows
-__global__ void __launch_bounds__(WARPS * 32, (NB == 1 ? EXL3_OCC : EXL3_OCC2) / WARPS)
+template <int CB, int NB>                  // NB: blocks of 8 activation rows
+__global__ void __launch_bounds__(EXL3_WARPS * 32, (NB == 1 ? EXL3_OCC : EXL3_OCC2) / EXL3_WARPS)
 exl3_gemv_kernel(const __grid_constant__ Exl3GemvArgs a) {
-  constexpr int WN = 8 / EXL3_TN, WK = WARPS / WN;              // WN warps share a k-tile's eight n-tiles
+  constexpr int WARPS = EXL3_WARPS, WN = 8 / EXL3_TN, WK = WARPS / WN;              // WN warps share a k-tile's eight n-tiles
   // (the argument block stays in constant memory: a local copy would put every field access on the stack)
   // Weight loads depend on no earlier launch; everything else is read after the dependency wait.
   const bool early = a.pair_expert == nullptr || a.pairs_early;
@@ -365,13 +365,12 @@ extern "C" int spark_exl3_gemv(const void* x, int ldx, const void* trellis, cons
   const uintptr_t xa = reinterpret_cast<uintptr_t>(x) | static_cast<uintptr_t>(ldx) * 2;
   a.x_align = (xa & 15) == 0 ? 16 : (xa & 7) == 0 ? 8 : 2;
   const bool two = rows_per_item > 8;
-  const int warps = EXL3_WARPS;
   const bool pairs = pair_expert && rows_per_item == 1;
   a.chunk = pairs ? (K / S % 256 == 0 ? 16 : 8) : K / S / 16;
   const int nch = K / 16 / S / a.chunk;
-  const size_t smem_bytes = static_cast<size_t>(rows_per_item) * ((K / S + 16) * 2 + nch * (S + warps * EXL3_TN / 8) * 128 * 4);
-  void (*kern)(Exl3GemvArgs) = codebook == 0 ? (two ? exl3_gemv_kernel<0, 2, EXL3_WARPS> : exl3_gemv_kernel<0, 1, EXL3_WARPS>)
-                                             : (two ? exl3_gemv_kernel<1, 2, EXL3_WARPS> : exl3_gemv_kernel<1, 1, EXL3_WARPS>);
+  const size_t smem_bytes = static_cast<size_t>(rows_per_item) * ((K / S + 16) * 2 + nch * (S + EXL3_WARPS * EXL3_TN / 8) * 128 * 4);
+  void (*kern)(Exl3GemvArgs) = codebook == 0 ? (two ? exl3_gemv_kernel<0, 2> : exl3_gemv_kernel<0, 1>)
+                                             : (two ? exl3_gemv_kernel<1, 2> : exl3_gemv_kernel<1, 1>);
   {
     static bool done[4] = {false, false, false, false};
     const int id = (codebook ? 2 : 0) + (two ? 1 : 0);
@@ -380,6 +379,6 @@ extern "C" int spark_exl3_gemv(const void* x, int ldx, const void* trellis, cons
       done[id] = true;
     }
   }
-  cudaError_t err = spark_launch_pdl(kern, dim3(N / 128, S, items), dim3(warps * 32), smem_bytes, s, dim3(1, S, 1), a);
+  cudaError_t err = spark_launch_pdl(kern, dim3(N / 128, S, items), dim3(EXL3_WARPS * 32), smem_bytes, s, dim3(1, S, 1), a);
   return err == cudaSuccess ? 0 : -4;
 }
