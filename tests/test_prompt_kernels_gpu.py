@@ -287,3 +287,32 @@ def test_sort_of_few_pairs(E, P):
     t = tiles[: ntile.item()].tolist()
     assert [e for _, _, e, _ in t] == [e for e in range(E) for _ in range(-(-int(n[e]) // 64))]
     assert sorted(r for row, _, _, m in t for r in range(row, row + m)) == list(range(len(order)))
+
+
+@pytest.mark.parametrize("rows,pos0,k", [(40, 200, 16), (129, 0, 8), (200, 1900, 256)])
+def test_masked_attention_on_the_selection_masks(rows, pos0, k):
+    """The masks as the selection leaves them, through the prompt tiles: attention over the tokens of its token list, in 64 bits."""
+    from spark_engine_b200.ops import cuda as cu, sparse as sp
+    P, g, D, Hq, Hkv = cu.P, _gen(rows), 64, 4, 2
+    ctx = pos0 + rows
+    q = torch.randn(rows, Hq, D, device=DEV, generator=g).bfloat16()
+    kv = torch.randn(2, ctx, Hkv, D, device=DEV, generator=g).bfloat16()
+    pos = torch.arange(pos0, ctx, dtype=torch.int32, device=DEV)
+    nb, mw = ctx // 4, (ctx + 127) // 128
+    score = torch.randint(0, 50, (rows, nb), device=DEV, generator=g).float()
+    sel, sel_n = sp.topk_select(score, nb, pos, 4, k)
+    mask = torch.full((rows, mw), -1, dtype=torch.int32, device=DEV)
+    cu.check(sp._dll().spark_topk_mask(P(score), nb, P(pos), rows, k, P(mask), mw, cu.stream(), 0), "spark_topk_mask")
+    out = torch.empty(rows, Hq, D, device=DEV, dtype=torch.bfloat16)
+    seg = torch.tensor([[0, 0, rows, pos0]], dtype=torch.int32, device=DEV)
+    row_kv = torch.zeros(rows, dtype=torch.int64, device=DEV)
+    cu.check(cu.lib().spark_attn_prefill_masked(P(q), P(kv[0]), P(kv[1]), P(row_kv), P(seg), 1, rows, P(q), Hq * D, 0, P(out), Hq, Hkv, D, D ** -0.5,
+                                                None, None, 0, rows, P(mask), mw, ctx, P(cu.status_word(torch.device(DEV))), cu.stream()), "masked")
+    assert cu.read_status(torch.device(DEV))[0] == 0
+    kk, vv = (t.double().repeat_interleave(Hq // Hkv, 1) for t in kv)
+    hide = torch.ones(rows, ctx, dtype=torch.bool, device=DEV)
+    for r in range(rows):
+        hide[r, sel[r, : sel_n[r]].long()] = False
+    s = torch.einsum("rhd,khd->hrk", q.double(), kk) * D ** -0.5
+    ref = torch.einsum("hrk,khd->rhd", torch.softmax(s.masked_fill(hide, -float("inf")), -1), vv)
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # as the token lists' test: two bf16 roundings and their sums
