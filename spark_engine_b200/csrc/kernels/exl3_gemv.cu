@@ -8,9 +8,10 @@
 // scratch, no atomics), applies the output Hadamard transform and scales.  Fixed reduction order => bitwise reproducible and independent of the rows in flight.
 // What bounds it: issue.  A tile of 256 weights takes about 35 instructions to decode and 46 in all; short slices add the transform of
 // the activations and the ends of the pipeline, so that pairs get as few slices as still fill the SMs (`_pick_slices`).  us, before (weights as the
-// 8-column operand of two products, a warp per 16 columns of every k-tile, slices of 256) and after: 40 pairs of 1024 x 2048 34.4 -> 27.8, of 2048 x 512
-// 20.1 -> 17.2; 160 pairs 122 -> 82 and 62 -> 52; 16 pairs of 3072 x 4096 74 -> 55, of 4096 x 1536 41 -> 33; one row of 12288 x 2048
-// 12.2 -> 10.4, of 2048 x 4096 9.0 -> 7.9.  160 pairs: 70 % of the issue slots of the busy SMs, 61 % over the launch.
+// 8-column operand of two products, a warp per 16 columns of every k-tile, slices of 256) and after: 40 pairs of 1024 x 2048 33.6 -> 27.6, of 2048 x 512,
+// gated, 18.5 -> 15.2; 160 pairs 120 -> 81 and 60 -> 46; 16 pairs of 3072 x 4096 74 -> 55, of 4096 x 1536, gated, 41 -> 33; one row of
+// 12288 x 2048 12.2 -> 10.2, of 2048 x 4096 8.9 -> 7.8.  40 pairs of 1024 x 2048: 51 instructions a tile in all, 65 % of the issue slots of the
+// busy SMs, 49 % over the launch.
 // M <= 16 is bandwidth / decode-ALU bound, so the warp-level MMA feeds it; GEMM-shaped EXL3 work goes
 // through exl3_reconstruct to the tcgen05 GEMM.
 // Replaces engine-rs/shim/qwen_exl3.cuh:427-626 (gemv_kernel / gemv_fused_kernel / finish_kernel) and

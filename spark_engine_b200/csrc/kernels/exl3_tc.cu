@@ -1,7 +1,7 @@
 // EXL3 grouped GEMM of prompt-size MoE batches on tcgen05: packed trellises -> fp16 operands in tensor memory.
 //   plain: y[rows, N]   = had128(xh @ inner_e) * svh_e                                   (fp32 or bf16)
 //   glu:   y[rows, F]   = had128(bf16(act(gate) * up) * suh2_e) as fp16, the input rows of the down product
-// with xh = had128(x * suh_e) in fp16, rows in expert order, work items of one expert and <= 128 rows.
+// with xh = had128(x * suh_e) in fp16, rows in expert order, work items of one expert and <= 192 rows.
 //
 // The product runs transposed: the weights are the 128-row M operand, the rows of the item the N operand (a multiple of 16, so
 // that 20 rows of an expert cost 32 columns and not 128).  A lane that takes four consecutive words of a packed tile owns all 16 k

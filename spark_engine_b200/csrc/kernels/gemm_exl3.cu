@@ -4,7 +4,8 @@
 // CTA pairs (cta_group::2): a pair computes 256 x BN, every CTA brings its 128 rows of A and half of the rows of W into its own shared
 // memory, and the leader issues for both.  What bounds it: a CTA by itself (128 x 256) asks L2 for 48 KB per 512 cycles of products, more than
 // the 64 bytes a cycle an SM gets; a pair asks for 32 KB per CTA.  The transform as a pass of its own wrote and read the products in fp32
-// (12 bytes per output where 2 are left).  4096 rows of 2048 x 12288 and 4096 x 2048, product and transform: 342 -> 215 us.
+// (12 bytes per output where 2 are left).  4096 rows of 2048 x 12288 and 4096 x 2048, product and transform: 342 -> 215 us.  Few rows of
+// wide matrices are left to the two launches (`exl3_linear`).
 //   warp 0      TMA: both CTAs' tiles are counted by the leader's barrier
 //   warp 1      the leader's issues the MMAs; commits reach both CTAs
 //   warps 2..5  epilogue of the CTA's 128 rows, two accumulator stages

@@ -406,9 +406,9 @@ def _pick_slices(K: int, items: int = 1, N: int = 128, pairs: bool = False) -> i
     depend on K and N only): as many as run at a time, and as keep the chains as short as slices of 256 had them (65536 x 2048, one / two
     slices: error against 64 bits 6.8e-7 / 3.7e-7, 38.8 / 34.9 us).  `pairs` of a row and an expert (summed in chunks of 256, whatever S is):
     the same for all `items`, and further while a slice keeps 1024 k and 2.2 waves hold all.  us, S = 1 / 2 / 4 / 8: 10 pairs of 1024 x 2048
-    14.0 / 13.3 / 11.3 / 10.5, 40 pairs 32.7 / 28.1 / 29.1 / 33.3, 160 pairs 82 / 85 / 96 / 118; 40 pairs of 2048 x 512 16.4 / 20.1; 16 pairs of
-    3072 x 4096, 2.08 waves at four - / 58.6 / 56.1 / 61.5, 12 of 4096 x 4096, 2.08 too - / 57.6 / 54.3 / 60.9, 32 of 2048 x 3072, 2.08 at three
-    52.0 with two, 57.4 with three; 24 of 4096 x 4096 98.9 with two, 102.7 with four (4.2 waves).  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS
+    14.7 / 13.3 / 11.3 / 10.3, 40 pairs 31.8 / 27.1 / 28.6 / 32.6, 160 pairs 81 / 84 / 95 / 116; 40 pairs of 2048 x 512 15.0 / 16.9; 16 pairs of
+    3072 x 4096, 2.08 waves at four - / 57.2 / 55.2 / 60.4, 12 of 4096 x 4096, 2.08 too - / 57.4 / 55.7 / 61.0, 32 of 2048 x 3072, 2.08 at three
+    50.6 with two, 56.1 with three; 24 of 4096 x 4096 98.3 with two, 102.3 with four (4.2 waves).  SPARK_EXL3_S / SPARK_EXL3_S_PAIRS
     force the count for single-matrix / per-pair launches."""
     blocks = K // 128
     forced = int(os.environ.get("SPARK_EXL3_S_PAIRS" if pairs else "SPARK_EXL3_S", "0"))
@@ -823,7 +823,7 @@ def _expert_gemv(x, w, pairs, pair_expert, pair_row, act, limit, out_f32, pairs_
 
 
 def moe_sort(ids, E, tile_rows=128):
-    """`tile_rows`: 128, or another number for the even tiles that `exl3_tc` (up to 192) and `moe_mxfp4_tc` (up to 128) alone take."""
+    """`tile_rows`: 128, or another number for the even tiles that `exl3_tc` (up to 192) and `moe_mxfp4_tc` (64) alone take."""
     Pn = ids.numel()
     dev = ids.device
     dbg.check_index("moe_sort expert ids", ids, 0, E, allow=-1)

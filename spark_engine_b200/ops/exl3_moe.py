@@ -34,7 +34,9 @@ def _fused(wgu, wd) -> bool:
 
 def tile_rows(wgu, wd, pairs: int, n_experts: int) -> int:
     """Rows of a tile for the products of these experts: 96 (two items' accumulators side by side) while an expert has up to 48 rows
-    on average, beyond 192 (an expert is decoded once, its rows are read out by the decoders)."""
+    on average, beyond 192 (an expert is decoded once, its rows are read out by the decoders).  Layer of 512 experts, every one as likely,
+    us with 96 / 128 / 192: 39 rows per expert 684 / 717 / 720, 59 757 / 800 / 800, 80 901 / 957 / 955, 98 1138 / 1089 / 1091.  The line is half
+    of a tile, below where even loads have it: real loads are uneven, and an expert with twice the average still is one tile of 96."""
     return 128 if not _fused(wgu, wd) else 96 if pairs <= 48 * n_experts else 192
 
 
