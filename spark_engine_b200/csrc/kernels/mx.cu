@@ -98,17 +98,24 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   __half* xs = reinterpret_cast<__half*>(smem_mx);              // [RB][XS]
   float* red = reinterpret_cast<float*>(smem_mx + static_cast<size_t>(RB) * XS * 2);   // [2][warps][16][16]
   const int item = blockIdx.y;
-  pdl_wait();
-  if (pair_expert && pair_expert[item] < 0) return;            // pair of an expert that lives on another rank
-  const int e = pair_expert ? pair_expert[item] : 0;
   const int R = rows_per_item;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * MXV_COLS * cgroups;
   constexpr int KI = FMT == 1 ? 128 : 64;                      // k per warp iteration (4 threads x 16 bytes)
   constexpr int KT = KI / 4;                                   // k per thread per iteration
   constexpr int STEPS = KT / 4;                                // mma k-steps per iteration
+  constexpr int U = 4;                                         // k-slices per batch
   const int iters = K / KI;
   const size_t row_bytes = FMT == 1 ? (K >> 1) : K;
+  if (!pair_expert && warp * U + t < iters) {
+    // the first batch of a single matrix starts on its way to L2, where the launch before leaves its stores: nothing is read ahead of the wait
+    const uint8_t* first = W + static_cast<size_t>(n0 + g) * row_bytes + (warp * U + t) * 64;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(first));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(first + 8 * row_bytes));
+  }
+  pdl_wait();
+  if (pair_expert && pair_expert[item] < 0) return;            // pair of an expert that lives on another rank
+  const int e = pair_expert ? pair_expert[item] : 0;
   const uint8_t* Wb = W + static_cast<size_t>(e) * w_expert_stride;
   const uint8_t* w_lo = Wb + static_cast<size_t>(n0 + g) * row_bytes + t * 16;
   const uint8_t* w_hi = w_lo + 8 * row_bytes;
@@ -130,7 +137,6 @@ mx_gemv_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const uint8_t* __re
   // of batch b+1 (the next U k-slices of this warp, or the first ones of the next column group) are issued before
   // the MMAs of batch b, so the memory pipe stays full across the per-group reductions.
   float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-  constexpr int U = 4;                                         // k-slices per batch
   const int nb = (iters + MXV_WARPS * U - 1) / (MXV_WARPS * U);      // batches per column group
   const int total = cgroups * nb;
   uint4 wl0[U], wh0[U], wl1[U], wh1[U];
