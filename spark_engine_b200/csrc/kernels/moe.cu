@@ -168,13 +168,15 @@ constexpr int ROUTER_RB = 16, ROUTER_WARPS = 16, ROUTER_COLS = 4;
 // 7.5 us, 16 rows 32 -> 15.2, 4 rows of the MXFP4 preset 37 -> 13.6 (before: a warp per column for all rows, the rows staged in shared
 // memory, two rows' choices after one another, one kernel for all kinds).  Tensor cores in place of the FP32 units (9.3, 13, 16 us) add
 // 16 products at a time with fewer bits: the logits' error grew 1.2 to 15 times over K = 256 .. 7168.
-// KIND: 0, 1 and 2 alone, 3 the others (the kernel is fetched anew in every layer: what a kind does not run costs instruction misses)
+// KIND: a kernel per kind (it is fetched anew in every layer: what a kind does not run costs instruction misses; kinds 3, 4 and 5 in one took
+// 11.9, 10.4 and 10.0 us for 4 rows of 2048 and 512 columns, alone 10.0, 7.1 and 7.0; all six in one 10.7, 7.9 and 8.1)
 template <int EPL, int NR, int KIND>                        // NR: rows of a warp (R <= 4 NR)
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 moe_router_topk_kernel(const __grid_constant__ RouterArgs a) {
   __shared__ int last_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int R = a.R, kind = KIND == 3 ? a.kind : KIND;
+  constexpr int kind = KIND;
+  const int R = a.R;
   const int NE = a.E + (a.shared_gate ? 1 : 0);
   const int n = blockIdx.x * ROUTER_COLS + (warp & 3), r0 = warp >> 2;
   const int KV = a.K >> 3;                                  // 16-byte vectors of a row
@@ -755,7 +757,8 @@ extern "C" int spark_moe_router_topk(const void* x, int ldx, const void* Wg, int
                   : pick(std::integral_constant<int, 4>{}, knd);
   };
   void (*kern)(RouterArgs) = kind == 0 ? of(std::integral_constant<int, 0>{}) : kind == 1 ? of(std::integral_constant<int, 1>{})
-                           : kind == 2 ? of(std::integral_constant<int, 2>{}) : of(std::integral_constant<int, 3>{});
+                           : kind == 2 ? of(std::integral_constant<int, 2>{}) : kind == 3 ? of(std::integral_constant<int, 3>{})
+                           : kind == 4 ? of(std::integral_constant<int, 4>{}) : of(std::integral_constant<int, 5>{});
   const cudaError_t err = spark_launch_pdl(kern, dim3((NE + ROUTER_COLS - 1) / ROUTER_COLS), dim3(ROUTER_WARPS * 32), 0, s, dim3(1, 1, 1), a);
   return err == cudaSuccess ? 0 : -4;
 }
