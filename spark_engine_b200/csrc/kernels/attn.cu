@@ -546,6 +546,39 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
   if (tid < D) out[(static_cast<size_t>(r) * Hq + h) * D + tid] = __float2bfloat16(res);
 }
 
+// Up to four splits: every thread has all statistics and its partial values in flight at once, with nothing to wait for in between (the same sums).
+// us with the attention in front: one row, one split, D = 256 8.4 -> 7.3; 300 rows
+// of one split 85 -> 75, of four 338 -> 328.
+constexpr int MERGE_FEW = 4;
+
+__global__ void __launch_bounds__(MERGE_T)
+attn_merge_few_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int nsplit, const __nv_bfloat16* __restrict__ qkv, int ld,
+                      int gated, int Hq, int D, __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
+  const int r = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
+  if (d >= D) return;
+  const size_t pb = (static_cast<size_t>(r) * Hq + h) * nsplit;
+  float m[MERGE_FEW], ls[MERGE_FEW], p[MERGE_FEW], g = 0.f;
+#pragma unroll
+  for (int u = 0; u < MERGE_FEW; ++u) {
+    const size_t at = pb + min(u, nsplit - 1);
+    m[u] = u < nsplit ? part_ml[2 * at] : -INFINITY;
+    ls[u] = part_ml[2 * at + 1];
+    p[u] = __ldcg(part_o + at * D + d);                        // (an empty split's is not written, and not used)
+  }
+  if (gated) g = __bfloat162float(qkv[static_cast<size_t>(r) * ld + h * 2 * D + D + d]);
+  float M = m[0], l = 0.f, o = 0.f;
+#pragma unroll
+  for (int u = 1; u < MERGE_FEW; ++u) M = fmaxf(M, m[u]);
+#pragma unroll
+  for (int u = 0; u < MERGE_FEW; ++u)
+    if (m[u] != -INFINITY) { const float w = __expf(m[u] - M); l += w * ls[u]; o += w * p[u]; }
+  float res = o / l;
+  if (gated) res = res / (1.f + __expf(-g));
+  out[(static_cast<size_t>(r) * Hq + h) * D + d] = __float2bfloat16(res);
+}
+
 }  // namespace spark
 
 using namespace spark;
@@ -608,11 +641,12 @@ static int attn_decode_launch(const void* qbuf, const void* kc, const void* vc, 
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return -4;
+  const auto merge = nsplit <= MERGE_FEW ? attn_merge_few_kernel : attn_merge_kernel;
   if (pdl)
-    err = spark_launch_pdl(attn_merge_kernel, dim3(R, Hq), dim3((D + 31) / 32 * 32), 0, s, dim3(1, 1, 1), (const float*)part_o, (const float*)part_ml,
+    err = spark_launch_pdl(merge, dim3(R, Hq), dim3((D + 31) / 32 * 32), 0, s, dim3(1, 1, 1), (const float*)part_o, (const float*)part_ml,
                            nsplit, (const __nv_bfloat16*)qkv, ld, gated, Hq, D, (__nv_bfloat16*)out);
   else {
-    attn_merge_kernel<<<dim3(R, Hq), (D + 31) / 32 * 32, 0, s>>>(part_o, part_ml, nsplit, (const __nv_bfloat16*)qkv, ld, gated, Hq, D, (__nv_bfloat16*)out);
+    merge<<<dim3(R, Hq), (D + 31) / 32 * 32, 0, s>>>(part_o, part_ml, nsplit, (const __nv_bfloat16*)qkv, ld, gated, Hq, D, (__nv_bfloat16*)out);
     err = cudaGetLastError();
   }
   return err == cudaSuccess ? 0 : -4;

@@ -316,3 +316,24 @@ def test_masked_attention_on_the_selection_masks(rows, pos0, k):
     s = torch.einsum("rhd,khd->hrk", q.double(), kk) * D ** -0.5
     ref = torch.einsum("hrk,khd->rhd", torch.softmax(s.masked_fill(hide, -float("inf")), -1), vv)
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # as the token lists' test: two bf16 roundings and their sums
+
+
+@pytest.mark.parametrize("D", [80, 128])
+@pytest.mark.parametrize("ctx", [3, 64, 250, 256, 257])
+def test_decode_attention_of_few_splits(D, ctx):
+    """Up to four splits and more, rows that see the first split only (the others are empty, their partial rows not written)."""
+    from spark_engine_b200.ops import cuda as cu
+    P, g, Hq, Hkv, ns = cu.P, _gen(ctx), 8, 4, (ctx + 63) // 64
+    q, qkv = torch.randn(2, Hq, D, device=DEV, generator=g).bfloat16(), torch.randn(2, 2 * Hq * D, device=DEV, generator=g).bfloat16()
+    kv = torch.randn(2, ctx, Hkv, D, device=DEV, generator=g).bfloat16()
+    pos = torch.tensor([ctx - 1, min(ctx - 1, 40)], dtype=torch.int32, device=DEV)
+    row_kv = torch.zeros(2, dtype=torch.int64, device=DEV)
+    po, pm = (torch.full((2 * Hq * ns * n,), float("nan"), device=DEV) for n in (D, 2))
+    out = torch.empty(2, Hq, D, device=DEV, dtype=torch.bfloat16)
+    cu.check(cu.lib().spark_attn_decode(P(q), P(kv[0]), P(kv[1]), None, None, 0, P(pos), P(row_kv), None, None, 0, P(po), P(pm), ns, P(qkv), 2 * Hq * D, 1,
+                                        2, Hq, Hkv, D, D ** -0.5, P(out), cu.stream(), None, None, None, 1), "spark_attn_decode")
+    kk, vv = (t.double().repeat_interleave(Hq // Hkv, 1) for t in kv)
+    s = torch.einsum("rhd,khd->hrk", q.double(), kk) * D ** -0.5
+    s = s.masked_fill(torch.arange(ctx, device=DEV) > pos.unsqueeze(1), -float("inf"))
+    ref = torch.einsum("hrk,khd->rhd", torch.softmax(s, -1), vv) * torch.sigmoid(qkv.view(2, Hq, 2, D)[:, :, 1].double())
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # probabilities and results in bf16
