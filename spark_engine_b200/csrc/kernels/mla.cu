@@ -195,12 +195,10 @@ __device__ __forceinline__ void mla_mma(float (&c)[4], const uint32_t (&a)[4], u
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// grid (R, ceil(nsplit / spc)); NW warps (16 where a CTA has 64 heads and an SM to itself, else 8); a CTA walks `spc` consecutive splits.  HM = 16-head MMA tiles (H <= 16*HM).  KW = kv_lora + rope (multiple of 16),
+// grid (R, ceil(nsplit / spc)); NW warps (8 or 16); a CTA walks `spc` consecutive splits.  HM = 16-head MMA tiles (H <= 16*HM).  KW = kv_lora + rope (multiple of 16),
 // L = kv_lora (multiple of 16).
-template <int HM> constexpr int mla_warps() { return HM == 4 ? 16 : 8; }
-
-template <int HM, bool SPLITP>
-__global__ void __launch_bounds__(mla_warps<HM>() * 32)
+template <int HM, bool SPLITP, int NW>
+__global__ void __launch_bounds__(NW * 32)
 mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
                   const __nv_bfloat16* __restrict__ lat,         // [tokens, KW]
                   const int* __restrict__ pos, const long long* __restrict__ row_kv, const int* __restrict__ sel,
@@ -210,7 +208,7 @@ mla_decode_kernel(const __nv_bfloat16* __restrict__ q_full,      // [R, H, KW]
                   const int* __restrict__ row_pos0, const int* __restrict__ row_j, const int* __restrict__ anc,
                   int lat_fp8, MlaPages pg) {
   extern __shared__ __align__(16) uint8_t smem_mla[];
-  constexpr int NW = mla_warps<HM>(), NT = NW * 32, HG = NW / 8, HMG = HM / HG;      // HG groups of eight warps split the head tiles
+  constexpr int NT = NW * 32, HG = NW / 8, HMG = HM / HG;      // HG groups of eight warps split the head tiles
   pdl_wait();
   pdl_trigger();
   const int LDK = KW + 8;
@@ -438,15 +436,15 @@ extern "C" int spark_mla_qrope(const void* qb, int ldq, int R, int H, int D, int
 
 namespace spark {
 
-template <int HM, bool SPLITP>
+template <int HM, bool SPLITP, int NW>
 static int launch_mla_decode(dim3 grid, int smem, cudaStream_t s, const void* q_full, const void* lat, const int* pos, const long long* row_kv,
                              const int* sel, const int* sel_n, int sel_ld, float* part_o, float* part_ml, int H, int KW, int L,
                              float scale, int nsplit, int spc, const int* row_pos0, const int* row_j, const int* anc, int lat_fp8,
                              MlaPages pg) {
-  auto kern = mla_decode_kernel<HM, SPLITP>;
+  auto kern = mla_decode_kernel<HM, SPLITP, NW>;
   static bool done = false;
   if (!done) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); done = true; }
-  const cudaError_t err = spark_launch_pdl(kern, grid, dim3(mla_warps<HM>() * 32), smem, s, dim3(1, 1, 1), (const __nv_bfloat16*)q_full,
+  const cudaError_t err = spark_launch_pdl(kern, grid, dim3(NW * 32), smem, s, dim3(1, 1, 1), (const __nv_bfloat16*)q_full,
                                            (const __nv_bfloat16*)lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, L, scale,
                                            nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg);
   return err == cudaSuccess ? 0 : -4;
@@ -468,11 +466,15 @@ static int mla_attn(const void* q_full, const void* lat, const int* pos, const l
   const int spc = R >= 128 ? nsplit : (R >= 32 ? 4 : 1);
   const dim3 grid(R, (nsplit + spc - 1) / spc);
   int rc;
-#define SPARK_MLA_DEC(HMV, SPV)                                                                                            \
-  rc = launch_mla_decode<HMV, SPV>(grid, smem, s, q_full, lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, kv_lora, \
-                              scale, nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg)
-  if (splitp) { if (HM == 1) SPARK_MLA_DEC(1, true); else if (HM == 2) SPARK_MLA_DEC(2, true); else SPARK_MLA_DEC(4, true); }
-  else { if (HM == 1) SPARK_MLA_DEC(1, false); else if (HM == 2) SPARK_MLA_DEC(2, false); else SPARK_MLA_DEC(4, false); }
+#define SPARK_MLA_DEC(HMV, SPV, NWV)                                                                                            \
+  rc = launch_mla_decode<HMV, SPV, NWV>(grid, smem, s, q_full, lat, pos, row_kv, sel, sel_n, sel_ld, part_o, part_ml, H, KW, kv_lora, \
+                                        scale, nsplit, spc, row_pos0, row_j, anc, lat_fp8, pg)
+  // sixteen warps where an SM holds one CTA: its tiles leave no room for two (228 KB, 1 KB of each reserved), or there are no more CTAs than SMs.
+  // Two of eight hide each other's phases (us, 8 / 16 warps, 64 heads, latents of 128 + 64: 16 rows of 3000 tokens 40 / 48, 200 of 400 77 / 89; one
+  // CTA per SM: 4 rows of 1500 13.7 / 12.2, 40 of 600 33 / 28; latents of 512 + 64, 200 rows of 400 242 / 220)
+  const bool wide = 2 * (smem + 1024) > 228 * 1024 || static_cast<long long>(grid.x) * grid.y <= 148;
+  if (splitp) { if (HM == 1) SPARK_MLA_DEC(1, true, 8); else if (HM == 2) SPARK_MLA_DEC(2, true, 8); else if (wide) SPARK_MLA_DEC(4, true, 16); else SPARK_MLA_DEC(4, true, 8); }
+  else { if (HM == 1) SPARK_MLA_DEC(1, false, 8); else if (HM == 2) SPARK_MLA_DEC(2, false, 8); else if (wide) SPARK_MLA_DEC(4, false, 16); else SPARK_MLA_DEC(4, false, 8); }
 #undef SPARK_MLA_DEC
   if (!rc) rc = launch_split_merge(part_o, part_ml, nsplit, sink, R, H, kv_lora, out, gate, ldg, pg.rows, 0, s);
   if (rc) return rc;

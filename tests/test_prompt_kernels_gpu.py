@@ -337,3 +337,29 @@ def test_decode_attention_of_few_splits(D, ctx):
     s = s.masked_fill(torch.arange(ctx, device=DEV) > pos.unsqueeze(1), -float("inf"))
     ref = torch.einsum("hrk,khd->rhd", torch.softmax(s, -1), vv) * torch.sigmoid(qkv.view(2, Hq, 2, D)[:, :, 1].double())
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # probabilities and results in bf16
+
+
+@pytest.mark.parametrize("H,L", [(64, 128), (40, 256), (64, 512)])
+def test_latent_attention_does_not_depend_on_the_warps(H, L):
+    """Few rows take sixteen warps per CTA, many eight (where two CTAs fit an SM): the bits of a row are the same."""
+    from spark_engine_b200.ops import cuda as cu
+    P, g, rope, ctx, rows = cu.P, _gen(H + L), 64, 200, 160
+    KW, ns = L + rope, (ctx + 63) // 64
+    q, lat = torch.randn(rows, H, KW, device=DEV, generator=g).bfloat16(), torch.randn(ctx, KW, device=DEV, generator=g).bfloat16()
+    pos = torch.arange(ctx - rows, ctx, dtype=torch.int32, device=DEV)
+    row_kv, sink = torch.zeros(rows, dtype=torch.int64, device=DEV), torch.randn(H, device=DEV, generator=g)
+
+    def run(lo, hi):
+        R = hi - lo
+        po, pm, out = torch.empty(R * H * ns * L, device=DEV), torch.empty(R * H * ns * 2, device=DEV), torch.empty(R, H, L, device=DEV, dtype=torch.bfloat16)
+        cu.check(cu.lib().spark_mla_attn(P(q[lo:hi]), P(lat), P(pos[lo:hi]), P(row_kv), None, None, 0, P(po), P(pm), ns, P(sink), R, H, L, rope, KW ** -0.5,
+                                         P(out), cu.stream(), None, None, None, 0), "spark_mla_attn")
+        return out
+    y = run(0, rows)
+    for lo, hi in ((0, 1), (7, 40), (100, 160)):
+        assert torch.equal(run(lo, hi), y[lo:hi])
+    s = torch.einsum("rhd,kd->hrk", q.double(), lat.double()) * KW ** -0.5
+    s = s.masked_fill(torch.arange(ctx, device=DEV) > pos.unsqueeze(1), -float("inf"))
+    w = torch.softmax(torch.cat((s, sink.double().view(H, 1, 1).expand(H, rows, 1)), -1), -1)[..., :-1]
+    ref = torch.einsum("hrk,kd->rhd", w, lat[:, :L].double())
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # probabilities and results in bf16
