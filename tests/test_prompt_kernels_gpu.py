@@ -363,3 +363,14 @@ def test_latent_attention_does_not_depend_on_the_warps(H, L):
     w = torch.softmax(torch.cat((s, sink.double().view(H, 1, 1).expand(H, rows, 1)), -1), -1)[..., :-1]
     ref = torch.einsum("hrk,kd->rhd", w, lat[:, :L].double())
     assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -7.5             # probabilities and results in bf16
+
+
+@pytest.mark.parametrize("K", [128, 512, 640])
+def test_rows_quantised_before_and_behind_their_gather(monkeypatch, K):
+    from spark_engine_b200.ops import mx
+    h = 3 * torch.randn(37, K, device=DEV, generator=_gen(K)).bfloat16()
+    rows = torch.randint(0, 37, (300,), device=DEV, generator=_gen(K), dtype=torch.int32)
+    behind = mx._quantised_rows(h, rows)
+    monkeypatch.setattr(mx, "QUANTISE_FIRST", 0)
+    for a, b in zip(mx._quantised_rows(h, rows), behind):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
