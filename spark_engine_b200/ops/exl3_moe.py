@@ -33,11 +33,11 @@ def _fused(wgu, wd) -> bool:
 
 
 def tile_rows(wgu, wd, pairs: int, n_experts: int) -> int:
-    """Rows of a tile for the products of these experts: 96 (two items' accumulators side by side) while an expert has up to 48 rows
-    on average, beyond 192 (an expert is decoded once, its rows are read out by the decoders).  Layer of 512 experts, every one as likely,
-    us with 96 / 128 / 192: 39 rows per expert 684 / 717 / 720, 59 757 / 800 / 800, 80 901 / 957 / 955, 98 1138 / 1089 / 1091.  The line is half
-    of a tile, below where even loads have it: real loads are uneven, and an expert with twice the average still is one tile of 96."""
-    return 128 if not _fused(wgu, wd) else 96 if pairs <= 48 * n_experts else 192
+    """Rows of a tile for the products of these experts: 96 (two items' accumulators side by side) while an expert has up to 64 rows
+    on average, beyond 192 (an expert is decoded once, its rows are read out by the decoders).  Sort and products of 512 experts of
+    [2048 x 1024], us with 96 / 192: every expert as likely, 53 rows on average 563 / 606, 66 623 / 667, 80 706 / 738, 102 986 / 869; likelihoods
+    falling as rank^-0.6 633 / 642, 681 / 691, 777 / 767, 902 / 869; as 1 / rank 666 / 665, 750 / 730, 828 / 790, 962 / 900."""
+    return 128 if not _fused(wgu, wd) else 96 if pairs <= 64 * n_experts else 192
 
 
 def exl3_grouped_experts(h, wgu, wd, ids, perm, tiles, ntile, max_tiles, c, tile_rows=128):
