@@ -18,7 +18,8 @@
 // What bounds it: the decode, about 35 integer instructions per 256 weights and sub-partition (194 us of 512 experts of [2048 x 1024] and
 // [512 x 2048], whatever the rows), and beyond some 100 rows of an expert the transforms of the read-out, 96 to 144 shuffles of 16 rows and
 // warp.  us of gate / up + down, one item per 128 rows and one ring of eight stages before: 1021 rows of ten experts 270 + 147 -> 262 + 144,
-// 8192 rows 865 + 551 -> 513 + 400 (items of 160 rows on average are decoded once instead of twice).
+// 8192 rows 865 + 551 -> 513 + 400 (items of 160 rows on average are decoded once instead of twice).  Where a CTA has one item at most, the two
+// groups' alternation lengthens its chain: 33 rows for each of 8 experts of [2048 x 1024] and [512 x 2048] 27.4 + 10.7 -> 29.2 + 11.6.
 //
 // Reference: engine-rs/shim/moe_exl3.cuh:521-1233 (gemm_grouped / gux / gu2 kernels, mma.sync m16n8k16).
 #include "exl3_common.cuh"
