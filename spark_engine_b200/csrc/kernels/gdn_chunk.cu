@@ -374,7 +374,8 @@ gdn_chunk_prep_kernel(const __nv_bfloat16* __restrict__ proj, int ldp, const __n
 // 32 value columns each) keep S, write it and U as K-major operands and store O.
 // What bounds it: the chain state -> product -> U -> product of a chunk, and the 128 KB per chunk that a CTA pulls from L2.
 // 64 chunks of 32 heads: 188 us (of 5473 cycles a chunk 3220 are the products, 860 writing S as an operand, 910 U); 293 with warp-level
-// TF32 products and the operands copied between them (four CTAs of 32 values a head).
+// TF32 products and the operands copied between them (four CTAs of 32 values a head).  Several segments, whole layer before and now: 4 x 1024
+// rows 1027 -> 689, 16 x 256 1011 -> 704, 64 x 64 1082 -> 787.
 constexpr int ST_SLOTS = 11, ST_SLOT = 16384, ST_THREADS = 10 * 32;
 constexpr int ST_B1 = GVS * GD * 4, ST_B2 = GVS * GC * 4;
 constexpr int ST_SMEM = ST_SLOTS * ST_SLOT + ST_B1 + ST_B2 + 256 + 1024;
